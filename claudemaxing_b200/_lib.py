@@ -52,6 +52,8 @@ SIGNATURES = {
     "soup_lmhead_finish": [_P] * 12 + [_L] * 4 + [_P],
     "soup_lmhead_finish_to": [_P] * 13 + [_I] + [_L] * 4 + [_P],
     "soup_lmhead_grad_scale": [_P, _P, _P, _L, _I, _P],
+    "soup_lmhead_totals": [_P] * 4 + [_I, _F] + [_P] * 4 + [_L, _P],
+    "soup_lmhead_backward": [_P] * 4 + [_L, _I, _P],
     "soup_xent_rows": [_P] * 5 + [_L, _L, _L, _I, _P],
     "soup_nf4_gemm_workspace_bytes": [_L, _L],
     "soup_nf4_linear_fwd": [_P, _P, _I, _P, _L, _L, _I, _I, _I, _P, _L, _P],
@@ -132,9 +134,11 @@ class _StreamOf(int):
 
 
 def stream_of(t):
-    """The current torch stream of `t`'s device, as the void* the C ABI takes."""
-    handle = _StreamOf(torch.cuda.current_stream(t.device).cuda_stream)
-    handle.device_index = t.device.index
+    """The current torch stream of `t`'s device, as the void* the C ABI takes. (The raw handle is
+    asked for directly: building a torch.cuda.Stream object for it costs 2 us per launch.)"""
+    index = t.get_device()
+    handle = _StreamOf(torch._C._cuda_getCurrentRawStream(index))
+    handle.device_index = index
     return handle
 
 
@@ -153,14 +157,20 @@ def require_cuda(*tensors):
             raise RuntimeError(f"libsoup_b200: tensors on {device} and {t.device} in one call")
 
 
+_entries = {}   # name -> ctypes function, filled on first use
+
+
 def call(name, *args):
     """Invokes an entry point. The launch, the library's per-device caches (SM count, status word,
     built-in scratch) and the stream all belong to one device: the one of the tensor `stream_of`
-    was asked about, which is made current for the duration of the call when it is not already."""
-    fn = getattr(lib(), name)
-    index = next((a.device_index for a in args if isinstance(a, _StreamOf)), None)
-    if index is not None and index != torch.cuda.current_device():
-        with torch.cuda.device(index):
+    was asked about (the stream is every launching entry's last argument), which is made current
+    for the duration of the call when it is not already."""
+    fn = _entries.get(name)
+    if fn is None:
+        fn = _entries.setdefault(name, getattr(lib(), name))
+    stream = args[-1] if args else None
+    if type(stream) is _StreamOf and stream.device_index != torch._C._cuda_getDevice():
+        with torch.cuda.device(stream.device_index):
             rc = fn(*args)
     else:
         rc = fn(*args)

@@ -1,7 +1,7 @@
 // Fused LM head + cross-entropy, forward and hidden-state gradient, without the logits in HBM.
 //
-// The vocabulary is walked in chunks of column tiles (256 columns each): a first chunk of one
-// wave of CTA pairs, then chunks of eight waves. Per chunk three kernels run back to back on the
+// The vocabulary is walked in chunks of column tiles (256 columns each): a small first chunk, then
+// chunks as large as the probability buffer allows (make_plan). Per chunk three kernels run back to back on the
 // caller's stream; a chunk's probabilities pass from the first to the third through a bf16 buffer
 // in HBM (the GEMMs leave more than 80 % of the memory bandwidth unused):
 //
@@ -14,20 +14,20 @@
 //                  P = bf16(e) (label column and unlabelled rows zeroed) through a swizzled staging
 //                  box and a TMA store. bf16 keeps fp32's exponent range, so a logit far above
 //                  everything seen so far cannot overflow P.
-//   row kernel     one warp per row: adds the tile sums to the running state (the state is kept
+//   row kernel     one CTA per row: adds the tile sums to the running state (the state is kept
 //                  normalised: run_max = lse so far, run_sum = 1), and sets the row's multiplier
 //                  exp(ref - base) for this chunk's gradient contribution.
 //   grad kernel    tcgen05 GEMM  dH += mult * P[rows,cols] * W[cols,K] on CTA pairs, 256 x 256
 //                  tiles with the vocabulary (K) dimension split so that all SMs have work; W is
 //                  the MN-major operand straight from its row-major storage. kind::f16 wants the
 //                  same element format for both operands, so this GEMM reads a bf16 copy of W
-//                  (made once per frozen weight by the caller). Partial sums are added with
-//                  fire-and-forget reductions; dH is kept relative to `base`, the lse after the
+//                  (made once per frozen weight by the caller). Partial sums are added by
+//                  the copy engine (tiled bulk reductions from shared memory); dH is kept relative to `base`, the lse after the
 //                  first chunk.
 //
 // The first chunk has no earlier lse: its statistics and its P are taken against each tile's own
-// maximum (two sweeps over the accumulator), the row kernel merges the tiles, and a small kernel
-// rescales the chunk's P in place to the merged lse. A last kernel
+// maximum (two sweeps over the accumulator), and the row kernel merges the tiles and rescales the
+// chunk's P in place to the merged lse. A last kernel
 // turns the state into loss / entropy / correct, rescales dH from `base` to the final lse and
 // adds (p_label - 1) * W[label] in fp32.
 //
@@ -74,7 +74,7 @@ constexpr int kIgnore = -100;
 constexpr int kEW = 16;                // accumulator columns per tcgen05.ld in the epilogues
 
 constexpr int kStageP = 4 * 2 * 4096;          // logits: per epilogue warp two 32 x 64 bf16 boxes
-constexpr int kStageT = 4 * 32 * 33 * 4;       // gradient: per epilogue warp a padded 32 x 32 fp32 block
+constexpr int kStageT = 4 * 2 * 4096;          // gradient: per epilogue warp two 32 x 32 fp32 boxes
 constexpr int kSmemLogits = kStages * kStageBytes + kStageP + 1024 + 256;
 constexpr int kSmemGrad = kStages * kStageBytes + kStageT + 1024 + 256;
 
@@ -173,10 +173,13 @@ __device__ __forceinline__ PairInit init_pair(const GemmSmem& s, int warp, int l
   return r;
 }
 
-__device__ __forceinline__ void finish_pair(const GemmSmem& s, int warp, uint32_t tmem) {
+__device__ __forceinline__ void finish_pair(const GemmSmem& s, int warp, uint32_t tmem, int* status,
+                                            int* sticky) {
   tc_fence_before_sync();
   __syncthreads();
   if (*s.abort_flag) {
+    // so that the failure outlives the call's workspace (soup_device_status)
+    if (threadIdx.x == 0 && sticky) atomicCAS(sticky, 0, *reinterpret_cast<volatile int*>(status));
     // A wait was abandoned: give copies that may still be in flight time to land before the
     // shared memory is released.
     for (int i = 0; i < 64; ++i) __nanosleep(2000);
@@ -221,6 +224,7 @@ struct LogitsArgs {
   int mode;                // LogitsMode
   int store_p;             // write P (gradient wanted)
   int* status;
+  int* sticky;             // the device's sticky status word (nullable)
 };
 
 // First chunk, first launch: statistics of one 128 x 256 tile for one thread (= one row) against
@@ -578,14 +582,20 @@ lmhead_logits_kernel(const __grid_constant__ CUtensorMap map_h,
     }
     if (lane == 0) tma_store_wait_read<0>();  // staging boxes fully read before shared memory goes away
   }
-  finish_pair(s, warp, tmem);
+  finish_pair(s, warp, tmem, a.status, a.sticky);
 }
 
 // ------------------------------------------------------------------------------------------
-// Row kernel: one warp per row merges the chunk's tile statistics into the running state.
+// Row kernel: one CTA per row merges the chunk's tile statistics into the running state.
 // The state is kept normalised: run_max = log-sum-exp so far, run_sum = 1, run_dot = sum of
 // softmax-so-far * z. For the gradient it also maintains `base` (the lse dH is relative to) and
-// writes the row's multiplier for this chunk's contribution.
+// writes the row's multiplier for this chunk's contribution. After the first chunk it brings that
+// chunk's P from "against its tile's maximum" to "against the lse" as well.
+//
+// Bound by latency: a row has up to a few hundred 16-byte statistics. One thread takes a few tiles
+// and the CTA exchanges through shared memory. (One warp per row took a serial chain of ten dependent
+// load and shuffle rounds per 320 tiles, and the rescale a launch of its own: 20 us per call at 2048
+// rows for the first chunk, 11.6 us now; 12.5 against 6.2 us at 128 rows.)
 // ------------------------------------------------------------------------------------------
 struct RowArgs {
   const float4* tile_stats;
@@ -597,7 +607,7 @@ struct RowArgs {
   float* base;      // [n_rows] lse that dH is relative to (set by the first chunk)
   float* mult;      // [n_rows] out: exp(ref - base) for the gradient kernel of this chunk
   float* dh;        // nullable: [n_rows, k_dim], touched only when a row is rebased
-  __nv_bfloat16* p; // nullable: the chunk's probabilities [n_rows, ld_p], touched only for hot rows
+  __nv_bfloat16* p; // nullable: the chunk's probabilities [n_rows, ld_p]
   int ld_p;
   int n_rows;
   int k_dim;
@@ -606,156 +616,32 @@ struct RowArgs {
   int mode;         // kModeTileMax (first chunk) or kModeCombined
   int want_grad;
   int* status;
+  int* sticky;
 };
 
-__global__ void __launch_bounds__(256) lmhead_row_kernel(const RowArgs a) {
-  const int lane = threadIdx.x & 31;
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (row >= a.n_rows) return;
-  const float ref = a.run_max[row];   // lse so far (-inf before the first chunk)
-  float run_dot = a.run_dot[row];
-  int best = a.best[row];
-  float best_val = a.mode == kModeTileMax ? -INFINITY : a.best_val[row];
-  float new_lse, new_dot;
-  bool hot_row = false;
-  if (a.mode == kModeTileMax) {
-    // statistics relative to each tile's own maximum: log-sum-exp merge
-    float run_max = -INFINITY, run_sum = 0.f;
-    run_dot = 0.f;
-    for (int t0 = 0; t0 < a.ct; t0 += 32) {
-      const int t = t0 + lane;
-      float4 st = make_float4(-INFINITY, 0.f, 0.f, 0.f);
-      if (t < a.ct) st = a.tile_stats[(size_t)row * a.ct_stride + t];
-      float gmax = st.x;
+constexpr int kRowThreads = 128;
+
+// Sums of two values over the CTA, in a fixed order; every thread gets both.
+__device__ __forceinline__ float2 row_sum2(float x, float y, float2* s_part, int warp, int lane) {
+  x = warp_sum(x);
+  y = warp_sum(y);
+  if (lane == 0) s_part[warp] = make_float2(x, y);
+  __syncthreads();
+  float2 t = s_part[0];
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
-      const unsigned holders = __ballot_sync(0xffffffffu, st.x == gmax);
-      const int first = __ffs(holders) - 1;  // lowest tile that holds the maximum
-      const int cand = __shfl_sync(0xffffffffu, __float_as_int(st.w), first);
-      if (gmax > best_val) { best_val = gmax; best = cand; }
-      const float new_max = fmaxf(run_max, gmax);
-      const float w = t < a.ct ? exp2f((st.x - new_max) * kLog2e) : 0.f;
-      const float part_sum = warp_sum(st.y * w);
-      const float part_dot = warp_sum(st.z * w);
-      const float rescale = exp2f((run_max - new_max) * kLog2e);  // exp(-inf) = 0 at the start
-      run_sum = run_sum * rescale + part_sum;
-      run_dot = run_dot * rescale + part_dot;
-      run_max = new_max;
-    }
-    new_lse = run_max + logf(run_sum);
-    new_dot = run_dot / run_sum;
-  } else {
-    // statistics relative to ref: the mass so far is exp(ref) * 1
-    float add_sum = 0.f, add_dot = 0.f;
-    for (int t0 = 0; t0 < a.ct; t0 += 32) {
-      const int t = t0 + lane;
-      float4 st = make_float4(-INFINITY, 0.f, 0.f, 0.f);
-      if (t < a.ct) st = a.tile_stats[(size_t)row * a.ct_stride + t];
-      float gmax = st.x;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) gmax = fmaxf(gmax, __shfl_xor_sync(0xffffffffu, gmax, o));
-      const unsigned holders = __ballot_sync(0xffffffffu, st.x == gmax);
-      const int first = __ffs(holders) - 1;
-      const int cand = __shfl_sync(0xffffffffu, __float_as_int(st.w), first);
-      if (gmax > best_val) { best_val = gmax; best = cand; }  // later tiles win only if larger
-      add_sum += warp_sum(st.y);
-      add_dot += warp_sum(st.z);
-    }
-    const float total = 1.0f + add_sum;
-    new_lse = ref + logf(total);
-    new_dot = (run_dot + add_dot) / total;
-    // Hot tiles (is_hot: written against their own maximum, not against ref) make the sums above
-    // meaningless for this row; best_val is then the largest of them. Redo the merge with every
-    // tile's own reference, relative to rho = best_val.
-    hot_row = is_hot(best_val, ref);
-    if (hot_row) {
-      const float rho = best_val;
-      const float w_ref = exp2f((ref - rho) * kLog2e);   // < e^-30
-      float sum = 0.f, dot = 0.f;
-      for (int t0 = 0; t0 < a.ct; t0 += 32) {
-        const int t = t0 + lane;
-        float4 st = make_float4(-INFINITY, 0.f, 0.f, 0.f);
-        if (t < a.ct) st = a.tile_stats[(size_t)row * a.ct_stride + t];
-        const float w = t < a.ct ? (is_hot(st.x, ref) ? exp2f((st.x - rho) * kLog2e) : w_ref) : 0.f;
-        sum += warp_sum(st.y * w);
-        dot += warp_sum(st.z * w);
-      }
-      const float total_hot = w_ref + sum;
-      new_lse = rho + logf(total_hot);
-      new_dot = (run_dot * w_ref + dot) / total_hot;
-    } else if (!(total < INFINITY) && lane == 0) {
-      atomicCAS(a.status, 0, 90);  // cannot happen: every non-hot tile sum is below 256 e^30
-    }
-  }
-  float mult = 1.0f;
-  if (a.want_grad) {
-    if (a.mode == kModeTileMax) {
-      if (lane == 0) a.base[row] = new_lse;   // the first chunk's P is written against this lse
-    } else if (hot_row) {
-      // The chunk's P of this row mixes references (ref for ordinary tiles, the tile maximum for
-      // hot ones). Bring all of it to rho = best_val, move dH of the row to the same reference and
-      // let the gradient kernel add the chunk with multiplier 1. Everything that was relative to
-      // ref shrinks by more than e^-30.
-      const float rho = best_val;
-      const float w_ref = exp2f((ref - rho) * kLog2e);
-      uint4* prow = reinterpret_cast<uint4*>(a.p + (size_t)row * a.ld_p);
-      for (int t = 0; t < a.ct; ++t) {
-        const float tm = a.tile_stats[(size_t)row * a.ct_stride + t].x;
-        const float f = is_hot(tm, ref) ? exp2f((tm - rho) * kLog2e) : w_ref;
-        if (f == 1.0f) continue;
-        uint4 v = prow[t * (kBN / 8) + lane];
-        uint32_t w[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const float2 e = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[k]));
-          __nv_bfloat162 h = __floats2bfloat162_rn(e.x * f, e.y * f);
-          w[k] = *reinterpret_cast<uint32_t*>(&h);
-        }
-        prow[t * (kBN / 8) + lane] = make_uint4(w[0], w[1], w[2], w[3]);
-      }
-      const float down = expf(a.base[row] - rho);
-      for (int i = lane; i < a.k_dim; i += 32) a.dh[(size_t)row * a.k_dim + i] *= down;
-      __syncwarp();
-      if (lane == 0) a.base[row] = rho;
-      mult = 1.0f;
-    } else {
-      float base = a.base[row];
-      if (ref - base > kRebase) {
-        // rare: the multiplier exp(ref - base) is getting large; bring dH of this row to ref
-        const float down = expf(base - ref);
-        for (int i = lane; i < a.k_dim; i += 32) a.dh[(size_t)row * a.k_dim + i] *= down;
-        base = ref;
-        __syncwarp();
-        if (lane == 0) a.base[row] = base;
-      }
-      mult = expf(ref - base);
-    }
-  }
-  if (lane == 0) {
-    a.run_max[row] = new_lse;
-    a.run_sum[row] = 1.0f;
-    a.run_dot[row] = new_dot;
-    a.best[row] = best;
-    a.best_val[row] = best_val;
-    if (a.want_grad) a.mult[row] = mult;
-  }
+  for (int w = 1; w < kRowThreads / 32; ++w) { t.x += s_part[w].x; t.y += s_part[w].y; }
+  return t;
 }
 
-// First chunk only: P was written as exp(z - tile maximum); bring it to exp(z - lse) in place, one
-// warp per row, one 16-byte vector (8 bf16) per lane and tile. A memory-bound pass over a chunk
-// that is still in L2, instead of a second GEMM pass over the chunk's logits.
-__global__ void __launch_bounds__(256)
-lmhead_rescale_first_kernel(__nv_bfloat16* __restrict__ p, int ld_p,
-                            const float4* __restrict__ tile_stats, int ct_stride,
-                            const float* __restrict__ lse, int n_rows, int ct) {
-  const int lane = threadIdx.x & 31;
-  const int row = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (row >= n_rows) return;
-  const float row_lse = lse[row];
-  uint4* prow = reinterpret_cast<uint4*>(p + (size_t)row * ld_p);
-#pragma unroll 2
-  for (int t = 0; t < ct; ++t) {
-    const float f = exp2f((tile_stats[(size_t)row * ct_stride + t].x - row_lse) * kLog2e);
+// Multiplies the row's P of this chunk tile by tile with factor(tile's maximum): a warp takes every
+// fourth tile, one 16-byte vector (8 bf16) per lane.
+template <typename F>
+__device__ __forceinline__ void rescale_row(const RowArgs& a, int row, int warp, int lane, F factor) {
+  uint4* prow = reinterpret_cast<uint4*>(a.p + (size_t)row * a.ld_p);
+  const float4* stats = a.tile_stats + (size_t)row * a.ct_stride;
+#pragma unroll 4
+  for (int t = warp; t < a.ct; t += kRowThreads / 32) {
+    const float f = factor(stats[t].x);
     uint4 v = prow[t * (kBN / 8) + lane];
     uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
@@ -768,30 +654,145 @@ lmhead_rescale_first_kernel(__nv_bfloat16* __restrict__ p, int ld_p,
   }
 }
 
+__global__ void __launch_bounds__(kRowThreads, 8) lmhead_row_kernel(const RowArgs a) {
+  __shared__ float s_max[kRowThreads / 32];
+  __shared__ int s_arg[kRowThreads / 32];
+  __shared__ float2 s_part[kRowThreads / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int row = blockIdx.x;
+  const bool first = a.mode == kModeTileMax;
+  const float4* stats = a.tile_stats + (size_t)row * a.ct_stride;
+  const float ref = a.run_max[row];   // lse so far (-inf before the first chunk)
+  const float old_dot = a.run_dot[row];
+  const float old_base = a.want_grad && !first ? a.base[row] : 0.f;
+  int best = a.best[row];
+  float best_val = first ? -INFINITY : a.best_val[row];
+  // the chunk's largest logit and its first column (tile order is column order: on equal maxima the
+  // lower column wins), and the plain sums that serve a later chunk's ordinary row
+  float m = -INFINITY, sum = 0.f, dot = 0.f;
+  int arg = INT32_MAX;
+  for (int t = threadIdx.x; t < a.ct; t += kRowThreads) {
+    const float4 st = stats[t];
+    if (st.x > m) { m = st.x; arg = __float_as_int(st.w); }
+    sum += st.y;
+    dot += st.z;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float om = __shfl_xor_sync(0xffffffffu, m, o);
+    const int oa = __shfl_xor_sync(0xffffffffu, arg, o);
+    if (om > m || (om == m && oa < arg)) { m = om; arg = oa; }
+  }
+  if (lane == 0) { s_max[warp] = m; s_arg[warp] = arg; }
+  float2 total = row_sum2(sum, dot, s_part, warp, lane);   // its barrier covers s_max / s_arg too
+  m = s_max[0];
+  arg = s_arg[0];
+#pragma unroll
+  for (int w = 1; w < kRowThreads / 32; ++w)
+    if (s_max[w] > m || (s_max[w] == m && s_arg[w] < arg)) { m = s_max[w]; arg = s_arg[w]; }
+  if (m > best_val) { best_val = m; best = arg; }   // earlier chunks keep a tie
+
+  // Hot tiles (is_hot: written against their own maximum, not against ref) make the plain sums
+  // meaningless for this row; best_val is then the largest of them. The merge is redone with every
+  // tile's own reference, relative to best_val, as for the first chunk.
+  const bool hot_row = !first && is_hot(best_val, ref);
+  const float rho = best_val;
+  const float w_ref = hot_row ? exp2f((ref - rho) * kLog2e) : 0.f;   // < e^-30
+  auto weight_of = [&](float tile_max) {
+    return first || is_hot(tile_max, ref) ? exp2f((tile_max - rho) * kLog2e) : w_ref;
+  };
+  float new_lse, new_dot;
+  if (first || hot_row) {
+    sum = dot = 0.f;
+    for (int t = threadIdx.x; t < a.ct; t += kRowThreads) {
+      const float4 st = stats[t];
+      const float w = weight_of(st.x);
+      sum += st.y * w;
+      dot += st.z * w;
+    }
+    __syncthreads();   // everybody has read the first pair of sums
+    total = row_sum2(sum, dot, s_part, warp, lane);
+    const float mass = w_ref + total.x;   // w_ref: the mass so far, exp(ref) * 1 (0 at the first chunk)
+    new_lse = rho + logf(mass);
+    new_dot = ((hot_row ? old_dot * w_ref : 0.f) + total.y) / mass;
+  } else {
+    const float mass = 1.0f + total.x;    // statistics relative to ref: the mass so far is exp(ref) * 1
+    new_lse = ref + logf(mass);
+    new_dot = (old_dot + total.y) / mass;
+    if (!(mass < INFINITY) && threadIdx.x == 0) {
+      atomicCAS(a.status, 0, 90);  // cannot happen: every non-hot tile sum is below 256 e^30
+      if (a.sticky) atomicCAS(a.sticky, 0, 90);
+    }
+  }
+  float mult = 1.0f, base = old_base;
+  if (a.want_grad) {
+    float down = 1.0f;   // what brings dH of this row to `base`
+    if (first) {
+      base = new_lse;
+      rescale_row(a, row, warp, lane, [&](float tile_max) { return exp2f((tile_max - new_lse) * kLog2e); });
+    } else if (hot_row) {
+      // The chunk's P of this row mixes references (ref for ordinary tiles, the tile maximum for
+      // hot ones). Bring all of it to rho = best_val, move dH of the row to the same reference and
+      // let the gradient kernel add the chunk with multiplier 1. Everything that was relative to
+      // ref shrinks by more than e^-30.
+      rescale_row(a, row, warp, lane, weight_of);
+      down = expf(old_base - rho);
+      base = rho;
+    } else {
+      if (ref - old_base > kRebase) {
+        // rare: the multiplier exp(ref - base) is getting large; bring dH of this row to ref
+        down = expf(old_base - ref);
+        base = ref;
+      }
+      mult = expf(ref - base);
+    }
+    if (!first && base != old_base)
+      for (int i = threadIdx.x; i < a.k_dim; i += kRowThreads) a.dh[(size_t)row * a.k_dim + i] *= down;
+  }
+  if (threadIdx.x == 0) {
+    a.run_max[row] = new_lse;
+    a.run_sum[row] = 1.0f;
+    a.run_dot[row] = new_dot;
+    a.best[row] = best;
+    a.best_val[row] = best_val;
+    if (a.want_grad) {
+      a.base[row] = base;
+      a.mult[row] = mult;
+    }
+  }
+}
+
 // ------------------------------------------------------------------------------------------
 // Gradient kernel: dH[rows, K] += mult[row] * P[rows, cols] * W[cols, K] for one chunk. A pair owns
-// a 256-row x 256-hidden-column output tile; a work unit is (tile, K split). The epilogue transposes
-// each 32 x 32 block of the accumulator through shared memory so that dH is touched in full
-// 128-byte rows.
+// a 256-row x 256-hidden-column output tile; a work unit is (tile, K split). The epilogue stages
+// each 32 x 32 block of the accumulator in shared memory (128-byte-swizzled) and the copy engine
+// adds it to dH (a tiled bulk reduction): the epilogue warps issue no atomics of their own, so that
+// splitting K over all CTA pairs costs little even when a unit has few K blocks (see pick_ksplit).
 // ------------------------------------------------------------------------------------------
 struct GradArgs {
-  float* dh;            // [n_rows, k_dim] fp32 of this row block, zeroed before the first chunk
   const float* mult;    // [n_rows]
+  int row0;             // first row of the block inside dH (TMA coordinate)
   int n_rows;
   int k_dim;            // hidden size (output columns)
   int col0;             // first shard column of the chunk (TMA row coordinate into W)
   int n_kb;             // 64-column blocks of the chunk
   int ksplit;           // K (vocabulary) splits per output tile
   int* status;
+  int* sticky;
 };
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsGemm, 1)
 lmhead_grad_kernel(const __grid_constant__ CUtensorMap map_p,
-                   const __grid_constant__ CUtensorMap map_w, const GradArgs a) {
+                   const __grid_constant__ CUtensorMap map_w,
+                   const __grid_constant__ CUtensorMap map_dh, const GradArgs a) {
   extern __shared__ uint8_t smem_raw[];
   const GemmSmem s = carve_smem<kStageT>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp == 0 && lane == 0) { prefetch_tensormap(&map_p); prefetch_tensormap(&map_w); }
+  if (warp == 0 && lane == 0) {
+    prefetch_tensormap(&map_p);
+    prefetch_tensormap(&map_w);
+    prefetch_tensormap(&map_dh);
+  }
   const PairInit pi = init_pair(s, warp, lane, a.status);
   if (!pi.run) return;
   const uint32_t tmem = pi.tmem, rank = pi.rank;
@@ -866,7 +867,7 @@ lmhead_grad_kernel(const __grid_constant__ CUtensorMap map_p,
     }
   } else {
     const int q = warp & 3;
-    float* tpose = reinterpret_cast<float*>(s.extra) + (warp - 2) * (32 * 33);
+    uint8_t* stage_warp = s.extra + (warp - 2) * 8192;   // two 32 x 32 fp32 boxes
     bool ok = true;
     int it = 0;
     for (int unit = pair; unit < n_units && ok; unit += n_pairs, ++it) {
@@ -881,47 +882,57 @@ lmhead_grad_kernel(const __grid_constant__ CUtensorMap map_p,
       const float my_mult = (row_base + lane < a.n_rows) ? a.mult[row_base + lane] : 0.f;
       const uint32_t taddr = tmem + (static_cast<uint32_t>(q * 32) << 16) + ab * kBN;
       const int col_base = tn * kBN;
+      // rows past the block are past dH as well (only the last block can be ragged): the reduction
+      // clips them, and columns past k_dim
+      const int n_boxes = row_base < a.n_rows ? min(kBN / 32, (a.k_dim - col_base + 31) / 32) : 0;
 #pragma unroll 1
-      for (int c = 0; c < kBN / 32; ++c) {
+      for (int c = 0; c < n_boxes; ++c) {
         uint32_t r[32];
         tmem_ld_32x32(taddr + c * 32, r);
+        uint8_t* box = stage_warp + (c & 1) * 4096;
+        if (lane == 0) tma_store_wait_read<1>();   // the reduction two boxes ago has read its source
+        __syncwarp();
         tmem_ld_wait_on(r);
-        __syncwarp();
+        uint8_t* mine = box + lane * 128;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) tpose[lane * 33 + j] = __uint_as_float(r[j]) * my_mult;
+        for (int j = 0; j < 8; ++j)
+          *reinterpret_cast<float4*>(mine + ((j ^ (lane & 7)) << 4)) =
+              make_float4(__uint_as_float(r[4 * j]) * my_mult, __uint_as_float(r[4 * j + 1]) * my_mult,
+                          __uint_as_float(r[4 * j + 2]) * my_mult, __uint_as_float(r[4 * j + 3]) * my_mult);
+        fence_proxy_async_smem();
         __syncwarp();
-        // Fire-and-forget reductions: with one K split exactly one CTA adds to an element per
-        // chunk and the result is deterministic; with several the order of the adds is not.
-        const int col = col_base + c * 32 + lane;
-        const bool col_ok = col < a.k_dim;
-#pragma unroll 8
-        for (int rr = 0; rr < 32; ++rr) {
-          const int row = row_base + rr;
-          if (col_ok && row < a.n_rows)
-            atomicAdd(a.dh + (size_t)row * a.k_dim + col, tpose[rr * 33 + lane]);
+        if (lane == 0) {
+          tma_reduce_add_2d(&map_dh, box, col_base + c * 32, a.row0 + row_base);
+          tma_store_commit();
         }
       }
       release_accumulator(s, ab, rank, lane);
     }
+    if (lane == 0) tma_store_wait_done();   // the sums have landed before the kernel ends
   }
-  finish_pair(s, warp, tmem);
+  finish_pair(s, warp, tmem, a.status, a.sticky);
 }
 
 // ------------------------------------------------------------------------------------------
 // Small kernels: state initialisation, merge across ranks, finish, backward scale.
 // ------------------------------------------------------------------------------------------
-__global__ void lmhead_init_state_kernel(float* run_max, float* run_sum, float* run_dot, int* best,
-                                         float* best_val, float* label_logit, float* grad_ref,
-                                         int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  run_max[i] = -INFINITY;
-  run_sum[i] = 0.f;
-  run_dot[i] = 0.f;
-  best[i] = 0;
-  best_val[i] = -INFINITY;
-  label_logit[i] = 0.f;
-  grad_ref[i] = 0.f;
+// Initial state of a call: the status word, the row states and (dh not NULL) the cleared gradient.
+__global__ void __launch_bounds__(256)
+lmhead_init_kernel(float* run_max, float* run_sum, float* run_dot, int* best, float* best_val,
+                   float* label_logit, float* grad_ref, int* status, float4* dh, int64_t dh_vec, int n) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) *status = 0;
+  if (i < n) {
+    run_max[i] = -INFINITY;
+    run_sum[i] = 0.f;
+    run_dot[i] = 0.f;
+    best[i] = 0;
+    best_val[i] = -INFINITY;
+    label_logit[i] = 0.f;
+    grad_ref[i] = 0.f;
+  }
+  if (dh)
+    for (int64_t v = i; v < dh_vec; v += (int64_t)gridDim.x * blockDim.x) dh[v] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // states: [n_ranks, n] each; out: [n]. Ranks are in ascending vocabulary order, so a later rank
@@ -977,14 +988,19 @@ struct FinishArgs {
   int dh_out_dtype;
 };
 
-__global__ void __launch_bounds__(256) lmhead_finish_kernel(const FinishArgs a) {
+// One CTA per row. Bound by memory: dH is read and written once, W[label] gathered. VEC: four columns
+// per thread and access (rows of a multiple of four columns, 16-byte aligned).
+constexpr int kFinishThreads = 128;
+template <bool VEC>
+__global__ void __launch_bounds__(kFinishThreads) lmhead_finish_kernel(const FinishArgs a) {
   const int row = blockIdx.x;
-  const float lse = a.run_max[row] + logf(a.run_sum[row]);
+  const float run_sum = a.run_sum[row], label_logit = a.label_logit[row];
+  const float lse = a.run_max[row] + logf(run_sum);
   const long long tg = a.target[row];
   const bool labelled = tg != kIgnore;
   if (threadIdx.x == 0 && a.token_loss) {
-    a.token_loss[row] = labelled ? lse - a.label_logit[row] : 0.f;
-    a.entropy[row] = lse - a.run_dot[row] / a.run_sum[row];
+    a.token_loss[row] = labelled ? lse - label_logit : 0.f;
+    a.entropy[row] = lse - a.run_dot[row] / run_sum;
     a.correct[row] = (labelled && (long long)a.best[row] == tg) ? 1 : 0;
   }
   if (!a.dh) return;
@@ -994,20 +1010,79 @@ __global__ void __launch_bounds__(256) lmhead_finish_kernel(const FinishArgs a) 
   const long long local = tg - a.col_offset;
   const bool mine = labelled && local >= 0 && local < a.v_shard;
   // the label's term, (p_label - 1) W[label], in fp32 (expm1 keeps it exact when p_label ~ 1)
-  const float label_term = mine ? expm1f(a.label_logit[row] - lse) * kGradScale : 0.f;
+  const float label_term = mine ? expm1f(label_logit - lse) * kGradScale : 0.f;
   const __half* w_row = a.weight + (size_t)(mine ? local : 0) * a.k_dim;
-  for (int c = threadIdx.x; c < a.k_dim; c += blockDim.x) {
-    float v = labelled ? dh_row[c] * scale : 0.f;
-    if (mine) v = fmaf(__half2float(w_row[c]), label_term, v);
-    if (a.dh_out) store1(a.dh_out, (int64_t)row * a.k_dim + c, a.dh_out_dtype, v);
-    else dh_row[c] = v;
+  if (VEC) {
+#pragma unroll 4
+    for (int c = threadIdx.x * 4; c < a.k_dim; c += kFinishThreads * 4) {
+      float v[4] = {0.f, 0.f, 0.f, 0.f};
+      if (labelled) {
+        const float4 d = *reinterpret_cast<const float4*>(dh_row + c);
+        v[0] = d.x * scale; v[1] = d.y * scale; v[2] = d.z * scale; v[3] = d.w * scale;
+      }
+      if (mine) {
+        float w[4];
+        loadv<4>(w_row, c, SOUP_F16, w);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) v[k] = fmaf(w[k], label_term, v[k]);
+      }
+      if (a.dh_out) storev<4>(a.dh_out, (int64_t)row * a.k_dim + c, a.dh_out_dtype, v);
+      else *reinterpret_cast<float4*>(dh_row + c) = make_float4(v[0], v[1], v[2], v[3]);
+    }
+  } else {
+    for (int c = threadIdx.x; c < a.k_dim; c += kFinishThreads) {
+      float v = labelled ? dh_row[c] * scale : 0.f;
+      if (mine) v = fmaf(__half2float(w_row[c]), label_term, v);
+      if (a.dh_out) store1(a.dh_out, (int64_t)row * a.k_dim + c, a.dh_out_dtype, v);
+      else dh_row[c] = v;
+    }
   }
+}
+
+// The step's numbers from the per-row terms, in one launch and a fixed order of additions:
+// loss = sum of token losses / divisor, hits, labelled rows; and divisor * GRAD_SCALE for backward.
+// The divisor is the labelled count, or *divisor_ptr, or divisor_value. One CTA: a few 10 KB.
+constexpr int kTotalsThreads = 1024;
+__global__ void __launch_bounds__(kTotalsThreads)
+lmhead_totals_kernel(const float* __restrict__ token_loss, const int* __restrict__ correct,
+                     const int64_t* __restrict__ target, const void* divisor_ptr, int divisor_kind,
+                     float divisor_value, float* loss, int64_t* hits, int64_t* labelled,
+                     float* grad_divisor, int64_t n) {
+  __shared__ float s_loss[32];
+  __shared__ int s_hits[32], s_lab[32];
+  float sum = 0.f;
+  int h = 0, l = 0;
+  for (int64_t i = threadIdx.x; i < n; i += kTotalsThreads) {
+    sum += token_loss[i];
+    h += correct[i];
+    l += target[i] != kIgnore;
+  }
+  sum = warp_sum(sum);
+  h = __reduce_add_sync(0xffffffffu, h);
+  l = __reduce_add_sync(0xffffffffu, l);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) { s_loss[warp] = sum; s_hits[warp] = h; s_lab[warp] = l; }
+  __syncthreads();
+  if (warp != 0) return;
+  sum = warp_sum(s_loss[lane]);
+  h = __reduce_add_sync(0xffffffffu, s_hits[lane]);
+  l = __reduce_add_sync(0xffffffffu, s_lab[lane]);
+  if (lane != 0) return;
+  float div = divisor_value;
+  if (divisor_kind == 1) div = (float)l;
+  else if (divisor_kind == 2) div = *reinterpret_cast<const float*>(divisor_ptr);
+  else if (divisor_kind == 3) div = (float)*reinterpret_cast<const int64_t*>(divisor_ptr);
+  *loss = __fdiv_rn(sum, div);
+  *hits = h;
+  *labelled = l;
+  *grad_divisor = div * kGradScale;
 }
 
 // grad = dh * scale, cast to the hidden dtype (the backward of the loss).
 __global__ void lmhead_scale_cast_kernel(const float* __restrict__ dh, void* __restrict__ out,
-                                         const float* __restrict__ scale_ptr, int64_t n, int odt) {
-  const float scale = *scale_ptr;
+                                         const float* __restrict__ scale_ptr,
+                                         const float* __restrict__ divisor_ptr, int64_t n, int odt) {
+  const float scale = divisor_ptr ? __fdiv_rn(*scale_ptr, *divisor_ptr) : *scale_ptr;
   const int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const int64_t n8 = n >> 3;
   if (v < n8) {
@@ -1021,25 +1096,25 @@ __global__ void lmhead_scale_cast_kernel(const float* __restrict__ dh, void* __r
     for (int64_t i = n8 << 3; i < n; ++i) store1(out, i, odt, dh[i] * scale);
 }
 
-// Copies a non-zero status of the call into the device's sticky status word (read and cleared by
-// soup_device_status), so that a failure outlives the call's workspace.
-__global__ void lmhead_publish_status_kernel(const int* call_status, int* sticky) {
-  const int code = *call_status;
-  if (code != 0) atomicCAS(sticky, 0, code);
-}
-
 inline int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 
-// K splits per gradient tile that minimise the makespan of `tiles` output tiles on `pairs` CTA
-// pairs (each pair runs its units one after another). 1 keeps the result deterministic.
+// K splits per gradient tile that minimise the makespan of `tiles` output tiles on `pairs` CTA pairs
+// (each pair runs its units one after another). A unit costs its K blocks plus kUnitCost blocks for
+// what the double-buffered accumulator does not hide. Up to kMaxSplit, so that few output tiles
+// (few rows) still reach every pair: 128 rows x 1536 have 6 tiles, which splits of at most four left
+// on 24 of the 74 pairs (215 us per call over 151936 columns, 93 us split over 72 of them; 1168 rows,
+// 30 tiles: 457 and 414 us). The order of units (tile fastest) keeps the pairs that run
+// together on one or two K ranges, whose rows of W they share through L2. 1 split keeps the result
+// deterministic.
+constexpr int kUnitCost = 8;
+constexpr int kMaxSplit = 80;
 inline int pick_ksplit(int tiles, int pairs, int n_kb, bool deterministic) {
   if (deterministic || tiles <= 0) return 1;
   int best = 1;
-  long best_span = (long)((tiles + pairs - 1) / pairs) * n_kb;
-  for (int ks = 2; ks <= 4; ++ks) {
-    if (n_kb / ks < 8) break;  // too little work per unit to amortise its epilogue
-    const long span = (long)((tiles * ks + pairs - 1) / pairs) * ((n_kb + ks - 1) / ks);
-    if (span * 10 < best_span * 9) { best = ks; best_span = span; }  // needs a 10 % gain
+  long best_span = (long)((tiles + pairs - 1) / pairs) * (n_kb + kUnitCost);
+  for (int ks = 2; ks <= kMaxSplit && ks <= n_kb; ++ks) {
+    const long span = (long)((tiles * ks + pairs - 1) / pairs) * ((n_kb + ks - 1) / ks + kUnitCost);
+    if (span < best_span) { best = ks; best_span = span; }
   }
   return best;
 }
@@ -1050,40 +1125,58 @@ struct Plan {
   int ct;          // column tiles of every later chunk (>= ct_first)
 };
 
-// Rows per block and column tiles per chunk. The first chunk is the one whose logits are computed
-// twice (once for its row statistics, once for its probabilities against them), so it is one wave
-// of CTA pairs wide and no wider. Every later chunk is written against the running statistics in
-// a single pass and can be large: eight waves (SOUP_LMHEAD_WAVES overrides), which cuts the
-// launches of a step, and the ramp and drain each one pays, from 55 to 13 at 2048 x 151936 (1.80 ->
-// 1.50 ms measured; four waves 1.56, sixteen 1.52). Its probabilities (bf16, 310 MB at 2048 rows)
-// then go through HBM instead of staying in L2, which these compute-bound kernels have bandwidth
-// to spare for. row_tiles * ct fills whole waves of CTA pairs. An override applies to all chunks.
+// Rows per block and column tiles per chunk. The first chunk needs two sweeps over its accumulators
+// and a rescale of its P, so it is small; every later chunk is written against the running
+// statistics in a single pass and is as large as the probability buffer allows, because each
+// launch pays its ramp and drain (55 launches instead of 13 at 2048 x 151936: 1.80 against 1.50 ms).
+// The probabilities then go through HBM instead of staying in L2, which these compute-bound
+// kernels have bandwidth to spare for. SOUP_LMHEAD_WAVES bounds a later chunk in waves of CTA pairs
+// at eight row tiles (default: kChunkBytes decides; 2048 and fewer rows then run in two chunks, which
+// saved one set of launches, 15 us, over chunks of eight waves); an override (`ct_override`) applies to all
+// chunks.
+//  - First chunk: the fewest column tiles whose rt * ct units fill whole waves of CTA pairs to 97 %
+//    or more, at least kFirstTiles of them (its gradient launch has four 64-column K blocks per
+//    tile to split).
+//  - Rows per block: 2048 for a full-width chunk; more when the shard is narrow (a rank of a
+//    vocabulary-parallel group), so that a launch still has a dozen tiles per CTA pair and the
+//    probability buffer stays around 600 MB. Whole multiples of 2048, at most 8192.
+constexpr int kFirstTiles = 16;
+constexpr int64_t kChunkBytes = 640ll << 20;
 inline Plan make_plan(int64_t n, int64_t v_shard, int sms, int ct_override) {
   Plan p;
   const int pairs = sms / 2 > 0 ? sms / 2 : 1;
   const int total_ct = (int)((v_shard + kBN - 1) / kBN);
-  int waves = 8;
+  int waves = 0;
   if (const char* e = getenv("SOUP_LMHEAD_WAVES")) { const int v = atoi(e); if (v >= 1 && v <= 64) waves = v; }
-  // A chunk is `wave` column tiles per wave of CTA pairs at eight row tiles (2048 rows).
-  int wave = 37;
-  for (int c = 40; c >= 8; --c)
-    if ((8 * c) % pairs == 0) { wave = c; break; }
-  p.ct_first = ct_override > 0 ? ct_override : wave;
-  p.ct = ct_override > 0 ? ct_override : waves * wave;
-  if (p.ct_first > total_ct) p.ct_first = total_ct;
-  if (p.ct_first < 1) p.ct_first = 1;
-  if (p.ct > total_ct) p.ct = total_ct;
-  if (p.ct < p.ct_first) p.ct = p.ct_first;
-  // Rows per block: 2048 for a full-width chunk; more when the shard is narrow (a rank of a
-  // vocabulary-parallel group), so that a launch still has a dozen tiles per CTA pair and the
-  // probability buffer stays around 600 MB. Whole multiples of 2048, at most 8192.
   int64_t rb = 2048;
   if (ct_override <= 0) {
-    rb = 2048 * (int64_t)((2 * waves * wave) / p.ct);
+    rb = 2048 * (int64_t)(592 / (total_ct < 296 ? (total_ct > 0 ? total_ct : 1) : 296));
     if (rb < 2048) rb = 2048;
     if (rb > 8192) rb = 8192;
   }
   p.row_block = (int)(n < rb ? (n < 1 ? 1 : n) : rb);
+  const int rt = (p.row_block + 2 * kBM - 1) / (2 * kBM);
+  if (ct_override > 0) {
+    p.ct_first = p.ct = ct_override;
+  } else {
+    p.ct_first = (kFirstTiles * rt + pairs - 1) / pairs * pairs / rt;   // whole waves, rounded down
+    for (int w = (kFirstTiles * rt + pairs - 1) / pairs; w <= 8; ++w) {
+      const int ct = w * pairs / rt;
+      if (rt * ct * 100 >= 97 * w * pairs) { p.ct_first = ct; break; }
+    }
+    p.ct = (int)(kChunkBytes / ((int64_t)p.row_block * kBN * 2));
+    if (waves && p.ct > waves * pairs / 2) p.ct = waves * pairs / 2;
+    // the later chunks of equal size
+    const int rest = total_ct - p.ct_first;
+    if (rest > 0 && p.ct < rest) {
+      const int chunks = (rest + p.ct - 1) / p.ct;
+      p.ct = (rest + chunks - 1) / chunks;
+    }
+  }
+  if (p.ct_first > total_ct) p.ct_first = total_ct;
+  if (p.ct_first < 1) p.ct_first = 1;
+  if (p.ct > total_ct) p.ct = total_ct;
+  if (p.ct < p.ct_first) p.ct = p.ct_first;
   return p;
 }
 
@@ -1199,6 +1292,20 @@ int encode_map_2d_16bit(CUtensorMap* map, const void* base, uint64_t rows, uint6
   return r == CUDA_SUCCESS ? 0 : -(int)r - 1000;
 }
 
+int encode_map_2d_f32(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
+                      uint64_t pitch_elems, uint32_t box_rows, uint32_t box_cols) {
+  EncodeTiledFn fn = get_encode_fn();
+  if (!fn) return -1;
+  const cuuint64_t dims[2] = {cols, rows};
+  const cuuint64_t strides[1] = {pitch_elems * 4};
+  const cuuint32_t box[2] = {box_cols, box_rows};
+  const cuuint32_t estr[2] = {1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<void*>(base), dims, strides,
+                        box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : -(int)r - 1000;
+}
+
 int encode_map_2d_bytes(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
                         uint64_t pitch_bytes, uint32_t box_rows, uint32_t box_cols) {
   EncodeTiledFn fn = get_encode_fn();
@@ -1259,22 +1366,25 @@ extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void
   const char* det_env = getenv("SOUP_LMHEAD_DETERMINISTIC");
   const bool deterministic = det_env && atoi(det_env) != 0;
 
-  CUtensorMap map_h, map_w_k, map_w_mn, map_p_ld, map_p_st;
+  CUtensorMap map_h, map_w_k, map_w_mn, map_p_ld, map_p_st, map_dh;
   if (umma::encode_map_2d_16bit(&map_h, hidden, (uint64_t)n, (uint64_t)h, (uint64_t)h, kBM, kBK, false) ||
       umma::encode_map_2d_16bit(&map_w_k, weight, (uint64_t)v_shard, (uint64_t)h, (uint64_t)h, kBN / 2, kBK, false) ||
       (want_grad &&
-       umma::encode_map_2d_16bit(&map_w_mn, weight_bf16, (uint64_t)v_shard, (uint64_t)h, (uint64_t)h, kBK, 64, true)) ||
+       (umma::encode_map_2d_16bit(&map_w_mn, weight_bf16, (uint64_t)v_shard, (uint64_t)h, (uint64_t)h, kBK, 64, true) ||
+        umma::encode_map_2d_f32(&map_dh, dh, (uint64_t)n, (uint64_t)h, (uint64_t)h, 32, 32))) ||
       umma::encode_map_2d_16bit(&map_p_ld, ws.p_buf, (uint64_t)plan.row_block, (uint64_t)ld_p,
                                 (uint64_t)ld_p, kBM, kBK, true) ||
       umma::encode_map_2d_16bit(&map_p_st, ws.p_buf, (uint64_t)plan.row_block, (uint64_t)ld_p,
                                 (uint64_t)ld_p, 32, 64, true))
     SOUP_FAIL(SOUP_ERR_DEVICE, "lmhead_ce: cuTensorMapEncodeTiled failed");
 
-  cudaMemsetAsync(ws.status, 0, 4, s);
-  if (want_grad) cudaMemsetAsync(dh, 0, (size_t)n * h * sizeof(float), s);
-  lmhead_init_state_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(
-      run_max, run_sum, run_dot, best, best_val, label_logit, grad_ref, (int)n);
-  SOUP_CHECK_LAUNCH("lmhead_init_state");
+  int* sticky = rowpipe::status_word();
+  const int64_t dh_vec = want_grad ? n * h / 4 : 0;   // h is a multiple of 8
+  const int64_t init_blocks = ((dh_vec > 4 * n ? dh_vec / 4 : n) + 255) / 256, init_cap = (n + 255) / 256 + 8 * sms;
+  lmhead_init_kernel<<<(unsigned)(init_blocks < init_cap ? init_blocks : init_cap), 256, 0, s>>>(
+      run_max, run_sum, run_dot, best, best_val, label_logit, grad_ref, ws.status,
+      want_grad ? reinterpret_cast<float4*>(dh) : nullptr, dh_vec, (int)n);
+  SOUP_CHECK_LAUNCH("lmhead_init");
 
   LaunchTimer timer(s);
   for (int64_t r0 = 0; r0 < n; r0 += plan.row_block) {
@@ -1299,6 +1409,7 @@ extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void
       la.ct_stride = plan.ct;
       la.store_p = want_grad;
       la.status = ws.status;
+      la.sticky = sticky;
       const int tiles1 = rt * ct;
       const unsigned grid1 = 2u * (unsigned)(tiles1 < max_pairs ? tiles1 : max_pairs);
 
@@ -1327,42 +1438,33 @@ extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void
       ra.mode = la.mode;
       ra.want_grad = want_grad;
       ra.status = ws.status;
+      ra.sticky = sticky;
       timer.mark(1);
-      lmhead_row_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(ra);
+      lmhead_row_kernel<<<(unsigned)rows, kRowThreads, 0, s>>>(ra);
       timer.mark(1);
       SOUP_CHECK_LAUNCH("lmhead_row");
 
       if (want_grad) {
-        if (first) {  // the first chunk's P from "against its tile maximum" to "against the lse"
-          timer.mark(1);
-          lmhead_rescale_first_kernel<<<(unsigned)((rows + 7) / 8), 256, 0, s>>>(
-              ws.p_buf, ld_p, ws.tile_stats, plan.ct, run_max + r0, rows, ct);
-          timer.mark(1);
-          SOUP_CHECK_LAUNCH("lmhead_rescale_first");
-        }
         GradArgs ga;
-        ga.dh = dh + r0 * h;
         ga.mult = ws.mult;
+        ga.row0 = (int)r0;
         ga.n_rows = rows;
         ga.k_dim = (int)h;
         ga.col0 = t0 * kBN;
         ga.n_kb = ct * (kBN / kBK);
         ga.status = ws.status;
+        ga.sticky = sticky;
         const int tiles2 = rt * (int)((h + kBN - 1) / kBN);
         ga.ksplit = pick_ksplit(tiles2, max_pairs, ga.n_kb, deterministic);
         const int units = tiles2 * ga.ksplit;
         const unsigned grid2 = 2u * (unsigned)(units < max_pairs ? units : max_pairs);
         timer.mark(2);
-        lmhead_grad_kernel<<<grid2, kThreadsGemm, kSmemGrad, s>>>(map_p_ld, map_w_mn, ga);
+        lmhead_grad_kernel<<<grid2, kThreadsGemm, kSmemGrad, s>>>(map_p_ld, map_w_mn, map_dh, ga);
         timer.mark(2);
         SOUP_CHECK_LAUNCH("lmhead_grad");
       }
       t0 += ct;
     }
-  }
-  if (int* sticky = rowpipe::status_word()) {
-    lmhead_publish_status_kernel<<<1, 1, 0, s>>>(ws.status, sticky);
-    SOUP_CHECK_LAUNCH("lmhead_publish_status");
   }
   timer.finish();
   return SOUP_OK;
@@ -1437,7 +1539,10 @@ extern "C" int soup_lmhead_finish_to(const float* run_max, const float* run_sum,
   a.dh_out = dh_out; a.dh_out_dtype = dh_out_dtype;
   a.n_rows = (int)n; a.k_dim = (int)h; a.v_shard = (int)v_shard; a.col_offset = (int)col_offset;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  lmhead_finish_kernel<<<(unsigned)n, 256, 0, s>>>(a);
+  const bool vec = h % 4 == 0 && (!dh || aligned16(dh)) && (!dh_out || aligned16(dh_out)) &&
+                   (reinterpret_cast<uintptr_t>(weight) & 7u) == 0;
+  if (vec) lmhead_finish_kernel<true><<<(unsigned)n, kFinishThreads, 0, s>>>(a);
+  else lmhead_finish_kernel<false><<<(unsigned)n, kFinishThreads, 0, s>>>(a);
   SOUP_CHECK_LAUNCH("lmhead_finish");
   return SOUP_OK;
 }
@@ -1452,16 +1557,37 @@ extern "C" int soup_lmhead_finish(const float* run_max, const float* run_sum, co
                                col_offset, stream);
 }
 
-extern "C" int soup_lmhead_grad_scale(const float* dh, void* out, const float* scale, int64_t n,
-                                      int out_dtype, void* stream) {
+extern "C" int soup_lmhead_totals(const float* token_loss, const int* correct, const int64_t* target,
+                                  const void* divisor, int divisor_kind, float divisor_value,
+                                  float* loss, int64_t* hits, int64_t* labelled, float* grad_divisor,
+                                  int64_t n, void* stream) {
+  using namespace soup;
+  if (n < 0 || n > INT32_MAX) SOUP_FAIL(SOUP_ERR_ARG, "lmhead_totals: bad shape");
+  if ((n && (!token_loss || !correct || !target)) || !loss || !hits || !labelled || !grad_divisor)
+    SOUP_FAIL(SOUP_ERR_ARG, "lmhead_totals: null pointer");
+  if (divisor_kind < 0 || divisor_kind > 3 || (divisor_kind >= 2 && !divisor))
+    SOUP_FAIL(SOUP_ERR_ARG, "lmhead_totals: divisor kind must be 0 (value), 1 (labelled rows), 2 (float*) or 3 (int64*)");
+  lmhead_totals_kernel<<<1, kTotalsThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      token_loss, correct, target, divisor, divisor_kind, divisor_value, loss, hits, labelled, grad_divisor, n);
+  SOUP_CHECK_LAUNCH("lmhead_totals");
+  return SOUP_OK;
+}
+
+extern "C" int soup_lmhead_backward(const float* dh, void* out, const float* grad_loss,
+                                    const float* grad_divisor, int64_t n, int out_dtype, void* stream) {
   using namespace soup;
   if (n == 0) return SOUP_OK;
-  if (!dh || !out || !scale || n < 0) SOUP_FAIL(SOUP_ERR_ARG, "lmhead_grad_scale: bad argument");
-  if (!is_float_dtype(out_dtype)) SOUP_FAIL(SOUP_ERR_ARG, "lmhead_grad_scale: unsupported dtype");
-  if (!aligned16(dh) || !aligned16(out)) SOUP_FAIL(SOUP_ERR_ARG, "lmhead_grad_scale: unaligned");
-  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (!dh || !out || !grad_loss || n < 0) SOUP_FAIL(SOUP_ERR_ARG, "lmhead_backward: bad argument");
+  if (!is_float_dtype(out_dtype)) SOUP_FAIL(SOUP_ERR_ARG, "lmhead_backward: unsupported dtype");
+  if (!aligned16(dh) || !aligned16(out)) SOUP_FAIL(SOUP_ERR_ARG, "lmhead_backward: unaligned");
   const int64_t n8 = (n >> 3) + 1;
-  lmhead_scale_cast_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, s>>>(dh, out, scale, n, out_dtype);
-  SOUP_CHECK_LAUNCH("lmhead_grad_scale");
+  lmhead_scale_cast_kernel<<<(unsigned)((n8 + 255) / 256), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+      dh, out, grad_loss, grad_divisor, n, out_dtype);
+  SOUP_CHECK_LAUNCH("lmhead_backward");
   return SOUP_OK;
+}
+
+extern "C" int soup_lmhead_grad_scale(const float* dh, void* out, const float* scale, int64_t n,
+                                      int out_dtype, void* stream) {
+  return soup_lmhead_backward(dh, out, scale, nullptr, n, out_dtype, stream);
 }

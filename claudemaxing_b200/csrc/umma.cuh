@@ -114,6 +114,14 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, const void*
                : "memory");
 }
 
+// The same box added to fp32 global memory (a tiled bulk reduction by the copy engine).
+__device__ __forceinline__ void tma_reduce_add_2d(const CUtensorMap* map, const void* smem_src, int32_t c0,
+                                                  int32_t c1) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];"
+               ::"l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(smem_src)), "r"(c0), "r"(c1)
+               : "memory");
+}
+
 __device__ __forceinline__ void tma_store_commit() {
   asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
@@ -358,6 +366,11 @@ __host__ __device__ constexpr uint32_t make_idesc_f16(int m, int n, uint32_t a_f
 // are not written.
 int encode_map_2d_16bit(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
                         uint64_t pitch_elems, uint32_t box_rows, uint32_t box_cols, bool bf16);
+
+// Row-major 2-D fp32 matrix; the box is [box_rows, box_cols] with box_cols * 4 == 128 bytes, in
+// shared memory with the 128-byte swizzle.
+int encode_map_2d_f32(CUtensorMap* map, const void* base, uint64_t rows, uint64_t cols,
+                      uint64_t pitch_elems, uint32_t box_rows, uint32_t box_cols);
 
 // Row-major 2-D byte matrix [rows, cols] with row pitch `pitch_bytes` (a multiple of 16); the box
 // is [box_rows, box_cols] with box_cols a multiple of 16, copied to shared memory row after row

@@ -54,7 +54,7 @@ int soup_row_status(int* host_status, void* stream);
 /* The same sticky word, for every kernel family: besides the row-kernel codes it receives the
  * code of a soup_lmhead_ce call whose bounded waits gave up (11-14 logits kernel, 21-24 gradient
  * kernel: producer, accumulator, operand and epilogue waits) or whose row merge met a non-finite
- * sum (90), copied from the call's workspace by the call's last launch, and 99 from
+ * sum (90), written by the launch that gave up, and 99 from
  * soup_wait_selftest. `clear` != 0 resets the word after reading it. Synchronises `stream`; meant
  * to be called where the host waits for the step's loss anyway. A non-zero word means outputs
  * since the last clear may be unwritten. No counterpart in the reference (its kernels cannot
@@ -330,7 +330,7 @@ int soup_lmhead_ce(const void* hidden, const void* weight, const void* weight_bf
 int soup_lmhead_set_timing(float* host_sink6);
 
 /* The tiling soup_lmhead_ce uses for a shape: rows per row block, 256-column tiles of the first
- * chunk (whose logits are computed twice) and of every later chunk. */
+ * chunk (written against its tiles' own maxima) and of every later chunk. */
 int soup_lmhead_plan(int64_t n, int64_t v_shard, int64_t chunk_tiles, int64_t* row_block,
                      int64_t* first_chunk_tiles, int64_t* tiles_per_chunk);
 
@@ -373,6 +373,21 @@ int soup_lmhead_finish_to(const float* run_max, const float* run_sum, const floa
 /* out = out_dtype(dh * scale[0]) — _FusedHeadLoss.backward, solution/lm_head_loss.py:248-254. */
 int soup_lmhead_grad_scale(const float* dh, void* out, const float* scale, int64_t n,
                            int out_dtype, void* stream);
+
+/* The step's numbers from the per-row terms in one launch: loss[0] = sum(token_loss) / divisor,
+ * hits[0] = sum(correct), labelled[0] = rows whose target is not -100, grad_divisor[0] = divisor *
+ * 1024 (what soup_lmhead_backward divides by). divisor_kind: 0 divisor_value, 1 the labelled rows,
+ * 2 a device float, 3 a device int64. Additions in a fixed order. Replaces the torch reductions
+ * around solution/lm_head_loss.py:238-245 and :268-282. */
+int soup_lmhead_totals(const float* token_loss, const int* correct, const int64_t* target,
+                       const void* divisor, int divisor_kind, float divisor_value, float* loss,
+                       int64_t* hits, int64_t* labelled, float* grad_divisor, int64_t n,
+                       void* stream);
+
+/* out = out_dtype(dh * (grad_loss[0] / grad_divisor[0])): soup_lmhead_grad_scale with the quotient
+ * formed on the device (grad_divisor NULL: 1). */
+int soup_lmhead_backward(const float* dh, void* out, const float* grad_loss,
+                         const float* grad_divisor, int64_t n, int out_dtype, void* stream);
 
 /* Loss / entropy / correct per row from materialised logits [n_rows, n_cols] (row pitch
  * row_stride elements). Replaces lm_head_xent_rows_kernel, solution/lm_head_loss.py:168-172

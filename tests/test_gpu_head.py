@@ -286,3 +286,35 @@ def test_finish_into_a_separate_typed_buffer_is_finish_then_one_rounding(out_dty
     assert torch.equal(out, raw.to(out_dtype))
     for a, b in zip(terms_a, terms_b):
         assert torch.equal(a, b)
+
+
+# (rows, hidden, vocabulary): one row; fewer rows than a CTA's 128; one past a CTA's, one past a
+# pair's 256; a ragged last row tile; a hidden size whose last 256-column output tile is ragged; one
+# column tile, one past the first chunk, a ragged last column tile. The contraction of the gradient
+# is split over all CTA pairs at every one of them.
+@pytest.mark.parametrize("dims", [(1, 64, 300), (24, 1536, 30000), (129, 904, 19200), (257, 512, 19201),
+                                  (1168, 264, 12000), (127, 1536, 255), (600, 72, 8193)])
+def test_gradient_split_over_all_pairs_at_the_edges_of_its_tiles(dims):
+    check(*make(*dims, seed=31, drop=0.0 if dims[0] == 1 else 0.3))   # one unlabelled row: 0 / 0
+
+
+@pytest.mark.parametrize("divisor", [None, 77, 77.0, torch.tensor(77), torch.tensor(77.0),
+                                     torch.tensor([77.0]), torch.tensor(77, dtype=torch.int32)])
+def test_totals_divide_by_every_kind_of_divisor(divisor):
+    """Loss, hits and labelled rows from one launch, and the gradient's divisor on the device,
+    for the labelled count, numbers, and tensors (of the dtypes the kernel reads and others)."""
+    from claudemaxing_b200.lm_head_loss import fused_head_loss
+
+    h, w, t = make(300, 64, 900, seed=33)
+    hd = h.to(DEV).requires_grad_(True)
+    loss, step = fused_head_loss(hd[None], w.to(DEV), None, num_items_in_batch=divisor, target=t.to(DEV)[None])
+    loss.sum().backward()
+    labelled = int((t != -100).sum())
+    div = labelled if divisor is None else 77
+    assert step.labelled.item() == labelled and step.labelled.dim() == 0
+    want = step.token_loss.double().sum().item() / div
+    assert abs(loss.item() - want) <= 1e-5 * abs(want)     # fp32 sums of 300 terms: 300 x 2^-24
+    from oracle.head_ce import head_ce
+
+    ref = head_ce(h, w, t, denominator=div)
+    assert_close_rel_max(hd.grad.cpu(), ref["dhidden"], 1e-2, "dhidden")
