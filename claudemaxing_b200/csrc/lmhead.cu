@@ -1105,14 +1105,17 @@ inline int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 // on 24 of the 74 pairs (215 us per call over 151936 columns, 93 us split over 72 of them; 1168 rows,
 // 30 tiles: 457 and 414 us). The order of units (tile fastest) keeps the pairs that run
 // together on one or two K ranges, whose rows of W they share through L2. 1 split keeps the result
-// deterministic.
+// deterministic. A unit has at least kMinUnit K blocks: the sums of more than two splits
+// arrive in any order, and a small model's fp16 step amplifies that (3000 columns, 48 blocks: two runs
+// differ by up to 1.4e-3 of a gradient with 47 splits, 9e-4 with four, not at all with two, for 5 us).
 constexpr int kUnitCost = 8;
+constexpr int kMinUnit = 20;
 constexpr int kMaxSplit = 80;
 inline int pick_ksplit(int tiles, int pairs, int n_kb, bool deterministic) {
   if (deterministic || tiles <= 0) return 1;
   int best = 1;
   long best_span = (long)((tiles + pairs - 1) / pairs) * (n_kb + kUnitCost);
-  for (int ks = 2; ks <= kMaxSplit && ks <= n_kb; ++ks) {
+  for (int ks = 2; ks <= kMaxSplit && ks * kMinUnit <= n_kb; ++ks) {
     const long span = (long)((tiles * ks + pairs - 1) / pairs) * ((n_kb + ks - 1) / ks + kUnitCost);
     if (span < best_span) { best = ks; best_span = span; }
   }
