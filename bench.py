@@ -539,9 +539,10 @@ def attention_suite(dev, tensor_peak):
             "ms": round(ms_own, 5), "tflops": round(flops / (ms_own * 1e-3) / 1e12, 1),
             "frac_of_measured_bf16_peak": round(flops / (ms_own * 1e-3) / 1e12 / tensor_peak, 4),
             "torch_varlen_flash_ms": round(ms_lib, 5), "launches": 1 if leg == "fwd" else 2,
-            "note": "latency-bound: ~150 CTAs each walking at most three key tiles; the backward "
-                    "launch count includes clearing the fp32 dK / dV buffers" if leg == "bwd" else
-                    "latency-bound: ~150 CTAs each walking at most three key tiles (score tiles resident in tensor memory between the two softmax passes)"}
+            "note": "latency-bound: ~150 CTAs each walking at most three query tiles; the backward's other "
+                    "launch clears the fp32 gradients and forms the rows' statistics (a torch cast of dq "
+                    "follows)" if leg == "bwd" else
+                    "latency-bound: ~150 CTAs each walking at most three key tiles, two CTAs per SM"}
     _lib.check_device_status()
     return out
 

@@ -26,18 +26,32 @@ OWN_FORWARD = os.environ.get("SOUP_ATTN_KERNEL", "1") != "0"
 OWN_BACKWARD = os.environ.get("SOUP_ATTN_BACKWARD", "1") != "0"
 
 
-def attention_gradients(q, k, v, out, lse, grad, cu_rows, scale):
-    """(dq fp16 [n, hq, 128], dk fp32 [n, hk, 128], dv fp32 [n, hk, 128]) of the segment attention
-    from this library's backward kernel (csrc/attention.cu)."""
+def attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, scale):
+    """(dq [n, hq, 128], dk [n, hk, 128], dv [n, hk, 128], flat): the fp32 gradients of the segment
+    attention from this library's backward kernel (csrc/attention.cu), and the one buffer the three
+    are consecutive parts of."""
     n, hq, d = q.shape
+    hk = k.shape[1]
     grad = grad if grad.is_contiguous() else grad.contiguous()
-    dq = torch.empty((n, hq, d), dtype=q.dtype, device=q.device)
-    dk, dv = torch.empty((2, n, k.shape[1], d), dtype=torch.float32, device=q.device)   # one clear
+    flat = torch.empty(n * (hq + 2 * hk) * d, dtype=torch.float32, device=q.device)
+    dq, dk, dv = _gradient_parts(flat, n, hq, hk, d)
+    stats = torch.empty(n * hq * 2, dtype=torch.float32, device=q.device)
     _lib.call("soup_attn_bwd", _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _lib.ptr(grad),
-              _lib.ptr(lse), _lib.ptr(cu_rows), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), n,
-              cu_rows.numel() - 1, hq, k.shape[1], d, q.stride(0), k.stride(0), v.stride(0),
+              _lib.ptr(lse), _lib.ptr(cu_rows), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(stats),
+              8 * n * hq, n, cu_rows.numel() - 1, hq, hk, d, q.stride(0), k.stride(0), v.stride(0),
               float(scale), _lib.stream_of(q))
-    return dq, dk, dv
+    return dq, dk, dv, flat
+
+
+def _gradient_parts(flat, n, hq, hk, d):
+    dq, dk, dv = flat.split((n * hq * d, n * hk * d, n * hk * d))
+    return dq.view(n, hq, d), dk.view(n, hk, d), dv.view(n, hk, d)
+
+
+def attention_gradients(q, k, v, out, lse, grad, cu_rows, scale):
+    """`attention_gradients_f32` with dq rounded to q's dtype: (dq, dk fp32, dv fp32)."""
+    dq, dk, dv, _ = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, scale)
+    return dq.to(q.dtype), dk, dv
 
 
 def mask_of_segments(cu_rows, n):
@@ -106,8 +120,8 @@ class SegmentAttention(torch.autograd.Function):
     def backward(ctx, grad):
         q, k, v, cu_rows, out, lse = ctx.saved_tensors
         if OWN_BACKWARD:
-            dq, dk, dv = attention_gradients(q, k, v, out, lse, grad, cu_rows, ctx.scale)
-            return dq, dk.to(k.dtype), dv.to(v.dtype), None, None, None
+            flat = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, ctx.scale)[3].to(q.dtype)
+            return (*_gradient_parts(flat, q.shape[0], q.shape[1], k.shape[1], q.shape[2]), None, None, None)
         rng_state = torch.empty(2, dtype=torch.uint64, device=q.device)   # no dropout: never read
         dq, dk, dv = torch.ops.torch_attn._varlen_attn_backward(
             grad.contiguous(), q, k, v, out, lse, cu_rows, cu_rows, ctx.longest, ctx.longest, True,

@@ -1,23 +1,24 @@
 // Causal attention inside the segments of one packed row (the batch rows of a packed training
 // batch), forward and backward, for head_dim 128 and fp16 q/k/v with grouped-query heads.
 //
-// Forward. One CTA owns 128 consecutive query tokens of one segment and one query head. The keys
-// and values it may see (its segment, up to its last token) arrive in tiles of 128 tokens by TMA
-// (keys through a two-stage ring). S = Q K^T of a tile is one tcgen05 product (M 128, N 128,
-// K 128) into a 128-column accumulator in tensor memory; the four softmax warps read it (thread =
-// query row). The softmax is done in two passes over the key tiles, so that the output
-// accumulator never has to be rescaled: the first pass only reduces the row maximum; the second
-// sums the exponentials, writes P = exp(S - max) as fp16 into a 128-byte-swizzled shared-memory
-// tile (the A operand) and accumulates O += P V in tensor memory (V as MN-major B operand). A
-// walk of up to three key tiles keeps all its score tiles in tensor memory between the passes
-// (S is formed once); a longer walk alternates two accumulators and forms every tile twice,
-// which at these sizes is cheap next to the latency of a rescale round trip through tensor
-// memory. The epilogue divides by the sum and writes fp16 rows and the log-sum-exp (natural log,
-// of the scaled scores) per row and head. The backward kernel is described where it starts.
+// Forward. A CTA owns 128 consecutive query tokens of one segment for NT query heads (one, or two
+// that share their key/value head) and walks the key tiles of 128 tokens these may see. Per tile
+// and head: S = Q K^T into 128 columns of tensor memory; the head's softmax warpgroup (thread =
+// query row) reads its row into registers, takes P = exp2(scale S - m) and writes it back as fp16
+// over S's columns; O += P V with P as the tensor-memory operand. m is the row maximum as of the
+// last rescale: O and the sum are rescaled only when the maximum has grown by more than 2^8 (P and
+// the sum stay far inside fp16 / fp32 range, and relative rounding does not depend on m), so almost
+// every tile goes without the round trip over O. The score product of the next tile is issued right
+// behind O += P V of this one; the commit that announces it also says that O may be rescaled.
 //
-// One CTA per SM (160 KB of shared memory, 512 columns of tensor memory): a CTA's walk is a chain
-// of dependent steps, so few large steps beat many small ones; CTAs take the tiles with the
-// longest walks first. Every wait is bounded (umma::mbar_wait).
+// What bounds it: on long walks the exponentials (16 a clock and SM: 1024 clocks a tile) and the
+// two products (1024 clocks a tile) alternate, so two tiles must be in flight on an SM. NT = 2 does
+// that inside a CTA and loads every key and value tile once for both heads; NT = 1 fits twice on an
+// SM (96 KB of shared memory, 256 columns) and does it with two CTAs: half the work per CTA and no
+// second wave where the row has few tiles. forward_heads_per_cta() draws the line.
+//
+// CTAs take the tiles with the longest walks first, over all heads. Every wait is bounded
+// (umma::mbar_wait).
 //
 // The reference calls torch SDPA here (solution/attention.py:332-343) on a [1, 1, N, N] mask
 // built by its packing (solution/lm_head_loss.py:300-337); this kernel takes the segment offsets.
@@ -32,29 +33,74 @@ namespace {
 
 using namespace umma;
 
-constexpr int kD = 128;          // head dimension
-constexpr int kBQ = 128;         // query rows per CTA
-constexpr int kBKV = 128;        // key/value rows per tile
-constexpr int kStages = 2;       // key tiles in flight (the value tile has one buffer)
+constexpr int kD = 128;                        // head dimension
+constexpr int kBQ = 128;                       // query rows per tile
+constexpr int kBKV = 128;                      // key/value rows per tile
 constexpr int kTileBytes = 128 * kD * 2;       // 32 KB: a [128 x 128] fp16 tile, two swizzled boxes
-constexpr int kQBytes = kBQ * kD * 2;          // 32 KB: two boxes of [128 rows x 64 cols]
-constexpr int kQBox = kBQ * 128;               // 16 KB
-constexpr int kKBytes = kBKV * kD * 2;         // 32 KB: two boxes of [128 rows x 64 cols]
-constexpr int kKVBox = kBKV * 128;             // 16 KB
-constexpr int kPBytes = kBQ * kBKV * 2;        // 32 KB: two boxes of [128 rows x 64 cols]
-constexpr int kThreads = 224;                  // warps 0-3 softmax, 4 key TMA, 5 MMA, 6 value TMA
-constexpr uint32_t kTmemCols = 512;            // score tiles from column 0, O behind them
+constexpr int kBox = kTileBytes / 2;           // one [128 rows x 64 cols] box
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kLn2 = 0.6931471805599453f;
+constexpr float kRescale = 8.0f;               // in powers of two: see the head of the file
 
-struct __align__(1024) Smem {
-  uint8_t q[kQBytes];
-  uint8_t k[kStages][kKBytes];
-  uint8_t v[kKBytes];
-  uint8_t p[kPBytes];
-  uint64_t q_full, k_full[kStages], k_empty[kStages], v_full, v_empty, s_full[3], s_empty[2], p_full,
-      p_empty, o_full;
-  uint32_t tmem_base;
-  int abort_flag;
+// Which tile a slot is. Slots go through the 128-row tiles of all segments in the order of their
+// depth inside the segment, deepest first (`depth` = tiles before it in its segment): the longest
+// walks of the forward, and, read from the other end, of the backward. More than 64 segments: plain
+// order. Called by whole warps; false for a slot past the last tile.
+struct Tile {
+  int seg_begin, seg_end, depth, tiles;   // tiles: of the whole segment
 };
+__device__ __forceinline__ bool locate_tile(const int32_t* cu, int segments, int slot, Tile& t) {
+  const int lane = threadIdx.x & 31;
+  if (segments <= 64) {
+    int b0 = 0, e0 = 0, b1 = 0, e1 = 0;
+    if (lane < segments) { b0 = cu[lane]; e0 = cu[lane + 1]; }
+    if (lane + 32 < segments) { b1 = cu[lane + 32]; e1 = cu[lane + 33]; }
+    const int n0 = (e0 - b0 + kBQ - 1) / kBQ, n1 = (e1 - b1 + kBQ - 1) / kBQ;
+    int left = slot;
+    for (int level = __reduce_max_sync(0xffffffffu, max(n0, n1)) - 1; level >= 0; --level) {
+      const uint32_t m0 = __ballot_sync(0xffffffffu, n0 > level), m1 = __ballot_sync(0xffffffffu, n1 > level);
+      const int c0 = __popc(m0), c = c0 + __popc(m1);
+      if (left < c) {
+        const bool low = left < c0;
+        const int src = __fns(low ? m0 : m1, 0, (low ? left : left - c0) + 1);
+        t.seg_begin = __shfl_sync(0xffffffffu, low ? b0 : b1, src);
+        t.seg_end = __shfl_sync(0xffffffffu, low ? e0 : e1, src);
+        t.tiles = __shfl_sync(0xffffffffu, low ? n0 : n1, src);
+        t.depth = level;
+        return true;
+      }
+      left -= c;
+    }
+    return false;
+  }
+  int base = 0;
+  for (int s0 = 0; s0 < segments; s0 += 32) {
+    int b = 0, e = 0;
+    if (s0 + lane < segments) { b = cu[s0 + lane]; e = cu[s0 + lane + 1]; }
+    const int n = (e - b + kBQ - 1) / kBQ;
+    int upto = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += y;
+    }
+    const uint32_t past = __ballot_sync(0xffffffffu, slot < base + upto);
+    if (past) {
+      const int src = __ffs(past) - 1;
+      t.seg_begin = __shfl_sync(0xffffffffu, b, src);
+      t.seg_end = __shfl_sync(0xffffffffu, e, src);
+      t.tiles = __shfl_sync(0xffffffffu, n, src);
+      t.depth = slot - base - (__shfl_sync(0xffffffffu, upto, src) - t.tiles);
+      return true;
+    }
+    base += __shfl_sync(0xffffffffu, upto, 31);
+  }
+  return false;
+}
+
+__device__ __forceinline__ uint32_t kstep(int k8) {   // K-major step of 16 columns, in descriptor units
+  return (uint32_t)(k8 >> 2) * (uint32_t)(kBox >> 4) + (uint32_t)(k8 & 3) * 2u;
+}
 
 struct AttnArgs {
   const int32_t* cu;     // [segments + 1]
@@ -62,293 +108,231 @@ struct AttnArgs {
   float* lse;            // [hq, n]
   int n, segments, hq, group;
   float scale_log2;      // softmax scale * log2(e)
-  float scale;
   int* status;
 };
 
-// Which (segment, first query token) a tile slot is: slots enumerate the 128-row tiles of the
-// segments in order. Returns false for a slot past the last tile.
-__device__ __forceinline__ bool locate(const int32_t* cu, int segments, int slot, int& seg_begin,
-                                       int& seg_end, int& q0) {
-  int base = 0;
-  for (int s = 0; s < segments; ++s) {
-    const int b = cu[s], e = cu[s + 1];
-    const int tiles = (e - b + kBQ - 1) / kBQ;
-    if (slot < base + tiles) {
-      seg_begin = b;
-      seg_end = e;
-      q0 = b + (slot - base) * kBQ;
-      return true;
-    }
-    base += tiles;
-  }
-  return false;
-}
+template <int NT>
+struct __align__(1024) FwdSmem {
+  static constexpr int kRing = 2 * NT;         // key and value tiles alternate: K0 V0 K1 V1 ...
+  uint8_t q[NT][kTileBytes];
+  uint8_t kv[kRing][kTileBytes];
+  uint64_t q_full, kv_full[kRing], kv_empty[kRing], s_full[NT], p_full[NT], o_full[NT];
+  uint32_t tmem_base;
+  int abort_flag;
+};
 
+template <int NT>
+constexpr int kFwdThreads = NT * 128 + 64;     // softmax warpgroups, then the TMA warp and the MMA warp
 
-// Four 16-byte chunks (32 fp16 columns starting at column `col0`, a multiple of 32) of row r of a
-// [128 x 128] fp16 tile stored as two 128-byte-swizzled boxes of 64 columns.
-__device__ __forceinline__ void write_tile_chunks(uint8_t* tile, int r, int col0, const uint32_t (&w)[16]) {
-  uint8_t* row = tile + (col0 >> 6) * (kTileBytes / 2) + r * 128;
-  const int j0 = (col0 & 63) >> 3;
+// One row of a score tile: its exponentials against the (possibly moved) reference m, as fp16 over
+// the score columns, and the row's sum. msl is m * scale_log2, rounded once and used everywhere, so
+// that its rounding cancels between P, the sum and the log-sum-exp.
+template <bool DIAG>
+__device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, int limit, bool first,
+                                             float sl, float& m, float& msl, float& l) {
+  uint32_t x[4][32];
 #pragma unroll
-  for (int j = 0; j < 4; ++j)
-    *reinterpret_cast<uint4*>(row + (((j0 + j) ^ (r & 7)) << 4)) =
-        make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
-}
-
-// Like `locate`, but the slots go through the tiles in the order of their walks' lengths: the
-// last tile of every segment first, then the ones before them, and so on.
-__device__ __forceinline__ bool locate_heavy_first(const int32_t* cu, int segments, int slot,
-                                                   int& seg_begin, int& seg_end, int& q0) {
-  if (segments > 64) return locate(cu, segments, slot, seg_begin, seg_end, q0);
-  int deepest = 0;
-  for (int s = 0; s < segments; ++s) deepest = max(deepest, (cu[s + 1] - cu[s] + kBQ - 1) / kBQ);
-  int base = 0;
-  for (int level = deepest - 1; level >= 0; --level)
-    for (int s = 0; s < segments; ++s) {
-      const int b = cu[s], e = cu[s + 1];
-      if ((e - b + kBQ - 1) / kBQ > level) {
-        if (slot == base) {
-          seg_begin = b;
-          seg_end = e;
-          q0 = b + level * kBQ;
-          return true;
-        }
-        ++base;
-      }
+  for (int c = 0; c < 4; ++c) tmem_ld_32x32(s_addr + c * 32, x[c]);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) tmem_ld_wait_on(x[c]);
+  float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      if (DIAG && c * 32 + j > limit) x[c][j] = 0xff800000u;   // -inf: no weight
+      mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(x[c][j]));
     }
-  return false;
+  const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+  if (first) {
+    m = top;
+    msl = m * sl;
+  } else {
+    const bool grow = (top - m) * sl > kRescale;
+    if (__any_sync(0xffffffffu, grow)) {   // rare
+      float f = 1.f;
+      if (grow) {
+        const float to = top * sl;
+        f = exp2f(msl - to);
+        m = top;
+        msl = to;
+      }
+      l *= f;
+#pragma unroll 1
+      for (int c = 0; c < kD; c += 16) {
+        uint32_t o[16];
+        tmem_ld_32x16(o_addr + c, o);
+        tmem_ld_wait_on(o);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
+        tmem_st_32x16(o_addr + c, o);
+      }
+      tmem_st_wait();
+    }
+  }
+  float s[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    uint32_t packed[16];
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      const float p0 = exp2f(fmaf(__uint_as_float(x[c][j]), sl, -msl));
+      const float p1 = exp2f(fmaf(__uint_as_float(x[c][j + 1]), sl, -msl));
+      s[j & 2] += p0;                      // the sum of exponentials, from the values before rounding
+      s[(j & 2) + 1] += p1;
+      __half2 hh = __floats2half2_rn(p0, p1);
+      packed[j >> 1] = *reinterpret_cast<uint32_t*>(&hh);
+    }
+    tmem_st_32x16(s_addr + c * 16, packed);
+  }
+  l += (s[0] + s[1]) + (s[2] + s[3]);
+  tmem_st_wait();
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+template <int NT>
+__global__ void __launch_bounds__(kFwdThreads<NT>, NT == 1 ? 2 : 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                const __grid_constant__ CUtensorMap map_v, AttnArgs a) {
+                const __grid_constant__ CUtensorMap map_v, const AttnArgs a) {
   extern __shared__ uint8_t raw[];
-  int seg_begin, seg_end, q0;
-  if (!locate_heavy_first(a.cu, a.segments, blockIdx.x, seg_begin, seg_end, q0)) return;   // the whole CTA leaves
+  using Smem = FwdSmem<NT>;
+  constexpr int kRing = Smem::kRing;
+  const int head_groups = a.hq / NT;
+  Tile tile;
+  // the whole CTA leaves when the slot is past the last tile
+  if (!locate_tile(a.cu, a.segments, blockIdx.x / head_groups, tile)) return;
   Smem& s = *reinterpret_cast<Smem*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y, hk = h / a.group;
-  const int q_end = min(seg_end, q0 + kBQ);                      // one past this tile's last token
-  const int n_kv = (q_end - seg_begin + kBKV - 1) / kBKV;        // key tiles it may see (>= 1)
+  const int h0 = (blockIdx.x % head_groups) * NT, hk = h0 / a.group;
+  const int q0 = tile.seg_begin + tile.depth * kBQ;
+  const int n_kv = tile.depth + 1;                               // key tiles it may see
+  constexpr int kLoadWarp = NT * 4, kMmaWarp = NT * 4 + 1;
   if (threadIdx.x == 0) {
     mbar_init(&s.q_full, 1);
-    for (int i = 0; i < kStages; ++i) {
-      mbar_init(&s.k_full[i], 1);
-      mbar_init(&s.k_empty[i], 1);
+    for (int i = 0; i < kRing; ++i) {
+      mbar_init(&s.kv_full[i], 1);
+      mbar_init(&s.kv_empty[i], 1);
     }
-    mbar_init(&s.v_full, 1);
-    mbar_init(&s.v_empty, 1);
-    for (int i = 0; i < 3; ++i) mbar_init(&s.s_full[i], 1);
-    for (int i = 0; i < 2; ++i) mbar_init(&s.s_empty[i], 4);
-    mbar_init(&s.p_full, 4);
-    mbar_init(&s.p_empty, 1);
-    mbar_init(&s.o_full, 1);
+    for (int t = 0; t < NT; ++t) {
+      mbar_init(&s.s_full[t], 1);
+      mbar_init(&s.p_full[t], 4);
+      mbar_init(&s.o_full[t], 1);
+    }
     s.abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == 4) {
-    tmem_alloc(&s.tmem_base, kTmemCols);
+  if (warp == kMmaWarp) {
+    tmem_alloc(&s.tmem_base, NT * 256);
     tmem_relinquish();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
-  const uint32_t tmem = s.tmem_base;
+  const uint32_t tmem = s.tmem_base;   // score columns of head t from t * 128, its O behind all scores
   volatile int* abort_flag = &s.abort_flag;
-  // Up to three key tiles (segments of up to 384 tokens): all score tiles stay in tensor memory
-  // (columns 0-383, O in 384-511), so the second pass reads them again instead of forming them
-  // again and the keys are loaded once. Longer walks alternate two score accumulators and form
-  // every tile twice (O in columns 256-383).
-  const bool resident = n_kv <= 3;
-  const uint32_t o_col = resident ? 3 * kBKV : 2 * kBKV;
 
-  if (warp == 4) {
-    // ---------------------------------------------------------------- Q and the key tiles
-    if (lane == 0) {
-      prefetch_tensormap(&map_q);
-      prefetch_tensormap(&map_k);
-      mbar_expect_tx(&s.q_full, kQBytes);
-      tma_load_2d(s.q, &map_q, h * kD, q0, &s.q_full);
-      tma_load_2d(s.q + kQBox, &map_q, h * kD + 64, q0, &s.q_full);
-      for (int g = 0; g < (resident ? n_kv : 2 * n_kv); ++g) {
-        const int st = g % kStages;
-        if (g >= kStages &&
-            !mbar_wait(&s.k_empty[st], ((g / kStages) & 1) ^ 1, abort_flag, a.status, 41))
-          break;
-        const int row = seg_begin + (g < n_kv ? g : g - n_kv) * kBKV;
-        mbar_expect_tx(&s.k_full[st], kKBytes);
-        tma_load_2d(s.k[st], &map_k, hk * kD, row, &s.k_full[st]);
-        tma_load_2d(s.k[st] + kKVBox, &map_k, hk * kD + 64, row, &s.k_full[st]);
-      }
-    }
-  } else if (warp == 6) {
-    // ---------------------------------------------------------------- the value tiles (pass 2)
+  if (warp == kLoadWarp) {
     if (lane == 0) {
       prefetch_tensormap(&map_v);
-      for (int t = 0; t < n_kv; ++t) {
-        if (t > 0 && !mbar_wait(&s.v_empty, (t - 1) & 1, abort_flag, a.status, 42)) break;
-        const int row = seg_begin + t * kBKV;
-        mbar_expect_tx(&s.v_full, kKBytes);
-        tma_load_2d(s.v, &map_v, hk * kD, row, &s.v_full);
-        tma_load_2d(s.v + kKVBox, &map_v, hk * kD + 64, row, &s.v_full);
+      mbar_expect_tx(&s.q_full, NT * kTileBytes);
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        tma_load_2d(s.q[t], &map_q, (h0 + t) * kD, q0, &s.q_full);
+        tma_load_2d(s.q[t] + kBox, &map_q, (h0 + t) * kD + 64, q0, &s.q_full);
+      }
+      for (int g = 0; g < 2 * n_kv; ++g) {
+        const int st = g % kRing;
+        if (g >= kRing && !mbar_wait(&s.kv_empty[st], ((g / kRing) & 1) ^ 1, abort_flag, a.status, 41)) break;
+        const CUtensorMap* map = (g & 1) ? &map_v : &map_k;
+        const int row = tile.seg_begin + (g >> 1) * kBKV;
+        mbar_expect_tx(&s.kv_full[st], kTileBytes);
+        tma_load_2d(s.kv[st], map, hk * kD, row, &s.kv_full[st]);
+        tma_load_2d(s.kv[st] + kBox, map, hk * kD + 64, row, &s.kv_full[st]);
       }
     }
-  } else if (warp == 5) {
-    // ---------------------------------------------------------------- MMA issue
+  } else if (warp == kMmaWarp) {
     if (lane == 0) {
       constexpr uint32_t idesc_s = make_idesc_f16(kBQ, kBKV, kFmtF16, kFmtF16, false, false);
       constexpr uint32_t idesc_o = make_idesc_f16(kBQ, kD, kFmtF16, kFmtF16, false, true);
-      const uint64_t dq = make_smem_desc(smem_u32(s.q), 16, 1024);
-      bool ok = mbar_wait(&s.q_full, 0, abort_flag, a.status, 43);
-      const uint64_t dp = make_smem_desc(smem_u32(s.p), 16, 1024);
-      const uint64_t dv = make_smem_desc(smem_u32(s.v), kKVBox, 1024);   // MN-major: boxes kKVBox apart
-      // S = Q K^T of the key tile in stage `st` into the accumulator at column `col`: 8 steps of
-      // 16 along the head dimension
-      auto mma_s = [&](int st, uint32_t col) {
-        const uint64_t dk = make_smem_desc(smem_u32(s.k[st]), 16, 1024);
-#pragma unroll
-        for (int k8 = 0; k8 < kD / 16; ++k8) {
-          const uint32_t qa = (uint32_t)(k8 >> 2) * (kQBox >> 4) + (uint32_t)(k8 & 3) * 2;
-          const uint32_t kb = (uint32_t)(k8 >> 2) * (kKVBox >> 4) + (uint32_t)(k8 & 3) * 2;
-          mma_f16_ss(tmem + col, dq + qa, dk + kb, idesc_s, k8 != 0);
-        }
+      auto full = [&](int g) {
+        return mbar_wait(&s.kv_full[g % kRing], (g / kRing) & 1, abort_flag, a.status, 44);
       };
-      // O (+)= P V along the key rows of the tile: P K-major, V MN-major
-      auto mma_pv = [&](int t) {
+      auto mma_s = [&](int t, int g) {   // S = Q K^T: 8 steps of 16 along the head dimension
+        const uint64_t dq = make_smem_desc(smem_u32(s.q[t]), 16, 1024);
+        const uint64_t dk = make_smem_desc(smem_u32(s.kv[g % kRing]), 16, 1024);
 #pragma unroll
-        for (int k8 = 0; k8 < kBKV / 16; ++k8) {
-          const uint32_t pa = (uint32_t)(k8 >> 2) * (kQBox >> 4) + (uint32_t)(k8 & 3) * 2;
-          mma_f16_ss(tmem + o_col, dp + pa, dv + k8 * (2048 >> 4), idesc_o, (t | k8) != 0);
-        }
+        for (int k8 = 0; k8 < kD / 16; ++k8)
+          mma_f16_ss(tmem + t * 128, dq + kstep(k8), dk + kstep(k8), idesc_s, k8 != 0);
+        tc_commit(&s.s_full[t]);
       };
-      auto issue_s = [&](int g) -> bool {   // the two-accumulator walk: tile g into accumulator g & 1
-        const int st = g % kStages, sb = g & 1;
-        if (!mbar_wait(&s.k_full[st], (g / kStages) & 1, abort_flag, a.status, 44)) return false;
-        if (g >= 2 && !mbar_wait(&s.s_empty[sb], ((g >> 1) & 1) ^ 1, abort_flag, a.status, 45))
-          return false;
+      bool ok = mbar_wait(&s.q_full, 0, abort_flag, a.status, 43) && full(0);
+      if (ok) {
         tc_fence_after_sync();
-        mma_s(st, sb * kBKV);
-        tc_commit(&s.s_full[sb]);
-        return true;
-      };
-      if (resident) {
-        for (int t = 0; t < n_kv && ok; ++t) {
-          ok = mbar_wait(&s.k_full[t % kStages], (t / kStages) & 1, abort_flag, a.status, 44);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) mma_s(t, 0);
+        tc_commit(&s.kv_empty[0]);
+      }
+      for (int i = 0; i < n_kv && ok; ++i) {
+        const int gv = 2 * i + 1, gk = 2 * i + 2;
+        const bool more = i + 1 < n_kv;
+        ok = full(gv);
+#pragma unroll
+        for (int t = 0; t < NT; ++t) {
+          ok = ok && mbar_wait(&s.p_full[t], i & 1, abort_flag, a.status, 47);
           if (!ok) break;
           tc_fence_after_sync();
-          mma_s(t % kStages, t * kBKV);
-          tc_commit(&s.s_full[t]);
-          tc_commit(&s.k_empty[t % kStages]);
-        }
-        for (int t = 0; t < n_kv && ok; ++t) {
-          ok = mbar_wait(&s.v_full, t & 1, abort_flag, a.status, 46);
-          if (ok) ok = mbar_wait(&s.p_full, t & 1, abort_flag, a.status, 47);
-          if (!ok) break;
-          tc_fence_after_sync();
-          mma_pv(t);
-          tc_commit(&s.v_empty);
-          tc_commit(&s.p_empty);
-        }
-      } else {
-        for (int g = 0; g < n_kv && ok; ++g) {   // pass 1: scores only
-          ok = issue_s(g);
-          if (ok) tc_commit(&s.k_empty[g % kStages]);
-        }
-        if (ok) ok = issue_s(n_kv);
-        for (int t = 0; t < n_kv && ok; ++t) {   // pass 2: scores of the next tile, then O += P V
-          const int g = n_kv + t;
-          if (t + 1 < n_kv) ok = issue_s(g + 1);
-          if (ok) ok = mbar_wait(&s.v_full, t & 1, abort_flag, a.status, 46);
-          if (ok) ok = mbar_wait(&s.p_full, t & 1, abort_flag, a.status, 47);
-          if (!ok) break;
-          tc_fence_after_sync();
-          mma_pv(t);
-          tc_commit(&s.k_empty[g % kStages]);
-          tc_commit(&s.v_empty);
-          tc_commit(&s.p_empty);
+          // O (+)= P V along the key rows of the tile: P from tensor memory, V MN-major
+          const uint64_t dv = make_smem_desc(smem_u32(s.kv[gv % kRing]), kBox, 1024);
+#pragma unroll
+          for (int k8 = 0; k8 < kBKV / 16; ++k8)
+            mma_f16_ts(tmem + (NT + t) * 128, tmem + t * 128 + k8 * 8, dv + k8 * (2048 >> 4), idesc_o, (i | k8) != 0);
+          if (t == NT - 1) tc_commit(&s.kv_empty[gv % kRing]);
+          if (more) {
+            if (t == 0) {
+              ok = full(gk);
+              if (!ok) break;
+              tc_fence_after_sync();
+            }
+            // over the columns of P, which the products above, in order before these, have read
+            mma_s(t, gk);
+            if (t == NT - 1) tc_commit(&s.kv_empty[gk % kRing]);
+          } else {
+            tc_commit(&s.o_full[t]);
+          }
         }
       }
-      if (ok) tc_commit(&s.o_full);
     }
   } else {
     // ---------------------------------------------------------------- softmax: thread = query row
-    const int r = threadIdx.x;
+    const int t = warp >> 2;
+    const int r = threadIdx.x & 127;
     const int q_idx = q0 + r;
-    const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
+    const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+    const uint32_t s_addr = lane_base + t * 128, o_addr = lane_base + (NT + t) * 128;
     const float sl = a.scale_log2;
-    float m = -INFINITY, l = 0.f;
+    float m = -INFINITY, msl = 0.f, l = 0.f;
     bool ok = true;
-    for (int g = 0; g < 2 * n_kv && ok; ++g) {
-      const int sb = g & 1;
-      const int tile = g < n_kv ? g : g - n_kv;
-      const uint32_t s_col = resident ? tile * kBKV : sb * kBKV;
-      if (!resident || g < n_kv) {   // resident tiles are complete once pass 1 has seen them
-        ok = resident ? mbar_wait(&s.s_full[tile], 0, abort_flag, a.status, 48)
-                      : mbar_wait(&s.s_full[sb], (g >> 1) & 1, abort_flag, a.status, 48);
-        ok = __all_sync(0xffffffffu, ok);
-        if (!ok) break;
-      }
+    for (int i = 0; i < n_kv; ++i) {
+      ok = __all_sync(0xffffffffu, mbar_wait(&s.s_full[t], i & 1, abort_flag, a.status, 48));
+      if (!ok) break;
       tc_fence_after_sync();
-      const int t = g < n_kv ? g : g - n_kv;
-      const int limit = q_idx - (seg_begin + t * kBKV);   // columns 0..limit are visible
-      if (g < n_kv) {   // pass 1: the row maximum only
-#pragma unroll 1
-        for (int c0 = 0; c0 < kBKV; c0 += 32) {
-          uint32_t x[32];
-          tmem_ld_32x32(lane_base + s_col + c0, x);
-          tmem_ld_wait_on(x);
-#pragma unroll
-          for (int c = 0; c < 32; ++c)
-            if (c0 + c <= limit) m = fmaxf(m, __uint_as_float(x[c]));
-        }
-        tc_fence_before_sync();
-        __syncwarp();
-        if (lane == 0 && !resident) mbar_arrive(&s.s_empty[sb]);
-      } else {          // pass 2: P = exp(S - max) as the fp16 A operand of O += P V
-        if (t > 0) {
-          ok = mbar_wait(&s.p_empty, (t - 1) & 1, abort_flag, a.status, 49);
-          ok = __all_sync(0xffffffffu, ok);
-          if (!ok) break;
-        }
-#pragma unroll 1
-        for (int c0 = 0; c0 < kBKV; c0 += 32) {
-          uint32_t x[32], packed[16];
-          tmem_ld_32x32(lane_base + s_col + c0, x);
-          tmem_ld_wait_on(x);
-#pragma unroll
-          for (int c = 0; c < 32; c += 2) {
-            const float p0 = c0 + c <= limit ? exp2f((__uint_as_float(x[c]) - m) * sl) : 0.f;
-            const float p1 = c0 + c + 1 <= limit ? exp2f((__uint_as_float(x[c + 1]) - m) * sl) : 0.f;
-            l += p0 + p1;       // the sum of exponentials, from the values before rounding
-            __half2 hh = __floats2half2_rn(p0, p1);
-            packed[c >> 1] = *reinterpret_cast<uint32_t*>(&hh);
-          }
-          write_tile_chunks(s.p, r, c0, packed);
-        }
-        tc_fence_before_sync();
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) {
-          if (!resident) mbar_arrive(&s.s_empty[sb]);
-          mbar_arrive(&s.p_full);
-        }
-      }
+      // only the last tile of the walk, the one on the diagonal, hides columns from a row
+      if (i + 1 < n_kv) softmax_tile<false>(s_addr, o_addr, 0, i == 0, sl, m, msl, l);
+      else softmax_tile<true>(s_addr, o_addr, r, i == 0, sl, m, msl, l);
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s.p_full[t]);
     }
-    if (ok) {
-      ok = mbar_wait(&s.o_full, 0, abort_flag, a.status, 50);
-      ok = __all_sync(0xffffffffu, ok);
-    }
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&s.o_full[t], 0, abort_flag, a.status, 50));
     if (ok) {
       tc_fence_after_sync();
       const float inv = 1.f / l;
-      const bool valid = q_idx < seg_end;
+      const bool valid = q_idx < tile.seg_end;
+      const int h = h0 + t;
       __half* dst = a.out + ((size_t)q_idx * a.hq + h) * kD;
 #pragma unroll
       for (int c0 = 0; c0 < kD; c0 += 32) {
         uint32_t o[32];
-        tmem_ld_32x32(lane_base + o_col + c0, o);
+        tmem_ld_32x32(o_addr + c0, o);
         tmem_ld_wait_on(o);
         if (valid) {
 #pragma unroll
@@ -364,107 +348,215 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           }
         }
       }
-      if (valid) a.lse[(size_t)h * a.n + q_idx] = m * a.scale + logf(l);
+      if (valid) a.lse[(size_t)h * a.n + q_idx] = (msl + log2f(l)) * kLn2;
       tc_fence_before_sync();
     }
   }
   __syncthreads();
-  if (warp == 4) {
+  if (s.abort_flag) {   // copies that may still be in flight land before the shared memory is released
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);
+    __syncthreads();
+  }
+  if (warp == kMmaWarp) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem, kTmemCols);
+    tmem_dealloc(tmem, NT * 256);
   }
 }
 
-}  // namespace
-}  // namespace soup
-
-namespace soup {
-namespace {
-
 // ------------------------------------------------------------------------------------------
-// Backward. Same decomposition as forward (a CTA owns 128 query tokens of one segment and one
-// query head and walks the key tiles it may see), but with key tiles of 128 tokens and one CTA
-// per SM: the walk is a chain of dependent steps, so fewer and larger steps are what shorten it.
-// Per key tile:
-//   S = Q K^T and dP = dO V^T            (two products into tensor-memory columns 0-127 / 128-255)
-//   P = exp(scale S - lse), dS = P (dP - D)   by the four row warps (D = rowsum(dO o O), formed
-//                                         by the same threads when the kernel starts)
-//   dV^T = dO^T P, dK^T = Q^T dS          (A and B both MN-major; into the columns S and dP left)
-//   dQ  += dS K                            (accumulates over the key tiles in columns 256-383)
-// dV^T and dK^T come out with the head dimension on the tensor-memory lanes; the row warps stage
-// them in shared memory as [key row][head dim] fp32 (over the V, P, dS and K tiles, all dead by
-// then) and bulk reductions (cp.reduce.async.bulk) add each key row to the fp32 dK / dV buffers:
-// the query heads of a group and the query tiles of a segment all add into the same rows. dQ
-// needs no atomics; it is scaled, rounded to fp16 and stored when the walk ends. CTAs take the
-// tiles with the longest walks first (`locate_heavy_first`), so that the few CTAs beyond one per
-// SM are short ones.
-constexpr int kBKVb = 128;                     // key rows per tile in backward
-constexpr uint32_t kTmemColsBwd = 512;         // S/dV^T [0,128) dP/dK^T [128,256) dQ [256,384)
+// Backward. A CTA owns one 128-token key/value tile of a segment and one query
+// head, keeps K, V and the accumulators dV and dK (tensor memory) and walks the query tiles from the
+// diagonal to the segment's end. Per query tile, everything transposed (lanes = key rows):
+//   S^T = K Q^T, dP^T = V dO^T               tensor-memory columns 0-127 / 128-255
+//   P^T = exp2(scale S^T - lse)              two compute warpgroups (64 query columns each), fp16 over S^T
+//   dV += P^T dO                             A from tensor memory, columns 256-383
+//   dS^T = P^T (dP^T - D)                    fp16 over dP^T, and to shared memory
+//   dK += dS^T Q                             A from tensor memory, columns 384-511
+//   dQ  = dS K                               A from shared memory, over dP^T's columns; a third
+//                                            warpgroup adds it to fp32 global memory (bulk reductions)
+// The score product of the next tile is issued as soon as dV has consumed P^T, so the exponentials of
+// tile i + 1 run under the dK / dQ products of tile i. dK and dV leave once per CTA.
+//
+// What bounds it: shared-memory bandwidth. The five products read 256 KB of operands per tile (S^T
+// and dP^T and dQ both operands, dV and dK one), staging and loads move 224 KB more: 3750 clocks at
+// 128 B a clock against 2560 clocks of products. (A query-stationary walk reads and moves 700 KB per
+// tile: it stages and adds dK and dV, 128 KB, where this one adds dQ, 64 KB. It took 35.8 us for 1280
+// tokens in 5 segments, 12 / 2 heads, and 790 us for 9215 tokens in 4; this one 22.8 and 300 us.)
+// ------------------------------------------------------------------------------------------
+constexpr int kBwdThreads = 448;   // warps 0-7 compute, 8-11 dQ, 12 loads, 13 products
+constexpr int kDqWarp = 8, kBwdLoadWarp = 12, kBwdMmaWarp = 13;
+constexpr uint32_t kColS = 0, kColP = 128, kColDv = 256, kColDk = 384;
 
-struct BwdSmem {
-  uint8_t q[kTileBytes];
-  uint8_t d_o[kTileBytes];
-  uint8_t v[kTileBytes];     // V_t; with p: the fp32 staging tile of dV
-  uint8_t p[kTileBytes];
-  uint8_t ds[kTileBytes];    // dS_t; with k: the fp32 staging tile of dK
+struct KvSmem {
   uint8_t k[kTileBytes];
-  uint64_t q_full, k_full, k_empty, v_full, v_empty, sdp_full, pds_full, grads_full, acc_free;
+  uint8_t v[kTileBytes];
+  uint8_t q[2][kTileBytes];    // k, v and q stage dV and dK (fp32) when the walk is over
+  uint8_t d_o[kTileBytes];
+  uint8_t ds[kTileBytes];      // dS^T [key rows x query columns]
+  uint8_t stage[4][8192];      // per dQ warp two 32 x 32 fp32 boxes
+  float2 stats[2][kBQ];        // (lse * log2 e, D) of the query tile's rows
+  uint64_t k_full, v_full, q_full[2], q_empty[2], do_full, do_empty, s_full, p_full, dp_full, ds_full,
+      dq_full, dq_free, stats_full[2], done;
   uint32_t tmem_base;
   int abort_flag;
 };
+static_assert(sizeof(KvSmem) <= 232448, "shared memory of one CTA");
 
-struct AttnBwdArgs {
+struct AttnKvArgs {
   const int32_t* cu;
-  const __half* out;     // [n, hq, 128]
-  const __half* d_out;   // [n, hq, 128]
-  const float* lse;      // [hq, n]
-  __half* dq;            // [n, hq, 128]
-  float* dk;             // [n, hk, 128] fp32, zero on entry
-  float* dv;             // [n, hk, 128] fp32, zero on entry
-  int n, segments, hq, hk, group;
+  const float2* stats;   // [hq, n]
+  int n, segments, hq, group;
   float scale_log2, scale;
   int* status;
 };
 
-// Adds `bytes` of fp32 values in shared memory to global memory (both 16-byte aligned, bytes a
-// multiple of 16) by one bulk asynchronous reduction; part of the thread's current bulk group.
-__device__ __forceinline__ void bulk_red_add_f32(float* gdst, const void* ssrc, uint32_t bytes) {
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
-               ::"l"(gdst), "r"(smem_u32(ssrc)), "r"(bytes)
-               : "memory");
+// D = rowsum(dO o O) and lse in powers of two per (token, head), and the cleared accumulators. 16
+// lanes per row of 128; bound by memory (512 B read, 512 B + cleared per row).
+constexpr int kPrepThreads = 256;
+__global__ void __launch_bounds__(kPrepThreads)
+attn_bwd_prep_kernel(const __half* __restrict__ out, const __half* __restrict__ d_out,
+                     const float* __restrict__ lse, float2* __restrict__ stats, float4* __restrict__ dq,
+                     float4* __restrict__ dk, float4* __restrict__ dv, int64_t rows_q, int64_t rows_k,
+                     int n, int hq) {
+  const int64_t row = (int64_t)blockIdx.x * (kPrepThreads / 16) + (threadIdx.x >> 4);
+  const int lane = threadIdx.x & 15;
+  const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (row < rows_k) {
+    dk[row * 32 + lane] = dk[row * 32 + 16 + lane] = zero;
+    dv[row * 32 + lane] = dv[row * 32 + 16 + lane] = zero;
+  }
+  float d = 0.f;
+  if (row < rows_q) {
+    const uint4 x = reinterpret_cast<const uint4*>(out)[row * 16 + lane];
+    const uint4 y = reinterpret_cast<const uint4*>(d_out)[row * 16 + lane];
+    const __half2* xh = reinterpret_cast<const __half2*>(&x);
+    const __half2* yh = reinterpret_cast<const __half2*>(&y);
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 xf = __half22float2(xh[e]), yf = __half22float2(yh[e]);
+      d = fmaf(xf.x, yf.x, fmaf(xf.y, yf.y, d));
+    }
+    dq[row * 32 + lane] = dq[row * 32 + 16 + lane] = zero;
+  }
+#pragma unroll
+  for (int o = 8; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+  if (row < rows_q && lane == 0) {
+    const int64_t token = row / hq;
+    const int64_t at = (row - token * hq) * n + token;
+    stats[at] = make_float2(lse[at] * kLog2e, d);
+  }
 }
 
-__device__ __forceinline__ void row_warps_sync() {   // the four row warps, named barrier 1
-  asm volatile("bar.sync 1, 128;" ::: "memory");
+// 32 fp32 columns of row `lane` of a 32 x 32 fp32 box with the 128-byte swizzle (8 pieces of 16 B).
+__device__ __forceinline__ void write_box_row(uint8_t* box, int lane, const uint32_t (&x)[32], float f, bool keep) {
+  uint8_t* mine = box + lane * 128;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    float4 v = make_float4(__uint_as_float(x[4 * j]) * f, __uint_as_float(x[4 * j + 1]) * f,
+                           __uint_as_float(x[4 * j + 2]) * f, __uint_as_float(x[4 * j + 3]) * f);
+    if (!keep) v = make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4*>(mine + ((j ^ (lane & 7)) << 4)) = v;
+  }
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
+// One query tile for one compute thread: key row r, query columns [64 * wg, 64 * wg + 64).
+struct ComputeTile {
+  uint32_t s_addr, dp_addr;   // this thread's lane, columns of its warpgroup
+  const float2* stats;        // its 64 columns
+  uint8_t* ds_box;            // its 64-column box of dS^T
+  int r;
+};
+
+template <bool DIAG>
+__device__ __forceinline__ void probabilities(const ComputeTile& t, int first_col, float sl, float (&p)[64]) {
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    uint32_t x[32], packed[16];
+    tmem_ld_32x32(t.s_addr + c * 32, x);
+    tmem_ld_wait_on(x);
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      // (lse, D) of two columns at a time; every thread of the warpgroup reads the same ones
+      const float4 st = *reinterpret_cast<const float4*>(t.stats + c * 32 + j);
+      float p0 = exp2f(fmaf(__uint_as_float(x[j]), sl, -st.x));
+      float p1 = exp2f(fmaf(__uint_as_float(x[j + 1]), sl, -st.z));
+      if (DIAG) {   // a query sees the keys up to its own row
+        if (first_col + c * 32 + j < t.r) p0 = 0.f;
+        if (first_col + c * 32 + j + 1 < t.r) p1 = 0.f;
+      }
+      p[c * 32 + j] = p0;
+      p[c * 32 + j + 1] = p1;
+      __half2 hh = __floats2half2_rn(p0, p1);
+      packed[j >> 1] = *reinterpret_cast<uint32_t*>(&hh);
+    }
+    tmem_st_32x16(t.s_addr + c * 16, packed);
+  }
+  tmem_st_wait();
+}
+
+__device__ __forceinline__ void score_gradients(const ComputeTile& t, const float (&p)[64]) {
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    uint32_t y[32], packed[16];
+    tmem_ld_32x32(t.dp_addr + c * 32, y);
+    tmem_ld_wait_on(y);
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+      const float4 st = *reinterpret_cast<const float4*>(t.stats + c * 32 + j);
+      const float p0 = p[c * 32 + j], p1 = p[c * 32 + j + 1];
+      __half2 hh = __floats2half2_rn(p0 * (__uint_as_float(y[j]) - st.y), p1 * (__uint_as_float(y[j + 1]) - st.w));
+      packed[j >> 1] = *reinterpret_cast<uint32_t*>(&hh);
+    }
+    tmem_st_32x16(t.dp_addr + c * 16, packed);
+    uint8_t* row = t.ds_box + t.r * 128;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      *reinterpret_cast<uint4*>(row + (((c * 4 + j) ^ (t.r & 7)) << 4)) =
+          make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
+  }
+  tmem_st_wait();
+}
+
+__global__ void __launch_bounds__(kBwdThreads, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_do,
-                const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
-                AttnBwdArgs a) {
-  extern __shared__ uint8_t raw[];
-  int seg_begin, seg_end, q0;
-  if (!locate_heavy_first(a.cu, a.segments, blockIdx.x, seg_begin, seg_end, q0)) return;
-  BwdSmem& s = *reinterpret_cast<BwdSmem*>((reinterpret_cast<uintptr_t>(raw) + 1023) & ~uintptr_t(1023));
+                   const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                   const __grid_constant__ CUtensorMap map_dq, const __grid_constant__ CUtensorMap map_dk,
+                   const __grid_constant__ CUtensorMap map_dv, const AttnKvArgs a) {
+  extern __shared__ __align__(1024) uint8_t raw_kv[];
+  Tile tile;
+  if (!locate_tile(a.cu, a.segments, blockIdx.x / a.hq, tile)) return;   // the whole CTA leaves
+  KvSmem& s = *reinterpret_cast<KvSmem*>(raw_kv);
+  if (smem_u32(raw_kv) & 1023) {   // the swizzled tiles and their descriptors want it; no room to align by hand
+    if (threadIdx.x == 0) atomicCAS(a.status, 0, 60);
+    return;
+  }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.y, hk = h / a.group;
-  const int q_end = min(seg_end, q0 + kBQ);
-  const int n_kv = (q_end - seg_begin + kBKVb - 1) / kBKVb;
+  const int h = blockIdx.x % a.hq, hk = h / a.group;
+  // depth counts from the walk's end: the tile with the longest walk is the segment's first
+  const int n_q = tile.depth + 1;                                   // query tiles of the walk
+  const int kv0 = tile.seg_begin + (tile.tiles - 1 - tile.depth) * kBKV;
   if (threadIdx.x == 0) {
-    mbar_init(&s.q_full, 1);
     mbar_init(&s.k_full, 1);
-    mbar_init(&s.k_empty, 1);
     mbar_init(&s.v_full, 1);
-    mbar_init(&s.v_empty, 1);
-    mbar_init(&s.sdp_full, 1);
-    mbar_init(&s.pds_full, 4);
-    mbar_init(&s.grads_full, 1);
-    mbar_init(&s.acc_free, 4);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&s.q_full[i], 1);
+      mbar_init(&s.q_empty[i], 1);
+      mbar_init(&s.stats_full[i], 4);
+    }
+    mbar_init(&s.do_full, 1);
+    mbar_init(&s.do_empty, 1);
+    mbar_init(&s.s_full, 1);
+    mbar_init(&s.p_full, 8);
+    mbar_init(&s.dp_full, 1);
+    mbar_init(&s.ds_full, 8);
+    mbar_init(&s.dq_full, 1);
+    mbar_init(&s.dq_free, 4);
+    mbar_init(&s.done, 1);
     s.abort_flag = 0;
     fence_barrier_init();
   }
-  if (warp == 4) {
-    tmem_alloc(&s.tmem_base, kTmemColsBwd);
+  if (warp == kBwdMmaWarp) {
+    tmem_alloc(&s.tmem_base, 512);
     tmem_relinquish();
   }
   tc_fence_before_sync();
@@ -472,216 +564,231 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc_fence_after_sync();
   const uint32_t tmem = s.tmem_base;
   volatile int* abort_flag = &s.abort_flag;
-  constexpr int kBox = kTileBytes / 2;   // one [128 rows x 64 cols] box
+  const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
 
-  if (warp == 4) {
-    if (lane == 0) {   // Q, dO, then the key tiles
-      prefetch_tensormap(&map_q);
-      prefetch_tensormap(&map_do);
-      prefetch_tensormap(&map_k);
-      mbar_expect_tx(&s.q_full, 2 * kTileBytes);
-      tma_load_2d(s.q, &map_q, h * kD, q0, &s.q_full);
-      tma_load_2d(s.q + kBox, &map_q, h * kD + 64, q0, &s.q_full);
-      tma_load_2d(s.d_o, &map_do, h * kD, q0, &s.q_full);
-      tma_load_2d(s.d_o + kBox, &map_do, h * kD + 64, q0, &s.q_full);
-      for (int t = 0; t < n_kv; ++t) {
-        if (t > 0 && !mbar_wait(&s.k_empty, (t - 1) & 1, abort_flag, a.status, 51)) break;
-        const int row = seg_begin + t * kBKVb;
-        mbar_expect_tx(&s.k_full, kTileBytes);
-        tma_load_2d(s.k, &map_k, hk * kD, row, &s.k_full);
-        tma_load_2d(s.k + kBox, &map_k, hk * kD + 64, row, &s.k_full);
-      }
-    }
-  } else if (warp == 6) {
-    if (lane == 0) {   // the value tiles
-      prefetch_tensormap(&map_v);
-      for (int t = 0; t < n_kv; ++t) {
-        if (t > 0 && !mbar_wait(&s.v_empty, (t - 1) & 1, abort_flag, a.status, 52)) break;
-        const int row = seg_begin + t * kBKVb;
-        mbar_expect_tx(&s.v_full, kTileBytes);
-        tma_load_2d(s.v, &map_v, hk * kD, row, &s.v_full);
-        tma_load_2d(s.v + kBox, &map_v, hk * kD + 64, row, &s.v_full);
-      }
-    }
-  } else if (warp == 5) {
+  if (warp == kBwdLoadWarp) {
     if (lane == 0) {
-      // every operand is a [128 x 128] fp16 tile of two swizzled boxes: K-major steps of 16
-      // columns advance 32 bytes inside a box (4 per box); MN-major steps of 16 rows advance
-      // 2048 bytes, the two boxes being the leading-dimension offset apart
-      constexpr uint32_t idesc_s = make_idesc_f16(kBQ, kBKVb, kFmtF16, kFmtF16, false, false);
-      constexpr uint32_t idesc_t = make_idesc_f16(kD, kBKVb, kFmtF16, kFmtF16, true, true);
-      constexpr uint32_t idesc_q = make_idesc_f16(kBQ, kD, kFmtF16, kFmtF16, false, true);
-      const uint64_t q_k = make_smem_desc(smem_u32(s.q), 16, 1024);
-      const uint64_t do_k = make_smem_desc(smem_u32(s.d_o), 16, 1024);
-      const uint64_t k_k = make_smem_desc(smem_u32(s.k), 16, 1024);
-      const uint64_t v_k = make_smem_desc(smem_u32(s.v), 16, 1024);
-      const uint64_t ds_k = make_smem_desc(smem_u32(s.ds), 16, 1024);
-      const uint64_t q_mn = make_smem_desc(smem_u32(s.q), kBox, 1024);
-      const uint64_t do_mn = make_smem_desc(smem_u32(s.d_o), kBox, 1024);
-      const uint64_t k_mn = make_smem_desc(smem_u32(s.k), kBox, 1024);
-      const uint64_t p_mn = make_smem_desc(smem_u32(s.p), kBox, 1024);
-      const uint64_t ds_mn = make_smem_desc(smem_u32(s.ds), kBox, 1024);
-      auto kstep = [](int k8) { return (uint32_t)(k8 >> 2) * (uint32_t)(kBox >> 4) + (uint32_t)(k8 & 3) * 2u; };
-      bool ok = mbar_wait(&s.q_full, 0, abort_flag, a.status, 53);
-      for (int t = 0; t < n_kv && ok; ++t) {
-        ok = mbar_wait(&s.k_full, t & 1, abort_flag, a.status, 54);
-        if (ok && t > 0) ok = mbar_wait(&s.acc_free, (t - 1) & 1, abort_flag, a.status, 56);
-        if (!ok) break;
-        tc_fence_after_sync();
-#pragma unroll
-        for (int k8 = 0; k8 < kD / 16; ++k8)
-          mma_f16_ss(tmem, q_k + kstep(k8), k_k + kstep(k8), idesc_s, k8 != 0);
-        ok = mbar_wait(&s.v_full, t & 1, abort_flag, a.status, 55);
-        if (!ok) break;
-        tc_fence_after_sync();
-#pragma unroll
-        for (int k8 = 0; k8 < kD / 16; ++k8)
-          mma_f16_ss(tmem + 128, do_k + kstep(k8), v_k + kstep(k8), idesc_s, k8 != 0);
-        tc_commit(&s.sdp_full);
-        ok = mbar_wait(&s.pds_full, t & 1, abort_flag, a.status, 57);
-        if (!ok) break;
-        tc_fence_after_sync();
-#pragma unroll
-        for (int k8 = 0; k8 < kBQ / 16; ++k8)   // along the query rows
-          mma_f16_ss(tmem, do_mn + k8 * (2048 >> 4), p_mn + k8 * (2048 >> 4), idesc_t, k8 != 0);
-#pragma unroll
-        for (int k8 = 0; k8 < kBQ / 16; ++k8)
-          mma_f16_ss(tmem + 128, q_mn + k8 * (2048 >> 4), ds_mn + k8 * (2048 >> 4), idesc_t, k8 != 0);
-#pragma unroll
-        for (int k8 = 0; k8 < kBKVb / 16; ++k8)  // along the key rows of the tile
-          mma_f16_ss(tmem + 256, ds_k + kstep(k8), k_mn + k8 * (2048 >> 4), idesc_q, (t | k8) != 0);
-        tc_commit(&s.grads_full);
+      auto tile_in = [&](uint8_t* dst, const CUtensorMap* map, int col, int row, uint64_t* bar) {
+        mbar_expect_tx(bar, kTileBytes);
+        tma_load_2d(dst, map, col, row, bar);
+        tma_load_2d(dst + kBox, map, col + 64, row, bar);
+      };
+      tile_in(s.k, &map_k, hk * kD, kv0, &s.k_full);
+      tile_in(s.q[0], &map_q, h * kD, kv0, &s.q_full[0]);
+      tile_in(s.v, &map_v, hk * kD, kv0, &s.v_full);
+      tile_in(s.d_o, &map_do, h * kD, kv0, &s.do_full);
+      for (int i = 1; i < n_q; ++i) {
+        const int row = kv0 + i * kBQ;
+        if (i >= 2 && !mbar_wait(&s.q_empty[i & 1], ((i >> 1) & 1) ^ 1, abort_flag, a.status, 61)) break;
+        tile_in(s.q[i & 1], &map_q, h * kD, row, &s.q_full[i & 1]);
+        if (!mbar_wait(&s.do_empty, (i - 1) & 1, abort_flag, a.status, 62)) break;
+        tile_in(s.d_o, &map_do, h * kD, row, &s.do_full);
       }
     }
-  } else {
-    const int r = threadIdx.x;
-    const int q_idx = q0 + r;
-    const bool valid = q_idx < seg_end;
-    const uint32_t lane_base = tmem + ((uint32_t)(warp * 32) << 16);
-    // D = rowsum(dO o O) and the row's log-sum-exp (in log2 units)
-    float delta = 0.f, lse2 = 0.f;
-    if (valid) {
-      const uint4* po = reinterpret_cast<const uint4*>(a.out + ((size_t)q_idx * a.hq + h) * kD);
-      const uint4* pg = reinterpret_cast<const uint4*>(a.d_out + ((size_t)q_idx * a.hq + h) * kD);
+  } else if (warp == kBwdMmaWarp) {
+    if (lane == 0) {
+      constexpr uint32_t idesc_nn = make_idesc_f16(128, 128, kFmtF16, kFmtF16, false, false);
+      constexpr uint32_t idesc_nt = make_idesc_f16(128, 128, kFmtF16, kFmtF16, false, true);
+      constexpr uint32_t idesc_tt = make_idesc_f16(128, 128, kFmtF16, kFmtF16, true, true);
+      const uint64_t k_k = make_smem_desc(smem_u32(s.k), 16, 1024), k_mn = make_smem_desc(smem_u32(s.k), kBox, 1024);
+      const uint64_t v_k = make_smem_desc(smem_u32(s.v), 16, 1024);
+      const uint64_t do_k = make_smem_desc(smem_u32(s.d_o), 16, 1024);
+      const uint64_t do_mn = make_smem_desc(smem_u32(s.d_o), kBox, 1024);
+      const uint64_t ds_mn = make_smem_desc(smem_u32(s.ds), kBox, 1024);
+      auto wait = [&](uint64_t* bar, int turn, int code) {
+        const bool got = mbar_wait(bar, turn & 1, abort_flag, a.status, code);
+        tc_fence_after_sync();
+        return got;
+      };
+      auto scores = [&](int i) {
+        const uint64_t q_k = make_smem_desc(smem_u32(s.q[i & 1]), 16, 1024);
 #pragma unroll
-      for (int i = 0; i < kD / 8; ++i) {
-        const uint4 x = po[i], y = pg[i];
-        const __half2* xh = reinterpret_cast<const __half2*>(&x);
-        const __half2* yh = reinterpret_cast<const __half2*>(&y);
+        for (int k8 = 0; k8 < 8; ++k8)
+          mma_f16_ss(tmem + kColS, k_k + kstep(k8), q_k + kstep(k8), idesc_nn, k8 != 0);
+        tc_commit(&s.s_full);
+      };
+      auto d_prob = [&]() {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float2 xf = __half22float2(xh[e]), yf = __half22float2(yh[e]);
-          delta = fmaf(xf.x, yf.x, fmaf(xf.y, yf.y, delta));
+        for (int k8 = 0; k8 < 8; ++k8)
+          mma_f16_ss(tmem + kColP, v_k + kstep(k8), do_k + kstep(k8), idesc_nn, k8 != 0);
+        tc_commit(&s.dp_full);
+      };
+      // columns of the 16 query tokens of step k8 in an fp16 operand that two warpgroups wrote over
+      // their own halves of 128 fp32 columns
+      auto packed_col = [](int k8) { return (uint32_t)((k8 >> 2) * 64 + (k8 & 3) * 8); };
+      bool ok = wait(&s.k_full, 0, 63) && wait(&s.q_full[0], 0, 64);
+      if (ok) scores(0);
+      ok = ok && wait(&s.v_full, 0, 65) && wait(&s.do_full, 0, 66);
+      if (ok) d_prob();
+      for (int i = 0; i < n_q && ok; ++i) {
+        const bool more = i + 1 < n_q;
+        ok = wait(&s.p_full, i, 67);
+        if (!ok) break;
+#pragma unroll
+        for (int k8 = 0; k8 < 8; ++k8)
+          mma_f16_ts(tmem + kColDv, tmem + kColS + packed_col(k8), do_mn + k8 * (2048 >> 4), idesc_nt, (i | k8) != 0);
+        tc_commit(&s.do_empty);
+        if (more) {   // over the columns of P^T, which the products above, in order before these, have read
+          ok = wait(&s.q_full[(i + 1) & 1], (i + 1) >> 1, 68);
+          if (!ok) break;
+          scores(i + 1);
+        }
+        ok = wait(&s.ds_full, i, 69);
+        if (!ok) break;
+        const uint64_t q_mn = make_smem_desc(smem_u32(s.q[i & 1]), kBox, 1024);
+#pragma unroll
+        for (int k8 = 0; k8 < 8; ++k8)
+          mma_f16_ts(tmem + kColDk, tmem + kColP + packed_col(k8), q_mn + k8 * (2048 >> 4), idesc_nt, (i | k8) != 0);
+        tc_commit(&s.q_empty[i & 1]);
+#pragma unroll
+        for (int k8 = 0; k8 < 8; ++k8)   // over the columns of dS^T, which the products above have read
+          mma_f16_ss(tmem + kColP, ds_mn + k8 * (2048 >> 4), k_mn + k8 * (2048 >> 4), idesc_tt, k8 != 0);
+        tc_commit(&s.dq_full);
+        if (more) {
+          ok = wait(&s.do_full, i + 1, 70) && wait(&s.dq_free, i, 71);
+          if (ok) d_prob();
         }
       }
-      lse2 = a.lse[(size_t)h * a.n + q_idx] * 1.4426950408889634f;
+      if (ok) tc_commit(&s.done);
     }
-    const float sl = a.scale_log2;
-    const int d_idx = warp * 32 + lane;          // this thread's row of dV^T / dK^T
+  } else if (warp >= kDqWarp) {
+    // ---------------------------------------------------------------- dQ, and the rows' statistics
+    const int r = threadIdx.x - kDqWarp * 32;
+    uint8_t* stage = s.stage[warp - kDqWarp];
+    const float2* stats = a.stats + (size_t)h * a.n;
+    auto fetch = [&](int i) {   // a query past the segment gets weight exp2(-inf) = 0
+      const int token = kv0 + i * kBQ + r;
+      return i < n_q && token < tile.seg_end ? stats[token] : make_float2(INFINITY, 0.f);
+    };
+    auto put = [&](int i, float2 v) {
+      s.stats[i & 1][r] = v;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s.stats_full[i & 1]);
+    };
+    put(0, fetch(0));
+    put(1, fetch(1));
     bool ok = true;
-    for (int t = 0; t < n_kv && ok; ++t) {
-      const int kv0 = seg_begin + t * kBKVb;
-      ok = mbar_wait(&s.sdp_full, t & 1, abort_flag, a.status, 58);
+    for (int i = 0; i < n_q; ++i) {
+      const float2 ahead = fetch(i + 2);
+      ok = __all_sync(0xffffffffu, mbar_wait(&s.dq_full, i & 1, abort_flag, a.status, 72));
+      if (!ok) break;
+      tc_fence_after_sync();
+      put(i + 2, ahead);   // dq_full(i): nobody reads the statistics of tile i any more
+      const bool keep = kv0 + i * kBQ + r < tile.seg_end;   // the tile's other rows belong to other segments
+      const int row0 = kv0 + i * kBQ + (warp - kDqWarp) * 32;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t x[32], y[32];
+        tmem_ld_32x32(lane_base + kColP + half * 64, x);
+        tmem_ld_32x32(lane_base + kColP + half * 64 + 32, y);
+        tmem_ld_wait_on(x);
+        tmem_ld_wait_on(y);
+        if (half == 1) {
+          tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&s.dq_free);
+        }
+        if (lane == 0) tma_store_wait_read<0>();   // both boxes have been read
+        __syncwarp();
+        write_box_row(stage, lane, x, a.scale, keep);
+        write_box_row(stage + 4096, lane, y, a.scale, keep);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && row0 < tile.seg_end) {
+          tma_reduce_add_2d(&map_dq, stage, h * kD + half * 64, row0);
+          tma_reduce_add_2d(&map_dq, stage + 4096, h * kD + half * 64 + 32, row0);
+          tma_store_commit();
+        }
+      }
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // the sums have landed
+  } else {
+    // ---------------------------------------------------------------- P^T and dS^T: thread = key row
+    const int wg = warp >> 2;
+    ComputeTile t;
+    t.r = threadIdx.x & 127;
+    t.s_addr = lane_base + kColS + wg * 64;
+    t.dp_addr = lane_base + kColP + wg * 64;
+    t.ds_box = s.ds + wg * kBox;
+    const float sl = a.scale_log2;
+    bool ok = true;
+    for (int i = 0; i < n_q; ++i) {
+      t.stats = s.stats[i & 1] + wg * 64;
+      ok = mbar_wait(&s.stats_full[i & 1], (i >> 1) & 1, abort_flag, a.status, 73) &&
+           mbar_wait(&s.s_full, i & 1, abort_flag, a.status, 74);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       tc_fence_after_sync();
-      const int limit = valid ? q_idx - kv0 : -1;    // columns 0..limit are visible
-#pragma unroll 1
-      for (int c0 = 0; c0 < kBKVb; c0 += 32) {
-        uint32_t x[32], y[32], pp[16], ds[16];
-        tmem_ld_32x32(lane_base + c0, x);
-        tmem_ld_32x32(lane_base + 128 + c0, y);
-        tmem_ld_wait_on(x);
-        tmem_ld_wait_on(y);
-#pragma unroll
-        for (int c = 0; c < 32; c += 2) {
-          float p0 = 0.f, p1 = 0.f;
-          if (c0 + c <= limit) p0 = exp2f(fmaf(__uint_as_float(x[c]), sl, -lse2));
-          if (c0 + c + 1 <= limit) p1 = exp2f(fmaf(__uint_as_float(x[c + 1]), sl, -lse2));
-          const float g0 = p0 * (__uint_as_float(y[c]) - delta);
-          const float g1 = p1 * (__uint_as_float(y[c + 1]) - delta);
-          __half2 ph = __floats2half2_rn(p0, p1), gh = __floats2half2_rn(g0, g1);
-          pp[c >> 1] = *reinterpret_cast<uint32_t*>(&ph);
-          ds[c >> 1] = *reinterpret_cast<uint32_t*>(&gh);
-        }
-        write_tile_chunks(s.p, r, c0, pp);
-        write_tile_chunks(s.ds, r, c0, ds);
-      }
-      fence_proxy_async_smem();
+      float p[64];
+      if (i == 0) probabilities<true>(t, wg * 64, sl, p);
+      else probabilities<false>(t, wg * 64, sl, p);
       tc_fence_before_sync();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&s.pds_full);
-      ok = mbar_wait(&s.grads_full, t & 1, abort_flag, a.status, 59);
-      ok = __all_sync(0xffffffffu, ok);
+      if (lane == 0) mbar_arrive(&s.p_full);
+      ok = __all_sync(0xffffffffu, mbar_wait(&s.dp_full, i & 1, abort_flag, a.status, 75));
       if (!ok) break;
       tc_fence_after_sync();
-      // dV^T and dK^T leave through shared memory: thread d writes its values as column d of a
-      // [128 key rows x 128] fp32 tile (dV over the V and P tiles, dK over the dS and K tiles, all
-      // four dead now), and thread r adds key row r of both to global memory with two bulk
-      // reductions: the copy engine does the atomic adds.
-      float* stage_v = reinterpret_cast<float*>(s.v);
-      float* stage_k = reinterpret_cast<float*>(s.ds);
-#pragma unroll 1
-      for (int c0 = 0; c0 < kBKVb; c0 += 32) {
-        uint32_t x[32], y[32];
-        tmem_ld_32x32(lane_base + c0, x);
-        tmem_ld_32x32(lane_base + 128 + c0, y);
-        tmem_ld_wait_on(x);
-        tmem_ld_wait_on(y);
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          stage_v[(c0 + c) * kD + d_idx] = __uint_as_float(x[c]);
-          stage_k[(c0 + c) * kD + d_idx] = __uint_as_float(y[c]) * a.scale;
-        }
-      }
+      score_gradients(t, p);
       tc_fence_before_sync();
       fence_proxy_async_smem();
-      row_warps_sync();
-      if (lane == 0) mbar_arrive(&s.acc_free);        // the accumulators have been read
-      if (kv0 + r < q_end) {                          // key row r of this tile exists for this CTA
-        const size_t row = ((size_t)(kv0 + r) * a.hk + hk) * kD;
-        bulk_red_add_f32(a.dv + row, stage_v + r * kD, kD * sizeof(float));
-        bulk_red_add_f32(a.dk + row, stage_k + r * kD, kD * sizeof(float));
-      }
-      tma_store_commit();
-      tma_store_wait_read<0>();    // the staged rows have been read: the tiles can be reloaded
-      row_warps_sync();
-      if (r == 0) {
-        mbar_arrive(&s.k_empty);
-        mbar_arrive(&s.v_empty);
-      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&s.ds_full);
     }
-    asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // this thread's reductions have landed
-    if (ok) {   // dQ: complete once the last tile's products are (grads_full of the last step)
-      __half* dst = a.dq + ((size_t)q_idx * a.hq + h) * kD;
-#pragma unroll
-      for (int c0 = 0; c0 < kD; c0 += 32) {
-        uint32_t o[32];
-        tmem_ld_32x32(lane_base + 256 + c0, o);
-        tmem_ld_wait_on(o);
-        if (valid) {
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            uint32_t w[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              __half2 hh = __floats2half2_rn(__uint_as_float(o[8 * j + 2 * e]) * a.scale,
-                                             __uint_as_float(o[8 * j + 2 * e + 1]) * a.scale);
-              w[e] = *reinterpret_cast<uint32_t*>(&hh);
-            }
-            *reinterpret_cast<uint4*>(dst + c0 + 8 * j) = make_uint4(w[0], w[1], w[2], w[3]);
-          }
+    if (ok) ok = __all_sync(0xffffffffu, mbar_wait(&s.done, 0, abort_flag, a.status, 76));
+    if (ok) {   // the first warpgroup adds dV, the second dK, through the tiles nobody reads any more
+      tc_fence_after_sync();
+      uint8_t* stage = s.k + warp * 16384;
+      const uint32_t src = lane_base + (wg == 0 ? kColDv : kColDk);
+      const float f = wg == 0 ? 1.f : a.scale;
+      const bool keep = kv0 + t.r < tile.seg_end;
+      const int row0 = kv0 + (warp & 3) * 32;
+#pragma unroll 1
+      for (int c = 0; c < 4; ++c) {
+        uint32_t x[32];
+        tmem_ld_32x32(src + c * 32, x);
+        tmem_ld_wait_on(x);
+        write_box_row(stage + c * 4096, lane, x, f, keep);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0 && row0 < tile.seg_end) {
+          tma_reduce_add_2d(wg == 0 ? &map_dv : &map_dk, stage + c * 4096, hk * kD + c * 32, row0);
+          tma_store_commit();
         }
       }
+      if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
       tc_fence_before_sync();
     }
   }
   __syncthreads();
-  if (warp == 4) {
+  if (s.abort_flag) {   // copies that may still be in flight land before the shared memory is released
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);
+    __syncthreads();
+  }
+  if (warp == kBwdMmaWarp) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem, kTmemColsBwd);
+    tmem_dealloc(tmem, 512);
   }
 }
+}  // namespace
+}  // namespace soup
+
+namespace soup {
+namespace {
+
+// every segment adds at most one partial tile to the tiles of the packed row
+inline int64_t tile_slots(int64_t n_tokens, int64_t n_segments) { return (n_tokens + kBQ - 1) / kBQ + n_segments; }
+
+// Heads of a forward CTA. Two per CTA (both heads use every key and value tile) pay once an SM has
+// more than about eight (tile, key tile) steps to walk, estimated from the mean segment; below, twice
+// as many CTAs of half the work finish earlier (12 query heads, 2 key heads, one and two heads: 1280
+// tokens in 5 segments 10.6 and 13.2 us, 4607 in 16 22.8 and 24.2, 4604 in 8 27.4 and 27.0, 4607 in 4
+// 41.0 and 39.6, 9215 in 4 110.9 and 101.2). The two heads share one key/value head.
+inline int forward_heads_per_cta(int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk) {
+  if ((hq / hk) % 2) return 1;
+  const double tiles = (double)n_tokens / kBQ, walk = (tiles / (double)n_segments + 1.0) / 2.0;
+  return tiles * walk * (double)hq > 8.0 * sm_count() ? 2 : 1;
+}
+
 }  // namespace
 }  // namespace soup
 
@@ -703,8 +810,11 @@ extern "C" int soup_attn_fwd(const void* q, const void* k, const void* v, const 
     SOUP_FAIL(SOUP_ERR_ARG, "attn_fwd: pointers must be 16-byte aligned");
   // a runtime call first: it makes the device's context current on this thread (autograd runs
   // backward on threads of its own), which the driver's tensor-map encoder needs
-  const size_t smem = sizeof(Smem) + 1024;
-  if (cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  const int heads = forward_heads_per_cta(n_tokens, n_segments, hq, hk);
+  const size_t smem = (heads == 1 ? sizeof(FwdSmem<1>) : sizeof(FwdSmem<2>)) + 1024;
+  if ((heads == 1 ? cudaFuncSetAttribute(attn_fwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
+                  : cudaFuncSetAttribute(attn_fwd_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem)) != cudaSuccess)
     SOUP_FAIL(SOUP_ERR_LAUNCH, "attn_fwd: shared memory attribute");
   CUtensorMap mq, mk, mv;
   if (umma::encode_map_2d_16bit(&mq, q, (uint64_t)n_tokens, (uint64_t)(hq * kD), (uint64_t)q_pitch, kBQ, 64, false) ||
@@ -719,71 +829,73 @@ extern "C" int soup_attn_fwd(const void* q, const void* k, const void* v, const 
   a.segments = (int)n_segments;
   a.hq = (int)hq;
   a.group = (int)(hq / hk);
-  a.scale = scale;
-  a.scale_log2 = scale * 1.4426950408889634f;
+  a.scale_log2 = scale * kLog2e;
   a.status = rowpipe::status_word();
-  // every segment adds at most one partial tile to the tiles of the packed row
-  const unsigned slots = (unsigned)((n_tokens + kBQ - 1) / kBQ + n_segments);
-  dim3 grid(slots, (unsigned)hq);
-  attn_fwd_kernel<<<grid, kThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(mq, mk, mv, a);
+  const int64_t ctas = tile_slots(n_tokens, n_segments) * (hq / heads);
+  if (ctas > INT32_MAX) SOUP_FAIL(SOUP_ERR_ARG, "attn_fwd: too many tokens, segments or heads");
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (heads == 1) attn_fwd_kernel<1><<<(unsigned)ctas, kFwdThreads<1>, smem, st>>>(mq, mk, mv, a);
+  else attn_fwd_kernel<2><<<(unsigned)ctas, kFwdThreads<2>, smem, st>>>(mq, mk, mv, a);
   SOUP_CHECK_LAUNCH("attn_fwd");
   return SOUP_OK;
 }
 
 extern "C" int soup_attn_bwd(const void* q, const void* k, const void* v, const void* out,
-                             const void* d_out, const float* lse, const int32_t* cu_rows, void* dq,
-                             float* dk, float* dv, int64_t n_tokens, int64_t n_segments, int64_t hq,
-                             int64_t hk, int64_t head_dim, int64_t q_pitch, int64_t k_pitch,
-                             int64_t v_pitch, float scale, void* stream) {
+                                 const void* d_out, const float* lse, const int32_t* cu_rows, float* dq,
+                                 float* dk, float* dv, void* workspace, int64_t workspace_bytes,
+                                 int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk,
+                                 int64_t head_dim, int64_t q_pitch, int64_t k_pitch, int64_t v_pitch,
+                                 float scale, void* stream) {
   using namespace soup;
-  if (n_tokens == 0 || n_segments == 0) return SOUP_OK;
-  if (!q || !k || !v || !out || !d_out || !lse || !cu_rows || !dq || !dk || !dv)
+  if (n_tokens == 0) return SOUP_OK;
+  if (!q || !k || !v || !out || !d_out || !lse || !cu_rows || !dq || !dk || !dv || !workspace)
     SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: null pointer");
   if (head_dim != kD) SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: head_dim must be 128");
   if (n_tokens < 0 || n_segments < 0 || hq <= 0 || hk <= 0 || hq % hk)
     SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: bad sizes (query heads must be a multiple of key heads)");
-  if (n_tokens > (1 << 30) || n_segments > 65535 || hq > 65535)
+  const int64_t ctas = tile_slots(n_tokens, n_segments) * hq;
+  if (n_tokens > (1 << 30) || n_segments > 65535 || hq > 65535 || ctas > INT32_MAX)
     SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: too many tokens, segments or heads");
   if (q_pitch < hq * kD || k_pitch < hk * kD || v_pitch < hk * kD || (q_pitch | k_pitch | v_pitch) & 7)
     SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: row pitches must cover the heads and be multiples of 8 elements");
-  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out) || !aligned16(d_out) || !aligned16(dq))
+  if (!aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(out) || !aligned16(d_out) ||
+      !aligned16(dq) || !aligned16(dk) || !aligned16(dv) || !aligned16(workspace))
     SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: pointers must be 16-byte aligned");
+  if (workspace_bytes < n_tokens * hq * (int64_t)sizeof(float2))
+    SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: workspace too small (%lld < %lld)", (long long)workspace_bytes,
+              (long long)(n_tokens * hq * (int64_t)sizeof(float2)));
   // a runtime call first (see soup_attn_fwd): backward usually runs on an autograd thread
-  const size_t smem = sizeof(BwdSmem) + 1024;
-  if (cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+  if (cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)sizeof(KvSmem)) != cudaSuccess)
     SOUP_FAIL(SOUP_ERR_LAUNCH, "attn_bwd: shared memory attribute");
-  CUtensorMap mq, mdo, mk, mv;
-  const int e_q = umma::encode_map_2d_16bit(&mq, q, (uint64_t)n_tokens, (uint64_t)(hq * kD), (uint64_t)q_pitch, kBQ, 64, false);
-  const int e_do = umma::encode_map_2d_16bit(&mdo, d_out, (uint64_t)n_tokens, (uint64_t)(hq * kD), (uint64_t)(hq * kD), kBQ, 64, false);
-  const int e_k = umma::encode_map_2d_16bit(&mk, k, (uint64_t)n_tokens, (uint64_t)(hk * kD), (uint64_t)k_pitch, kBKVb, 64, false);
-  const int e_v = umma::encode_map_2d_16bit(&mv, v, (uint64_t)n_tokens, (uint64_t)(hk * kD), (uint64_t)v_pitch, kBKVb, 64, false);
-  if (e_q || e_do || e_k || e_v)
-    SOUP_FAIL(SOUP_ERR_LAUNCH, "attn_bwd: cuTensorMapEncodeTiled failed (q %d, d_out %d, k %d, v %d)", e_q, e_do, e_k, e_v);
+  CUtensorMap mq, mdo, mk, mv, mdq, mdk, mdv;
+  const uint64_t n = (uint64_t)n_tokens, wq = (uint64_t)(hq * kD), wk = (uint64_t)(hk * kD);
+  if (umma::encode_map_2d_16bit(&mq, q, n, wq, (uint64_t)q_pitch, kBQ, 64, false) ||
+      umma::encode_map_2d_16bit(&mdo, d_out, n, wq, wq, kBQ, 64, false) ||
+      umma::encode_map_2d_16bit(&mk, k, n, wk, (uint64_t)k_pitch, kBKV, 64, false) ||
+      umma::encode_map_2d_16bit(&mv, v, n, wk, (uint64_t)v_pitch, kBKV, 64, false) ||
+      umma::encode_map_2d_f32(&mdq, dq, n, wq, wq, 32, 32) || umma::encode_map_2d_f32(&mdk, dk, n, wk, wk, 32, 32) ||
+      umma::encode_map_2d_f32(&mdv, dv, n, wk, wk, 32, 32))
+    SOUP_FAIL(SOUP_ERR_LAUNCH, "attn_bwd: cuTensorMapEncodeTiled failed");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  const size_t kv_bytes = (size_t)n_tokens * hk * kD * sizeof(float);
-  const bool adjacent = reinterpret_cast<char*>(dk) + kv_bytes == reinterpret_cast<char*>(dv);
-  if (cudaMemsetAsync(dk, 0, adjacent ? 2 * kv_bytes : kv_bytes, st) != cudaSuccess ||
-      (!adjacent && cudaMemsetAsync(dv, 0, kv_bytes, st) != cudaSuccess))
-    SOUP_FAIL(SOUP_ERR_LAUNCH, "attn_bwd: clearing dk / dv failed");
-  AttnBwdArgs a;
+  const int64_t rows = n_tokens * hq;
+  attn_bwd_prep_kernel<<<(unsigned)((rows + kPrepThreads / 16 - 1) / (kPrepThreads / 16)), kPrepThreads, 0, st>>>(
+      reinterpret_cast<const __half*>(out), reinterpret_cast<const __half*>(d_out), lse,
+      reinterpret_cast<float2*>(workspace), reinterpret_cast<float4*>(dq), reinterpret_cast<float4*>(dk),
+      reinterpret_cast<float4*>(dv), rows, n_tokens * hk, (int)n_tokens, (int)hq);
+  SOUP_CHECK_LAUNCH("attn_bwd_prep");
+  if (n_segments == 0) return SOUP_OK;
+  AttnKvArgs a;
   a.cu = cu_rows;
-  a.out = reinterpret_cast<const __half*>(out);
-  a.d_out = reinterpret_cast<const __half*>(d_out);
-  a.lse = lse;
-  a.dq = reinterpret_cast<__half*>(dq);
-  a.dk = dk;
-  a.dv = dv;
+  a.stats = reinterpret_cast<const float2*>(workspace);
   a.n = (int)n_tokens;
   a.segments = (int)n_segments;
   a.hq = (int)hq;
-  a.hk = (int)hk;
   a.group = (int)(hq / hk);
   a.scale = scale;
-  a.scale_log2 = scale * 1.4426950408889634f;
+  a.scale_log2 = scale * kLog2e;
   a.status = rowpipe::status_word();
-  const unsigned slots = (unsigned)((n_tokens + kBQ - 1) / kBQ + n_segments);
-  dim3 grid(slots, (unsigned)hq);
-  attn_bwd_kernel<<<grid, kThreads, smem, st>>>(mq, mdo, mk, mv, a);
+  attn_bwd_kernel<<<(unsigned)ctas, kBwdThreads, sizeof(KvSmem), st>>>(mq, mdo, mk, mv, mdq, mdk, mdv, a);
   SOUP_CHECK_LAUNCH("attn_bwd");
   return SOUP_OK;
 }

@@ -122,6 +122,6 @@ extern "C" int soup_device_status(int* host_status, int clear, void* stream) {
   return SOUP_OK;
 }
 
-extern "C" int soup_version(void) { return 2; }
+extern "C" int soup_version(void) { return 3; }
 
 extern "C" const char* soup_last_error_string(void) { return soup::g_error; }

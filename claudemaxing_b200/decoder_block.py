@@ -43,7 +43,7 @@ import torch
 from . import _lib
 from . import attention as attention_mod
 from . import lora as lora_mod
-from .attention import attention_gradients, segment_attention
+from .attention import attention_gradients_f32, segment_attention
 from .rmsnorm import fp16_copy_of
 from .rope import rotate_into
 from .swiglu_recompute import _silu_mul_bwd, _silu_mul_fwd
@@ -328,9 +328,8 @@ class _QKVRope(torch.autograd.Function):
         plan, (n, d, nq, nk, hq, hk) = ctx.plan, ctx.sizes
         if ctx.attends:
             cos, sin, q_out, k_out, v_out, attended, lse, cu_rows = ctx.saved_tensors
-            dq, dk, dv = attention_gradients(q_out, k_out, v_out, attended, lse,
-                                             grads[0].reshape(n, hq, d), cu_rows, ctx.scale)
-            dk = dk.to(F16)   # the pipelined rotation wants q and k of one element size
+            dq, dk, dv, _ = attention_gradients_f32(q_out, k_out, v_out, attended, lse,
+                                                    grads[0].reshape(n, hq, d), cu_rows, ctx.scale)
         else:
             cos, sin = ctx.saved_tensors
             dq, dk, dv = grads

@@ -203,16 +203,17 @@ int soup_attn_fwd(const void* q, const void* k, const void* v, const int32_t* cu
                   void* stream);
 
 /* Backward of soup_attn_fwd: from q, k, v, the forward's out and lse, and d_out, the gradients
- *   dq [n_tokens, hq, 128] fp16 contiguous (every token inside a segment is written),
- *   dk, dv [n_tokens, hk, 128] fp32 contiguous: cleared here, then accumulated with atomic adds over
- *   the query heads of a group and the query tiles of a segment (their last bits can differ
- *   between runs).
- * out and d_out are [n_tokens, hq, 128] fp16 contiguous; the rest as in soup_attn_fwd. In the
- * reference this is the backward of torch SDPA (solution/attention.py:332-343). */
+ *   dq [n_tokens, hq, 128], dk and dv [n_tokens, hk, 128], fp32 contiguous: cleared here (tokens
+ *   outside every segment get zeros), then accumulated with atomic adds, dq over the key tiles of a
+ *   segment, dk and dv over the query heads of a group (their last bits can differ between runs).
+ * out and d_out are [n_tokens, hq, 128] fp16 contiguous; `workspace` holds 8 bytes per token and query
+ * head; the rest as in soup_attn_fwd. In the reference this is the backward of torch SDPA
+ * (solution/attention.py:332-343). (Before version 3 dq was fp16 and there was no workspace.) */
 int soup_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* d_out,
-                  const float* lse, const int32_t* cu_rows, void* dq, float* dk, float* dv,
-                  int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk, int64_t head_dim,
-                  int64_t q_pitch, int64_t k_pitch, int64_t v_pitch, float scale, void* stream);
+                  const float* lse, const int32_t* cu_rows, float* dq, float* dk, float* dv,
+                  void* workspace, int64_t workspace_bytes, int64_t n_tokens, int64_t n_segments,
+                  int64_t hq, int64_t hk, int64_t head_dim, int64_t q_pitch, int64_t k_pitch,
+                  int64_t v_pitch, float scale, void* stream);
 
 /* out = round_out(round_gate?(silu(gate)) * up). Replaces silu_mul_fwd_persistent at
  * solution/swiglu_recompute.py:98-100 and :176-178 (kernel :36-48). */

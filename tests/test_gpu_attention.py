@@ -55,6 +55,8 @@ def test_attention_kernels_on_the_reference_kernels_golden_vectors(tag):
     (6, 1, [1000, 3]),
     (4, 2, [40] * 100 + [3]),        # more than 64 segments: the plain tile order
     (2, 1, [2500]),                  # twenty key tiles: many turns of every barrier
+    (12, 2, [2500, 700, 1]),         # long enough for two heads per forward CTA
+    (3, 1, [129, 255]),              # an odd group: one head per CTA whatever the size
 ])
 def test_attention_kernels_against_fp32_with_the_fp16_sdpa_error_as_the_bar(hq, hk, lens):
     from oracle import attention as oat
@@ -81,6 +83,30 @@ def test_attention_kernels_against_fp32_with_the_fp16_sdpa_error_as_the_bar(hq, 
         err, allowed = rel_norm(got.float().cpu(), exact.float()), rel_norm(lib.float().cpu(), exact.float())
         assert err <= 3 * allowed + 1e-4, (name, err, allowed)
     assert dk.dtype == dv.dtype == torch.float32 and dq.dtype == torch.float16
+    assert (lse.double().cpu() - want_lse).abs().max() < 2e-3
+
+
+@pytest.mark.parametrize("hq,hk,lens", [(4, 2, [700, 130]), (12, 2, [2600, 520])])
+def test_attention_forward_when_the_row_maximum_keeps_growing(hq, hk, lens):
+    """Scores that grow along the keys (by far more than the 2^8 a stale maximum may lag), then fall:
+    every row's accumulator is rescaled, some rows of a warp earlier than others. One and two heads
+    per CTA. P is rounded to fp16 relative to a reference up to 2^8 below the maximum, which leaves
+    its relative rounding, 2^-11 an element, as it is: the bound of the plain cases."""
+    from oracle import attention as oat
+
+    torch.manual_seed(2)
+    n, d = sum(lens), 128
+    q, k, v = (torch.randn(n, h, d, device=DEV) for h in (hq, hk, hk))
+    ramp = torch.cat([torch.cat([torch.linspace(0.05, 8, L - L // 4), torch.linspace(8, 0.5, L // 4)]) for L in lens])
+    k = (k * ramp.to(DEV)[:, None, None]).half()
+    q, v = q.half(), v.half()
+    grad = torch.randn(n, hq, d, device=DEV).half()
+    cu = _cu(lens)
+    out, lse, dq, dk, dv = _run(q, k, v, cu, grad)
+    want_out, want_lse = oat.segment_attention(q.cpu(), k.cpu(), v.cpu(), cu)
+    want = (want_out,) + oat.segment_attention_backward(q.cpu(), k.cpu(), v.cpu(), cu, grad.cpu())
+    for name, got, exact in zip(("out", "dq", "dk", "dv"), (out, dq, dk, dv), want):
+        assert rel_norm(got.float().cpu(), exact.float()) < 2e-3, name
     assert (lse.double().cpu() - want_lse).abs().max() < 2e-3
 
 
