@@ -341,6 +341,118 @@ __device__ __forceinline__ void unpack_smem(const char* row, int vi, int dt, flo
 // A dtype that is a template constant (>= 0) is folded by the compiler; -1 takes the run-time code.
 template <int C> __device__ __forceinline__ int dt_sel(int rt) { return C >= 0 ? C : rt; }
 
+// ------------------------------------------------------------------------------------------
+// One CTA per row (four rows of up to 256 columns), eight columns per thread, everything a row needs
+// requested at once: bound by memory when many rows are in flight, by one row's latency when few are.
+// The ring kernels below spend the latter on ring set-up, a serial walk of the row by one or two warps
+// and, in backward, on the weight's copy in shared memory; with fp32 rows this form is faster at every
+// row count (1536 columns, 10 B and 16 B an element: forward 7.6 -> 5.6 us at 1280 rows, 44.6 -> 41.2 at
+// 16384; backward with the residual 14.8 -> 8.5 and 87.6 -> 71.1 us, the latter 5.7 TB/s; 64 rows 5.4 ->
+// 1.8 and 7.7 -> 2.3). A 16-bit row is half the bytes for the same threads, and the ring wins once more
+// rows are waiting than fit (5.0 -> 4.3 us at 1280 rows, 6.3 -> 5.6 at 2560, but 7.4 -> 9.6 at 4608):
+// `row_kernel_covers`.
+// ------------------------------------------------------------------------------------------
+constexpr int kRowMaxThreads = 512;   // rows of up to 4096 columns
+
+// Sum over a row's threads (every thread gets it), in a fixed order; one warp or the whole CTA.
+__device__ __forceinline__ float cta_sum(float v, float* s_red) {
+  v = warp_sum(v);
+  const int warps = (int)(blockDim.x >> 5);
+  if (warps == 1) return v;
+  if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  float t = 0.f;
+  for (int w = 0; w < warps; ++w) t += s_red[w];
+  return t;
+}
+
+template <int XDT, int WDT, int ODT>
+__global__ void __launch_bounds__(kRowMaxThreads)
+rmsnorm_fwd_row_kernel(const void* __restrict__ x, const void* __restrict__ w, void* __restrict__ out,
+                       float* __restrict__ rstd_out, void* __restrict__ low, const int32_t* __restrict__ slot,
+                       void* __restrict__ small, int64_t n_small, int64_t n_rows, int n_cols, float eps,
+                       int xdt_rt, int wdt_rt, int odt_rt) {
+  __shared__ float s_red[kRowMaxThreads / 32];
+  const int xdt = dt_sel<XDT>(xdt_rt), wdt = dt_sel<WDT>(wdt_rt), odt = dt_sel<ODT>(odt_rt);
+  const int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y, at = row * n_cols + threadIdx.x * 8;
+  if (row >= n_rows) return;   // only where a warp is a row: nobody waits for it
+  const int col = threadIdx.x * 8;
+  const bool mine = col < n_cols;
+  float xv[8], wv[8];
+  int sl[8];
+  float ss = 0.f;
+  if (mine) {
+    load8(x, at, xdt, xv);
+    load8(w, col, wdt, wv);
+    if (low) load_slots<8>(slot, col, sl);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) ss += xv[k] * xv[k];
+  }
+  ss = cta_sum(ss, s_red);
+  const float rstd = 1.0f / sqrtf(ss * (1.0f / (float)n_cols) + eps);
+  if (threadIdx.x == 0) rstd_out[row] = rstd;
+  if (!mine) return;
+  float o[8], nrm[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    nrm[k] = round_through(xv[k] * rstd, xdt);
+    o[k] = nrm[k] * wv[k];
+  }
+  store8(out, at, odt, o);
+  if (low) {
+    store8(low, at, SOUP_F16, o);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      if (sl[k] >= 0) store1(small, row * n_small + sl[k], SOUP_F16, nrm[k]);
+  }
+}
+
+// The 4-bit model's backward: fp32 dy, the fp16 copy of the forward's output as the saved tensor, fp32
+// weight and dx, optionally the residual gradient added and an fp16 copy of the sum written.
+__global__ void __launch_bounds__(kRowMaxThreads)
+rmsnorm_bwd_saved_row_kernel(const float* __restrict__ dy, const __half* __restrict__ saved,
+                             const float* __restrict__ w, const float* __restrict__ rstd_in,
+                             const float* __restrict__ add, float* __restrict__ dx, __half* __restrict__ dx16,
+                             const int32_t* __restrict__ slot, const __half* __restrict__ small, int64_t n_small,
+                             int64_t n_rows, int n_cols) {
+  __shared__ float s_red[kRowMaxThreads / 32];
+  const int64_t row = (int64_t)blockIdx.x * blockDim.y + threadIdx.y, at = row * n_cols + threadIdx.x * 8;
+  if (row >= n_rows) return;   // only where a warp is a row: nobody waits for it
+  const int col = threadIdx.x * 8;
+  const bool mine = col < n_cols;
+  const float rstd = rstd_in[row];
+  float yv[8], nrm[8], extra[8];
+  float dot = 0.f;
+  if (mine) {
+    float xv[8], wv[8];
+    int sl[8];
+    load8(dy, at, SOUP_F32, yv);
+    load8(saved, at, SOUP_F16, xv);
+    if (add) load8(add, at, SOUP_F32, extra);
+    load8(w, col, SOUP_F32, wv);
+    load_slots<8>(slot, col, sl);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      // the normalised value: saved / w, except in the side-buffer columns (|w| tiny)
+      nrm[k] = xv[k] * (1.0f / wv[k]);
+      if (sl[k] >= 0) nrm[k] = __half2float(small[row * n_small + sl[k]]);
+      yv[k] *= wv[k];
+      dot += yv[k] * nrm[k];
+    }
+  }
+  const float mean_dot = cta_sum(dot, s_red) * (1.0f / (float)n_cols);
+  if (!mine) return;
+  float o[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) o[k] = (yv[k] - nrm[k] * mean_dot) * rstd;
+  if (add) {   // the gradient that reaches the same tensor along the residual connection
+#pragma unroll
+    for (int k = 0; k < 8; ++k) o[k] += extra[k];
+  }
+  store8(dx, at, SOUP_F32, o);
+  if (dx16) store8(dx16, at, SOUP_F16, o);   // and its fp16 copy, for the projection backward that receives it next
+}
+
 // XDT / WDT / ODT: compile-time dtype codes of the hot combinations, or -1 for "read the argument".
 template <int XB, int XDT, int WDT, int ODT>
 __global__ void __launch_bounds__(rowpipe::kMaxWarps * 32, 2)
@@ -575,155 +687,6 @@ rmsnorm_bwd_pipe_kernel(const void* __restrict__ dy, const void* __restrict__ xi
   }
 }
 
-// The 4-bit model's backward: fp32 dy, the fp16 copy of the forward's output as the saved tensor,
-// fp32 weight and dx. Only dy travels through the warp's ring; the saved row, half as many bytes,
-// comes through plain 8-byte loads into registers one row ahead (as RoPE's cos/sin rows do). That
-// halves the bulk copies per row (the copy engine has a cost per copy) and leaves the ring two
-// stages where a slot of dy + saved row had room for one. NVX: 4-element vectors per lane.
-template <int NVX>
-__global__ void __launch_bounds__(rowpipe::kMaxWarps * 32, 2)
-rmsnorm_bwd_saved_kernel(const float* __restrict__ dy, const __half* __restrict__ saved,
-                         const float* __restrict__ w, const float* __restrict__ rstd_in,
-                         const float* __restrict__ add, float* __restrict__ dx,
-                         __half* __restrict__ dx16, const int32_t* __restrict__ slot,
-                         const __half* __restrict__ small, int64_t n_small, int64_t n_rows,
-                         int n_cols, int stages, int team, int w_offset, int* status) {
-  constexpr int EPV = 4;
-  extern __shared__ __align__(128) char smem[];
-  __shared__ int s_abort;
-  __shared__ float s_part[2 * rowpipe::kMaxWarps];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  const int member = team == 2 ? (warp & 1) : 0;
-  const int n_vec = n_cols / EPV / team, v0 = member * n_vec;
-  const uint32_t y_bytes = (uint32_t)n_cols * 4 / team;
-  const int64_t y_pitch = (int64_t)n_cols * 4;
-  if (threadIdx.x == 0) s_abort = 0;
-  rowpipe::Ring ring;
-  ring.init(smem, y_bytes, stages, warp, lane);
-  __syncthreads();
-  const int64_t row0 = (int64_t)blockIdx.x * (warps / team) + warp / team;
-  const int64_t stride = (int64_t)gridDim.x * (warps / team);
-  const char* yb = reinterpret_cast<const char*>(dy) + (size_t)member * y_bytes;
-  const __half* xb = saved + (size_t)v0 * EPV;
-  int64_t next = row0;
-  if (lane == 0) {
-    for (int s = 0; s < stages && next < n_rows; ++s, next += stride) {
-      umma::mbar_expect_tx(&ring.bars[s], y_bytes);
-      rowpipe::bulk_load(ring.slot_ptr(s), yb + next * y_pitch, y_bytes, &ring.bars[s]);
-    }
-  }
-  next = __shfl_sync(0xffffffffu, next, 0);
-  // The weight and its reciprocal, needed by every row, sit in shared memory behind the ring
-  // (registers are taken by the two saved rows in flight and the normalised values).
-  float* s_w = reinterpret_cast<float*>(smem + w_offset);
-  float* s_winv = s_w + n_cols;
-  for (int c = threadIdx.x; c < n_cols; c += blockDim.x) {
-    const float wc = w[c];
-    s_w[c] = wc;
-    s_winv[c] = 1.0f / wc;
-  }
-  __syncthreads();
-  uint32_t slot_mask = 0;
-#pragma unroll
-  for (int v = 0; v < NVX; ++v) {
-    const int vi = lane + 32 * v;
-    if (vi < n_vec) {
-      int sl[EPV];
-      load_slots<EPV>(slot, (v0 + vi) * EPV, sl);
-#pragma unroll
-      for (int k = 0; k < EPV; ++k)
-        if (sl[k] >= 0) slot_mask |= 1u << v;
-    }
-  }
-  Raw<8> xcur[NVX], xnxt[NVX];
-  auto fetch_saved = [&](int64_t row, Raw<8> (&dst)[NVX]) {
-#pragma unroll
-    for (int v = 0; v < NVX; ++v) {
-      const int vi = lane + 32 * v;
-      if (vi < n_vec) dst[v] = ld_raw<8>(xb, (row * n_cols + (int64_t)vi * EPV) * 2);
-    }
-  };
-  if (row0 < n_rows) fetch_saved(row0, xcur);
-  const float inv_cols = 1.0f / (float)n_cols;
-  int iter = 0;
-  for (int64_t row = row0; row < n_rows; row += stride, ++iter) {
-    if (row + stride < n_rows) fetch_saved(row + stride, xnxt);
-    if (!ring.wait(&s_abort, status, 12)) {
-      ring.drain((int)((next - row) / stride));
-      if (team == 2) asm volatile("bar.arrive %0, 64;" ::"r"((warp >> 1) + 1) : "memory");
-      return;
-    }
-    const char* ysrc = ring.slot_ptr(ring.slot);
-    const float rstd = rstd_in[row];
-    // the normalised value: saved / w, except in the side-buffer columns (|w| tiny)
-    float nrm[NVX][EPV];
-    float dot = 0.f;
-#pragma unroll
-    for (int v = 0; v < NVX; ++v) {
-      const int vi = lane + 32 * v;
-      if (vi < n_vec) {
-        float yv[EPV], xv[EPV];
-        unpack_smem<EPV, 4>(ysrc, vi, SOUP_F32, yv);
-        unpack<EPV, 2>(xcur[v], SOUP_F16, xv);
-        const float4 wq = *reinterpret_cast<const float4*>(s_w + (v0 + vi) * EPV);
-        const float4 iq = *reinterpret_cast<const float4*>(s_winv + (v0 + vi) * EPV);
-        const float wv[EPV] = {wq.x, wq.y, wq.z, wq.w}, winv[EPV] = {iq.x, iq.y, iq.z, iq.w};
-        int sl[EPV];
-#pragma unroll
-        for (int k = 0; k < EPV; ++k) sl[k] = -1;
-        if (slot_mask >> v & 1u) load_slots<EPV>(slot, (v0 + vi) * EPV, sl);
-#pragma unroll
-        for (int k = 0; k < EPV; ++k) {
-          nrm[v][k] = sl[k] >= 0 ? __half2float(small[row * n_small + sl[k]]) : xv[k] * winv[k];
-          dot += yv[k] * wv[k] * nrm[v][k];
-        }
-      }
-    }
-    dot = warp_sum(dot);
-    if (team == 2) dot = rowpipe::team_sum2(dot, s_part, warp, lane, iter);
-    const float mean_dot = dot * inv_cols;
-#pragma unroll
-    for (int v = 0; v < NVX; ++v) {
-      const int vi = lane + 32 * v;
-      if (vi < n_vec) {
-        float yv[EPV];
-        unpack_smem<EPV, 4>(ysrc, vi, SOUP_F32, yv);
-        const float4 wq = *reinterpret_cast<const float4*>(s_w + (v0 + vi) * EPV);
-        float4 o;
-        o.x = (yv[0] * wq.x - nrm[v][0] * mean_dot) * rstd;
-        o.y = (yv[1] * wq.y - nrm[v][1] * mean_dot) * rstd;
-        o.z = (yv[2] * wq.z - nrm[v][2] * mean_dot) * rstd;
-        o.w = (yv[3] * wq.w - nrm[v][3] * mean_dot) * rstd;
-        const int64_t at = row * n_cols + (int64_t)(v0 + vi) * EPV;
-        if (add) {   // the gradient that reaches the same tensor along the residual connection
-          const float4 r = *reinterpret_cast<const float4*>(add + at);
-          o.x += r.x; o.y += r.y; o.z += r.z; o.w += r.w;
-        }
-        *reinterpret_cast<float4*>(dx + at) = o;
-        if (dx16) {  // and its fp16 copy, for the projection backward that receives it next
-          __half2 lo = __floats2half2_rn(o.x, o.y), hi = __floats2half2_rn(o.z, o.w);
-          uint2 packed;
-          packed.x = *reinterpret_cast<uint32_t*>(&lo);
-          packed.y = *reinterpret_cast<uint32_t*>(&hi);
-          *reinterpret_cast<uint2*>(dx16 + at) = packed;
-        }
-      }
-    }
-    __syncwarp();
-    if (next < n_rows) {
-      if (lane == 0) {
-        umma::fence_proxy_async_smem();
-        umma::mbar_expect_tx(&ring.bars[ring.slot], y_bytes);
-        rowpipe::bulk_load(ring.slot_ptr(ring.slot), yb + next * y_pitch, y_bytes, &ring.bars[ring.slot]);
-      }
-      next += stride;
-    }
-    ring.advance();
-#pragma unroll
-    for (int v = 0; v < NVX; ++v) xcur[v] = xnxt[v];
-  }
-}
-
 // YB / XB: bytes per element of dy and of the saved tensor (x, or the fp16 copy of the output).
 template <int NV, int YB, int XB, bool DW>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
@@ -873,6 +836,19 @@ inline int64_t bwd_ctas(int64_t n_rows) {
   return n_rows < cap ? (n_rows < 1 ? 1 : n_rows) : cap;
 }
 
+// Launch shape of the row kernels: a row's threads, and rows per CTA.
+inline dim3 row_block(int64_t n_cols) {
+  const unsigned threads = (unsigned)((n_cols / 8 + 31) / 32 * 32);
+  return dim3(threads, threads == 32 ? 4 : 1);
+}
+inline unsigned row_grid(int64_t n_rows, dim3 block) { return (unsigned)((n_rows + block.y - 1) / block.y); }
+
+// fp32 rows always, 16-bit rows while at most two waves of their threads wait (see the kernels).
+inline bool row_kernel_covers(int64_t n_rows, int64_t n_cols, int dtype) {
+  if (n_cols > kRowMaxThreads * 8) return false;
+  return dtype == SOUP_F32 || n_rows * row_block(n_cols).x <= 2ll * sm_count() * 2048;
+}
+
 }  // namespace
 }  // namespace soup
 
@@ -901,6 +877,17 @@ extern "C" int soup_rmsnorm_fwd(const void* x, const void* w, void* out, float* 
     rmsnorm_fwd_scalar_kernel<<<(unsigned)n_rows, 256, 0, s>>>(x, w, out, rstd, low, slot, small,
                                                                n_small, (int)n_cols, eps, x_dtype,
                                                                w_dtype, out_dtype);
+  } else if (row_kernel_covers(n_rows, n_cols, x_dtype)) {
+    const dim3 block = row_block(n_cols);
+#define SOUP_RMS_FWD_R(X_, W_, O_)                                                               \
+  rmsnorm_fwd_row_kernel<X_, W_, O_><<<row_grid(n_rows, block), block, 0, s>>>(                  \
+      x, w, out, rstd, low, slot, small, n_small, n_rows, (int)n_cols, eps, x_dtype, w_dtype, out_dtype)
+    const bool same = x_dtype == w_dtype && x_dtype == out_dtype;
+    if (same && x_dtype == SOUP_F32) SOUP_RMS_FWD_R(SOUP_F32, SOUP_F32, SOUP_F32);
+    else if (same && x_dtype == SOUP_F16) SOUP_RMS_FWD_R(SOUP_F16, SOUP_F16, SOUP_F16);
+    else if (same && x_dtype == SOUP_BF16) SOUP_RMS_FWD_R(SOUP_BF16, SOUP_BF16, SOUP_BF16);
+    else SOUP_RMS_FWD_R(-1, -1, -1);
+#undef SOUP_RMS_FWD_R
   } else if (plan.stages && status) {
 #define SOUP_RMS_FWD_P(XB_, X_, W_, O_)                                                          \
   do {                                                                                            \
@@ -1042,34 +1029,15 @@ int rmsnorm_bwd_any(const void* dy, const void* xin, const void* w, const float*
     const bool same = dy_dtype == xin_dtype && dy_dtype == w_dtype && dy_dtype == dx_dtype;
     const bool four_bit = saved_output && dy_dtype == SOUP_F32 && xin_dtype == SOUP_F16 &&
                           w_dtype == SOUP_F32 && dx_dtype == SOUP_F32;
-    // the 4-bit model's path with the saved row through registers: the ring carries dy only
-    const rowpipe::Plan plan_y = four_bit ? rowpipe::make_plan((size_t)n_cols * 4, 0, (n_cols * 2) % 32 == 0, n_rows)
-                                          : rowpipe::Plan{8, 0, 1, 1, 0, 0};
-    const int per_lane = plan_y.stages ? (int)((n_cols / 4 / plan_y.team + 31) / 32) : 0;
-    // weight and reciprocal behind the ring; two CTAs of this size must still fit an SM
-    const size_t w_off = (plan_y.smem + 15) / 16 * 16;
-    const size_t smem_y = w_off + 2 * (size_t)n_cols * sizeof(float);
-    const bool saved_kernel = four_bit && plan_y.stages >= 1 && per_lane >= 1 && per_lane <= 8 &&
-                              smem_y <= 112 * 1024;
-    if ((add || dx16) && !saved_kernel)
+    const bool rows = four_bit && row_kernel_covers(n_rows, n_cols, SOUP_F32) && (!dx16 || aligned16(dx16));
+    if ((add || dx16) && !(rows && n_cols <= 2048))
       SOUP_FAIL(SOUP_ERR_ARG, "rmsnorm_bwd_residual: this shape does not take the residual form");
-    if (saved_kernel) {
-      grid = plan_y.grid;
-#define SOUP_RMS_BWD_S(NVX_)                                                                     \
-  do {                                                                                            \
-    auto kernel = rmsnorm_bwd_saved_kernel<NVX_>;                                                 \
-    cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_y);       \
-    kernel<<<plan_y.grid, plan_y.warps * 32, smem_y, s>>>(                                        \
-        reinterpret_cast<const float*>(dy), reinterpret_cast<const __half*>(xin),                 \
-        reinterpret_cast<const float*>(w), rstd, add, reinterpret_cast<float*>(dx), dx16, slot,   \
-        reinterpret_cast<const __half*>(small), n_small, n_rows, (int)n_cols, plan_y.stages,      \
-        plan_y.team, (int)w_off, status);                                                         \
-  } while (0)
-      if (per_lane <= 2) SOUP_RMS_BWD_S(2);
-      else if (per_lane <= 4) SOUP_RMS_BWD_S(4);
-      else if (per_lane <= 6) SOUP_RMS_BWD_S(6);
-      else SOUP_RMS_BWD_S(8);
-#undef SOUP_RMS_BWD_S
+    if (rows) {
+      const dim3 block = row_block(n_cols);
+      rmsnorm_bwd_saved_row_kernel<<<row_grid(n_rows, block), block, 0, s>>>(
+          reinterpret_cast<const float*>(dy), reinterpret_cast<const __half*>(xin),
+          reinterpret_cast<const float*>(w), rstd, add, reinterpret_cast<float*>(dx), dx16, slot,
+          reinterpret_cast<const __half*>(small), n_small, n_rows, (int)n_cols);
     } else if (four_bit)
       SOUP_RMS_BWD_P(4, 2, SOUP_F32, SOUP_F16, SOUP_F32, SOUP_F32, 1);
     else if (!saved_output && same && dy_dtype == SOUP_F16)
