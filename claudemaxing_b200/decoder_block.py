@@ -276,6 +276,13 @@ def _norm_and_residual(norm, hidden):
     return norm(hidden), hidden
 
 
+def _plain_tables(cos, sin, n):
+    """Whether the rotary tables are what soup_qkv_rope_* take: fp32, one row per token, 16-byte aligned
+    (both are contiguous already)."""
+    return (cos.dtype == sin.dtype == F32 and cos.shape[1] == sin.shape[1] == n
+            and (cos.data_ptr() | sin.data_ptr()) % 16 == 0)
+
+
 class _QKVRope(torch.autograd.Function):
     """(x16 @ [Wq; Wk; Wv]^T + bias) split into q (+ adapter), k, v (+ adapter); q and k rotated;
     all three returned as fp16 [tokens, heads, head_dim]. With `cu_rows` (segment offsets of the
@@ -300,14 +307,22 @@ class _QKVRope(torch.autograd.Function):
         def heads_first(t, h):   # [n, h*d] (any row stride) seen as [1, h, n, d]
             return t.unflatten(-1, (h, d)).unsqueeze(0).transpose(1, 2)
 
-        rotate_into(heads_first(qkv[:, :nq], hq),
-                    None if lora_q is None else heads_first(lora_q.reshape(n, nq), hq),
-                    heads_first(qkv[:, nq:nq + nk], hk), cos, sin,
-                    q_out.unsqueeze(0).transpose(1, 2), k_out.unsqueeze(0).transpose(1, 2))
-        v_rows = qkv[:, nq + nk:]
-        v_out = v_rows.contiguous() if lora_v is None else v_rows + lora_v.reshape(n, nk)
+        v_out = torch.empty(n, nk, dtype=F16, device=x16.device)
+        shapes = tuple(None if t is None else t.shape for t in (lora_q, lora_v))
+        lora_q, lora_v = (None if t is None else t.reshape(n, -1) for t in (lora_q, lora_v))
+        if _plain_tables(cos, sin, n) and qkv.is_contiguous() and all(
+                t is None or (t.dtype == F16 and t.is_contiguous() and t.data_ptr() % 16 == 0)
+                for t in (lora_q, lora_v)):
+            _lib.call("soup_qkv_rope_fwd", _lib.ptr(qkv), qkv.stride(0), _lib.ptr(lora_q), _lib.ptr(lora_v),
+                      _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(q_out), _lib.ptr(k_out), _lib.ptr(v_out), n, hq, hk,
+                      d, _lib.stream_of(qkv))
+        else:
+            rotate_into(heads_first(qkv[:, :nq], hq), None if lora_q is None else heads_first(lora_q, hq),
+                        heads_first(qkv[:, nq:nq + nk], hk), cos, sin,
+                        q_out.unsqueeze(0).transpose(1, 2), k_out.unsqueeze(0).transpose(1, 2))
+            v_out.copy_(qkv[:, nq + nk:] if lora_v is None else qkv[:, nq + nk:] + lora_v)
         ctx.plan, ctx.sizes, ctx.x_shape = plan, (n, d, nq, nk, hq, hk), x.shape
-        ctx.lora_shapes = (None if lora_q is None else lora_q.shape, None if lora_v is None else lora_v.shape)
+        ctx.lora_shapes = shapes
         ctx.attends = cu_rows is not None
         v_out = v_out.view(n, hk, d)
         if not ctx.attends:
@@ -333,15 +348,19 @@ class _QKVRope(torch.autograd.Function):
         else:
             cos, sin = ctx.saved_tensors
             dq, dk, dv = grads
-        dq, dk = (g if g.stride(-1) == 1 else g.contiguous() for g in (dq, dk))
         dqkv = torch.empty(n, nq + 2 * nk, dtype=F16, device=dq.device)
+        if ctx.attends and _plain_tables(cos, sin, n):
+            _lib.call("soup_qkv_rope_bwd", _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(cos), _lib.ptr(sin),
+                      _lib.ptr(dqkv), dqkv.stride(0), n, hq, hk, d, _lib.stream_of(dq))
+        else:
+            dq, dk = (g if g.stride(-1) == 1 else g.contiguous() for g in (dq, dk))
 
-        def heads_first(t, h):
-            return t.unflatten(-1, (h, d)).unsqueeze(0).transpose(1, 2)
+            def heads_first(t, h):
+                return t.unflatten(-1, (h, d)).unsqueeze(0).transpose(1, 2)
 
-        rotate_into(dq.unsqueeze(0).transpose(1, 2), None, dk.unsqueeze(0).transpose(1, 2), cos, sin,
-                    heads_first(dqkv[:, :nq], hq), heads_first(dqkv[:, nq:nq + nk], hk), backward=True)
-        dqkv[:, nq + nk:].copy_(dv.reshape(n, nk))
+            rotate_into(dq.unsqueeze(0).transpose(1, 2), None, dk.unsqueeze(0).transpose(1, 2), cos, sin,
+                        heads_first(dqkv[:, :nq], hq), heads_first(dqkv[:, nq:nq + nk], hk), backward=True)
+            dqkv[:, nq + nk:].copy_(dv.reshape(n, nk))
         dx = None
         if ctx.needs_input_grad[0]:
             bases = [_base(m) for m in (plan.q, plan.k, plan.v)]

@@ -188,6 +188,18 @@ int soup_rope_sum(const void* q, const void* q_add, const void* k, const void* c
                   int q_dtype, int q_add_dtype, int k_dtype, int cs_dtype, int q_out_dtype,
                   int k_out_dtype, int backward, void* stream);
 
+/* The rows [q | k | v] of a q/k/v projection (fp16, row pitch qkv_pitch) as rotated q (+ add_q), rotated
+ * k and v (+ add_v): fp16 [n, h, d] contiguous, sums and rotation in fp32, one rounding. add_q [n, hq*d]
+ * and add_v [n, hk*d] fp16 contiguous or NULL; cos, sin fp32 [n, d]. One launch for what the reference
+ * reaches with its adapter sums, its rotation (solution/rope.py:17-43) and the attention's casts. */
+int soup_qkv_rope_fwd(const void* qkv, int64_t qkv_pitch, const void* add_q, const void* add_v,
+                      const float* cos, const float* sin, void* q, void* k, void* v, int64_t n, int64_t hq,
+                      int64_t hk, int64_t d, void* stream);
+/* Its transpose: fp32 dq, dk (rotated back) and dv ([n, h, d] contiguous) as rows of dqkv, fp16. */
+int soup_qkv_rope_bwd(const float* dq, const float* dk, const float* dv, const float* cos, const float* sin,
+                      void* dqkv, int64_t dqkv_pitch, int64_t n, int64_t hq, int64_t hk, int64_t d,
+                      void* stream);
+
 /* Causal attention inside the segments of one packed row, forward: for every token i of segment s,
  * out[i, h] = softmax_j(scale * q[i, h] . k[j, h / (hq/hk)]) v[j, h / (hq/hk)] over the tokens j <= i
  * of the same segment. Stands where the reference calls torch SDPA on the [1, 1, N, N] mask of its

@@ -284,6 +284,81 @@ def test_rope_of_a_sum_into_strided_outputs_is_the_chain_it_replaces(dims, with_
     assert (buf[:, (h + kv) * d:] == 7.0).all()    # the v block is not this kernel's to write
 
 
+@pytest.mark.parametrize("dims", [(1280, 12, 2, 128), (37, 4, 4, 64), (5, 3, 1, 16), (1, 1, 1, 256)])
+@pytest.mark.parametrize("with_terms", [True, False])
+def test_qkv_split_and_rotation_is_the_rotation_and_the_sums_it_replaces(dims, with_terms):
+    """`soup_qkv_rope_fwd` / `_bwd` against `rotate_into` and torch's sum and copy, bit for bit (the
+    same fp32 operations and one rounding each), with a row pitch wider than the three blocks."""
+    from claudemaxing_b200 import _lib
+    from claudemaxing_b200.rope import rotate_into
+
+    t, h, kv, d = dims
+    gen = torch.Generator().manual_seed(4)
+    cols, pitch = (h + 2 * kv) * d, (h + 2 * kv) * d + 8
+    qkv = torch.randn(t, pitch, generator=gen).half().to(DEV)
+    add_q = torch.randn(t, h * d, generator=gen).half().to(DEV) if with_terms else None
+    add_v = torch.randn(t, kv * d, generator=gen).half().to(DEV) if with_terms else None
+    emb = torch.randn(1, t, d, generator=gen) * 3
+    cos, sin = emb.cos().to(DEV), emb.sin().to(DEV)
+
+    def heads_first(x, heads):
+        return x.unflatten(-1, (heads, d)).unsqueeze(0).transpose(1, 2)
+
+    q, k, v = (torch.empty(t, heads, d, dtype=F16, device=DEV) for heads in (h, kv, kv))
+    _lib.call("soup_qkv_rope_fwd", _lib.ptr(qkv), pitch, _lib.ptr(add_q), _lib.ptr(add_v), _lib.ptr(cos),
+              _lib.ptr(sin), _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), t, h, kv, d, _lib.stream_of(q))
+    wq, wk = torch.empty_like(q), torch.empty_like(k)
+    rotate_into(heads_first(qkv[:, :h * d], h), None if add_q is None else heads_first(add_q, h),
+                heads_first(qkv[:, h * d:(h + kv) * d], kv), cos, sin,
+                wq.unsqueeze(0).transpose(1, 2), wk.unsqueeze(0).transpose(1, 2))
+    wv = qkv[:, (h + kv) * d:cols]
+    assert torch.equal(q, wq) and torch.equal(k, wk)
+    assert torch.equal(v.view(t, -1), wv if add_v is None else wv + add_v)
+    dq, dk, dv = (torch.randn(t, heads, d, generator=gen).to(DEV) for heads in (h, kv, kv))
+    got, want = torch.full((2, t, pitch), 7.0, dtype=F16, device=DEV)
+    _lib.call("soup_qkv_rope_bwd", _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(cos), _lib.ptr(sin),
+              _lib.ptr(got), pitch, t, h, kv, d, _lib.stream_of(dq))
+    rotate_into(dq.unsqueeze(0).transpose(1, 2), None, dk.unsqueeze(0).transpose(1, 2), cos, sin,
+                heads_first(want[:, :h * d], h), heads_first(want[:, h * d:(h + kv) * d], kv), backward=True)
+    want[:, (h + kv) * d:cols] = dv.reshape(t, -1)
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("cols", [8, 248, 256, 264, 4096, 4104])
+@pytest.mark.parametrize("rows", [1, 5, 4000])
+def test_rmsnorm_row_kernels_at_the_edges_of_their_shapes(rows, cols):
+    """One CTA per row, four rows of one warp, and the ring kernels beside them (more than 4096 columns;
+    many 16-bit rows): forward in fp32 and fp16 and the saved-output backward against float64. Bounds:
+    fp32 sums of up to 4104 terms (1e-5); one rounding to fp16 after another (2^-10)."""
+    import importlib
+
+    from claudemaxing_b200 import _lib
+
+    rms = importlib.import_module("claudemaxing_b200.rmsnorm")
+    gen = torch.Generator().manual_seed(cols + rows)
+    x = torch.randn(rows, cols, generator=gen).to(DEV)
+    w = (torch.rand(cols, generator=gen) + 0.5).to(DEV)
+    w[cols // 2] = 1e-5
+    dy = torch.randn(rows, cols, generator=gen).to(DEV)
+
+    def exact(t, weight):
+        t = t.double()
+        return t * torch.rsqrt(t.pow(2).mean(-1, keepdim=True) + 1e-6) * weight.double()
+
+    out, rstd, low, slots, small = rms._forward_launch(x, w, 1e-6, F32, True)
+    assert_close_rel_max(out, exact(x, w).float(), 1e-5)
+    out16 = rms._forward_launch(x.half(), w.half(), 1e-6, F16, False)[0]
+    assert_close_rel_max(out16.float(), exact(x.half(), w.half()).float(), 2 ** -10)
+    dx = torch.empty_like(x)
+    _lib.call("soup_rmsnorm_bwd", _lib.ptr(dy), _lib.ptr(low), _lib.ptr(w), _lib.ptr(rstd), _lib.ptr(dx), None,
+              None, _lib.ptr(slots), _lib.ptr(small), small.shape[-1], rows, cols, _lib.F32, _lib.F16, _lib.F32,
+              _lib.F32, 1, _lib.stream_of(dy))
+    leaf = x.double().requires_grad_()
+    exact(leaf, w).backward(dy.double())
+    # the saved normalised values carry fp16's rounding
+    assert_close_rel_max(dx, leaf.grad.float(), 2 ** -9)
+
+
 @pytest.mark.parametrize("rows,cols", [(1280, 1536), (37, 256), (5, 4096)])
 @pytest.mark.parametrize("with_residual", [True, False])
 def test_rmsnorm_backward_with_the_residual_gradient_folded_in(rows, cols, with_residual):
