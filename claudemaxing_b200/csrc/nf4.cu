@@ -1,9 +1,13 @@
 // NF4 dequantisation with the nested 8-bit absmax fused in: an HBM-streaming kernel.
 //
-// One thread turns 16 packed bytes (one 128-bit load) into 32 outputs (four 128-bit fp16 stores,
-// or eight for fp32). The 32 outputs of a thread share one absmax block because every supported
-// blocksize is a multiple of 32, so the scale is computed once per load. The arithmetic is the
-// reference's, operation for operation, with explicitly unfused fp32 intrinsics:
+// A thread turns kGroups groups of 8 packed bytes (one 64-bit load each) into 16 outputs each: fp16 in
+// one 256-bit store, fp32 in two, so that a lane fills whole 32-byte sectors and a warp 1 KB in a row.
+// (Groups of 16 bytes stored as four 128-bit pieces wrote every sector in two halves, from different
+// instructions: the 46.8 M weights of a Qwen2.5-1.5B block took 27.8 us to fp16 and 86.0 us to fp32, now
+// 20.8 and 34.8 us, 5.7 and 6.1 TB/s.) The 16 outputs of a group share one absmax block because every supported
+// blocksize is a multiple of 32. All loads a thread needs are issued before the first is used; the
+// 256-entry table is read through L1, eight or fewer entries a warp. The arithmetic is the reference's,
+// operation for operation, with explicitly unfused fp32 intrinsics:
 //   scale = code2[absmax8[b]] * absmax2[b / blocksize2]   (__fmul_rn)
 //   scale = scale + offset                                 (__fadd_rn)
 //   out   = round(code[nibble] * scale)                    (__fmul_rn, then RN to the out dtype)
@@ -14,18 +18,23 @@ namespace soup {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr int kVecPerThread = 2;  // independent 128-bit loads in flight per thread
+constexpr int kGroups = 4;        // independent 64-bit loads in flight per thread
 
 template <bool NESTED>
-__device__ __forceinline__ float block_scale(const void* absmax, const float* s_code2,
-                                             const float* absmax2, float offset, int64_t blk,
-                                             int shift2) {
+__device__ __forceinline__ float block_scale(const void* absmax, const float* code2, const float* absmax2,
+                                             float offset, int64_t blk, int shift2) {
   if (NESTED) {
     const uint32_t q8 = reinterpret_cast<const uint8_t*>(absmax)[blk];
-    const float a2 = __ldg(absmax2 + (blk >> shift2));
-    return __fadd_rn(__fmul_rn(s_code2[q8], a2), offset);
+    return __fadd_rn(__fmul_rn(__ldg(code2 + q8), __ldg(absmax2 + (blk >> shift2))), offset);
   }
   return __ldg(reinterpret_cast<const float*>(absmax) + blk);
+}
+
+// 32 bytes to a 32-byte aligned address in one store.
+__device__ __forceinline__ void store32(void* p, const uint32_t (&w)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(p), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+               : "memory");
 }
 
 // One CTA's share of one tensor: blocks [0, n_blocks) of the tensor, this CTA being `block`.
@@ -37,65 +46,81 @@ nf4_dequant_body(const uint8_t* __restrict__ packed, const void* __restrict__ ab
                  void* __restrict__ out, int64_t n_bytes, int shift, int shift2, int64_t block,
                  int64_t n_blocks) {
   __shared__ float s_code[16];
-  __shared__ float s_code2[256];
-  if (threadIdx.x < 16) s_code[threadIdx.x] = code[threadIdx.x];
-  if (NESTED) s_code2[threadIdx.x] = code2[threadIdx.x];  // kThreads == 256
-  __syncthreads();
-  const float offset = NESTED ? __ldg(offset_ptr) : 0.f;
-
-  const int64_t n_vec = n_bytes >> 4;  // whole 16-byte groups
-  const int64_t v_base = block * (kThreads * kVecPerThread) + threadIdx.x;
-
-  uint4 raw[kVecPerThread];
+  const bool wide = (reinterpret_cast<uintptr_t>(out) & 31u) == 0;   // else 16-byte aligned
+  const int64_t n_groups = n_bytes >> 3;
+  const int64_t g_base = block * (kThreads * kGroups) + threadIdx.x;
+  uint2 raw[kGroups];
+  uint32_t q8[kGroups];
+  float top[kGroups];   // absmax2 of the group's block (nested), or its absmax
 #pragma unroll
-  for (int u = 0; u < kVecPerThread; ++u) {
-    const int64_t v = v_base + (int64_t)u * kThreads;
-    if (v < n_vec) raw[u] = __ldcs(reinterpret_cast<const uint4*>(packed) + v);
+  for (int u = 0; u < kGroups; ++u) {
+    const int64_t g = g_base + (int64_t)u * kThreads;
+    if (g < n_groups) {
+      raw[u] = __ldcs(reinterpret_cast<const uint2*>(packed) + g);
+      const int64_t blk = (g << 4) >> shift;
+      if (NESTED) {
+        q8[u] = __ldg(reinterpret_cast<const uint8_t*>(absmax) + blk);
+        top[u] = __ldg(absmax2 + (blk >> shift2));
+      } else {
+        top[u] = __ldg(reinterpret_cast<const float*>(absmax) + blk);
+      }
+    }
   }
+  const float offset = NESTED ? __ldg(offset_ptr) : 0.f;
+  if (threadIdx.x < 16) s_code[threadIdx.x] = code[threadIdx.x];
+  __syncthreads();
 #pragma unroll
-  for (int u = 0; u < kVecPerThread; ++u) {
-    const int64_t v = v_base + (int64_t)u * kThreads;
-    if (v >= n_vec) continue;
-    const int64_t e0 = v << 5;  // first output element of this group
-    const float scale = block_scale<NESTED>(absmax, s_code2, absmax2, offset, e0 >> shift, shift2);
-    const uint32_t w[4] = {raw[u].x, raw[u].y, raw[u].z, raw[u].w};
+  for (int u = 0; u < kGroups; ++u) {
+    const int64_t g = g_base + (int64_t)u * kThreads;
+    if (g >= n_groups) continue;
+    const int64_t e0 = g << 4;  // first output element of this group
+    const float scale = NESTED ? __fadd_rn(__fmul_rn(__ldg(code2 + q8[u]), top[u]), offset) : top[u];
+    const uint32_t w[2] = {raw[u].x, raw[u].y};
     if (OUT_F16) {
-      uint4* o = reinterpret_cast<uint4*>(reinterpret_cast<__half*>(out) + e0);
+      uint32_t h[8];
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {  // one 32-bit word = 4 bytes = 8 outputs = one 128-bit store
-        uint32_t h[4];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-          const uint32_t byte = (w[k] >> (8 * b)) & 0xffu;
-          const float hi = __fmul_rn(s_code[byte >> 4], scale);
-          const float lo = __fmul_rn(s_code[byte & 15u], scale);
-          __half2 p = __floats2half2_rn(hi, lo);
-          h[b] = *reinterpret_cast<uint32_t*>(&p);
-        }
-        __stcs(o + k, make_uint4(h[0], h[1], h[2], h[3]));
+      for (int b = 0; b < 8; ++b) {
+        const uint32_t byte = (w[b >> 2] >> (8 * (b & 3))) & 0xffu;
+        const float hi = __fmul_rn(s_code[byte >> 4], scale);
+        const float lo = __fmul_rn(s_code[byte & 15u], scale);
+        __half2 p = __floats2half2_rn(hi, lo);
+        h[b] = *reinterpret_cast<uint32_t*>(&p);
+      }
+      __half* o = reinterpret_cast<__half*>(out) + e0;
+      if (wide) {
+        store32(o, h);
+      } else {
+        reinterpret_cast<uint4*>(o)[0] = make_uint4(h[0], h[1], h[2], h[3]);
+        reinterpret_cast<uint4*>(o)[1] = make_uint4(h[4], h[5], h[6], h[7]);
       }
     } else {
-      float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + e0);
+      float* o = reinterpret_cast<float*>(out) + e0;
 #pragma unroll
-      for (int k = 0; k < 4; ++k) {
+      for (int half = 0; half < 2; ++half) {
+        uint32_t f[8];
 #pragma unroll
-        for (int b = 0; b < 4; b += 2) {
-          const uint32_t b0 = (w[k] >> (8 * b)) & 0xffu, b1 = (w[k] >> (8 * b + 8)) & 0xffu;
-          __stcs(o + k * 2 + (b >> 1),
-                 make_float4(__fmul_rn(s_code[b0 >> 4], scale), __fmul_rn(s_code[b0 & 15u], scale),
-                             __fmul_rn(s_code[b1 >> 4], scale), __fmul_rn(s_code[b1 & 15u], scale)));
+        for (int b = 0; b < 4; ++b) {
+          const uint32_t byte = (w[half] >> (8 * b)) & 0xffu;
+          f[2 * b] = __float_as_uint(__fmul_rn(s_code[byte >> 4], scale));
+          f[2 * b + 1] = __float_as_uint(__fmul_rn(s_code[byte & 15u], scale));
+        }
+        if (wide) {
+          store32(o + 8 * half, f);
+        } else {
+          reinterpret_cast<uint4*>(o)[2 * half] = make_uint4(f[0], f[1], f[2], f[3]);
+          reinterpret_cast<uint4*>(o)[2 * half + 1] = make_uint4(f[4], f[5], f[6], f[7]);
         }
       }
     }
   }
 
-  // Ragged tail (n_bytes not a multiple of 16): the last block's first threads go byte by byte.
+  // Ragged tail (n_bytes not a multiple of 8): the last block's first threads go byte by byte.
   if (block == n_blocks - 1) {
-    const int64_t tail0 = n_vec << 4;
+    const int64_t tail0 = n_groups << 3;
     for (int64_t i = tail0 + threadIdx.x; i < n_bytes; i += kThreads) {
       const uint32_t byte = packed[i];
       const int64_t e = i << 1;
-      const float scale = block_scale<NESTED>(absmax, s_code2, absmax2, offset, e >> shift, shift2);
+      const float scale = block_scale<NESTED>(absmax, code2, absmax2, offset, e >> shift, shift2);
       const float hi = __fmul_rn(s_code[byte >> 4], scale);
       const float lo = __fmul_rn(s_code[byte & 15u], scale);
       if (OUT_F16) {
@@ -109,6 +134,11 @@ nf4_dequant_body(const uint8_t* __restrict__ packed, const void* __restrict__ ab
   }
 }
 
+inline int64_t blocks_of(int64_t n_bytes) {
+  const int64_t blocks = ((n_bytes >> 3) + kThreads * kGroups - 1) / (kThreads * kGroups);
+  return blocks < 1 ? 1 : blocks;
+}
+
 template <bool NESTED, bool OUT_F16>
 __global__ void __launch_bounds__(kThreads)
 nf4_dequant_kernel(const uint8_t* __restrict__ packed, const void* __restrict__ absmax,
@@ -119,23 +149,24 @@ nf4_dequant_kernel(const uint8_t* __restrict__ packed, const void* __restrict__ 
                                     shift, shift2, blockIdx.x, gridDim.x);
 }
 
-// Several tensors in one launch (blockIdx.y = tensor): removes the per-launch latency that
-// dominates the small projection weights (k/v of Qwen2.5-1.5B are 0.4 M elements each).
+// Several tensors in one launch: removes the per-launch latency that dominates the small projection
+// weights (k/v of Qwen2.5-1.5B are 0.4 M elements each). Their blocks follow one another in the grid.
 constexpr int kMaxBatch = 8;
 struct Nf4Batch {
   soup_nf4_item item[kMaxBatch];
-  int64_t n_blocks[kMaxBatch];
+  int64_t first_block[kMaxBatch + 1];
+  int count;
 };
 
 template <bool NESTED, bool OUT_F16>
 __global__ void __launch_bounds__(kThreads)
-nf4_dequant_batch_kernel(const Nf4Batch b, const float* __restrict__ code, int shift, int shift2) {
-  const soup_nf4_item& it = b.item[blockIdx.y];
-  const int64_t n_blocks = b.n_blocks[blockIdx.y];
-  if ((int64_t)blockIdx.x >= n_blocks) return;
+nf4_dequant_batch_kernel(const __grid_constant__ Nf4Batch b, const float* __restrict__ code, int shift, int shift2) {
+  int i = 0;
+  while (i + 1 < b.count && (int64_t)blockIdx.x >= b.first_block[i + 1]) ++i;
+  const soup_nf4_item& it = b.item[i];
   nf4_dequant_body<NESTED, OUT_F16>(reinterpret_cast<const uint8_t*>(it.packed), it.absmax, code,
                                     it.code2, it.absmax2, it.offset, it.out, it.n_elems >> 1, shift,
-                                    shift2, blockIdx.x, n_blocks);
+                                    shift2, blockIdx.x - b.first_block[i], b.first_block[i + 1] - b.first_block[i]);
 }
 
 inline int log2_exact(int v) {
@@ -169,10 +200,7 @@ extern "C" int soup_nf4_dequant(const void* packed, const void* absmax, const fl
   if (!aligned16(packed) || !aligned16(out))
     SOUP_FAIL(SOUP_ERR_ARG, "nf4_dequant: packed and out must be 16-byte aligned");
   const int64_t n_bytes = n_elems >> 1;
-  const int64_t n_vec = n_bytes >> 4;
-  const int64_t per_block = kThreads * kVecPerThread;
-  int64_t blocks = (n_vec + per_block - 1) / per_block;
-  if (blocks < 1) blocks = 1;
+  const int64_t blocks = blocks_of(n_bytes);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
 #define SOUP_NF4_LAUNCH(N_, F_)                                                              \
   nf4_dequant_kernel<N_, F_><<<(unsigned)blocks, kThreads, 0, s>>>(                          \
@@ -206,11 +234,10 @@ extern "C" int soup_nf4_dequant_batch(const soup_nf4_item* items, int count, con
   if (out_dtype != SOUP_F16 && out_dtype != SOUP_F32)
     SOUP_FAIL(SOUP_ERR_ARG, "nf4_dequant_batch: out dtype must be fp16 or fp32");
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const int64_t per_block = kThreads * kVecPerThread;
   for (int i0 = 0; i0 < count; i0 += kMaxBatch) {
     Nf4Batch b;
     int m = 0;
-    int64_t max_blocks = 1;
+    b.first_block[0] = 0;
     for (int i = i0; i < count && m < kMaxBatch; ++i) {
       const soup_nf4_item& it = items[i];
       if (it.n_elems == 0) continue;
@@ -219,14 +246,12 @@ extern "C" int soup_nf4_dequant_batch(const soup_nf4_item* items, int count, con
           !aligned16(it.out))
         SOUP_FAIL(SOUP_ERR_ARG, "nf4_dequant_batch: item %d is malformed", i);
       b.item[m] = it;
-      int64_t blocks = (((it.n_elems >> 1) >> 4) + per_block - 1) / per_block;
-      if (blocks < 1) blocks = 1;
-      b.n_blocks[m] = blocks;
-      if (blocks > max_blocks) max_blocks = blocks;
+      b.first_block[m + 1] = b.first_block[m] + blocks_of(it.n_elems >> 1);
       ++m;
     }
     if (m == 0) continue;
-    dim3 grid((unsigned)max_blocks, (unsigned)m);
+    b.count = m;
+    const unsigned grid = (unsigned)b.first_block[m];
     if (nested) {
       if (out_dtype == SOUP_F16) nf4_dequant_batch_kernel<true, true><<<grid, kThreads, 0, s>>>(b, code, shift, shift2);
       else nf4_dequant_batch_kernel<true, false><<<grid, kThreads, 0, s>>>(b, code, shift, shift2);

@@ -62,6 +62,27 @@ def test_nf4_bit_exact_vs_oracle(shape, nested):
     assert torch.equal(out32.half().cpu(), ref16)
 
 
+@pytest.mark.parametrize("nested", [True, False])
+@pytest.mark.parametrize("shape", [(1, 16), (33, 1000), (2, 4096 * 8 + 6)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_nf4_outputs_on_16_byte_boundaries_and_ragged_tails(shape, nested, shift):
+    """An output that is 16- but not 32-byte aligned takes two stores per group; byte counts off a
+    multiple of 8, and just over one CTA's share (8 KB), take the tail and the second CTA."""
+    from claudemaxing_b200.nf4 import dequantize_nf4
+    from oracle import nf4 as onf4
+
+    gen = torch.Generator().manual_seed(shape[1])
+    packed, state = onf4.quantize_nf4((torch.randn(*shape, generator=gen) * 0.05).half(), nested=nested)
+    n = shape[0] * shape[1]
+    for dtype in (F16, F32):
+        step = 16 // torch.empty((), dtype=dtype).element_size() * shift
+        buf = torch.full((n + step + 8,), 7.0, dtype=dtype, device=DEV)
+        out = buf[step:step + n].view(shape)
+        dequantize_nf4(packed.to(DEV), state.to(DEV), dtype, out=out)
+        assert torch.equal(_bits(out.cpu()), _bits(onf4.dequantize_nf4(packed, state, dtype)))
+        assert (buf[:step] == 7.0).all() and (buf[step + n:] == 7.0).all()
+
+
 def test_nf4_quantiser_matches_oracle_and_roundtrip_is_idempotent():
     from claudemaxing_b200 import qlora
     from claudemaxing_b200.nf4 import dequantize_nf4
