@@ -27,30 +27,35 @@ OWN_BACKWARD = os.environ.get("SOUP_ATTN_BACKWARD", "1") != "0"
 
 
 def attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, scale):
-    """(dq [n, hq, 128], dk [n, hk, 128], dv [n, hk, 128], flat): the fp32 gradients of the segment
-    attention from this library's backward kernel (csrc/attention.cu), and the one buffer the three
-    are consecutive parts of."""
+    """The fp32 gradients of the segment attention from this library's backward kernel
+    (csrc/attention.cu) as one flat buffer: dq [n, hq, 128], dk [n, hk, 128], dv [n, hk, 128] one after
+    another (`gradient_parts`)."""
     n, hq, d = q.shape
     hk = k.shape[1]
     grad = grad if grad.is_contiguous() else grad.contiguous()
     flat = torch.empty(n * (hq + 2 * hk) * d, dtype=torch.float32, device=q.device)
-    dq, dk, dv = _gradient_parts(flat, n, hq, hk, d)
     stats = torch.empty(n * hq * 2, dtype=torch.float32, device=q.device)
+    dq = flat.data_ptr()
+    dk = dq + 4 * n * hq * d
     _lib.call("soup_attn_bwd", _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _lib.ptr(grad),
-              _lib.ptr(lse), _lib.ptr(cu_rows), _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(stats),
+              _lib.ptr(lse), _lib.ptr(cu_rows), dq, dk, dk + 4 * n * hk * d, _lib.ptr(stats),
               8 * n * hq, n, cu_rows.numel() - 1, hq, hk, d, q.stride(0), k.stride(0), v.stride(0),
               float(scale), _lib.stream_of(q))
-    return dq, dk, dv, flat
+    return flat
 
 
-def _gradient_parts(flat, n, hq, hk, d):
-    dq, dk, dv = flat.split((n * hq * d, n * hk * d, n * hk * d))
-    return dq.view(n, hq, d), dk.view(n, hk, d), dv.view(n, hk, d)
+def gradient_parts(flat, n, hq, hk, d):
+    """(dq, dk, dv) views of `attention_gradients_f32`'s buffer, or of a copy of it."""
+    at = n * hq * d
+    return (torch.as_strided(flat, (n, hq, d), (hq * d, d, 1)),
+            torch.as_strided(flat, (n, hk, d), (hk * d, d, 1), at),
+            torch.as_strided(flat, (n, hk, d), (hk * d, d, 1), at + n * hk * d))
 
 
 def attention_gradients(q, k, v, out, lse, grad, cu_rows, scale):
-    """`attention_gradients_f32` with dq rounded to q's dtype: (dq, dk fp32, dv fp32)."""
-    dq, dk, dv, _ = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, scale)
+    """`attention_gradients_f32` as three tensors, dq rounded to q's dtype: (dq, dk fp32, dv fp32)."""
+    flat = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, scale)
+    dq, dk, dv = gradient_parts(flat, q.shape[0], q.shape[1], k.shape[1], q.shape[2])
     return dq.to(q.dtype), dk, dv
 
 
@@ -120,8 +125,9 @@ class SegmentAttention(torch.autograd.Function):
     def backward(ctx, grad):
         q, k, v, cu_rows, out, lse = ctx.saved_tensors
         if OWN_BACKWARD:
-            flat = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, ctx.scale)[3].to(q.dtype)
-            return (*_gradient_parts(flat, q.shape[0], q.shape[1], k.shape[1], q.shape[2]), None, None, None)
+            # one rounding launch for all three: they are adjacent
+            flat = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, ctx.scale).to(q.dtype)
+            return (*gradient_parts(flat, q.shape[0], q.shape[1], k.shape[1], q.shape[2]), None, None, None)
         rng_state = torch.empty(2, dtype=torch.uint64, device=q.device)   # no dropout: never read
         dq, dk, dv = torch.ops.torch_attn._varlen_attn_backward(
             grad.contiguous(), q, k, v, out, lse, cu_rows, cu_rows, ctx.longest, ctx.longest, True,

@@ -43,7 +43,7 @@ import torch
 from . import _lib
 from . import attention as attention_mod
 from . import lora as lora_mod
-from .attention import attention_gradients_f32, segment_attention
+from .attention import attention_gradients_f32, gradient_parts, segment_attention
 from .rmsnorm import fp16_copy_of
 from .rope import rotate_into
 from .swiglu_recompute import _silu_mul_bwd, _silu_mul_fwd
@@ -60,6 +60,8 @@ def _plain_precision(fn):
 
     @functools.wraps(fn)
     def wrapped(*args, **kwargs):
+        if not torch.is_autocast_enabled("cuda"):   # backward: nothing to switch off
+            return fn(*args, **kwargs)
         with torch.autocast("cuda", enabled=False):
             return fn(*args, **kwargs)
 
@@ -343,16 +345,18 @@ class _QKVRope(torch.autograd.Function):
         plan, (n, d, nq, nk, hq, hk) = ctx.plan, ctx.sizes
         if ctx.attends:
             cos, sin, q_out, k_out, v_out, attended, lse, cu_rows = ctx.saved_tensors
-            dq, dk, dv, _ = attention_gradients_f32(q_out, k_out, v_out, attended, lse,
-                                                    grads[0].reshape(n, hq, d), cu_rows, ctx.scale)
+            flat = attention_gradients_f32(q_out, k_out, v_out, attended, lse, grads[0].reshape(n, hq, d),
+                                           cu_rows, ctx.scale)
         else:
             cos, sin = ctx.saved_tensors
-            dq, dk, dv = grads
-        dqkv = torch.empty(n, nq + 2 * nk, dtype=F16, device=dq.device)
+        dqkv = torch.empty(n, nq + 2 * nk, dtype=F16, device=cos.device)
         if ctx.attends and _plain_tables(cos, sin, n):
-            _lib.call("soup_qkv_rope_bwd", _lib.ptr(dq), _lib.ptr(dk), _lib.ptr(dv), _lib.ptr(cos), _lib.ptr(sin),
-                      _lib.ptr(dqkv), dqkv.stride(0), n, hq, hk, d, _lib.stream_of(dq))
+            dq = flat.data_ptr()
+            dk = dq + 4 * n * nq
+            _lib.call("soup_qkv_rope_bwd", dq, dk, dk + 4 * n * nk, _lib.ptr(cos), _lib.ptr(sin),
+                      _lib.ptr(dqkv), dqkv.stride(0), n, hq, hk, d, _lib.stream_of(cos))
         else:
+            dq, dk, dv = gradient_parts(flat, n, hq, hk, d) if ctx.attends else grads
             dq, dk = (g if g.stride(-1) == 1 else g.contiguous() for g in (dq, dk))
 
             def heads_first(t, h):

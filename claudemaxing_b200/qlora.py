@@ -145,12 +145,22 @@ class _DequantBuffers:
         self.order = []                # buffer indices, least recently used first
 
     def holds(self, group, key):
-        for i, owner in enumerate(self.owner):
-            if owner is not None and owner() is group and self.key[i] == key:
+        i = group.last   # where the group was found or filled last: the owner decides, as for any other
+        if i is not None and i < len(self.owner) and self._is(i, group, key):
+            return i
+        for i in range(len(self.owner)):
+            if self._is(i, group, key):
+                group.last = i
                 return i
         return None
 
+    def _is(self, i, group, key):
+        owner = self.owner[i]
+        return owner is not None and owner() is group and self.key[i] == key
+
     def touch(self, i):
+        if self.order and self.order[-1] == i:
+            return
         if i in self.order:
             self.order.remove(i)
         self.order.append(i)
@@ -211,6 +221,7 @@ class NF4Group:
         for n in self.sizes:
             self.offsets.append(self.offsets[-1] + (n + 127) // 128 * 128)  # 256-byte aligned slices
         self.next = self.prev = None   # neighbours in forward order (set by `chain`)
+        self.last = None               # see _DequantBuffers.holds
         for l in self.layers:
             l.group = self
 
@@ -223,15 +234,17 @@ class NF4Group:
     def _key(self):
         return tuple(l.packed._version for l in self.layers) + tuple(l.packed.data_ptr() for l in self.layers)
 
-    def _views(self, flat):
-        return [flat[o:o + n].view(l.out_features, l.in_features)
-                for l, o, n in zip(self.layers, self.offsets, self.sizes)]
+    def _view(self, flat, j):
+        layer = self.layers[j]
+        return torch.as_strided(flat, (layer.out_features, layer.in_features), (layer.in_features, 1),
+                                self.offsets[j])
 
     def _fill(self, bufs, i, dtype):
         from .nf4 import dequantize_nf4_batch
 
+        flat = bufs.flat[i]
         dequantize_nf4_batch([(l.packed, l.quant_state) for l in self.layers], dtype,
-                             outs=self._views(bufs.flat[i]))
+                             outs=[self._view(flat, j) for j in range(len(self.layers))])
         bufs.owner[i], bufs.key[i] = weakref.ref(self), self._key()
 
     def stacked(self, layers, dtype, probe=False):
@@ -247,12 +260,17 @@ class NF4Group:
             return None
         if probe:
             return True
-        first = self.weight(layers[0], dtype)
-        flat = first.reshape(-1)
+        flat = self._resident(dtype)
         total = sum(l.out_features for l in layers)
-        return torch.as_strided(flat, (total, layers[0].in_features), (layers[0].in_features, 1))
+        return torch.as_strided(flat, (total, layers[0].in_features), (layers[0].in_features, 1),
+                                self.offsets[index[0]])
 
     def weight(self, layer, dtype):
+        return self._view(self._resident(dtype), self.layers.index(layer))
+
+    def _resident(self, dtype):
+        """The buffer that holds this group's weights now, filled first if none does."""
+        layer = self.layers[0]
         device = layer.packed.device
         bufs = NF4Group._buffers.get((device, dtype))
         if bufs is None or bufs.numel < self.offsets[-1]:
@@ -263,7 +281,7 @@ class NF4Group:
             i = bufs.take(self.resident_blocks(bufs.numel, dtype))
             self._fill(bufs, i, dtype)
         bufs.touch(i)
-        return self._views(bufs.flat[i])[self.layers.index(layer)]
+        return bufs.flat[i]
 
 
 class NF4Linear(torch.nn.Module):
