@@ -33,6 +33,8 @@ SIGNATURES = {
     "soup_rope": [_P, _P, _P, _P, _P, _P] + [_L] * 13 + [_I] * 6 + [_P],
     "soup_rope_sum": [_P, _P, _P, _P, _P, _P, _P] + [_L] * 22 + [_I] * 7 + [_P],
     "soup_attn_fwd": [_P, _P, _P, _P, _P, _P] + [_L] * 8 + [_F, _P],
+    "soup_lora_pair_gain": [_P, _L, _L, _P, _L, _L] + [_P] * 6 + [_F, _F, _L, _L, _P],
+    "soup_lora_pair_input": [_P] * 8 + [_F, _F] + [_L] * 3 + [_P],
     "soup_qkv_rope_fwd": [_P, _L] + [_P] * 7 + [_L] * 4 + [_P],
     "soup_qkv_rope_bwd": [_P] * 6 + [_L] * 5 + [_P],
     "soup_attn_bwd": [_P] * 11 + [_L] * 9 + [_F, _P],

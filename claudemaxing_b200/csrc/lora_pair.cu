@@ -1,0 +1,421 @@
+// Backward of a block's two rank-16 adapters (q_proj's and v_proj's, sharing their input) in two
+// launches: everything that reads the output gradients, and everything that reads the shared input.
+//
+// As torch products the pair takes eight launches at a few thousand tokens (two per weight gradient,
+// two for the rank-16 gradients, a batched product back to the input's width and the mask kernel),
+// 45 us a block at 1280 tokens, most of it launches of GEMMs with an extent of 16, and writes and
+// reads four [tokens, hidden] fp16 tensors in between. Here a rank of 16 is one k step (or one m tile)
+// of mma.sync.m16n8k16, operands go from global memory to fragments without shared memory, and a
+// fragment's transpose is a movmatrix away, so that each [tokens, width] tensor is read once and the
+// only one written is the input gradient. (A tcgen05 tile would be 128 wide where these are 16.)
+// Bound by latency at the step's token counts: 8.2 + 6.3 us at 1280 tokens (hidden 1536, outputs 1536
+// and 256) where the eight launches take 37.2 us, 10.8 + 19.1 and 70.0 us at 4608.
+//
+// Roundings are those of the products they replace: fp32 accumulators, the rank-16 gradient and the
+// product back to the input's width rounded to fp16 once, weight gradients added in fp32 (by
+// reductions, in any order).
+#include "common.cuh"
+#include "umma.cuh"
+
+namespace soup {
+namespace {
+
+constexpr int kRank = 16;
+
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t x) {
+  uint32_t y;
+  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
+  return y;
+}
+
+// c += a b: A [16 x 16] row, B [16 x 8] column fragments.
+__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// Adds `bytes` of fp32 values in shared memory to global memory (both 16-byte aligned).
+__device__ __forceinline__ void bulk_add(float* gdst, const float* ssrc, uint32_t bytes) {
+  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
+               ::"l"(gdst), "r"(umma::smem_u32(ssrc)), "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ void red_add4(float* p, float x, float y, float z, float w) {
+  asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w));
+}
+
+// The order of indices inside a product is free as long as both operands agree, so that a lane can move
+// contiguous bytes: of 16 ranks, "index 2t, 2t + 1 of 8-block i" is rank 4t + 2i, 4t + 2i + 1, and of 32
+// columns, "index 2t, 2t + 1 of 8-block j" is column 8t + 2j, 8t + 2j + 1 (t = lane % 4). With the plain
+// order a fragment is four 4-byte loads a lane, 16 bytes of each of 8 rows, and the load unit is what
+// bounds the kernel.
+__device__ __forceinline__ int rank_of(int block, int index) { return 4 * (index >> 1) + 2 * block + (index & 1); }
+__device__ __forceinline__ int column_of(int block, int index) { return 8 * (index >> 1) + 2 * block + (index & 1); }
+
+// The A fragment of rows row0 .. row0 + 15 of a row-major fp16 [n_rows, 16] matrix; rows past n_rows read
+// as zero.
+__device__ __forceinline__ void load_rank_fragment(const __half* m, int64_t row0, int64_t n_rows, int lane,
+                                                   uint32_t (&f)[4]) {
+  const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {   // f[0], f[1]: rows g, g + 8 of block 0; f[2], f[3]: of block 1
+    const int64_t row = row0 + g + half * 8;
+    const uint2 v = row < n_rows ? __ldg(reinterpret_cast<const uint2*>(m + row * kRank + 4 * t)) : make_uint2(0u, 0u);
+    f[half] = v.x;
+    f[2 + half] = v.y;
+  }
+}
+
+// ------------------------------------------------------------------------------------------
+// gain = g B (fp16 [rows, 16], B already scaled) and dB += alpha g^T a, for both adapters. A CTA owns 32
+// rows; its 16 warps take 32-column chunks of the gradients in turn: a chunk's fragments are an operand
+// of the first product as they are and, transposed, of the second. The warps' partial gains meet in
+// shared memory and are summed in a fixed order; a chunk's 32 x 16 values of dB are 2 KB in a row and are
+// added by the copy engine. A chain of a few dependent loads, 8.0 us at 128 rows as at 1280. (With the
+// plain order of columns, four-byte loads, 10.0 us; 128 rows per cluster of eight CTAs 18.1 us, the
+// partial gains crossing the cluster one value at a time.)
+// ------------------------------------------------------------------------------------------
+constexpr int kGainBlocks = 2, kGainRows = 16 * kGainBlocks, kGainWarps = 16, kChunk = 32;
+constexpr int kGainValues = kGainRows * kRank;   // of one adapter
+constexpr int kGainStage = kChunk * kRank;       // one chunk of dB; two per warp
+constexpr int kGainSmem = kGainWarps * (2 * kGainValues + 2 * kGainStage) * (int)sizeof(float);
+
+struct GainArgs {
+  const __half* g[2];
+  int64_t pitch[2];
+  int out[2];             // columns of each gradient, a multiple of 16
+  const __half* a;        // [2, rows, 16]
+  const __half* b[2];     // [out, 16]
+  float* db[2];           // [out, 16]
+  float alpha[2];
+  __half* gain;           // [2, rows, 16]
+  int64_t rows;
+};
+
+__global__ void __launch_bounds__(kGainWarps * 32) lora_gain_kernel(const __grid_constant__ GainArgs p) {
+  extern __shared__ __align__(128) float s_gain[];   // [kGainWarps][2][kGainValues], then the warps' stages
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int g = lane >> 2, t = lane & 3;
+  const int64_t row0 = (int64_t)blockIdx.x * kGainRows;
+  float* stages = s_gain + kGainWarps * 2 * kGainValues + warp * 2 * kGainStage;
+  int turn = 0;
+#pragma unroll 1
+  for (int w = 0; w < 2; ++w) {
+    // a, rows along the contraction: B fragments [16 rows x 8 ranks] of the row blocks
+    uint32_t ab[kGainBlocks][2][2];   // [row block][rank block][row half]
+#pragma unroll
+    for (int rb = 0; rb < kGainBlocks; ++rb) {
+      uint32_t f[4];
+      load_rank_fragment(p.a + (int64_t)w * p.rows * kRank, row0 + rb * 16, p.rows, lane, f);
+      ab[rb][0][0] = transpose8x8(f[0]);
+      ab[rb][0][1] = transpose8x8(f[1]);
+      ab[rb][1][0] = transpose8x8(f[2]);
+      ab[rb][1][1] = transpose8x8(f[3]);
+    }
+    float gain[kGainBlocks][2][4] = {};   // [row block][rank block]
+    const int out = p.out[w];
+    const float al = p.alpha[w];
+#pragma unroll 2
+    for (int col0 = warp * kChunk; col0 < out; col0 += kGainWarps * kChunk) {
+      const int left = out - col0;   // 16 in the last chunk of an odd number of sixteens
+      uint32_t gf[kGainBlocks][2][4];   // [row block][row half][column block]
+#pragma unroll
+      for (int rb = 0; rb < kGainBlocks; ++rb)
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const int64_t row = row0 + rb * 16 + g + half * 8;
+          const uint4 v = row < p.rows && 8 * t < left
+                              ? __ldg(reinterpret_cast<const uint4*>(p.g[w] + row * p.pitch[w] + col0 + 8 * t))
+                              : make_uint4(0u, 0u, 0u, 0u);
+          gf[rb][half][0] = v.x;
+          gf[rb][half][1] = v.y;
+          gf[rb][half][2] = v.z;
+          gf[rb][half][3] = v.w;
+        }
+      uint32_t bf[4][2];   // [column block][rank block]
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int col = column_of(j, g);
+        const uint2 v = col < left ? __ldg(reinterpret_cast<const uint2*>(p.b[w] + (int64_t)(col0 + col) * kRank + 4 * t))
+                                   : make_uint2(0u, 0u);
+        bf[j][0] = transpose8x8(v.x);
+        bf[j][1] = transpose8x8(v.y);
+      }
+      float db[2][2][4] = {};   // [16-column half][rank block]
+#pragma unroll
+      for (int rb = 0; rb < kGainBlocks; ++rb)
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+          const uint32_t ga[4] = {gf[rb][0][2 * s], gf[rb][1][2 * s], gf[rb][0][2 * s + 1], gf[rb][1][2 * s + 1]};
+          mma16816(gain[rb][0], ga, bf[2 * s][0], bf[2 * s + 1][0]);
+          mma16816(gain[rb][1], ga, bf[2 * s][1], bf[2 * s + 1][1]);
+          const uint32_t gt[4] = {transpose8x8(ga[0]), transpose8x8(ga[2]), transpose8x8(ga[1]), transpose8x8(ga[3])};
+          mma16816(db[s][0], gt, ab[rb][0][0], ab[rb][0][1]);
+          mma16816(db[s][1], gt, ab[rb][1][0], ab[rb][1][1]);
+        }
+      float* stage = stages + turn * kGainStage;
+      turn ^= 1;
+      if (lane == 0) umma::tma_store_wait_read<1>();   // the stage used two chunks ago has been read
+      __syncwarp();
+#pragma unroll
+      for (int s = 0; s < 2; ++s)
+#pragma unroll
+        for (int half = 0; half < 2; ++half)
+          *reinterpret_cast<float4*>(stage + column_of(2 * s + half, g) * kRank + 4 * t) =
+              make_float4(db[s][0][2 * half] * al, db[s][0][2 * half + 1] * al, db[s][1][2 * half] * al,
+                          db[s][1][2 * half + 1] * al);
+      umma::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        bulk_add(p.db[w] + (int64_t)col0 * kRank, stage, min(left, kChunk) * kRank * sizeof(float));
+        umma::tma_store_commit();
+      }
+    }
+#pragma unroll
+    for (int rb = 0; rb < kGainBlocks; ++rb)
+#pragma unroll
+      for (int half = 0; half < 2; ++half)
+        *reinterpret_cast<float4*>(s_gain + (warp * 2 + w) * kGainValues + (rb * 16 + g + half * 8) * kRank + 4 * t) =
+            make_float4(gain[rb][0][2 * half], gain[rb][0][2 * half + 1], gain[rb][1][2 * half],
+                        gain[rb][1][2 * half + 1]);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * kGainValues; i += kGainWarps * 32) {
+    float sum = 0.f;   // in the warps' order: the same bits every time
+#pragma unroll
+    for (int k = 0; k < kGainWarps; ++k) sum += s_gain[k * 2 * kGainValues + i];
+    const int w = i / kGainValues, e = i - w * kGainValues;
+    if (row0 + e / kRank < p.rows) p.gain[((int64_t)w * p.rows + row0) * kRank + e] = __float2half_rn(sum);
+  }
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // the sums have landed
+}
+
+// ------------------------------------------------------------------------------------------
+// From the shared input x (fp16) and the two masks: dx = sum over the adapters of
+// keep * scale * fp16(gain A), and dA += gain^T (keep * scale * x). A warp owns 32 columns and walks
+// every fourth 16-row block of its CTA; the CTA's four warps on the same columns add up their dA in
+// shared memory first, because the reductions into dA, the same [16, hidden] for every block of rows,
+// are what bounds it (8.4 us at 1280 rows and 22.0 at 4608 with a reduction per warp, now 6.3 and 19.1).
+// ------------------------------------------------------------------------------------------
+constexpr int kInputStrips = 2, kInputGroups = 4;   // per CTA: 32-column strips, warps on each
+
+struct InputArgs {
+  const __half* x;
+  const uint8_t* bits[2];
+  const __half* gain;     // [2, rows, 16]
+  const __half* a;        // [2, 16, hidden]
+  float* dx;
+  float* da[2];           // [16, hidden]
+  float scale[2];
+  int64_t rows;
+  int hidden, strips, blocks_per_cta;   // strips: hidden / 32
+};
+
+__global__ void __launch_bounds__(kInputStrips * kInputGroups * 32)
+lora_input_kernel(const __grid_constant__ InputArgs p) {
+  __shared__ float4 s_da[kInputStrips][kInputGroups][8][32];   // [..][adapter, row half, column half][lane]
+  const int lane = threadIdx.x & 31, group = (threadIdx.x >> 5) % kInputGroups;
+  const int local = (threadIdx.x >> 5) / kInputGroups;
+  const int strip = min((int)blockIdx.x * kInputStrips + local, p.strips - 1);   // the odd last one twice
+  const bool mine = blockIdx.x * kInputStrips + local < p.strips;
+  const int g = lane >> 2, t = lane & 3;
+  const int col = strip * 32 + t * 8;
+  // A of both adapters: B fragments [16 x 8] of the four tiles
+  uint32_t af[2][4][2];
+#pragma unroll
+  for (int w = 0; w < 2; ++w)
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const uint4 v = *reinterpret_cast<const uint4*>(p.a + ((int64_t)w * kRank + rank_of(half, g)) * p.hidden + col);
+      const uint32_t r[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) af[w][j][half] = transpose8x8(r[j]);
+    }
+  float da[2][4][4] = {};
+  const int64_t n_blocks = (p.rows + 15) / 16;
+  const int64_t begin = (int64_t)blockIdx.y * p.blocks_per_cta;
+  const int64_t end = begin + p.blocks_per_cta < n_blocks ? begin + p.blocks_per_cta : n_blocks;
+  const int64_t first = begin + group, last = mine ? end : 0;
+  const int bit_shift = t * 8;
+  auto fetch = [&](int64_t rb, uint4 (&x)[2], uint32_t (&bits)[2][2], uint32_t (&gf)[2][4]) {
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int64_t row = rb * 16 + g + half * 8;
+      const bool ok = row < p.rows;
+      const int64_t at = row * p.hidden + col;
+      x[half] = ok ? *reinterpret_cast<const uint4*>(p.x + at) : make_uint4(0u, 0u, 0u, 0u);
+#pragma unroll
+      for (int w = 0; w < 2; ++w)
+        bits[w][half] = ok ? *reinterpret_cast<const uint32_t*>(p.bits[w] + ((at - t * 8) >> 3)) : 0u;
+    }
+#pragma unroll
+    for (int w = 0; w < 2; ++w)
+      load_rank_fragment(p.gain + (int64_t)w * p.rows * kRank, rb * 16, p.rows, lane, gf[w]);
+  };
+  uint4 x[2];
+  uint32_t bits[2][2], gf[2][4];
+  if (first < last) fetch(first, x, bits, gf);
+#pragma unroll 1
+  for (int64_t rb = first; rb < last; rb += kInputGroups) {
+    uint4 nx[2];
+    uint32_t nbits[2][2], ngf[2][4];
+    if (rb + kInputGroups < last) fetch(rb + kInputGroups, nx, nbits, ngf);
+    float sum[2][8];   // dx of rows g and g + 8
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      const float scale = p.scale[w];
+      const uint32_t gt[4] = {transpose8x8(gf[w][0]), transpose8x8(gf[w][2]), transpose8x8(gf[w][1]),
+                              transpose8x8(gf[w][3])};
+      const uint32_t keep[2] = {bits[w][0] >> bit_shift, bits[w][1] >> bit_shift};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float c[4] = {0.f, 0.f, 0.f, 0.f};
+        mma16816(c, gf[w], af[w][j][0], af[w][j][1]);
+        uint32_t xf[2];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const uint32_t raw = j == 0 ? x[half].x : j == 1 ? x[half].y : j == 2 ? x[half].z : x[half].w;
+          const float2 xv = __half22float2(*reinterpret_cast<const __half2*>(&raw));
+          const bool k0 = (keep[half] >> (2 * j)) & 1u, k1 = (keep[half] >> (2 * j + 1)) & 1u;
+          __half2 dropped = __floats2half2_rn(k0 ? __fmul_rn(xv.x, scale) : 0.f, k1 ? __fmul_rn(xv.y, scale) : 0.f);
+          xf[half] = transpose8x8(*reinterpret_cast<uint32_t*>(&dropped));
+          // the product rounded to fp16, as a tensor of its own would be
+          const float g0 = __half2float(__float2half_rn(c[2 * half])), g1 = __half2float(__float2half_rn(c[2 * half + 1]));
+          const float d0 = k0 ? __fmul_rn(g0, scale) : 0.f, d1 = k1 ? __fmul_rn(g1, scale) : 0.f;
+          sum[half][2 * j] = w ? __fadd_rn(sum[half][2 * j], d0) : d0;
+          sum[half][2 * j + 1] = w ? __fadd_rn(sum[half][2 * j + 1], d1) : d1;
+        }
+        mma16816(da[w][j], gt, xf[0], xf[1]);
+      }
+    }
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const int64_t row = rb * 16 + g + half * 8;
+      if (row < p.rows) {
+        float4* dst = reinterpret_cast<float4*>(p.dx + row * p.hidden + col);
+        dst[0] = make_float4(sum[half][0], sum[half][1], sum[half][2], sum[half][3]);
+        dst[1] = make_float4(sum[half][4], sum[half][5], sum[half][6], sum[half][7]);
+      }
+    }
+    if (rb + kInputGroups < last) {
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        x[half] = nx[half];
+        bits[0][half] = nbits[0][half];
+        bits[1][half] = nbits[1][half];
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { gf[0][i] = ngf[0][i]; gf[1][i] = ngf[1][i]; }
+    }
+  }
+#pragma unroll
+  for (int w = 0; w < 2; ++w)
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+#pragma unroll
+      for (int q = 0; q < 2; ++q)
+        s_da[local][group][w * 4 + half * 2 + q][lane] =
+            make_float4(da[w][2 * q][2 * half], da[w][2 * q][2 * half + 1], da[w][2 * q + 1][2 * half],
+                        da[w][2 * q + 1][2 * half + 1]);
+  __syncthreads();
+  // the strip's four warps finish two of its eight pieces each
+#pragma unroll
+  for (int e = 0; e < 8 / kInputGroups; ++e) {
+    const int piece = group * (8 / kInputGroups) + e, w = piece >> 2, half = (piece >> 1) & 1, q = piece & 1;
+    float4 sum = s_da[local][0][piece][lane];
+#pragma unroll
+    for (int k = 1; k < kInputGroups; ++k) {
+      const float4 v = s_da[local][k][piece][lane];
+      sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+    }
+    if (mine) red_add4(p.da[w] + (int64_t)rank_of(half, g) * p.hidden + col + q * 4, sum.x, sum.y, sum.z, sum.w);
+  }
+}
+
+inline bool aligned4(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 3u) == 0; }
+
+}  // namespace
+}  // namespace soup
+
+extern "C" int soup_lora_pair_gain(const void* g_first, int64_t pitch_first, int64_t out_first, const void* g_second,
+                                   int64_t pitch_second, int64_t out_second, const void* a, const void* b_first,
+                                   const void* b_second, void* gain, float* db_first, float* db_second,
+                                   float alpha_first, float alpha_second, int64_t rows, int64_t rank, void* stream) {
+  using namespace soup;
+  if (rows < 0 || rank != kRank) SOUP_FAIL(SOUP_ERR_ARG, "lora_pair_gain: the rank must be 16");
+  if (out_first <= 0 || out_second <= 0 || out_first % 16 || out_second % 16 || out_first > (1 << 24) ||
+      out_second > (1 << 24))
+    SOUP_FAIL(SOUP_ERR_ARG, "lora_pair_gain: output widths must be multiples of 16");
+  if (pitch_first < out_first || pitch_second < out_second || (pitch_first | pitch_second) & 7)
+    SOUP_FAIL(SOUP_ERR_ARG, "lora_pair_gain: row pitches must cover the outputs and be multiples of 8");
+  if (rows == 0) return SOUP_OK;
+  if (!g_first || !g_second || !a || !b_first || !b_second || !gain || !db_first || !db_second)
+    SOUP_FAIL(SOUP_ERR_ARG, "lora_pair_gain: null pointer");
+  if (!aligned16(g_first) || !aligned16(g_second) || !aligned16(a) || !aligned16(b_first) || !aligned16(b_second) ||
+      !aligned16(db_first) || !aligned16(db_second))
+    SOUP_FAIL(SOUP_ERR_ARG, "lora_pair_gain: unaligned pointer");
+  GainArgs p;
+  p.g[0] = reinterpret_cast<const __half*>(g_first);
+  p.g[1] = reinterpret_cast<const __half*>(g_second);
+  p.pitch[0] = pitch_first;
+  p.pitch[1] = pitch_second;
+  p.out[0] = (int)out_first;
+  p.out[1] = (int)out_second;
+  p.a = reinterpret_cast<const __half*>(a);
+  p.b[0] = reinterpret_cast<const __half*>(b_first);
+  p.b[1] = reinterpret_cast<const __half*>(b_second);
+  p.db[0] = db_first;
+  p.db[1] = db_second;
+  p.alpha[0] = alpha_first;
+  p.alpha[1] = alpha_second;
+  p.gain = reinterpret_cast<__half*>(gain);
+  p.rows = rows;
+  if (cudaFuncSetAttribute(lora_gain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGainSmem) != cudaSuccess)
+    SOUP_FAIL(SOUP_ERR_LAUNCH, "lora_pair_gain: shared memory attribute");
+  lora_gain_kernel<<<(unsigned)((rows + kGainRows - 1) / kGainRows), kGainWarps * 32, kGainSmem,
+                     reinterpret_cast<cudaStream_t>(stream)>>>(p);
+  SOUP_CHECK_LAUNCH("lora_pair_gain");
+  return SOUP_OK;
+}
+
+extern "C" int soup_lora_pair_input(const void* x16, const uint8_t* bits_first, const uint8_t* bits_second,
+                                    const void* gain, const void* a_pair, float* dx, float* da_first,
+                                    float* da_second, float scale_first, float scale_second, int64_t rows,
+                                    int64_t hidden, int64_t rank, void* stream) {
+  using namespace soup;
+  if (rows < 0 || rank != kRank) SOUP_FAIL(SOUP_ERR_ARG, "lora_pair_input: the rank must be 16");
+  if (hidden <= 0 || hidden % 32 || hidden > (1 << 24))
+    SOUP_FAIL(SOUP_ERR_ARG, "lora_pair_input: the input width must be a multiple of 32");
+  if (rows == 0) return SOUP_OK;
+  if (!x16 || !bits_first || !bits_second || !gain || !a_pair || !dx || !da_first || !da_second)
+    SOUP_FAIL(SOUP_ERR_ARG, "lora_pair_input: null pointer");
+  if (!aligned16(x16) || !aligned4(bits_first) || !aligned4(bits_second) || !aligned16(gain) || !aligned16(a_pair) ||
+      !aligned16(dx) || !aligned16(da_first) || !aligned16(da_second))
+    SOUP_FAIL(SOUP_ERR_ARG, "lora_pair_input: unaligned pointer");
+  InputArgs p;
+  p.x = reinterpret_cast<const __half*>(x16);
+  p.bits[0] = bits_first;
+  p.bits[1] = bits_second;
+  p.gain = reinterpret_cast<const __half*>(gain);
+  p.a = reinterpret_cast<const __half*>(a_pair);
+  p.dx = dx;
+  p.da[0] = da_first;
+  p.da[1] = da_second;
+  p.scale[0] = scale_first;
+  p.scale[1] = scale_second;
+  p.rows = rows;
+  p.hidden = (int)hidden;
+  p.strips = (int)(hidden / 32);
+  // row blocks per CTA, whole rounds of its four warps, that leave about one CTA per SM
+  const int64_t columns = (p.strips + kInputStrips - 1) / kInputStrips, n_blocks = (rows + 15) / 16;
+  int64_t per = (columns * n_blocks + sm_count() - 1) / sm_count();
+  if (per < (n_blocks + 65534) / 65535) per = (n_blocks + 65534) / 65535;
+  per = (per + kInputGroups - 1) / kInputGroups * kInputGroups;
+  if (per > (1 << 20)) SOUP_FAIL(SOUP_ERR_ARG, "lora_pair_input: too many rows");
+  p.blocks_per_cta = (int)per;
+  const dim3 grid((unsigned)columns, (unsigned)((n_blocks + per - 1) / per));
+  lora_input_kernel<<<grid, kInputStrips * kInputGroups * 32, 0, reinterpret_cast<cudaStream_t>(stream)>>>(p);
+  SOUP_CHECK_LAUNCH("lora_pair_input");
+  return SOUP_OK;
+}

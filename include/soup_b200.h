@@ -188,6 +188,24 @@ int soup_rope_sum(const void* q, const void* q_add, const void* k, const void* c
                   int q_dtype, int q_add_dtype, int k_dtype, int cs_dtype, int q_out_dtype,
                   int k_out_dtype, int backward, void* stream);
 
+/* Backward of a block's two rank-16 adapters on one input (the reference's two LoRA branches,
+ * solution/lora.py:94-134, with B scaled beforehand), in two launches. First, from the output gradients g
+ * (fp16 [rows, out], row pitch in elements a multiple of 8, out of 16): gain[i] = fp16(g_i b_i), fp16
+ * [2, rows, 16], and db_i += alpha_i * g_i^T a[i] (fp32 [out, 16]); a is fp16 [2, rows, 16], b_i fp16
+ * [out, 16]. */
+int soup_lora_pair_gain(const void* g_first, int64_t pitch_first, int64_t out_first, const void* g_second,
+                        int64_t pitch_second, int64_t out_second, const void* a, const void* b_first,
+                        const void* b_second, void* gain, float* db_first, float* db_second,
+                        float alpha_first, float alpha_second, int64_t rows, int64_t rank, void* stream);
+/* Then, from the shared input x16 (fp16 [rows, hidden], hidden a multiple of 32), the packed masks and
+ * a_pair (fp16 [2, 16, hidden]): dx = sum_i keep_i * scale_i * fp16(gain_i a_i) (fp32) and
+ * da_i += gain_i^T fp16(keep_i * scale_i * x16) (fp32 [16, hidden]). The sums into da and db are added in
+ * any order. */
+int soup_lora_pair_input(const void* x16, const uint8_t* bits_first, const uint8_t* bits_second,
+                         const void* gain, const void* a_pair, float* dx, float* da_first, float* da_second,
+                         float scale_first, float scale_second, int64_t rows, int64_t hidden, int64_t rank,
+                         void* stream);
+
 /* The rows [q | k | v] of a q/k/v projection (fp16, row pitch qkv_pitch) as rotated q (+ add_q), rotated
  * k and v (+ add_v): fp16 [n, h, d] contiguous, sums and rotation in fp32, one rounding. add_q [n, hq*d]
  * and add_v [n, hk*d] fp16 contiguous or NULL; cos, sin fp32 [n, d]. One launch for what the reference

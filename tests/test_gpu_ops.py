@@ -345,6 +345,50 @@ def test_qkv_split_and_rotation_is_the_rotation_and_the_sums_it_replaces(dims, w
     assert torch.equal(got, want)
 
 
+@pytest.mark.parametrize("rows", [1, 16, 33, 1280])
+@pytest.mark.parametrize("hidden,outs", [(1536, (1536, 256)), (32, (16, 16)), (160, (48, 144))])
+def test_lora_pair_backward_in_two_launches(rows, hidden, outs):
+    """`soup_lora_pair_gain` / `soup_lora_pair_input` against the products they replace in float64, with
+    fp16 roundings where those have them; ragged row blocks, strips that leave warps of a CTA idle, a
+    row pitch of its own, sums added to what the buffers hold. Bounds: one fp16 ulp where a sum in
+    another order rounds the other way (2^-10 of the value, 2^-10 of the largest), fp32 sums (1e-4)."""
+    from claudemaxing_b200 import _lib
+
+    gen = torch.Generator().manual_seed(rows + hidden)
+
+    def rand(*shape, std=1.0):
+        return (torch.randn(*shape, generator=gen) * std).half().to(DEV)
+
+    pitch = outs[0] + 2 * outs[1]
+    wide = rand(rows, pitch, std=0.1)
+    g = (wide[:, :outs[0]], wide[:, outs[0] + outs[1]:])   # column blocks, on 16-byte boundaries
+    a, a_pair = rand(2, rows, 16), rand(2, 16, hidden, std=0.05)
+    b = tuple(rand(o, 16, std=0.05) for o in outs)
+    x16 = rand(rows, hidden)
+    keep = (torch.rand(2, rows * hidden, generator=gen) > 0.1).to(DEV)
+    bits = (keep.view(2, -1, 8).to(torch.int32) << torch.arange(8, device=DEV, dtype=torch.int32)).sum(-1).to(torch.uint8)
+    scales, alphas = (1 / 0.9, 1 / 0.8), (2.0, 0.5)
+    gain = torch.empty(2, rows, 16, dtype=F16, device=DEV)
+    db = [torch.ones(o, 16, device=DEV) for o in outs]
+    da = [torch.ones(16, hidden, device=DEV) for _ in outs]
+    dx = torch.full((rows, hidden), float("nan"), device=DEV)
+    stream = _lib.stream_of(dx)
+    _lib.call("soup_lora_pair_gain", _lib.ptr(g[0]), pitch, outs[0], _lib.ptr(g[1]), pitch, outs[1], _lib.ptr(a),
+              _lib.ptr(b[0]), _lib.ptr(b[1]), _lib.ptr(gain), _lib.ptr(db[0]), _lib.ptr(db[1]), *alphas, rows, 16, stream)
+    want_dx = torch.zeros(rows, hidden, dtype=torch.float64, device=DEV)
+    for i in (0, 1):
+        assert_close_rel_max(gain[i], (g[i].double() @ b[i].double()).float(), 2 ** -10, "gain")
+        assert_close_rel_max(db[i], (1 + alphas[i] * (g[i].double().t() @ a[i].double())).float(), 1e-4, "dB")
+    _lib.call("soup_lora_pair_input", _lib.ptr(x16), _lib.ptr(bits[0]), _lib.ptr(bits[1]), _lib.ptr(gain),
+              _lib.ptr(a_pair), _lib.ptr(dx), _lib.ptr(da[0]), _lib.ptr(da[1]), *scales, rows, hidden, 16, stream)
+    for i in (0, 1):
+        k = keep[i].view(rows, hidden)
+        xd = torch.where(k, x16.float() * scales[i], torch.zeros((), device=DEV)).half()
+        want_dx += k * scales[i] * (gain[i].double() @ a_pair[i].double()).half().double()
+        assert_close_rel_max(da[i], (1 + gain[i].double().t() @ xd.double()).float(), 1e-4, "dA")
+    assert_close_rel_max(dx, want_dx.float(), 2 ** -10, "dx")
+
+
 @pytest.mark.parametrize("cols", [8, 248, 256, 264, 4096, 4104])
 @pytest.mark.parametrize("rows", [1, 5, 4000])
 def test_rmsnorm_row_kernels_at_the_edges_of_their_shapes(rows, cols):
