@@ -3,7 +3,7 @@
 //
 // As torch products the pair takes eight launches at a few thousand tokens (two per weight gradient,
 // two for the rank-16 gradients, a batched product back to the input's width and the mask kernel),
-// 45 us a block at 1280 tokens, most of it launches of GEMMs with an extent of 16, and writes and
+// 37 us a block at 1280 tokens, most of it launches of GEMMs with an extent of 16, and writes and
 // reads four [tokens, hidden] fp16 tensors in between. Here a rank of 16 is one k step (or one m tile)
 // of mma.sync.m16n8k16, operands go from global memory to fragments without shared memory, and a
 // fragment's transpose is a movmatrix away, so that each [tokens, width] tensor is read once and the
