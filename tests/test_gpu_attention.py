@@ -88,10 +88,9 @@ def test_attention_kernels_against_fp32_with_the_fp16_sdpa_error_as_the_bar(hq, 
 
 @pytest.mark.parametrize("hq,hk,lens", [(4, 2, [700, 130]), (12, 2, [2600, 520])])
 def test_attention_forward_when_the_row_maximum_keeps_growing(hq, hk, lens):
-    """Scores that grow along the keys (by far more than the 2^8 a stale maximum may lag), then fall:
-    every row's accumulator is rescaled, some rows of a warp earlier than others. One and two heads
-    per CTA. P is rounded to fp16 relative to a reference up to 2^8 below the maximum, which leaves
-    its relative rounding, 2^-11 an element, as it is: the bound of the plain cases."""
+    """Scores that grow along the keys, then fall: every row's accumulator is rescaled, some rows of a
+    warp earlier than others. One and two heads per CTA. P is rounded to fp16 relative to the row's
+    maximum so far, 2^-11 an element: the bound of the plain cases."""
     from oracle import attention as oat
 
     torch.manual_seed(2)
