@@ -389,6 +389,69 @@ def test_lora_pair_backward_in_two_launches(rows, hidden, outs):
     assert_close_rel_max(dx, want_dx.float(), 2 ** -10, "dx")
 
 
+def _rows_of(kind, rows, out, gen):
+    """An output gradient [1, rows, out]: a tensor of its own, a column block, one row broadcast over
+    the tokens, or rows whose pitch is not a multiple of 16 bytes."""
+    if kind == "broadcast":
+        return (torch.randn(1, 1, out, generator=gen) * 0.1).half().to(DEV).expand(1, rows, out)
+    wide = (torch.randn(1, rows, out + (3 if kind == "ragged" else 64), generator=gen) * 0.1).half().to(DEV)
+    return wide[..., :out].contiguous() if kind == "plain" else wide[..., -out:] if kind == "block" else wide[..., :out]
+
+
+@pytest.mark.parametrize("rank,rows,outs,kinds,launches", [
+    (16, 80, (160, 48), ("plain", "plain"), 2),
+    (16, 33, (160, 48), ("block", "plain"), 2),
+    (16, 40, (160, 48), ("plain", "broadcast"), 0),   # a row pitch of zero
+    (16, 40, (160, 48), ("ragged", "plain"), 0),
+    (16, 40, (168, 48), ("plain", "plain"), 0),       # a width off the kernel's tiles
+    (8, 40, (160, 48), ("plain", "plain"), 0),
+])
+def test_lora_pair_in_place_is_two_single_branches_whichever_way_its_backward_runs(
+        rank, rows, outs, kinds, launches, monkeypatch):
+    """The pair's backward adding into preset gradients against two LoRABranch nodes with the same
+    dropout draws: through its two launches where they take the operands, through the products they
+    replace otherwise. Bounds: an fp16 rank-r gradient that rounds the other way, 2^-10 of the largest
+    value, in everything formed from it."""
+    from claudemaxing_b200 import _lib
+    from claudemaxing_b200.lora import LoRABranch, LoRABranchPair
+
+    hidden, ps, scalings = 96, (0.1, 0.25), (2.0, 0.5)
+    gen = torch.Generator().manual_seed(rank + rows)
+    x = torch.randn(1, rows, hidden, generator=gen).to(DEV)
+    x16 = x.half()
+    weights = [(torch.randn(*shape, generator=gen) * 0.05).to(DEV)
+               for out in outs for shape in ((rank, hidden), (out, rank))]
+    preset = [torch.randn(w.shape, generator=gen).to(DEV) for w in weights]
+    grads = [_rows_of(kind, rows, out, gen) for kind, out in zip(kinds, outs)]
+    entry, made = _lib.call, []
+    monkeypatch.setattr(_lib, "call", lambda name, *args: (made.append(name), entry(name, *args))[1])
+
+    def run(pair):
+        leaf = x.clone().requires_grad_()
+        ws = [w.clone().requires_grad_() for w in weights]
+        for w, g in zip(ws, preset):
+            w.grad = g.clone()
+        torch.cuda.manual_seed(5)
+        b16s = [(ws[2 * i + 1].detach() * scalings[i]).half() for i in (0, 1)]
+        if pair:
+            monkeypatch.setattr(LoRABranch, "accumulate_in_place", True)
+            a16_pair = torch.stack([ws[0].detach().half(), ws[2].detach().half()])
+            out = LoRABranchPair.apply(leaf, x16, *ws, *ps, *scalings, a16_pair, *b16s)
+        else:
+            out = [LoRABranch.apply(leaf, x16, ws[2 * i], ws[2 * i + 1], ps[i], scalings[i],
+                                    ws[2 * i].detach().half(), b16s[i], True) for i in (0, 1)]
+        torch.autograd.backward(list(out), grads)
+        monkeypatch.setattr(LoRABranch, "accumulate_in_place", False)
+        return [*(t.detach() for t in out), leaf.grad, *(w.grad for w in ws)]
+
+    want = run(False)
+    made.clear()
+    got = run(True)
+    assert sum(name.startswith("soup_lora_pair") for name in made) == launches
+    for name, a, b in zip(("out", "out", "dx", "dA", "dB", "dA", "dB"), got, want):
+        assert_close_rel_max(a, b, 2 ** -10, name)
+
+
 @pytest.mark.parametrize("cols", [8, 248, 256, 264, 4096, 4104])
 @pytest.mark.parametrize("rows", [1, 5, 4000])
 def test_rmsnorm_row_kernels_at_the_edges_of_their_shapes(rows, cols):
