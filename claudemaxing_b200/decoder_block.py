@@ -278,10 +278,10 @@ def _norm_and_residual(norm, hidden):
     return norm(hidden), hidden
 
 
-def _plain_tables(cos, sin, n):
-    """Whether the rotary tables are what soup_qkv_rope_* take: fp32, one row per token, 16-byte aligned
-    (both are contiguous already)."""
-    return (cos.dtype == sin.dtype == F32 and cos.shape[1] == sin.shape[1] == n
+def _plain_tables(cos, sin, n, d):
+    """Whether the rotary tables are what soup_qkv_rope_* take: fp32, one row of the head dimension per
+    token, 16-byte aligned (both are contiguous already)."""
+    return (cos.dtype == sin.dtype == F32 and cos.shape == sin.shape == (1, n, d)
             and (cos.data_ptr() | sin.data_ptr()) % 16 == 0)
 
 
@@ -295,6 +295,7 @@ class _QKVRope(torch.autograd.Function):
     @staticmethod
     @_plain_precision
     def forward(ctx, x, x16, lora_q, lora_v, cos, sin, plan, cu_rows=None, scale=None):
+        _lib.require_cuda(x16, lora_q, lora_v, cos, sin)
         bases = [_base(m) for m in (plan.q, plan.k, plan.v)]
         n, d = x16.numel() // x16.shape[-1], plan.head_dim
         nq, nk = bases[0].out_features, bases[1].out_features
@@ -311,8 +312,8 @@ class _QKVRope(torch.autograd.Function):
 
         v_out = torch.empty(n, nk, dtype=F16, device=x16.device)
         shapes = tuple(None if t is None else t.shape for t in (lora_q, lora_v))
-        lora_q, lora_v = (None if t is None else t.reshape(n, -1) for t in (lora_q, lora_v))
-        if _plain_tables(cos, sin, n) and qkv.is_contiguous() and all(
+        lora_q, lora_v = (None if t is None else t.reshape(n, w_out) for t, w_out in ((lora_q, nq), (lora_v, nk)))
+        if _plain_tables(cos, sin, n, d) and qkv.is_contiguous() and all(
                 t is None or (t.dtype == F16 and t.is_contiguous() and t.data_ptr() % 16 == 0)
                 for t in (lora_q, lora_v)):
             _lib.call("soup_qkv_rope_fwd", _lib.ptr(qkv), qkv.stride(0), _lib.ptr(lora_q), _lib.ptr(lora_v),
@@ -350,7 +351,7 @@ class _QKVRope(torch.autograd.Function):
         else:
             cos, sin = ctx.saved_tensors
         dqkv = torch.empty(n, nq + 2 * nk, dtype=F16, device=cos.device)
-        if ctx.attends and _plain_tables(cos, sin, n):
+        if ctx.attends and _plain_tables(cos, sin, n, d):
             dq = flat.data_ptr()
             dk = dq + 4 * n * nq
             _lib.call("soup_qkv_rope_bwd", dq, dk, dk + 4 * n * nk, _lib.ptr(cos), _lib.ptr(sin),

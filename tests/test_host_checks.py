@@ -5,6 +5,7 @@ import pytest
 import torch
 
 from claudemaxing_b200 import _lib
+from claudemaxing_b200 import decoder_block as D
 from claudemaxing_b200 import lm_head_loss as L
 
 
@@ -33,3 +34,48 @@ def test_head_refuses_a_target_of_another_length_than_the_hidden_states(launches
     assert not launches
     L.fused_head_loss(hidden, weight, None, target=torch.zeros(1, 8, dtype=torch.int64))
     assert [name for name, _ in launches] == ["soup_lmhead_ce", "soup_lmhead_finish", "soup_lmhead_totals"]
+
+
+class _Projection:
+    def __init__(self, out_features, weight):
+        self.out_features, self.group, self._weight = out_features, self, weight
+
+    def stacked(self, bases, dtype):
+        return self._weight
+
+
+class _Plan:
+    head_dim = 16
+
+    def __init__(self, heads, kv_heads, hidden):
+        weight = torch.randn((heads + 2 * kv_heads) * 16, hidden).half()
+        self.q, self.k, self.v = (_Projection(h * 16, weight) for h in (heads, kv_heads, kv_heads))
+
+    @staticmethod
+    def qkv_bias(device):
+        return None
+
+
+def _qkv(lora_q_width=64, lora_v_width=32, tables=((1, 5, 16), (1, 5, 16))):
+    x = torch.randn(1, 5, 32, requires_grad=True)
+    lora_q, lora_v = (torch.randn(1, 5, width).half() for width in (lora_q_width, lora_v_width))
+    cos, sin = (torch.randn(*shape) for shape in tables)
+    return D._QKVRope.apply(x, x.detach().half(), lora_q, lora_v, cos, sin, _Plan(4, 2, 32)), cos, sin
+
+
+def test_qkv_split_reads_adapter_terms_and_tables_of_its_own_shape_and_device_only(launches, monkeypatch):
+    """The launch takes bare pointers: an adapter term narrower than its projection is refused, tables
+    of another shape go to the rotation that reads their strides, and every tensor that is read has
+    been checked to be on the device."""
+    checked = []
+    monkeypatch.setattr(_lib, "require_cuda", lambda *tensors: checked.extend(tensors))
+    (q, k, v), cos, sin = _qkv()
+    assert [name for name, _ in launches] == ["soup_qkv_rope_fwd"]
+    assert any(t is cos for t in checked) and any(t is sin for t in checked)
+    assert q.shape == (5, 4, 16) and k.shape == v.shape == (5, 2, 16)
+    for width in (dict(lora_q_width=48), dict(lora_v_width=16), dict(lora_q_width=80)):
+        with pytest.raises(RuntimeError, match="invalid for input of size"):
+            _qkv(**width)
+    launches.clear()
+    _qkv(tables=((1, 5, 16), (1, 5, 8)))
+    assert [name for name, _ in launches] == ["soup_rope_sum"]
