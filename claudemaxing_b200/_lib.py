@@ -141,6 +141,8 @@ def stream_of(t):
     """The current torch stream of `t`'s device, as the void* the C ABI takes. (The raw handle is
     asked for directly: building a torch.cuda.Stream object for it costs 2 us per launch.)"""
     index = t.get_device()
+    if index < 0:
+        raise ValueError(f"libsoup_b200: expected a CUDA tensor, but got one on {t.device}")
     handle = _StreamOf(torch._C._cuda_getCurrentRawStream(index))
     handle.device_index = index
     return handle

@@ -19,6 +19,13 @@ def launches(monkeypatch):
     return made
 
 
+def test_a_cpu_tensor_has_no_stream(monkeypatch):
+    """A launch whose operands nobody else has checked ends here, not on a stream with host pointers."""
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda index: 0, raising=False)
+    with pytest.raises(ValueError, match="cpu"):
+        _lib.stream_of(torch.zeros(2))
+
+
 @pytest.mark.parametrize("targets", [7, 9, 12])
 @pytest.mark.parametrize("grad", [True, False])
 def test_head_refuses_a_target_of_another_length_than_the_hidden_states(launches, targets, grad):
