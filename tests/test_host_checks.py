@@ -43,6 +43,23 @@ def test_head_refuses_a_target_of_another_length_than_the_hidden_states(launches
     assert [name for name, _ in launches] == ["soup_lmhead_ce", "soup_lmhead_finish", "soup_lmhead_totals"]
 
 
+def test_head_gradient_of_several_losses_is_refused(launches):
+    """A divisor of several elements makes a loss of several; its gradient is no single factor."""
+    def loss_of(divisor):
+        hidden = torch.randn(1, 8, 64).half().requires_grad_()
+        return L.fused_head_loss(hidden, torch.randn(300, 64).half(), None, num_items_in_batch=divisor,
+                                 target=torch.zeros(1, 8, dtype=torch.int64))[0]
+
+    several = loss_of(torch.tensor([2.0, 4.0]))
+    assert several.shape == (2,)
+    with pytest.raises(RuntimeError, match="one loss"):
+        several.sum().backward()
+    assert "soup_lmhead_backward" not in [name for name, _ in launches]
+    for divisor in (None, 3, torch.tensor([2.0]), torch.tensor(2.0)):
+        loss_of(divisor).sum().backward()
+    assert [name for name, _ in launches].count("soup_lmhead_backward") == 4
+
+
 class _Projection:
     def __init__(self, out_features, weight):
         self.out_features, self.group, self._weight = out_features, self, weight
