@@ -108,6 +108,7 @@ struct AttnArgs {
   float* lse;            // [hq, n]
   int n, segments, hq, group;
   float scale_log2;      // softmax scale * log2(e)
+  float scale_far;       // the power of two at or above it (softmax_tile)
   int* status;
 };
 
@@ -124,18 +125,39 @@ struct __align__(1024) FwdSmem {
 template <int NT>
 constexpr int kFwdThreads = NT * 128 + 64;     // softmax warpgroups, then the TMA warp and the MMA warp
 
-// One row of a score tile: its exponentials against the (possibly moved) reference m, as fp16 over
-// the score columns, and the row's sum. msl is m * scale_log2, rounded once and used everywhere, so
-// that its rounding cancels between P, the sum and the log-sum-exp.
+// What a row's exponentials are taken against: exp2(x * sl - msl), msl being the row's maximum so far
+// times sl, rounded once and used everywhere, so that its rounding cancels between P, the sum and the
+// log-sum-exp. sl is the softmax scale (times log2 e), except that from kFarScore on that rounding is more
+// than 2^3, for which P's fp16 range has no room, and scores that differ at all differ by 2^4: there a power
+// of two takes its place, whose products are exact, and only the largest score has weight either way.
+// (It costs 119.3 against 116.5 us for 9215 tokens in 4 segments with two heads per CTA, 130.8 against 126.3
+// with one, 11.4 against 11.3 for 1280 in 5; subtracting the maximum from every score 118.1, 135.4 and 11.6.)
+// A row whose scores so far are all -inf has the finite maximum kLowest: they weigh nothing.
+constexpr float kFarScore = 268435456.f;   // 2^28
+constexpr float kLowest = -1e30f;          // below any product of 128 finite fp16 pairs
+struct RowRef {
+  float sl, msl;
+  __device__ __forceinline__ void set(float top, float scale, float scale_far) {
+    sl = scale;
+    msl = __fmul_rn(top, scale);
+    if (fabsf(msl) >= kFarScore) {
+      sl = scale_far;
+      msl = top * scale_far;
+    }
+  }
+};
+
+// One row of a score tile: its exponentials, as fp16 over the score columns, against the (possibly moved)
+// reference, and the row's sum l.
 template <bool DIAG>
 __device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, int limit, bool first,
-                                             float sl, float& m, float& msl, float& l) {
+                                             float scale, float scale_far, RowRef& ref, float& l) {
   uint32_t x[4][32];
 #pragma unroll
   for (int c = 0; c < 4; ++c) tmem_ld_32x32(s_addr + c * 32, x[c]);
 #pragma unroll
   for (int c = 0; c < 4; ++c) tmem_ld_wait_on(x[c]);
-  float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  float mx[4] = {kLowest, kLowest, kLowest, kLowest};
 #pragma unroll
   for (int c = 0; c < 4; ++c)
 #pragma unroll
@@ -145,17 +167,15 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, i
     }
   const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
   if (first) {
-    m = top;
-    msl = m * sl;
+    ref.set(top, scale, scale_far);
   } else {
-    const bool grow = (top - m) * sl > 0.f;
+    const bool grow = __fmul_rn(top, ref.sl) > ref.msl;
     if (__any_sync(0xffffffffu, grow)) {
       float f = 1.f;
-      if (grow) {
-        const float to = top * sl;
-        f = exp2f(msl - to);
-        m = top;
-        msl = to;
+      if (grow) {   // from one reference, as it was used, to the next; a far one is left behind by 2^4 at least
+        const float old = fabsf(ref.msl) < kFarScore ? ref.msl : -INFINITY;
+        ref.set(top, scale, scale_far);
+        f = exp2f(fabsf(ref.msl) < kFarScore ? old - ref.msl : -fmaf(top, scale, -old));
       }
       l *= f;
 #pragma unroll 1
@@ -176,8 +196,8 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, i
     uint32_t packed[16];
 #pragma unroll
     for (int j = 0; j < 32; j += 2) {
-      const float p0 = exp2f(fmaf(__uint_as_float(x[c][j]), sl, -msl));
-      const float p1 = exp2f(fmaf(__uint_as_float(x[c][j + 1]), sl, -msl));
+      const float p0 = exp2f(fmaf(__uint_as_float(x[c][j]), ref.sl, -ref.msl));
+      const float p1 = exp2f(fmaf(__uint_as_float(x[c][j + 1]), ref.sl, -ref.msl));
       s[j & 2] += p0;                      // the sum of exponentials, from the values before rounding
       s[(j & 2) + 1] += p1;
       __half2 hh = __floats2half2_rn(p0, p1);
@@ -308,16 +328,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int q_idx = q0 + r;
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     const uint32_t s_addr = lane_base + t * 128, o_addr = lane_base + (NT + t) * 128;
-    const float sl = a.scale_log2;
-    float m = -INFINITY, msl = 0.f, l = 0.f;
+    RowRef ref = {};
+    float l = 0.f;
     bool ok = true;
     for (int i = 0; i < n_kv; ++i) {
       ok = __all_sync(0xffffffffu, mbar_wait(&s.s_full[t], i & 1, abort_flag, a.status, 48));
       if (!ok) break;
       tc_fence_after_sync();
       // only the last tile of the walk, the one on the diagonal, hides columns from a row
-      if (i + 1 < n_kv) softmax_tile<false>(s_addr, o_addr, 0, i == 0, sl, m, msl, l);
-      else softmax_tile<true>(s_addr, o_addr, r, i == 0, sl, m, msl, l);
+      if (i + 1 < n_kv) softmax_tile<false>(s_addr, o_addr, 0, i == 0, a.scale_log2, a.scale_far, ref, l);
+      else softmax_tile<true>(s_addr, o_addr, r, i == 0, a.scale_log2, a.scale_far, ref, l);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&s.p_full[t]);
@@ -348,7 +368,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           }
         }
       }
-      if (valid) a.lse[(size_t)h * a.n + q_idx] = (msl + log2f(l)) * kLn2;
+      if (valid) a.lse[(size_t)h * a.n + q_idx] = (ref.msl * (ref.sl == a.scale_log2 ? 1.f : a.scale_log2 / ref.sl) + log2f(l)) * kLn2;
       tc_fence_before_sync();
     }
   }
@@ -830,6 +850,7 @@ extern "C" int soup_attn_fwd(const void* q, const void* k, const void* v, const 
   a.hq = (int)hq;
   a.group = (int)(hq / hk);
   a.scale_log2 = scale * kLog2e;
+  a.scale_far = exp2f(ceilf(log2f(a.scale_log2)));
   a.status = rowpipe::status_word();
   const int64_t ctas = tile_slots(n_tokens, n_segments) * (hq / heads);
   if (ctas > INT32_MAX) SOUP_FAIL(SOUP_ERR_ARG, "attn_fwd: too many tokens, segments or heads");

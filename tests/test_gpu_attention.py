@@ -18,10 +18,9 @@ def _cu(lens):
     return torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32)
 
 
-def _run(q, k, v, cu, grad, scale=None):
-    """(out, lse, dq, dk, dv) of the kernels on [N, h, 128] fp16 views (any row pitch)."""
+def _forward(q, k, v, cu, scale=None):
+    """(out, lse) of the forward kernel on [N, h, 128] fp16 views (any row pitch)."""
     from claudemaxing_b200 import _lib
-    from claudemaxing_b200.attention import attention_gradients
 
     n, hq, d = q.shape
     scale = d ** -0.5 if scale is None else scale
@@ -31,6 +30,18 @@ def _run(q, k, v, cu, grad, scale=None):
     _lib.call("soup_attn_fwd", _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(cu), _lib.ptr(out),
               _lib.ptr(lse), n, cu.numel() - 1, hq, k.shape[1], d, q.stride(0), k.stride(0),
               v.stride(0), float(scale), _lib.stream_of(q))
+    _lib.check_device_status()
+    return out, lse
+
+
+def _run(q, k, v, cu, grad, scale=None):
+    """(out, lse, dq, dk, dv) of the kernels on [N, h, 128] fp16 views (any row pitch)."""
+    from claudemaxing_b200 import _lib
+    from claudemaxing_b200.attention import attention_gradients
+
+    out, lse = _forward(q, k, v, cu, scale)
+    scale = q.shape[2] ** -0.5 if scale is None else scale
+    cu = cu.to(DEV)
     dq, dk, dv = attention_gradients(q, k, v, out, lse, grad, cu, scale)
     _lib.check_device_status()
     return out, lse, dq, dk, dv
@@ -107,6 +118,52 @@ def test_attention_forward_when_the_row_maximum_keeps_growing(hq, hk, lens):
     for name, got, exact in zip(("out", "dq", "dk", "dv"), (out, dq, dk, dv), want):
         assert rel_norm(got.float().cpu(), exact.float()) < 2e-3, name
     assert (lse.double().cpu() - want_lse).abs().max() < 2e-3
+
+
+@pytest.mark.parametrize("hq,hk,lens", [(4, 2, [700, 130]), (12, 2, [4100, 520])])
+@pytest.mark.parametrize("case", ["far", "masked", "mixed"])
+def test_attention_forward_at_scores_far_from_zero_and_at_minus_infinity(hq, hk, lens, case):
+    """One and two heads per CTA. "far": scores around 1e8, where every row attends to one key; "mixed":
+    every other row's are small, so a warp holds both kinds; "masked": keys whose scores are -inf, a
+    whole key tile and two keys of the next, in front of finite ones. Scores are exact to fp32's 2^-24 of
+    products of 1e9, far under the gap of the two largest (asserted), so the far rows give the value of one
+    key, and the log-sum-exp is that score."""
+    from oracle import attention as oat
+
+    gen = torch.Generator().manual_seed(8)
+    n, d = sum(lens), 128
+    q, k, v = (torch.randn(n, h, d, generator=gen) for h in (hq, hk, hk))
+    rows = torch.arange(n)
+    far = rows >= 0 if case == "far" else rows % 2 == 0 if case == "mixed" else rows < 0
+    q[far] *= 8000
+    if case != "masked":
+        k *= 8000 if case == "far" else 4000
+        q[~far] /= 4000
+    else:
+        q[..., 0] = q[..., 0].abs() + 0.1
+        k[:130, :, 0] = float("-inf")
+    q, k, v = q.half(), k.half(), v.half()
+    cu = _cu(lens)
+    q_d, k_d, v_d = q.to(DEV), k.to(DEV), v.to(DEV)
+    out, lse = _forward(q_d, k_d, v_d, cu)
+    want, want_lse = oat.segment_attention(q, k, v, cu)
+    if case == "masked":      # the first 130 rows see nothing else
+        assert torch.isfinite(out[130:]).all()
+        assert rel_norm(out[130:].float().cpu(), want[130:].float()) < 2e-3
+        assert (lse[:, 130:].double().cpu() - want_lse[:, 130:]).abs().max() < 2e-3
+        return
+    gap = torch.full((hq, n), float("inf"), dtype=torch.float64)
+    for b, e in zip(cu.tolist(), cu.tolist()[1:]):
+        z = torch.einsum("qhd,khd->hqk", q_d[b:e].double(), k_d[b:e].double().repeat_interleave(hq // hk, 1))
+        z.masked_fill_(~torch.ones(e - b, e - b, dtype=torch.bool, device=DEV).tril(), float("-inf"))
+        two = z.topk(2, -1).values.cpu()
+        gap[:, b:e] = two[..., 0] - two[..., 1]
+    clear = (gap > 2e4) | ~far          # of ten thousand rows one has two keys that close
+    assert clear.double().mean() > 0.99
+    close = clear.t()[..., None]
+    assert rel_norm((out.float().cpu() * close), (want.float() * close)) < 2e-3
+    error = (lse.double().cpu() - want_lse).abs()
+    assert (error <= 2e-3 + 2.0 ** -16 * want_lse.abs()).all()
 
 
 def test_attention_kernels_read_q_k_v_as_column_blocks_and_leave_other_rows_alone():
