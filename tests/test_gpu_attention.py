@@ -66,7 +66,8 @@ def test_attention_kernels_on_the_reference_kernels_golden_vectors(tag):
     (6, 1, [1000, 3]),
     (4, 2, [40] * 100 + [3]),        # more than 64 segments: the plain tile order
     (2, 1, [2500]),                  # twenty key tiles: many turns of every barrier
-    (12, 2, [2500, 700, 1]),         # long enough for two heads per forward CTA
+    (12, 2, [2500, 700, 1]),         # long walks, one head per forward CTA
+    (12, 2, [3500, 700, 1]),         # long enough for two
     (3, 1, [129, 255]),              # an odd group: one head per CTA whatever the size
 ])
 def test_attention_kernels_against_fp32_with_the_fp16_sdpa_error_as_the_bar(hq, hk, lens):
@@ -97,7 +98,7 @@ def test_attention_kernels_against_fp32_with_the_fp16_sdpa_error_as_the_bar(hq, 
     assert (lse.double().cpu() - want_lse).abs().max() < 2e-3
 
 
-@pytest.mark.parametrize("hq,hk,lens", [(4, 2, [700, 130]), (12, 2, [2600, 520])])
+@pytest.mark.parametrize("hq,hk,lens", [(4, 2, [700, 130]), (12, 2, [2600, 520]), (12, 2, [4100, 520])])
 def test_attention_forward_when_the_row_maximum_keeps_growing(hq, hk, lens):
     """Scores that grow along the keys, then fall: every row's accumulator is rescaled, some rows of a
     warp earlier than others. One and two heads per CTA. P is rounded to fp16 relative to the row's
@@ -123,11 +124,11 @@ def test_attention_forward_when_the_row_maximum_keeps_growing(hq, hk, lens):
 @pytest.mark.parametrize("hq,hk,lens", [(4, 2, [700, 130]), (12, 2, [4100, 520])])
 @pytest.mark.parametrize("case", ["far", "masked", "mixed"])
 def test_attention_forward_at_scores_far_from_zero_and_at_minus_infinity(hq, hk, lens, case):
-    """One and two heads per CTA. "far": scores around 1e8, where every row attends to one key; "mixed":
+    """One and two heads per CTA. "far": scores up to 1e9, where every row attends to one key; "mixed":
     every other row's are small, so a warp holds both kinds; "masked": keys whose scores are -inf, a
-    whole key tile and two keys of the next, in front of finite ones. Scores are exact to fp32's 2^-24 of
-    products of 1e9, far under the gap of the two largest (asserted), so the far rows give the value of one
-    key, and the log-sum-exp is that score."""
+    whole key tile and two keys of the next, in front of finite ones. An fp32 sum of 128 products is
+    within 2^-17 of their magnitudes' sum, about twice the largest score here: the log-sum-exp's bound,
+    and far under the gap of the two largest scores (asserted), so that a far row is one key's value."""
     from oracle import attention as oat
 
     gen = torch.Generator().manual_seed(8)
@@ -135,14 +136,14 @@ def test_attention_forward_at_scores_far_from_zero_and_at_minus_infinity(hq, hk,
     q, k, v = (torch.randn(n, h, d, generator=gen) for h in (hq, hk, hk))
     rows = torch.arange(n)
     far = rows >= 0 if case == "far" else rows % 2 == 0 if case == "mixed" else rows < 0
-    q[far] *= 8000
+    q[far] *= 12000
     if case != "masked":
-        k *= 8000 if case == "far" else 4000
-        q[~far] /= 4000
+        k *= 12000
+        q[~far] /= 12000
     else:
         q[..., 0] = q[..., 0].abs() + 0.1
         k[:130, :, 0] = float("-inf")
-    q, k, v = q.half(), k.half(), v.half()
+    q, k, v = q.clamp(-6e4, 6e4).half(), (k if case == "masked" else k.clamp(-6e4, 6e4)).half(), v.half()
     cu = _cu(lens)
     q_d, k_d, v_d = q.to(DEV), k.to(DEV), v.to(DEV)
     out, lse = _forward(q_d, k_d, v_d, cu)
@@ -158,10 +159,10 @@ def test_attention_forward_at_scores_far_from_zero_and_at_minus_infinity(hq, hk,
         z.masked_fill_(~torch.ones(e - b, e - b, dtype=torch.bool, device=DEV).tril(), float("-inf"))
         two = z.topk(2, -1).values.cpu()
         gap[:, b:e] = two[..., 0] - two[..., 1]
-    clear = (gap > 2e4) | ~far          # of ten thousand rows one has two keys that close
+    clear = (gap > 1e5) | ~far          # of ten thousand rows one has two keys that close
     assert clear.double().mean() > 0.99
-    close = clear.t()[..., None]
-    assert rel_norm((out.float().cpu() * close), (want.float() * close)) < 2e-3
+    keep = clear.t()[..., None]
+    assert rel_norm(out.float().cpu() * keep, want.float() * keep) < 2e-3
     error = (lse.double().cpu() - want_lse).abs()
     assert (error <= 2e-3 + 2.0 ** -16 * want_lse.abs()).all()
 
