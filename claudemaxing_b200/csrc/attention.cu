@@ -6,7 +6,7 @@
 // and head: S = Q K^T into 128 columns of tensor memory; the head's softmax warpgroup (thread =
 // query row) reads its row into registers, takes P = exp2(scale S - m) and writes it back as fp16
 // over S's columns; O += P V with P as the tensor-memory operand. m is the row's maximum so far: O and
-// the sum are rescaled when it grows. (Letting it lag by up to 2^8 saves those round trips, 101 against
+// the sum are rescaled when it grows. (Letting it lag by up to 2^8 saved those round trips, 101 against
 // 117 us for 9215 tokens in 4 segments, but the largest P is then no longer 1, which fp16 holds exactly,
 // and the output's error against float64 rises by up to a tenth on peaked rows.) The score product of
 // the next tile is issued right behind O += P V of this one; the commit that announces it also says that
@@ -799,14 +799,16 @@ namespace {
 inline int64_t tile_slots(int64_t n_tokens, int64_t n_segments) { return (n_tokens + kBQ - 1) / kBQ + n_segments; }
 
 // Heads of a forward CTA. Two per CTA (both heads use every key and value tile) pay once an SM has
-// more than about eight (tile, key tile) steps to walk, estimated from the mean segment; below, twice
-// as many CTAs of half the work finish earlier (12 query heads, 2 key heads, one and two heads: 1280
-// tokens in 5 segments 10.6 and 13.2 us, 4607 in 16 22.8 and 24.2, 4604 in 8 27.4 and 27.0, 4607 in 4
-// 41.0 and 39.6, 9215 in 4 110.9 and 101.2). The two heads share one key/value head.
+// more than about fourteen (tile, key tile) steps to walk, estimated from the mean segment; below, twice
+// as many CTAs of half the work finish earlier. One and two heads, in us, by steps per SM: 12 query and 2
+// key heads 1: 11.4 and 13.8 (1280 tokens in 5 segments), 5: 24.1 and 25.2 (4607 in 16), 8: 28.7 and 28.0
+// (4604 in 8), 11: 42.2 and 46.7 (2048 in 1), 15: 46.5 and 47.2 (4607 in 4), 29: 72.9 and 69.9 (9212 in 8),
+// 55: 130.6 and 119.4 (9215 in 4); 32 and 8 heads 13: 51.7 and 54.8 (4607 in 16), 16: 36.3 and 33.3 (2048 in
+// 2), 39: 98.2 and 92.3 (4607 in 4). The two heads share one key/value head.
 inline int forward_heads_per_cta(int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk) {
   if ((hq / hk) % 2) return 1;
   const double tiles = (double)n_tokens / kBQ, walk = (tiles / (double)n_segments + 1.0) / 2.0;
-  return tiles * walk * (double)hq > 8.0 * sm_count() ? 2 : 1;
+  return tiles * walk * (double)hq > 14.0 * sm_count() ? 2 : 1;
 }
 
 }  // namespace
