@@ -1139,7 +1139,10 @@ struct Plan {
 // chunks.
 //  - First chunk: the fewest column tiles whose rt * ct units fill whole waves of CTA pairs to 97 %
 //    or more, at least kFirstTiles of them (its gradient launch has four 64-column K blocks per
-//    tile to split).
+//    tile to split) and at most one for every two pairs: its probabilities are rounded to bf16 twice,
+//    and with one row tile a whole wave of it was 18944 columns (the probability part of dHidden at up
+//    to 256 rows, 32000 columns and flat logits: 9.40e-4 from float64, 8.93e-4 with half of that; the
+//    later chunks take as many waves either way).
 //  - Rows per block: 2048 for a full-width chunk; more when the shard is narrow (a rank of a
 //    vocabulary-parallel group), so that a launch still has a dozen tiles per CTA pair and the
 //    probability buffer stays around 600 MB. Whole multiples of 2048, at most 8192.
@@ -1167,6 +1170,7 @@ inline Plan make_plan(int64_t n, int64_t v_shard, int sms, int ct_override) {
       const int ct = w * pairs / rt;
       if (rt * ct * 100 >= 97 * w * pairs) { p.ct_first = ct; break; }
     }
+    if (p.ct_first > pairs / 2) p.ct_first = pairs / 2;
     p.ct = (int)(kChunkBytes / ((int64_t)p.row_block * kBN * 2));
     if (waves && p.ct > waves * pairs / 2) p.ct = waves * pairs / 2;
     // the later chunks of equal size

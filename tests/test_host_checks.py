@@ -1,5 +1,7 @@
 """What the Python side refuses before a launch reads or writes anything, on CPU tensors with the
-launches replaced by a recorder."""
+launches replaced by a recorder, and the plans the library makes on the host."""
+
+import ctypes
 
 import pytest
 import torch
@@ -58,6 +60,22 @@ def test_head_gradient_of_several_losses_is_refused(launches):
     for divisor in (None, 3, torch.tensor([2.0]), torch.tensor(2.0)):
         loss_of(divisor).sum().backward()
     assert [name for name, _ in launches].count("soup_lmhead_backward") == 4
+
+
+def _head_plan(rows, columns, chunk_tiles=0):
+    """(rows per block, column tiles of the first chunk, of a later one); without a device the library
+    plans for 148 SMs."""
+    out = [ctypes.c_int64() for _ in range(3)]
+    _lib.lib().soup_lmhead_plan(rows, columns, chunk_tiles, *(ctypes.byref(x) for x in out))
+    return tuple(x.value for x in out)
+
+
+@pytest.mark.parametrize("columns", [300, 32000, 50257, 151936])
+def test_head_rounds_no_more_of_the_vocabulary_twice_than_37_tiles(columns):
+    """The first chunk's probabilities are rounded against their tile's maximum and again after the merge."""
+    for rows in (1, 24, 128, 256, 257, 512, 600, 1168, 2048, 4096, 8192):
+        first = _head_plan(rows, columns)[1]
+        assert 1 <= first <= 37, rows
 
 
 class _Projection:
