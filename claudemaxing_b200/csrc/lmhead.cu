@@ -1143,10 +1143,12 @@ struct Plan {
 //    and with one row tile a whole wave of it was 18944 columns (the probability part of dHidden at up
 //    to 256 rows, 32000 columns and flat logits: 9.40e-4 from float64, 8.93e-4 with half of that; the
 //    later chunks take as many waves either way).
-//  - Rows per block: 2048 for a full-width chunk; more when the shard is narrow (a rank of a
+//  - Rows per block: 4096 for a full-width chunk; more when the shard is narrow (a rank of a
 //    vocabulary-parallel group), so that a launch still has a dozen tiles per CTA pair and the
-//    probability buffer stays around 600 MB. Whole multiples of 2048, at most 8192.
+//    probability buffer stays around 600 MB. Whole multiples of 2048, at most 8192: twice the
+//    tiles of kRowWaves waves (or of SOUP_LMHEAD_WAVES) at eight row tiles.
 constexpr int kFirstTiles = 16;
+constexpr int kRowWaves = 8;
 constexpr int64_t kChunkBytes = 640ll << 20;
 inline Plan make_plan(int64_t n, int64_t v_shard, int sms, int ct_override) {
   Plan p;
@@ -1156,7 +1158,8 @@ inline Plan make_plan(int64_t n, int64_t v_shard, int sms, int ct_override) {
   if (const char* e = getenv("SOUP_LMHEAD_WAVES")) { const int v = atoi(e); if (v >= 1 && v <= 64) waves = v; }
   int64_t rb = 2048;
   if (ct_override <= 0) {
-    rb = 2048 * (int64_t)(592 / (total_ct < 296 ? (total_ct > 0 ? total_ct : 1) : 296));
+    const int wide = (waves ? waves : kRowWaves) * pairs / 2;   // column tiles
+    rb = 2048 * (int64_t)(2 * wide / (total_ct < wide ? (total_ct > 0 ? total_ct : 1) : wide));
     if (rb < 2048) rb = 2048;
     if (rb > 8192) rb = 8192;
   }

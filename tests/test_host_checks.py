@@ -78,6 +78,19 @@ def test_head_rounds_no_more_of_the_vocabulary_twice_than_37_tiles(columns):
         assert 1 <= first <= 37, rows
 
 
+def test_head_row_block_follows_the_waves_a_chunk_may_have(monkeypatch):
+    """Rows per block: twice the column tiles of so many waves of 74 pairs at eight row tiles, over the
+    shard's tiles (594 at full width, 75 of eight ranks), in multiples of 2048 up to 8192."""
+    def blocks():
+        return [_head_plan(65536, columns)[0] for columns in (151936, 37984, 18992)]
+
+    assert blocks() == [4096, 6144, 8192]
+    monkeypatch.setenv("SOUP_LMHEAD_WAVES", "4")
+    assert blocks() == [4096, 4096, 6144]
+    monkeypatch.setenv("SOUP_LMHEAD_WAVES", "16")
+    assert blocks() == [4096, 8192, 8192]
+
+
 class _Projection:
     def __init__(self, out_features, weight):
         self.out_features, self.group, self._weight = out_features, self, weight
