@@ -48,6 +48,7 @@ SIGNATURES = {
     "soup_dropout_pack2": [_P] * 7 + [_L, _F, _F, _I, _P],
     "soup_dropout_unpack2": [_P] * 8 + [_L, _F, _F, _P],
     "soup_lmhead_workspace_bytes": [_L, _L, _L, _L],
+    "soup_lmhead_forward_workspace_bytes": [_L, _L, _L, _L],
     "soup_lmhead_ce": [_P] * 13 + [_L] * 6 + [_I, _P],
     "soup_lmhead_set_timing": [_P],
     "soup_lmhead_plan": [_L, _L, _L, _P, _P, _P],
@@ -63,8 +64,8 @@ SIGNATURES = {
     "soup_nf4_linear_fwd": [_P, _P, _I, _P, _L, _L, _I, _I, _I, _P, _L, _P],
     "soup_nf4_linear_dx": [_P, _I, _P, _P, _I, _L, _L, _I, _I, _I, _P, _L, _P],
 }
-_RESTYPE = {"soup_lmhead_workspace_bytes": _L, "soup_rmsnorm_bwd_partials": _L,
-            "soup_nf4_gemm_workspace_bytes": _L}
+_RESTYPE = {"soup_lmhead_workspace_bytes": _L, "soup_lmhead_forward_workspace_bytes": _L,
+            "soup_rmsnorm_bwd_partials": _L, "soup_nf4_gemm_workspace_bytes": _L}
 SIGNATURES["soup_rmsnorm_bwd_partials"] = [_L, _L]
 
 class Nf4Item(ctypes.Structure):

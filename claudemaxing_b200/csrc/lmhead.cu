@@ -1176,9 +1176,9 @@ inline Plan make_plan(int64_t n, int64_t v_shard, int sms, int ct_override) {
     if (p.ct_first > pairs / 2) p.ct_first = pairs / 2;
     p.ct = (int)(kChunkBytes / ((int64_t)p.row_block * kBN * 2));
     if (waves && p.ct > waves * pairs / 2) p.ct = waves * pairs / 2;
-    // the later chunks of equal size
+    // the later chunks of equal size, and no larger than what there is
     const int rest = total_ct - p.ct_first;
-    if (rest > 0 && p.ct < rest) {
+    if (rest > 0) {
       const int chunks = (rest + p.ct - 1) / p.ct;
       p.ct = (rest + chunks - 1) / chunks;
     }
@@ -1191,26 +1191,25 @@ inline Plan make_plan(int64_t n, int64_t v_shard, int sms, int ct_override) {
 }
 
 struct Workspace {
-  __nv_bfloat16* p_buf;   // [row_block, ct * 256]
-  float4* tile_stats;     // [row_block, ct]
+  int* status;            // first: found without knowing whether the call wants the gradient
   float* mult;            // [row_block]
-  int* status;
+  float4* tile_stats;     // [row_block, ct]
+  __nv_bfloat16* p_buf;   // [row_block, ct * 256], with the gradient only
   int64_t bytes;
 };
 
-inline Workspace carve_workspace(void* base, const Plan& p) {
+inline Workspace carve_workspace(void* base, const Plan& p, bool want_grad) {
   Workspace w;
   uint8_t* b = reinterpret_cast<uint8_t*>(base);
   int64_t off = 0;
-  const int64_t ld_p = (int64_t)p.ct * kBN;
-  w.p_buf = reinterpret_cast<__nv_bfloat16*>(b + off);
-  off += round_up((int64_t)p.row_block * ld_p * 2, 1024);
-  w.tile_stats = reinterpret_cast<float4*>(b + off);
-  off += round_up((int64_t)p.row_block * p.ct * 16, 1024);
-  w.mult = reinterpret_cast<float*>(b + off);
-  off += round_up((int64_t)p.row_block * 4, 1024);
   w.status = reinterpret_cast<int*>(b + off);
   off += 1024;
+  w.mult = reinterpret_cast<float*>(b + off);
+  off += round_up((int64_t)p.row_block * 4, 1024);
+  w.tile_stats = reinterpret_cast<float4*>(b + off);
+  off += round_up((int64_t)p.row_block * p.ct * 16, 1024);
+  w.p_buf = want_grad ? reinterpret_cast<__nv_bfloat16*>(b + off) : nullptr;
+  if (want_grad) off += round_up((int64_t)p.row_block * p.ct * kBN * 2, 1024);
   w.bytes = off;
   return w;
 }
@@ -1337,8 +1336,14 @@ extern "C" int64_t soup_lmhead_workspace_bytes(int64_t n, int64_t h, int64_t v_s
                                                int64_t chunk_tiles) {
   using namespace soup;
   (void)h;
-  const Plan p = make_plan(n, v_shard, sm_count(), (int)chunk_tiles);
-  return carve_workspace(nullptr, p).bytes;
+  return carve_workspace(nullptr, make_plan(n, v_shard, sm_count(), (int)chunk_tiles), true).bytes;
+}
+
+extern "C" int64_t soup_lmhead_forward_workspace_bytes(int64_t n, int64_t h, int64_t v_shard,
+                                                       int64_t chunk_tiles) {
+  using namespace soup;
+  (void)h;
+  return carve_workspace(nullptr, make_plan(n, v_shard, sm_count(), (int)chunk_tiles), false).bytes;
 }
 
 extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void* weight_bf16,
@@ -1367,7 +1372,7 @@ extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void
   const int max_pairs = sms / 2;
   if (max_pairs < 1) SOUP_FAIL(SOUP_ERR_DEVICE, "lmhead_ce: needs at least two SMs");
   const Plan plan = make_plan(n, v_shard, sms, (int)chunk_tiles);
-  const Workspace ws = carve_workspace(workspace, plan);
+  const Workspace ws = carve_workspace(workspace, plan, want_grad != 0);
   if (workspace_bytes < ws.bytes)
     SOUP_FAIL(SOUP_ERR_ARG, "lmhead_ce: workspace too small (%lld < %lld)",
               (long long)workspace_bytes, (long long)ws.bytes);
@@ -1381,12 +1386,13 @@ extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void
       umma::encode_map_2d_16bit(&map_w_k, weight, (uint64_t)v_shard, (uint64_t)h, (uint64_t)h, kBN / 2, kBK, false) ||
       (want_grad &&
        (umma::encode_map_2d_16bit(&map_w_mn, weight_bf16, (uint64_t)v_shard, (uint64_t)h, (uint64_t)h, kBK, 64, true) ||
-        umma::encode_map_2d_f32(&map_dh, dh, (uint64_t)n, (uint64_t)h, (uint64_t)h, 32, 32))) ||
-      umma::encode_map_2d_16bit(&map_p_ld, ws.p_buf, (uint64_t)plan.row_block, (uint64_t)ld_p,
-                                (uint64_t)ld_p, kBM, kBK, true) ||
-      umma::encode_map_2d_16bit(&map_p_st, ws.p_buf, (uint64_t)plan.row_block, (uint64_t)ld_p,
-                                (uint64_t)ld_p, 32, 64, true))
+        umma::encode_map_2d_f32(&map_dh, dh, (uint64_t)n, (uint64_t)h, (uint64_t)h, 32, 32) ||
+        umma::encode_map_2d_16bit(&map_p_ld, ws.p_buf, (uint64_t)plan.row_block, (uint64_t)ld_p,
+                                  (uint64_t)ld_p, kBM, kBK, true) ||
+        umma::encode_map_2d_16bit(&map_p_st, ws.p_buf, (uint64_t)plan.row_block, (uint64_t)ld_p,
+                                  (uint64_t)ld_p, 32, 64, true))))
     SOUP_FAIL(SOUP_ERR_DEVICE, "lmhead_ce: cuTensorMapEncodeTiled failed");
+  if (!want_grad) map_p_st = map_h;   // nothing is stored through it
 
   int* sticky = rowpipe::status_word();
   const int64_t dh_vec = want_grad ? n * h / 4 : 0;   // h is a multiple of 8
@@ -1499,7 +1505,7 @@ extern "C" int soup_lmhead_status(const void* workspace, int64_t n, int64_t v_sh
                                   int64_t chunk_tiles, int* host_status, void* stream) {
   using namespace soup;
   const Plan plan = make_plan(n, v_shard, sm_count(), (int)chunk_tiles);
-  const Workspace ws = carve_workspace(const_cast<void*>(workspace), plan);
+  const Workspace ws = carve_workspace(const_cast<void*>(workspace), plan, false);
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (cudaMemcpyAsync(host_status, ws.status, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess)

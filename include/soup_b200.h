@@ -343,10 +343,12 @@ int soup_nf4_linear_dx(const soup_nf4_gemm_item* items, int n_items, const float
  * weight_bf16: the same weight rounded to bf16 (needed when want_grad != 0; the gradient GEMM
  * multiplies bf16 probabilities with it, and the tensor core takes one format for both operands).
  * col_offset = global index of the shard's first column. chunk_tiles = 256-column tiles per
- * chunk (0 = library default). workspace: soup_lmhead_workspace_bytes() bytes, 16-byte aligned.
+ * chunk (0 = library default). workspace: soup_lmhead_workspace_bytes() bytes, 16-byte aligned;
+ * with want_grad == 0 soup_lmhead_forward_workspace_bytes() are enough (no probabilities are kept).
  * With SOUP_LMHEAD_DETERMINISTIC=1 in the environment the gradient GEMM does not split its
  * reduction dimension and dh is bit-reproducible (at a lower SM occupancy). */
 int64_t soup_lmhead_workspace_bytes(int64_t n, int64_t h, int64_t v_shard, int64_t chunk_tiles);
+int64_t soup_lmhead_forward_workspace_bytes(int64_t n, int64_t h, int64_t v_shard, int64_t chunk_tiles);
 int soup_lmhead_ce(const void* hidden, const void* weight, const void* weight_bf16,
                    const int64_t* target, float* run_max, float* run_sum, float* run_dot, int* best,
                    float* best_val, float* label_logit, float* grad_ref, float* dh, void* workspace,

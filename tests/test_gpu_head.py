@@ -298,6 +298,26 @@ def test_gradient_split_over_all_pairs_at_the_edges_of_its_tiles(dims):
     check(*make(*dims, seed=31, drop=0.0 if dims[0] == 1 else 0.3))   # one unlabelled row: 0 / 0
 
 
+@pytest.mark.parametrize("dims", [(1, 64, 300), (257, 512, 19201), (600, 72, 40000)])
+def test_forward_pass_stays_inside_its_smaller_workspace(dims):
+    """The workspace of a forward-only pass, with a guard behind it: the terms are the training pass's
+    to the bit, and the guard is untouched."""
+    from claudemaxing_b200 import _lib
+    from claudemaxing_b200 import lm_head_loss as L
+
+    h, w, t = (x.to(DEV) for x in make(*dims, seed=35))
+    state, raw = L.head_partial(h, w, t)
+    nbytes = _lib.lib().soup_lmhead_forward_workspace_bytes(dims[0], dims[1], dims[2], 0)
+    buf = torch.full((nbytes + 65536,), 165, dtype=torch.uint8, device=DEV)
+    mine = L.HeadState(dims[0], DEV)
+    _lib.call("soup_lmhead_ce", _lib.ptr(h), _lib.ptr(w), None, _lib.ptr(t), *mine.pointers(), None, _lib.ptr(buf),
+              nbytes, dims[0], dims[1], dims[2], 0, 0, 0, _lib.stream_of(h))
+    _lib.check_device_status()
+    for a, b in zip(state.tensors()[:6], mine.tensors()[:6]):
+        assert torch.equal(a, b)
+    assert (buf[nbytes:] == 165).all()
+
+
 @pytest.mark.parametrize("divisor", [None, 77, 77.0, torch.tensor(77), torch.tensor(77.0),
                                      torch.tensor([77.0]), torch.tensor(77, dtype=torch.int32)])
 def test_totals_divide_by_every_kind_of_divisor(divisor):

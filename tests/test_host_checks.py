@@ -91,6 +91,26 @@ def test_head_row_block_follows_the_waves_a_chunk_may_have(monkeypatch):
     assert blocks() == [4096, 8192, 8192]
 
 
+@pytest.mark.parametrize("rows", [1, 128, 1168, 2048, 8192])
+def test_head_workspace_holds_no_more_probabilities_than_a_chunk_has(launches, rows):
+    """bf16 probabilities of the largest chunk with the gradient, none without; a call is handed the
+    workspace of its own kind."""
+    block, first, later = _head_plan(rows, 151936)
+    assert later == max(first, -(-(594 - first) // -(-(594 - first) // later)))   # equal chunks, none larger
+    lib = _lib.lib()
+    full = lib.soup_lmhead_workspace_bytes(rows, 64, 151936, 0)
+    forward = lib.soup_lmhead_forward_workspace_bytes(rows, 64, 151936, 0)
+    assert full - forward == -(-block * later * 512 // 1024) * 1024
+    assert forward <= block * (later * 16 + 4) + 4096
+    hidden, weight = torch.zeros(rows, 64).half(), torch.zeros(300, 64).half()
+    for grad in (True, False):
+        L.head_partial(hidden, weight, torch.zeros(rows, dtype=torch.int64), want_grad=grad,
+                       w_bf16=weight.bfloat16())
+        _, args = launches.pop()
+        wanted = lib.soup_lmhead_workspace_bytes if grad else lib.soup_lmhead_forward_workspace_bytes
+        assert args[13] == wanted(rows, 64, 300, 0)
+
+
 class _Projection:
     def __init__(self, out_features, weight):
         self.out_features, self.group, self._weight = out_features, self, weight
