@@ -345,12 +345,15 @@ template <int C> __device__ __forceinline__ int dt_sel(int rt) { return C >= 0 ?
 // One CTA per row (four rows of up to 256 columns), eight columns per thread, everything a row needs
 // requested at once: bound by memory when many rows are in flight, by one row's latency when few are.
 // The ring kernels below spend the latter on ring set-up, a serial walk of the row by one or two warps
-// and, in backward, on the weight's copy in shared memory; with fp32 rows this form is faster at every
-// row count (1536 columns, 10 B and 16 B an element: forward 7.6 -> 5.6 us at 1280 rows, 44.6 -> 41.2 at
-// 16384; backward with the residual 14.8 -> 8.5 and 87.6 -> 71.1 us, the latter 5.7 TB/s; 64 rows 5.4 ->
-// 1.8 and 7.7 -> 2.3). A 16-bit row is half the bytes for the same threads, and the ring wins once more
-// rows are waiting than fit (5.0 -> 4.3 us at 1280 rows, 6.3 -> 5.6 at 2560, but 7.4 -> 9.6 at 4608):
-// `row_kernel_covers`.
+// and, in backward, on the weight's copy in shared memory. With fp32 rows this form was the faster one at 1536
+// columns and every row count (10 B and 16 B an element: forward 7.4 -> 5.3 us at 1280 rows, 44.9 -> 41.8 at
+// 16384; backward with the residual 14.4 -> 7.6 and 87.6 -> 68.4; 64 rows 5.5 -> 1.9 and 8.1 -> 2.5), and from 8
+// to 4096 columns but for: the forward without the fp16 copy at 2048 to 3072 columns and more than 2000 rows,
+// 6 % faster to 10 % slower (2048 x 2300 7.9 -> 8.6, x 16384 48.5 -> 46.4; 3072 x 16384 68 -> 71), and the backward without
+// the residual at 65536 rows of 64 to 384 columns and 16384 of 2048, 4 to 7 % slower (384 columns 57.5 ->
+// 61.5). A 16-bit row is half the bytes for the same threads, and the ring wins once more rows are waiting
+// than fit: `row_kernel_covers`. The residual form keeps the 2048 columns it always took: wider rows are
+// three launches.
 // ------------------------------------------------------------------------------------------
 constexpr int kRowMaxThreads = 512;   // rows of up to 4096 columns
 
@@ -843,10 +846,15 @@ inline dim3 row_block(int64_t n_cols) {
 }
 inline unsigned row_grid(int64_t n_rows, dim3 block) { return (unsigned)((n_rows + block.y - 1) / block.y); }
 
-// fp32 rows always, 16-bit rows while at most two waves of their threads wait (see the kernels).
+// Whether the row kernel is the faster one (see there). fp32 rows: always. 16-bit rows: while at most two
+// waves of them wait, counted in threads, of which the kernel's registers leave 1152 on an SM (ring and row
+// kernel, in us: 1536 columns 4.9 -> 4.1 at 1280 rows but 5.1 -> 5.5 at 2000, 2048 columns 5.1 -> 4.6 at 1200 but
+// 5.8 -> 6.9 at 2300, 3584 columns 6.0 -> 7.6 at 1100, 768 columns 4.7 -> 4.4 at 3200 but 4.6 -> 5.6 at 4608).
+// Rows of one warp need no barrier and win up to three and a half (128 columns 7.0 -> 5.2 at 16384 rows).
 inline bool row_kernel_covers(int64_t n_rows, int64_t n_cols, int dtype) {
   if (n_cols > kRowMaxThreads * 8) return false;
-  return dtype == SOUP_F32 || n_rows * row_block(n_cols).x <= 2ll * sm_count() * 2048;
+  const unsigned threads = row_block(n_cols).x;
+  return dtype == SOUP_F32 || n_rows * threads <= 2ll * sm_count() * (threads == 32 ? 2048 : 1152);
 }
 
 }  // namespace
