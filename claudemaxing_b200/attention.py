@@ -26,6 +26,12 @@ OWN_FORWARD = os.environ.get("SOUP_ATTN_KERNEL", "1") != "0"
 OWN_BACKWARD = os.environ.get("SOUP_ATTN_BACKWARD", "1") != "0"
 
 
+def own_backward():
+    """Whether gradients come from this library's backward kernel. It adds into all three in any order;
+    under torch.use_deterministic_algorithms torch's does the work, which has a fixed order then."""
+    return OWN_BACKWARD and not torch.are_deterministic_algorithms_enabled()
+
+
 def attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, scale):
     """The fp32 gradients of the segment attention from this library's backward kernel
     (csrc/attention.cu) as one flat buffer: dq [n, hq, 128], dk [n, hk, 128], dv [n, hk, 128] one after
@@ -107,7 +113,7 @@ class SegmentAttention(torch.autograd.Function):
     """Causal attention inside the segments of a packed row on fp16 [tokens, heads, 128] tensors:
     forward and backward by this library's tcgen05 kernels (csrc/attention.cu). The forward also
     returns the row log-sum-exps in the layout torch's variable-length flash-attention backward
-    takes ([heads, tokens]), which `SOUP_ATTN_BACKWARD=0` uses instead of this library's."""
+    takes ([heads, tokens]), which stands in where `own_backward` says so."""
 
     @staticmethod
     def forward(ctx, q, k, v, cu_rows, longest, scale):
@@ -124,10 +130,11 @@ class SegmentAttention(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad):
         q, k, v, cu_rows, out, lse = ctx.saved_tensors
-        if OWN_BACKWARD:
+        if own_backward():
             # one rounding launch for all three: they are adjacent
             flat = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, ctx.scale).to(q.dtype)
             return (*gradient_parts(flat, q.shape[0], q.shape[1], k.shape[1], q.shape[2]), None, None, None)
+        _varlen()   # registers the operator
         rng_state = torch.empty(2, dtype=torch.uint64, device=q.device)   # no dropout: never read
         dq, dk, dv = torch.ops.torch_attn._varlen_attn_backward(
             grad.contiguous(), q, k, v, out, lse, cu_rows, cu_rows, ctx.longest, ctx.longest, True,

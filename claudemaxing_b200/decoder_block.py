@@ -512,7 +512,7 @@ def fused_block_forward(layer, hidden_states, attention_mask=None, position_ids=
     cos, sin = position_embeddings
     cu = kwargs["cu_seq_lens_q"]
     scale = layer.self_attn.scaling
-    if (plan.head_dim == 128 and attention_mod.OWN_FORWARD and attention_mod.OWN_BACKWARD
+    if (plan.head_dim == 128 and attention_mod.OWN_FORWARD and attention_mod.own_backward()
             and cu.dtype == torch.int32 and cu.is_cuda):
         attended = _QKVRope.apply(x, x16, branches[0], branches[2], cos.contiguous(), sin.contiguous(),
                                   plan, cu, plan.head_dim ** -0.5 if scale is None else scale)

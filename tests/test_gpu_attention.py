@@ -121,6 +121,31 @@ def test_attention_forward_when_the_row_maximum_keeps_growing(hq, hk, lens):
     assert (lse.double().cpu() - want_lse).abs().max() < 2e-3
 
 
+def test_attention_gradients_are_reproducible_when_torch_is_told_to_be():
+    """torch.use_deterministic_algorithms: no sums in any order; the gradients of several key tiles and
+    a group of heads come out the same twice, and within the two kernels' fp16 rounding of the others."""
+    from claudemaxing_b200.attention import SegmentAttention
+
+    gen = torch.Generator().manual_seed(6)
+    lens = [700, 333]
+    q, k, v = (torch.randn(sum(lens), h, 128, generator=gen).half().to(DEV).requires_grad_() for h in (12, 2, 2))
+    grad = torch.randn(q.shape, generator=gen).half().to(DEV)
+    cu = _cu(lens).to(DEV)
+
+    def gradients():
+        return torch.autograd.grad(SegmentAttention.apply(q, k, v, cu, max(lens), 128 ** -0.5), (q, k, v), grad)
+
+    own = gradients()
+    torch.use_deterministic_algorithms(True)
+    try:
+        first, second = gradients(), gradients()
+    finally:
+        torch.use_deterministic_algorithms(False)
+    for name, a, b, c in zip("qkv", first, second, own):
+        assert torch.equal(a, b), name
+        assert rel_norm(a.float(), c.float()) < 2e-3, name
+
+
 @pytest.mark.parametrize("hq,hk,lens", [(4, 2, [700, 130]), (12, 2, [4100, 520])])
 @pytest.mark.parametrize("case", ["far", "masked", "mixed"])
 def test_attention_forward_at_scores_far_from_zero_and_at_minus_infinity(hq, hk, lens, case):

@@ -395,7 +395,7 @@ def _rows_of(kind, rows, out, gen):
     if kind == "broadcast":
         return (torch.randn(1, 1, out, generator=gen) * 0.1).half().to(DEV).expand(1, rows, out)
     wide = (torch.randn(1, rows, out + (3 if kind == "ragged" else 64), generator=gen) * 0.1).half().to(DEV)
-    return wide[..., :out].contiguous() if kind == "plain" else wide[..., -out:] if kind == "block" else wide[..., :out]
+    return wide[..., :out].contiguous() if kind in ("plain", "ordered") else wide[..., -out:] if kind == "block" else wide[..., :out]
 
 
 @pytest.mark.parametrize("rank,rows,outs,kinds,launches", [
@@ -405,6 +405,7 @@ def _rows_of(kind, rows, out, gen):
     (16, 40, (160, 48), ("ragged", "plain"), 0),
     (16, 40, (168, 48), ("plain", "plain"), 0),       # a width off the kernel's tiles
     (8, 40, (160, 48), ("plain", "plain"), 0),
+    (16, 80, (160, 48), ("plain", "ordered"), 0),     # torch.use_deterministic_algorithms
 ])
 def test_lora_pair_in_place_is_two_single_branches_whichever_way_its_backward_runs(
         rank, rows, outs, kinds, launches, monkeypatch):
@@ -423,6 +424,8 @@ def test_lora_pair_in_place_is_two_single_branches_whichever_way_its_backward_ru
                for out in outs for shape in ((rank, hidden), (out, rank))]
     preset = [torch.randn(w.shape, generator=gen).to(DEV) for w in weights]
     grads = [_rows_of(kind, rows, out, gen) for kind, out in zip(kinds, outs)]
+    if "ordered" in kinds:   # the switch itself would refuse cuBLAS without a workspace setting
+        monkeypatch.setattr(torch, "are_deterministic_algorithms_enabled", lambda: True)
     entry, made = _lib.call, []
     monkeypatch.setattr(_lib, "call", lambda name, *args: (made.append(name), entry(name, *args))[1])
 
