@@ -1105,9 +1105,10 @@ inline int64_t round_up(int64_t v, int64_t m) { return (v + m - 1) / m * m; }
 // on 24 of the 74 pairs (215 us per call over 151936 columns, 93 us split over 72 of them; 1168 rows,
 // 30 tiles: 457 and 414 us). The order of units (tile fastest) keeps the pairs that run
 // together on one or two K ranges, whose rows of W they share through L2. 1 split keeps the result
-// deterministic. A unit has at least kMinUnit K blocks: the sums of more than two splits
-// arrive in any order, and a small model's fp16 step amplifies that (3000 columns, 48 blocks: two runs
-// differ by up to 1.4e-3 of a gradient with 47 splits, 9e-4 with four, not at all with two, for 5 us).
+// deterministic. A unit has at least kMinUnit K blocks, for small vocabularies: the sums of more than
+// two splits arrive in any order, and a small model's fp16 step amplifies that (3000 columns, 48 blocks: two
+// runs differ by up to 1.4e-3 of a gradient with 47 splits, 9e-4 with four, not at all with two, for 5 us).
+// Larger ones have up to kMaxSplit sums in any order; SOUP_LMHEAD_DETERMINISTIC is the switch for one order.
 constexpr int kUnitCost = 8;
 constexpr int kMinUnit = 20;
 constexpr int kMaxSplit = 80;
@@ -1498,6 +1499,21 @@ extern "C" int soup_lmhead_plan(int64_t n, int64_t v_shard, int64_t chunk_tiles,
   if (row_block) *row_block = p.row_block;
   if (first_chunk_tiles) *first_chunk_tiles = p.ct_first;
   if (tiles_per_chunk) *tiles_per_chunk = p.ct;
+  return SOUP_OK;
+}
+
+extern "C" int soup_lmhead_grad_units(int64_t n, int64_t h, int64_t v_shard, int64_t chunk_tiles,
+                                      int64_t* first_chunk, int64_t* later_chunk, int64_t* pairs) {
+  using namespace soup;
+  if (n <= 0 || h <= 0 || v_shard <= 0) SOUP_FAIL(SOUP_ERR_ARG, "lmhead_grad_units: bad shape");
+  const Plan p = make_plan(n, v_shard, sm_count(), (int)chunk_tiles);
+  const int total_ct = (int)((v_shard + kBN - 1) / kBN), rest = total_ct - p.ct_first;
+  const int tiles = (p.row_block + 2 * kBM - 1) / (2 * kBM) * (int)((h + kBN - 1) / kBN);
+  const int max_pairs = sm_count() / 2;
+  auto units = [&](int ct) { return ct > 0 ? tiles * pick_ksplit(tiles, max_pairs, ct * (kBN / kBK), false) : 0; };
+  if (first_chunk) *first_chunk = units(p.ct_first);
+  if (later_chunk) *later_chunk = units(rest < p.ct ? rest : p.ct);
+  if (pairs) *pairs = max_pairs;
   return SOUP_OK;
 }
 

@@ -367,6 +367,12 @@ int soup_lmhead_set_timing(float* host_sink6);
 int soup_lmhead_plan(int64_t n, int64_t v_shard, int64_t chunk_tiles, int64_t* row_block,
                      int64_t* first_chunk_tiles, int64_t* tiles_per_chunk);
 
+/* The work units (output tiles x splits of the contraction) of its gradient launches for the first
+ * row block's first chunk and for a later one (0 when there is none), and the CTA pairs that take
+ * them. Without SOUP_LMHEAD_DETERMINISTIC. */
+int soup_lmhead_grad_units(int64_t n, int64_t h, int64_t v_shard, int64_t chunk_tiles,
+                           int64_t* first_chunk, int64_t* later_chunk, int64_t* pairs);
+
 /* Reads back the device status word of the last soup_lmhead_ce on this workspace (synchronises
  * `stream`): 0 = every bounded wait completed; otherwise the code of the wait that gave up. */
 int soup_lmhead_status(const void* workspace, int64_t n, int64_t v_shard, int64_t chunk_tiles,

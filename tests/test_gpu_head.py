@@ -290,12 +290,46 @@ def test_finish_into_a_separate_typed_buffer_is_finish_then_one_rounding(out_dty
 
 # (rows, hidden, vocabulary): one row; fewer rows than a CTA's 128; one past a CTA's, one past a
 # pair's 256; a ragged last row tile; a hidden size whose last 256-column output tile is ragged; one
-# column tile, one past the first chunk, a ragged last column tile. The contraction of the gradient
-# is split over all CTA pairs at every one of them.
+# column tile, one past the first chunk, a ragged last column tile. One split, a few, or enough for
+# most CTA pairs.
 @pytest.mark.parametrize("dims", [(1, 64, 300), (24, 1536, 30000), (129, 904, 19200), (257, 512, 19201),
                                   (1168, 264, 12000), (127, 1536, 255), (600, 72, 8193)])
-def test_gradient_split_over_all_pairs_at_the_edges_of_its_tiles(dims):
+def test_gradient_at_the_edges_of_its_tiles(dims):
     check(*make(*dims, seed=31, drop=0.0 if dims[0] == 1 else 0.3))   # one unlabelled row: 0 / 0
+
+
+@pytest.mark.parametrize("dims", [(1300, 1544, 40001), (1100, 2056, 30000)])
+def test_gradient_with_more_units_than_cta_pairs_at_ragged_tiles(dims):
+    """A pair runs several units: both accumulators and both staging boxes are used again, at ragged
+    row, output and column tiles."""
+    import ctypes
+
+    from claudemaxing_b200 import _lib
+
+    first, later, pairs = (ctypes.c_int64() for _ in range(3))
+    n, hidden, vocab = dims
+    _lib.call("soup_lmhead_grad_units", n, hidden, vocab, 0, *(ctypes.byref(x) for x in (first, later, pairs)))
+    tiles = -(-n // 256) * -(-hidden // 256)
+    assert later.value > pairs.value and later.value > 2 * tiles and n % 256 and hidden % 256 and vocab % 256
+    check(*make(*dims, seed=31))
+
+
+def test_drop_in_function_is_the_head_s_own_entry():
+    """`_FusedHeadLoss.apply`, the reference's signature, against fused_head_loss: the same launches, so
+    the same bits, with a divisor on the host and on the device."""
+    from claudemaxing_b200.lm_head_loss import _FusedHeadLoss, fused_head_loss
+
+    h, w, t = (x.to(DEV) for x in make(300, 64, 900, seed=34))
+    for divisor in (77, torch.tensor(77, device=DEV), torch.tensor([77.0], device=DEV)):
+        mine, theirs = (h[None].clone().requires_grad_() for _ in range(2))
+        loss, token_loss, entropy, correct = _FusedHeadLoss.apply(mine, w, t[None], divisor, torch.float16, None, True)
+        want, terms = fused_head_loss(theirs, w, None, num_items_in_batch=divisor, target=t[None])
+        (loss * 64).sum().backward()
+        (want * 64).sum().backward()
+        assert loss.shape == want.shape and correct.shape == token_loss.shape == (1, 300)
+        for a, b in ((loss, want), (token_loss, terms.token_loss), (entropy, terms.token_entropy),
+                     (correct.sum(), terms.correct), (mine.grad, theirs.grad)):
+            assert torch.equal(a, b)
 
 
 @pytest.mark.parametrize("dims", [(1, 64, 300), (257, 512, 19201), (600, 72, 40000)])
