@@ -800,24 +800,10 @@ LOSS_SCALE = 4096.0   # the loss is scaled as a trainer's GradScaler does: fp16 
 C5A_TOKENS = 65536
 
 
-def recorded_traffic():
-    """DRAM bytes per step of the two GEMM kernels at config 1 on one GPU, as recorded from an ncu
-    capture in the line `traffic_bytes_per_step logits=<bytes> grad=<bytes>` of
-    profiles/lmhead_c1_kernels_full.md (None when the file or the line is missing)."""
-    try:
-        with open(os.path.join(ROOT, "profiles", "lmhead_c1_kernels_full.md")) as f:
-            for line in f:
-                if line.startswith("traffic_bytes_per_step"):
-                    return {k: float(v) for k, v in (kv.split("=") for kv in line.split()[1:])}
-    except Exception:  # noqa: BLE001
-        pass
-    return None
-
-
 def head_launches(n_rows, v_local, world):
-    """Kernels of this library one head pass over n_rows x v_local launches: state init, per row
-    block and chunk (logits, row merge, gradient) plus the first chunk's rescale, status publish,
-    finish, backward scale (or rounding before the reduce-scatter); at N>1 also the merge."""
+    """Kernels of this library one head pass over n_rows x v_local launches: initialisation, per row
+    block and chunk (logits, row merge, gradient), finish; on one GPU the step's totals and the backward
+    scale, at N>1 the merge of the ranks' states."""
     from claudemaxing_b200 import _lib
 
     rb, ct1, ct = ctypes.c_int64(), ctypes.c_int64(), ctypes.c_int64()
@@ -825,7 +811,7 @@ def head_launches(n_rows, v_local, world):
     row_blocks = -(-n_rows // rb.value)
     col_tiles = -(-v_local // 256)
     chunks = 1 + -(-max(col_tiles - ct1.value, 0) // ct.value)
-    return 1 + row_blocks * (chunks * 3 + 1) + 1 + 1 + 1 + (1 if world > 1 else 0)
+    return 1 + row_blocks * chunks * 3 + 1 + (1 if world > 1 else 2)
 
 
 class HeadJob:
@@ -1124,8 +1110,6 @@ def main():
     tf = lambda ms: flops_gemm / (ms * 1e-3) / 1e12 if ms > 0 else 0.0  # noqa: E731
     tensor_peak = peak["bf16_tflops"]
     logits_tf, grad_tf = tf(k_ms[0]), tf(k_ms[2])
-    traffic = recorded_traffic() if (world == 1 and args.workload == "c1") else None
-    minimum_bytes = 2.0 * v_local * HIDDEN + 2.0 * n_tokens * HIDDEN + 4.0 * n_tokens * HIDDEN
     roofline = {
         "kernel": "lmhead_logits_kernel (tcgen05 GEMM + softmax-statistics epilogue)",
         "bound": "tensor", "achieved": round(logits_tf, 1), "peak": tensor_peak, "unit": "TFLOP/s",
@@ -1133,17 +1117,6 @@ def main():
         "frac_of_sustained": round(logits_tf / peak["bf16_tflops_sustained"], 4),
         "frac_of_nominal_2250": round(logits_tf / 2250.0, 4),
         "ms_per_launch": round(k_ms[0] / max(k_launch[0], 1), 5), "launches_per_step": k_launch[0],
-        # DRAM bytes (read + write) of the logits launches of one step divided by their number,
-        # from the ncu capture recorded in profiles/; config 1 on one GPU only
-        "traffic": None if not traffic else round(traffic["logits"] / max(k_launch[0], 1)),
-        "traffic_per_step": None if not traffic else {
-            "logits_kernel": traffic["logits"], "grad_kernel": traffic["grad"],
-            "both": traffic["logits"] + traffic["grad"],
-            "minimum_w_once_hidden_dh": minimum_bytes,
-            "ratio_to_minimum": round((traffic["logits"] + traffic["grad"]) / minimum_bytes, 2),
-            "note": "the probabilities of a chunk pass from the logits to the gradient kernel "
-                    "through a bf16 buffer and the gradient GEMM reads a bf16 copy of W: that "
-                    "traffic is measured here and is not part of the minimum"},
         "grad_kernel": {"achieved": round(grad_tf, 1), "frac": round(grad_tf / tensor_peak, 4),
                         "ms_per_launch": round(k_ms[2] / max(k_launch[2], 1), 5),
                         "launches_per_step": k_launch[2]},
