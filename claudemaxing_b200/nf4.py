@@ -101,7 +101,7 @@ def dequantize_nf4_batch(weights, dtype=None, outs=None):
             code2, absmax2 = st.state2.code.contiguous(), st.state2.absmax.contiguous()
             offset = st.offset
             if not (type(offset) is torch.Tensor and offset.dtype == torch.float32
-                    and offset.device == packed.device):
+                    and offset.device == packed.device and offset.numel() == 1):
                 offset = _offset_tensor(offset, packed.device)
             keep += (code2, absmax2, offset)
             item.code2, item.absmax2, item.offset = code2.data_ptr(), absmax2.data_ptr(), offset.data_ptr()

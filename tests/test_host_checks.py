@@ -111,6 +111,24 @@ def test_head_workspace_holds_no_more_probabilities_than_a_chunk_has(launches, r
         assert args[13] == wanted(rows, 64, 300, 0)
 
 
+def test_nf4_batch_takes_one_offset_per_weight(launches, monkeypatch):
+    from types import SimpleNamespace
+
+    from claudemaxing_b200 import nf4
+
+    def weight(offset):
+        second = SimpleNamespace(code=torch.zeros(256), absmax=torch.zeros(1), blocksize=256)
+        state = SimpleNamespace(shape=(2, 64), dtype=torch.float16, nested=True, blocksize=64, code=torch.zeros(16),
+                                absmax=torch.zeros(2, dtype=torch.uint8), state2=second, offset=offset)
+        return torch.zeros(64, dtype=torch.uint8), state
+
+    for offset in (torch.tensor(0.5), torch.tensor([0.5]), 0.5, torch.tensor(0.5, dtype=torch.float64)):
+        assert nf4.dequantize_nf4_batch([weight(offset)])[0].shape == (2, 64)
+    with pytest.raises(RuntimeError):
+        nf4.dequantize_nf4_batch([weight(torch.tensor([0.5, 0.25]))])
+    assert [name for name, _ in launches] == ["soup_nf4_dequant_batch"] * 4
+
+
 class _Projection:
     def __init__(self, out_features, weight):
         self.out_features, self.group, self._weight = out_features, self, weight
