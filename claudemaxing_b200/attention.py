@@ -1,11 +1,12 @@
 """Attention of the packed training row, and grouped-query attention without repeating k/v.
 
-Attention stays a library call, as in the reference (solution/attention.py:332-343 calls torch
-SDPA). Two routes replace transformers' "sdpa" attention function:
+The reference calls torch SDPA (solution/attention.py:332-343). Two routes replace transformers'
+"sdpa" attention function:
 
 * a packed row whose batch rows are given as segment offsets (`cu_seq_lens_q` / `cu_seq_lens_k`,
-  the keyword names transformers uses for packed sequences) runs torch's variable-length causal
-  attention: work and memory are linear in the packed length times the longest segment, and no
+  the keyword names transformers uses for packed sequences) runs this library's kernels
+  (csrc/attention.cu; fp16, head dimension 128) or torch's variable-length causal attention (other
+  16-bit operands): work and memory are linear in the packed length times the longest segment, and no
   [N, N] mask exists. The reference's packed route builds that mask (solution/lm_head_loss.py:
   300-337); this is the same attention pattern stated as segments.
 * a boolean 4-D mask on a grouped-query model runs one SDPA call with `enable_gqa`, which gives

@@ -397,9 +397,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 // The score product of the next tile is issued as soon as dV has consumed P^T, so the exponentials of
 // tile i + 1 run under the dK / dQ products of tile i. dK and dV leave once per CTA.
 //
-// What bounds it: shared-memory bandwidth. The five products read 256 KB of operands per tile (S^T
-// and dP^T and dQ both operands, dV and dK one), staging and loads move 224 KB more: 3750 clocks at
-// 128 B a clock against 2560 clocks of products. (A query-stationary walk reads and moves 700 KB per
+// What bounds it: the chain of hand-overs of a tile, one CTA per SM deep. 9215 tokens in 4 segments take
+// about 7000 clocks a tile, the tensor pipe active 37 % of them; the products need 2560, and shared memory
+// 3750 by count: they read 256 KB of operands per tile (S^T and dP^T and dQ both operands, dV and dK one),
+// staging and loads move 224 KB more, at 128 B a clock. (A query-stationary walk reads and moves 700 KB per
 // tile: it stages and adds dK and dV, 128 KB, where this one adds dQ, 64 KB. It took 35.8 us for 1280
 // tokens in 5 segments, 12 / 2 heads, and 790 us for 9215 tokens in 4; this one 22.8 and 300 us.)
 // ------------------------------------------------------------------------------------------

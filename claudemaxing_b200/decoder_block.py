@@ -8,16 +8,17 @@ kernels costs a launch and a pass over [tokens, hidden]: about a quarter of the 
 module computes the same block with those passes folded into the kernels next to them:
 
 * q, k and v come from one GEMM on the block's dequantised weights (adjacent in the buffer all of
-  a block's projections are dequantised into) and stay fp16; `soup_rope_sum` adds the adapter
-  output to q in fp32, rotates q and k and writes them as fp16 [tokens, heads, head_dim], which
-  are exactly the values the reference chain reaches (fp32 sum, fp32 rotation, one rounding to
-  fp16 at the attention's cast); v + adapter is one fp16 add (fp32 inside, one rounding);
+  a block's projections are dequantised into) and stay fp16; `soup_qkv_rope_fwd` adds the adapter
+  outputs to q and v in fp32, rotates q and k and writes the three as fp16 [tokens, heads, head_dim],
+  which are exactly the values the reference chain reaches (fp32 sum, fp32 rotation, one rounding to
+  fp16 at the attention's cast); rotary tables it does not read take `soup_rope_sum` and an add;
 * attention is causal attention inside the segments of the packed row (attention.py; for heads
   of 128 this library's kernels, called from the same autograd node as the projection);
-* the block's two adapters are one node (lora.LoRABranchPair: both packed and unpacked by one
-  launch each, one batched product with A), their weights cast once per decoder forward;
+* the block's two adapters are one node (lora.LoRABranchPair: both packed by one launch, one batched
+  product with A, backward in two launches where it adds into gradients that exist), their weights
+  cast once per decoder forward;
 * o_proj and down_proj add the fp32 residual in the GEMM's epilogue and write fp32;
-* backward rotates dq and dk straight into column blocks of one [tokens, q+k+v] fp16 buffer and
+* backward rotates dq and dk, and rounds dv, straight into one [tokens, q+k+v] fp16 buffer and
   forms the input gradient of the three projections in one GEMM with fp32 output; the MLP's two
   input gradients accumulate in one fp32 output as well;
 * each norm and the residual connection that leaves the same tensor are one node (`_NormResidual`):
@@ -290,7 +291,8 @@ class _QKVRope(torch.autograd.Function):
     all three returned as fp16 [tokens, heads, head_dim]. With `cu_rows` (segment offsets of the
     packed row) the causal attention inside the segments runs here as well, on this library's
     kernels, and its output [tokens, heads, head_dim] is what is returned: backward then hands the
-    attention kernel's fp32 dV straight to the copy into the projection's gradient buffer."""
+    attention kernel's fp32 gradients straight to the launch that rotates dq and dk back and writes the
+    projection's gradient (`soup_qkv_rope_bwd`)."""
 
     @staticmethod
     @_plain_precision
