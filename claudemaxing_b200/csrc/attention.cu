@@ -23,6 +23,7 @@
 //
 // The reference calls torch SDPA here (solution/attention.py:332-343) on a [1, 1, N, N] mask
 // built by its packing (solution/lm_head_loss.py:300-337); this kernel takes the segment offsets.
+#include <cfloat>
 #include <cuda.h>
 
 #include "common.cuh"
@@ -107,7 +108,7 @@ struct AttnArgs {
   __half* out;           // [n, hq, 128]
   float* lse;            // [hq, n]
   int n, segments, hq, group;
-  float scale_log2;      // softmax scale * log2(e)
+  float scale_log2;      // softmax scale * log2(e), above zero (attn_fwd_kernel's NEG has the sign)
   float scale_far;       // the power of two at or above it (softmax_tile)
   int* status;
 };
@@ -148,8 +149,8 @@ struct RowRef {
 };
 
 // One row of a score tile: its exponentials, as fp16 over the score columns, against the (possibly moved)
-// reference, and the row's sum l.
-template <bool DIAG>
+// reference, and the row's sum l. NEG: of the negated scores (a softmax scale below zero).
+template <bool DIAG, bool NEG>
 __device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, int limit, bool first,
                                              float scale, float scale_far, RowRef& ref, float& l) {
   uint32_t x[4][32];
@@ -162,6 +163,7 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, i
   for (int c = 0; c < 4; ++c)
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
+      if (NEG) x[c][j] ^= 0x80000000u;
       if (DIAG && c * 32 + j > limit) x[c][j] = 0xff800000u;   // -inf: no weight
       mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(x[c][j]));
     }
@@ -209,7 +211,7 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, i
   tmem_st_wait();
 }
 
-template <int NT>
+template <int NT, bool NEG>
 __global__ void __launch_bounds__(kFwdThreads<NT>, NT == 1 ? 2 : 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const AttnArgs a) {
@@ -336,8 +338,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (!ok) break;
       tc_fence_after_sync();
       // only the last tile of the walk, the one on the diagonal, hides columns from a row
-      if (i + 1 < n_kv) softmax_tile<false>(s_addr, o_addr, 0, i == 0, a.scale_log2, a.scale_far, ref, l);
-      else softmax_tile<true>(s_addr, o_addr, r, i == 0, a.scale_log2, a.scale_far, ref, l);
+      if (i + 1 < n_kv) softmax_tile<false, NEG>(s_addr, o_addr, 0, i == 0, a.scale_log2, a.scale_far, ref, l);
+      else softmax_tile<true, NEG>(s_addr, o_addr, r, i == 0, a.scale_log2, a.scale_far, ref, l);
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&s.p_full[t]);
@@ -833,11 +835,11 @@ extern "C" int soup_attn_fwd(const void* q, const void* k, const void* v, const 
     SOUP_FAIL(SOUP_ERR_ARG, "attn_fwd: pointers must be 16-byte aligned");
   // a runtime call first: it makes the device's context current on this thread (autograd runs
   // backward on threads of its own), which the driver's tensor-map encoder needs
-  const int heads = forward_heads_per_cta(n_tokens, n_segments, hq, hk);
+  const bool negative = scale < 0.f;
+  const int heads = negative ? 1 : forward_heads_per_cta(n_tokens, n_segments, hq, hk);
+  const auto kernel = negative ? attn_fwd_kernel<1, true> : heads == 1 ? attn_fwd_kernel<1, false> : attn_fwd_kernel<2, false>;
   const size_t smem = (heads == 1 ? sizeof(FwdSmem<1>) : sizeof(FwdSmem<2>)) + 1024;
-  if ((heads == 1 ? cudaFuncSetAttribute(attn_fwd_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)
-                  : cudaFuncSetAttribute(attn_fwd_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem)) != cudaSuccess)
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
     SOUP_FAIL(SOUP_ERR_LAUNCH, "attn_fwd: shared memory attribute");
   CUtensorMap mq, mk, mv;
   if (umma::encode_map_2d_16bit(&mq, q, (uint64_t)n_tokens, (uint64_t)(hq * kD), (uint64_t)q_pitch, kBQ, 64, false) ||
@@ -852,14 +854,14 @@ extern "C" int soup_attn_fwd(const void* q, const void* k, const void* v, const 
   a.segments = (int)n_segments;
   a.hq = (int)hq;
   a.group = (int)(hq / hk);
-  a.scale_log2 = scale * kLog2e;
+  // a scale of zero as the smallest above it: x * scale is as good as zero, and a hidden key's -inf stays -inf
+  a.scale_log2 = fmaxf(fabsf(scale) * kLog2e, FLT_MIN);
   a.scale_far = exp2f(ceilf(log2f(a.scale_log2)));
   a.status = rowpipe::status_word();
   const int64_t ctas = tile_slots(n_tokens, n_segments) * (hq / heads);
   if (ctas > INT32_MAX) SOUP_FAIL(SOUP_ERR_ARG, "attn_fwd: too many tokens, segments or heads");
   cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-  if (heads == 1) attn_fwd_kernel<1><<<(unsigned)ctas, kFwdThreads<1>, smem, st>>>(mq, mk, mv, a);
-  else attn_fwd_kernel<2><<<(unsigned)ctas, kFwdThreads<2>, smem, st>>>(mq, mk, mv, a);
+  kernel<<<(unsigned)ctas, heads == 1 ? kFwdThreads<1> : kFwdThreads<2>, smem, st>>>(mq, mk, mv, a);
   SOUP_CHECK_LAUNCH("attn_fwd");
   return SOUP_OK;
 }

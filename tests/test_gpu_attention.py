@@ -121,6 +121,26 @@ def test_attention_forward_when_the_row_maximum_keeps_growing(hq, hk, lens):
     assert (lse.double().cpu() - want_lse).abs().max() < 2e-3
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.05])
+@pytest.mark.parametrize("hq,hk,lens", [(4, 2, [300, 130]), (12, 2, [4100, 520])])
+def test_attention_with_a_scale_of_zero_or_less(hq, hk, lens, scale):
+    """Every visible key weighs the same, or the smaller scores more; hidden keys weigh nothing either way.
+    One and two heads per CTA; bounds of the plain cases."""
+    from oracle import attention as oat
+
+    gen = torch.Generator().manual_seed(12)
+    q, k, v, grad = (torch.randn(sum(lens), h, 128, generator=gen).half() for h in (hq, hk, hk, hq))
+    cu = _cu(lens)
+    got = _run(q.to(DEV), k.to(DEV), v.to(DEV), cu, grad.to(DEV), scale=scale)
+    out, lse = oat.segment_attention(q, k, v, cu, scale)
+    want = (out, lse) + oat.segment_attention_backward(q, k, v, cu, grad, scale)
+    for name, a, b in zip(("out", "lse", "dq", "dk", "dv"), got, want):
+        if scale == 0.0 and name in ("dq", "dk"):
+            assert (a == 0).all(), name
+        else:
+            assert rel_norm(a.float().cpu(), b.float()) < 2e-3, name
+
+
 def test_attention_gradients_are_reproducible_when_torch_is_told_to_be():
     """torch.use_deterministic_algorithms: no sums in any order; the gradients of several key tiles and
     a group of heads come out the same twice, and within the two kernels' fp16 rounding of the others."""
