@@ -242,6 +242,39 @@ def test_rope_vs_oracle(dims, dtype, cos_batch_one):
         assert_close_rel_max(val.detach().cpu(), r, tol, name)
 
 
+@pytest.mark.parametrize("heads", [(12, 2), (3, 2), (1, 1), (7, 0), (0, 5)])
+@pytest.mark.parametrize("dtype", [F32, F16, BF16])
+def test_rope_gradients_have_the_layout_of_their_inputs(heads, dtype):
+    """Gradients of [b, h, t, d] outputs: heads that do and do not fill a thread's share, one of q and k
+    alone; laid out as the projections q and k are views of, or as the contiguous tensors they are."""
+    from claudemaxing_b200.rope import rope
+    from oracle import elementwise as ew
+
+    gen = torch.Generator().manual_seed(4)
+    b, t, d = 2, 45, 128
+    cos, sin = ew.rope_tables(torch.arange(t), d, dtype=dtype)
+    rows = [torch.randn(b, t, max(h, 1) * d, generator=gen).to(dtype) for h in heads]
+    grads = [torch.randn(b, max(h, 1), t, d, generator=gen).to(dtype) for h in heads]
+    views = [x.view(b, t, -1, d).transpose(1, 2) for x in rows]
+    want = ew.rope_fwd_bwd(*views, cos, sin, *grads)[2:]
+    for contiguous in (False, True):
+        leaves = [x.to(DEV).requires_grad_(h > 0) for x, h in zip(rows, heads)]
+        inputs = [x.view(b, t, -1, d).transpose(1, 2) for x in leaves]
+        if contiguous:
+            inputs = [x.contiguous() for x in inputs]
+        seen = [None, None]
+        for i, x in enumerate(inputs):
+            if x.requires_grad:
+                x.register_hook(lambda g, i=i: seen.__setitem__(i, g.stride()))
+        out = rope(*inputs, cos.to(DEV), sin.to(DEV))
+        torch.autograd.backward(out, [g.to(DEV) for g in grads])
+        for x, leaf, w, strides, h in zip(inputs, leaves, want, seen, heads):
+            if h:
+                assert strides == x.stride()
+                assert_close_rel_max(leaf.grad.view(b, t, -1, d).transpose(1, 2).cpu(), w,
+                                     {F32: 1e-5, F16: 2e-3, BF16: 1.6e-2}[dtype], "gradient")
+
+
 def test_rope_packed_positions_restart_per_row():
     # benchmark config 3: one packed row of lengths {512,384,640,512}, positions restart at 0
     from claudemaxing_b200.rope import rope
