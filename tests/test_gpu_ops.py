@@ -172,6 +172,27 @@ def test_rmsnorm_vs_oracle(shape, dtypes, train_w):
         assert wd.grad is None
 
 
+@pytest.mark.parametrize("cols", [256, 264, 512, 4088, 4096, 4104])
+@pytest.mark.parametrize("rows", [1, 3, 4, 1783])   # 1783: three rows a step, a second step for some CTAs, a remainder
+def test_rmsnorm_weight_gradient_at_the_edges_of_its_kernels(cols, rows):
+    from claudemaxing_b200.rmsnorm import rmsnorm
+
+    gen = torch.Generator().manual_seed(rows)
+    x, dy = (torch.randn(rows, cols, generator=gen).half() for _ in range(2))
+    w = (1 + 0.5 * torch.randn(cols, generator=gen)).half()
+    norm = x.double() * (x.double().square().mean(-1, keepdim=True) + 1e-6).rsqrt()
+    gn = dy.double() * w.double()
+    want_dx = (gn - norm * (gn * norm).mean(-1, keepdim=True)) * (x.double().square().mean(-1, keepdim=True) + 1e-6).rsqrt()
+    leaves = [t.to(DEV).requires_grad_() for t in (x, w)]
+    rmsnorm(*leaves, 1e-6).backward(dy.to(DEV))
+    # fp16: a rounding of dy * w and of the result each, half an ulp (4.9e-4) of their value
+    assert_close_rel_max(leaves[0].grad.cpu(), want_dx.float(), 2e-3, "dx")
+    assert_close_rel_max(leaves[1].grad.cpu(), (dy.double() * norm).sum(0).float(), 2e-3, "dw")
+    again = [t.to(DEV).requires_grad_() for t in (x, w)]
+    rmsnorm(*again, 1e-6).backward(dy.to(DEV))
+    assert torch.equal(leaves[1].grad, again[1].grad)   # a fixed order of additions
+
+
 def test_rmsnorm_fp16_copy_path_and_tiny_weights():
     # fp32 x, frozen fp32 w: forward leaves an fp16 copy for the next layers, backward uses it;
     # a 2e5 "massive activation" channel and tiny / zero weights (tests_local/test_rmsnorm.py:197-277)
