@@ -101,52 +101,68 @@ def _grouped_sdpa(query, key, value, attention_mask, scaling):
 
 
 def _token_major(t):
-    """[tokens, heads, 128] view of a [1, heads, tokens, 128] tensor if its heads are adjacent in
-    memory (a transposed view of a [tokens, heads * 128] matrix), else None."""
-    x = t.transpose(1, 2)[0]
-    if x.stride(2) == 1 and x.stride(1) == x.shape[2] and x.stride(0) >= x.shape[1] * x.shape[2] \
-            and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0:
-        return x
-    return None
+    """Whether the heads of a [1, heads, tokens, 128] tensor are adjacent in memory (a transposed view of a
+    [tokens, heads * 128] matrix)."""
+    _, sh, st, sd = t.stride()
+    _, heads, _, d = t.shape
+    return sd == 1 and sh == d and st >= heads * d and st % 8 == 0 and t.data_ptr() % 16 == 0
+
+
+def _rows(t):
+    """[tokens, heads, 128] view of a [1, heads, tokens, 128] tensor, or the tensor itself when it is one."""
+    return t if t.dim() == 3 else t[0].transpose(0, 1)
 
 
 class SegmentAttention(torch.autograd.Function):
-    """Causal attention inside the segments of a packed row on fp16 [tokens, heads, 128] tensors:
-    forward and backward by this library's tcgen05 kernels (csrc/attention.cu). The forward also
+    """Causal attention inside the segments of a packed row on fp16 [tokens, heads, 128] tensors, or
+    [1, heads, tokens, 128] ones whose heads are adjacent in memory (`_token_major`; the output is then [1,
+    tokens, heads, 128]; the views are taken in here because a select of a tensor that carries gradients
+    costs a fill and a copy of it in backward: six launches for q, k and v, 37 of 490 us of device time at
+    9215 tokens): forward and backward by this library's tcgen05 kernels (csrc/attention.cu). The forward also
     returns the row log-sum-exps in the layout torch's variable-length flash-attention backward
     takes ([heads, tokens]), which stands in where `own_backward` says so."""
 
     @staticmethod
     def forward(ctx, q, k, v, cu_rows, longest, scale):
+        inputs, ctx.batched = (q, k, v), q.dim() == 4
+        q, k, v = map(_rows, inputs)
         n, hq, d = q.shape
         out = torch.empty((n, hq, d), dtype=q.dtype, device=q.device)
         lse = torch.empty((hq, n), dtype=torch.float32, device=q.device)
         _lib.call("soup_attn_fwd", _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(cu_rows),
                   _lib.ptr(out), _lib.ptr(lse), n, cu_rows.numel() - 1, hq, k.shape[1], d,
                   q.stride(0), k.stride(0), v.stride(0), float(scale), _lib.stream_of(q))
-        ctx.save_for_backward(q, k, v, cu_rows, out, lse)
+        ctx.save_for_backward(*inputs, cu_rows, out, lse)
         ctx.longest, ctx.scale = int(longest), float(scale)
-        return out
+        return out.unsqueeze(0) if ctx.batched else out
 
     @staticmethod
     def backward(ctx, grad):
-        q, k, v, cu_rows, out, lse = ctx.saved_tensors
+        *inputs, cu_rows, out, lse = ctx.saved_tensors
+        q, k, v = map(_rows, inputs)
+        if ctx.batched:
+            grad = grad[0]
         if own_backward():
             # one rounding launch for all three: they are adjacent
             flat = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, ctx.scale).to(q.dtype)
-            return (*gradient_parts(flat, q.shape[0], q.shape[1], k.shape[1], q.shape[2]), None, None, None)
-        _varlen()   # registers the operator
-        rng_state = torch.empty(2, dtype=torch.uint64, device=q.device)   # no dropout: never read
-        dq, dk, dv = torch.ops.torch_attn._varlen_attn_backward(
-            grad.contiguous(), q, k, v, out, lse, cu_rows, cu_rows, ctx.longest, ctx.longest, True,
-            rng_state, ctx.scale, [-1, 0])
-        return dq, dk, dv, None, None, None
+            grads = gradient_parts(flat, q.shape[0], q.shape[1], k.shape[1], q.shape[2])
+        else:
+            _varlen()   # registers the operator
+            rng_state = torch.empty(2, dtype=torch.uint64, device=q.device)   # no dropout: never read
+            grads = torch.ops.torch_attn._varlen_attn_backward(
+                grad.contiguous(), q, k, v, out, lse, cu_rows, cu_rows, ctx.longest, ctx.longest, True,
+                rng_state, ctx.scale, [-1, 0])
+        if ctx.batched:
+            grads = tuple(g.transpose(0, 1).unsqueeze(0) for g in grads)
+        return (*grads, None, None, None)
 
 
 def _own_forward_covers(q, k, v, cu_rows):
-    return (OWN_FORWARD and q is not None and k is not None and v is not None
-            and q.dtype == torch.float16 and k.dtype == v.dtype == torch.float16
-            and q.shape[2] == 128 and cu_rows.dtype == torch.int32 and cu_rows.is_cuda
+    """For [1, heads, tokens, head_dim] tensors."""
+    return (OWN_FORWARD and q.dtype == torch.float16 and k.dtype == v.dtype == torch.float16
+            and q.shape[0] == k.shape[0] == v.shape[0] == 1
+            and q.shape[3] == 128 and cu_rows.dtype == torch.int32 and cu_rows.is_cuda
+            and all(_token_major(t) for t in (q, k, v))
             and hasattr(torch.ops, "torch_attn") and hasattr(torch.ops.torch_attn, "_varlen_attn_backward"))
 
 
@@ -161,11 +177,9 @@ def segment_attention(query, key, value, cu_rows, longest, scaling):
     if (varlen_attn is None or not query.is_cuda or dtype not in _LOW or query.shape[-1] > 256
             or query.shape[-1] % 8 or query.shape[1] % key.shape[1]):
         return _grouped_sdpa(query, key, value, mask_of_segments(cu_rows, query.shape[2]), scaling)
-    if dtype == torch.float16 and all(t.dtype == dtype for t in (query, key, value)):
-        rows = [_token_major(t) for t in (query, key, value)]
-        if _own_forward_covers(*rows, cu_rows):
-            scale = query.shape[-1] ** -0.5 if scaling is None else scaling
-            return SegmentAttention.apply(*rows, cu_rows, longest, scale).unsqueeze(0)
+    if dtype == torch.float16 and _own_forward_covers(query, key, value, cu_rows):
+        scale = query.shape[-1] ** -0.5 if scaling is None else scaling
+        return SegmentAttention.apply(query, key, value, cu_rows, longest, scale)
     q, k, v = (t.transpose(1, 2)[0] if t.dtype == dtype else t.transpose(1, 2)[0].to(dtype)
                for t in (query, key, value))
     out = varlen_attn(q, k, v, cu_rows, cu_rows, int(longest), int(longest),

@@ -251,3 +251,31 @@ def test_attention_kernels_refuse_what_they_do_not_cover():
     with pytest.raises(RuntimeError, match="multiple of key heads"):
         _lib.call("soup_attn_fwd", _lib.ptr(q), _lib.ptr(q), _lib.ptr(q), _lib.ptr(cu), _lib.ptr(q),
                   _lib.ptr(lse), 8, 1, 3, 2, 128, 384, 384, 384, 0.1, _lib.stream_of(q))
+
+
+@pytest.mark.parametrize("pitch", [0, 64])
+def test_gradients_pass_through_the_views_of_a_decoder_block(pitch):
+    """[1, heads, tokens, 128] views of token-major rows (dense, or column blocks of a wider matrix): the
+    numbers of the [tokens, heads, 128] form, and no gradient of another layout that views would copy."""
+    from claudemaxing_b200.attention import SegmentAttention, segment_attention
+
+    gen = torch.Generator().manual_seed(8)
+    lens, heads = [130, 1, 77], (4, 2, 2)
+    n = sum(lens)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV)
+    wide = [torch.randn(n, h * 128 + pitch, generator=gen).half().to(DEV) for h in heads]
+    grad = torch.randn(1, n, heads[0], 128, generator=gen).half().to(DEV)
+    flat = [w[:, :h * 128].unflatten(1, (h, 128)).detach().requires_grad_() for w, h in zip(wide, heads)]
+    want = SegmentAttention.apply(*flat, cu, max(lens), 0.1)
+    want.backward(grad[0])
+    leaves = [w[:, :h * 128].unflatten(1, (h, 128)).detach().requires_grad_() for w, h in zip(wide, heads)]
+    views = [x.unsqueeze(0).transpose(1, 2) for x in leaves]
+    seen = []
+    for x in views:
+        x.register_hook(lambda g: seen.append(g.transpose(1, 2)[0].is_contiguous()))
+    out = segment_attention(*views, cu, max(lens), 0.1)
+    assert out.shape == (1, n, heads[0], 128) and torch.equal(out[0], want)
+    out.backward(grad)
+    assert seen == [True] * 3
+    for x, w in zip(leaves, flat):   # sums of up to two tiles in any order
+        assert (x.grad.float() - w.grad.float()).abs().max() <= 2e-3 * w.grad.float().abs().max()
