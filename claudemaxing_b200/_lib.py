@@ -35,6 +35,10 @@ SIGNATURES = {
     "soup_attn_fwd": [_P, _P, _P, _P, _P, _P] + [_L] * 8 + [_F, _P],
     "soup_lora_pair_gain": [_P, _L, _L, _P, _L, _L] + [_P] * 6 + [_F, _F, _L, _L, _P],
     "soup_lora_pair_input": [_P] * 8 + [_F, _F] + [_L] * 3 + [_P],
+    "soup_lora_up": [_P] * 5 + [_F] + [_L] * 4 + [_P],
+    "soup_lora_branch_workspace_bytes": [_L] * 3,
+    "soup_lora_branch_bwd": [_P, _L] + [_P] * 8 + [_I] * 3 + [_F] * 3 + [_P] + [_L] * 5 + [_P],
+    "soup_lora_cast": [_P] * 4 + [_L, _L, _I, _I, _P],
     "soup_qkv_rope_fwd": [_P, _L] + [_P] * 7 + [_L] * 4 + [_P],
     "soup_qkv_rope_bwd": [_P] * 6 + [_L] * 5 + [_P],
     "soup_attn_bwd": [_P] * 11 + [_L] * 9 + [_F, _P],
@@ -66,7 +70,8 @@ SIGNATURES = {
     "soup_nf4_linear_dx": [_P, _I, _P, _P, _I, _L, _L, _I, _I, _I, _P, _L, _P],
 }
 _RESTYPE = {"soup_lmhead_workspace_bytes": _L, "soup_lmhead_forward_workspace_bytes": _L,
-            "soup_rmsnorm_bwd_partials": _L, "soup_nf4_gemm_workspace_bytes": _L}
+            "soup_rmsnorm_bwd_partials": _L, "soup_nf4_gemm_workspace_bytes": _L,
+            "soup_lora_branch_workspace_bytes": _L}
 SIGNATURES["soup_rmsnorm_bwd_partials"] = [_L, _L]
 
 class Nf4Item(ctypes.Structure):

@@ -15,25 +15,13 @@
 // product back to the input's width rounded to fp16 once, weight gradients added in fp32 (by
 // reductions, in any order).
 #include "common.cuh"
+#include "rank16.cuh"
 #include "umma.cuh"
 
 namespace soup {
 namespace {
 
-constexpr int kRank = 16;
-
-__device__ __forceinline__ uint32_t transpose8x8(uint32_t x) {
-  uint32_t y;
-  asm("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(y) : "r"(x));
-  return y;
-}
-
-// c += a b: A [16 x 16] row, B [16 x 8] column fragments.
-__device__ __forceinline__ void mma16816(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
+using namespace rank16;
 
 // Adds `bytes` of fp32 values in shared memory to global memory (both 16-byte aligned).
 __device__ __forceinline__ void bulk_add(float* gdst, const float* ssrc, uint32_t bytes) {
@@ -43,28 +31,6 @@ __device__ __forceinline__ void bulk_add(float* gdst, const float* ssrc, uint32_
 }
 __device__ __forceinline__ void red_add4(float* p, float x, float y, float z, float w) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w));
-}
-
-// The order of indices inside a product is free as long as both operands agree, so that a lane can move
-// contiguous bytes: of 16 ranks, "index 2t, 2t + 1 of 8-block i" is rank 4t + 2i, 4t + 2i + 1, and of 32
-// columns, "index 2t, 2t + 1 of 8-block j" is column 8t + 2j, 8t + 2j + 1 (t = lane % 4). With the plain
-// order a fragment is four 4-byte loads a lane, 16 bytes of each of 8 rows, and the load unit is what
-// bounds the kernel.
-__device__ __forceinline__ int rank_of(int block, int index) { return 4 * (index >> 1) + 2 * block + (index & 1); }
-__device__ __forceinline__ int column_of(int block, int index) { return 8 * (index >> 1) + 2 * block + (index & 1); }
-
-// The A fragment of rows row0 .. row0 + 15 of a row-major fp16 [n_rows, 16] matrix; rows past n_rows read
-// as zero.
-__device__ __forceinline__ void load_rank_fragment(const __half* m, int64_t row0, int64_t n_rows, int lane,
-                                                   uint32_t (&f)[4]) {
-  const int g = lane >> 2, t = lane & 3;
-#pragma unroll
-  for (int half = 0; half < 2; ++half) {   // f[0], f[1]: rows g, g + 8 of block 0; f[2], f[3]: of block 1
-    const int64_t row = row0 + g + half * 8;
-    const uint2 v = row < n_rows ? __ldg(reinterpret_cast<const uint2*>(m + row * kRank + 4 * t)) : make_uint2(0u, 0u);
-    f[half] = v.x;
-    f[2 + half] = v.y;
-  }
 }
 
 // ------------------------------------------------------------------------------------------
@@ -210,6 +176,7 @@ struct InputArgs {
   float scale[2];
   int64_t rows;
   int hidden, strips, blocks_per_cta;   // strips: hidden / 32
+  int wide_dx;            // dx is 32-byte aligned
 };
 
 __global__ void __launch_bounds__(kInputStrips * kInputGroups * 32)
@@ -293,9 +260,13 @@ lora_input_kernel(const __grid_constant__ InputArgs p) {
     for (int half = 0; half < 2; ++half) {
       const int64_t row = rb * 16 + g + half * 8;
       if (row < p.rows) {
-        float4* dst = reinterpret_cast<float4*>(p.dx + row * p.hidden + col);
-        dst[0] = make_float4(sum[half][0], sum[half][1], sum[half][2], sum[half][3]);
-        dst[1] = make_float4(sum[half][4], sum[half][5], sum[half][6], sum[half][7]);
+        float* dst = p.dx + row * p.hidden + col;
+        if (p.wide_dx) {
+          store_sector(dst, sum[half]);
+        } else {
+          reinterpret_cast<float4*>(dst)[0] = make_float4(sum[half][0], sum[half][1], sum[half][2], sum[half][3]);
+          reinterpret_cast<float4*>(dst)[1] = make_float4(sum[half][4], sum[half][5], sum[half][6], sum[half][7]);
+        }
       }
     }
     if (rb + kInputGroups < last) {
@@ -406,6 +377,7 @@ extern "C" int soup_lora_pair_input(const void* x16, const uint8_t* bits_first, 
   p.scale[1] = scale_second;
   p.rows = rows;
   p.hidden = (int)hidden;
+  p.wide_dx = aligned32(dx);
   p.strips = (int)(hidden / 32);
   // row blocks per CTA, whole rounds of its four warps, that leave about one CTA per SM
   const int64_t columns = (p.strips + kInputStrips - 1) / kInputStrips, n_blocks = (rows + 15) / 16;

@@ -280,7 +280,7 @@ rmsnorm_bwd_scalar_kernel(const void* __restrict__ dy, const void* __restrict__ 
 
 // dw[c] = sum over partial rows, fixed order, rounded once to the weight dtype. 32 columns a CTA, every
 // sixteenth partial row a warp: a chain of 37 loads for 592 partial rows, where one thread a column had 592
-// (11.8 us at 1536 columns).
+// (11.8 -> 5.0 us at 1536 columns).
 constexpr int kReduceWarps = 16;
 __global__ void __launch_bounds__(kReduceWarps * 32)
 rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, void* __restrict__ dw, int n_partials,

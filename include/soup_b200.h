@@ -206,6 +206,25 @@ int soup_lora_pair_input(const void* x16, const uint8_t* bits_first, const uint8
                          float scale_first, float scale_second, int64_t rows, int64_t hidden, int64_t rank,
                          void* stream);
 
+/* out = fp16(fp16(low b16^T) * scale) of a rank-16 adapter, or of two (b16_second not NULL): low fp16
+ * [adapters, rows, 16], b16 fp16 [out, 16] (out a multiple of 8), out fp16 [rows, out]. The product with B and
+ * the scaling of solution/lora.py:94-116. */
+int soup_lora_up(const void* low, const void* b16_first, const void* b16_second, void* out_first, void* out_second,
+                 float scale, int64_t rows, int64_t width_first, int64_t width_second, int64_t rank, void* stream);
+/* Backward of one rank-16 LoRA branch (solution/lora.py:118-134) from the output gradient g (fp16, row pitch g_pitch,
+ * a multiple of 8): with gs = fp16(g * g_scale) and gain = fp16(gs B), dx = keep * keep_scale * fp16(gain A)
+ * (fp32), dA = gain^T fp16(keep * keep_scale * x16) (fp32 [16, in]) and dB = db_alpha * gs^T low (fp32 [out, 16]);
+ * add_*: to what the buffer holds. Sums are formed in a fixed order. */
+int64_t soup_lora_branch_workspace_bytes(int64_t rows, int64_t in, int64_t out);
+int soup_lora_branch_bwd(const void* g, int64_t g_pitch, const void* x16, const uint8_t* bits, const void* low,
+                         const void* a16, const void* b16, float* dx, float* da, float* db, int add_dx, int add_da,
+                         int add_db, float keep_scale, float g_scale, float db_alpha, void* workspace,
+                         int64_t workspace_bytes, int64_t rows, int64_t in, int64_t out, int64_t rank,
+                         void* stream);
+/* fp16 copies of an adapter's two weights (n_a and n_b elements, multiples of 8) in one launch. */
+int soup_lora_cast(const void* a, const void* b, void* a16, void* b16, int64_t n_a, int64_t n_b, int a_dtype,
+                   int b_dtype, void* stream);
+
 /* The rows [q | k | v] of a q/k/v projection (fp16, row pitch qkv_pitch) as rotated q (+ add_q), rotated
  * k and v (+ add_v): fp16 [n, h, d] contiguous, sums and rotation in fp32, one rounding. add_q [n, hq*d]
  * and add_v [n, hk*d] fp16 contiguous or NULL; cos, sin fp32 [n, d]. One launch for what the reference

@@ -736,6 +736,43 @@ def test_lora_branch_with_cast_scaled_weights_and_in_place_gradients(scaling, mo
         assert rel_norm(fast.float().cpu(), plain.float().cpu()) < 2e-3, name
 
 
+@pytest.mark.parametrize("rows", [1, 15, 17, 1000])
+@pytest.mark.parametrize("width,out", [(32, 8), (96, 40), (1568, 520)])
+@pytest.mark.parametrize("scaling,given", [(2.0, False), (0.3, False), (0.3, True)])
+def test_rank16_branch_at_the_edges_of_its_tiles(rows, width, out, scaling, given):
+    """Against the products in float64 with fp16 roundings where those have them: row tiles, strips and
+    chunks with remainders, a gradient row pitch of its own. Bounds: one fp16 ulp of the largest value per
+    rounding that may go the other way (2^-10; two of them, the product and its scaling, in the output and in dx),
+    fp32 sums (1e-4) of terms whose factors may round the other way."""
+    from claudemaxing_b200.lora import LoRABranch
+
+    gen = torch.Generator().manual_seed(rows + width)
+    x = torch.randn(1, rows, width, generator=gen).to(DEV).requires_grad_()
+    a, b = (((torch.randn(*shape, generator=gen) * 0.1).to(DEV)).requires_grad_() for shape in ((16, width), (out, 16)))
+    g = torch.randn(1, rows, out + 8, generator=gen).half().to(DEV)[..., :out]
+    a16, b16 = a.detach().half(), ((b.detach() * scaling) if given else b.detach()).half()
+    torch.manual_seed(3)
+    got = LoRABranch.apply(x, x.detach().half(), a, b, 0.1, scaling, *((a16, b16, True) if given else ()))
+    got.backward(g)
+    torch.manual_seed(3)
+    mask = torch.native_dropout(x.detach(), 0.1, True)[1][0]
+    keep = mask / 0.9
+    f64 = lambda t: t.detach().double()
+    once = lambda t: t.half().double()
+    xd = once(mask * (x.detach()[0] * (1 / 0.9)))
+    low = once(xd @ f64(a16).t())
+    outer = 1.0 if given else scaling
+    want = once(once(low @ f64(b16).t()) * outer)
+    gs = once(f64(g[0]) * outer)
+    gain = once(gs @ f64(b16))
+    want_dx = once(gain @ f64(a16)) * keep.double()
+    x16d = once(mask * (x.detach().half()[0].float() * (1 / 0.9)))
+    assert_close_rel_max(got.detach()[0], want.half(), 2 ** -9, "out")
+    assert_close_rel_max(x.grad[0], want_dx.float(), 2 ** -9, "dx")
+    assert_close_rel_max(a.grad, (gain.t() @ x16d).float(), 2 ** -10, "dA")
+    assert_close_rel_max(b.grad, (gs.t() @ low * (scaling if given else 1.0)).float(), 2 ** -10, "dB")
+
+
 def test_paired_lora_branches_are_the_two_single_branches():
     """LoRABranchPair (one packing launch, one batched product with A, one unpacking launch that
     sums the input gradients) against two LoRABranch calls with the same dropout draws: outputs
