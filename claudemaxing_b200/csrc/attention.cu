@@ -392,19 +392,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 //   S^T = K Q^T, dP^T = V dO^T               tensor-memory columns 0-127 / 128-255
 //   P^T = exp2(scale S^T - lse)              two compute warpgroups (64 query columns each), fp16 over S^T
 //   dV += P^T dO                             A from tensor memory, columns 256-383
-//   dS^T = P^T (dP^T - D)                    fp16 over dP^T, and to shared memory
-//   dK += dS^T Q                             A from tensor memory, columns 384-511
+//   dS^T = P^T (dP^T - D)                    fp16 to shared memory
 //   dQ  = dS K                               A from shared memory, over dP^T's columns; a third
 //                                            warpgroup adds it to fp32 global memory (bulk reductions)
+//   dK += dS^T Q                             A from shared memory, columns 384-511, while dQ is read out
 // The score product of the next tile is issued as soon as dV has consumed P^T, so the exponentials of
-// tile i + 1 run under the dK / dQ products of tile i. dK and dV leave once per CTA.
+// tile i + 1 run under the dQ / dK products of tile i. dK and dV leave once per CTA.
 //
-// What bounds it: the chain of hand-overs of a tile, one CTA per SM deep. 9215 tokens in 4 segments take
-// about 7000 clocks a tile, the tensor pipe active 37 % of them; the products need 2560, and shared memory
-// 3750 by count: they read 256 KB of operands per tile (S^T and dP^T and dQ both operands, dV and dK one),
-// staging and loads move 224 KB more, at 128 B a clock. (A query-stationary walk reads and moves 700 KB per
-// tile: it stages and adds dK and dV, 128 KB, where this one adds dQ, 64 KB. It took 35.8 us for 1280
-// tokens in 5 segments, 12 / 2 heads, and 790 us for 9215 tokens in 4; this one 22.8 and 300 us.)
+// What bounds it: shared memory, at 128 B a clock. A tile's products read 288 KB of operands (S^T, dP^T, dQ and dK
+// both of theirs, dV one), loads, dS^T and the staging of dQ move 224 KB more and the rows' statistics 32: 4250
+// clocks by count, about 5200 measured between tiles (9215 tokens in 4 segments: 266 us), and the thread that
+// issues the products waits on none of the warps for long. The tensor core needs 2560. With dS^T in tensor memory as
+// dK's operand 32 KB fewer are read, but dQ, over the same columns, has to wait for dK and the next dP^T for both:
+// 5600 clocks, 290 us. (A query-stationary walk reads and moves 700 KB per tile: it stages and adds dK and dV, 128
+// KB, where this one adds dQ, 64 KB. It took 35.8 us for 1280 tokens in 5 segments, 12 / 2 heads, and 790 us for
+// 9215 tokens in 4; this one 20 and 266 us.)
 // ------------------------------------------------------------------------------------------
 constexpr int kBwdThreads = 448;   // warps 0-7 compute, 8-11 dQ, 12 loads, 13 products
 constexpr int kDqWarp = 8, kBwdLoadWarp = 12, kBwdMmaWarp = 13;
@@ -417,7 +419,7 @@ struct KvSmem {
   uint8_t d_o[kTileBytes];
   uint8_t ds[kTileBytes];      // dS^T [key rows x query columns]
   uint8_t stage[4][8192];      // per dQ warp two 32 x 32 fp32 boxes
-  float2 stats[2][kBQ];        // (lse * log2 e, D) of the query tile's rows
+  float lse[2][kBQ], d[2][kBQ];   // lse * log2 e and D of the query tile's rows
   uint64_t k_full, v_full, q_full[2], q_empty[2], do_full, do_empty, s_full, p_full, dp_full, ds_full,
       dq_full, dq_free, stats_full[2], done;
   uint32_t tmem_base;
@@ -485,32 +487,37 @@ __device__ __forceinline__ void write_box_row(uint8_t* box, int lane, const uint
 // One query tile for one compute thread: key row r, query columns [64 * wg, 64 * wg + 64).
 struct ComputeTile {
   uint32_t s_addr, dp_addr;   // this thread's lane, columns of its warpgroup
-  const float2* stats;        // its 64 columns
+  const float *lse, *d;       // of its 64 columns
   uint8_t* ds_box;            // its 64-column box of dS^T
   int r;
 };
 
 template <bool DIAG>
 __device__ __forceinline__ void probabilities(const ComputeTile& t, int first_col, float sl, float (&p)[64]) {
+  uint32_t x[2][32];
+  tmem_ld_32x32(t.s_addr, x[0]);
+  tmem_ld_32x32(t.s_addr + 32, x[1]);
+  tmem_ld_wait_on(x[0]);
+  tmem_ld_wait_on(x[1]);
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
-    uint32_t x[32], packed[16];
-    tmem_ld_32x32(t.s_addr + c * 32, x);
-    tmem_ld_wait_on(x);
+    uint32_t packed[16];
 #pragma unroll
-    for (int j = 0; j < 32; j += 2) {
-      // (lse, D) of two columns at a time; every thread of the warpgroup reads the same ones
-      const float4 st = *reinterpret_cast<const float4*>(t.stats + c * 32 + j);
-      float p0 = exp2f(fmaf(__uint_as_float(x[j]), sl, -st.x));
-      float p1 = exp2f(fmaf(__uint_as_float(x[j + 1]), sl, -st.z));
-      if (DIAG) {   // a query sees the keys up to its own row
-        if (first_col + c * 32 + j < t.r) p0 = 0.f;
-        if (first_col + c * 32 + j + 1 < t.r) p1 = 0.f;
+    for (int j = 0; j < 32; j += 4) {
+      // four columns' lse at a time; every thread of the warpgroup reads the same ones
+      const float4 l = *reinterpret_cast<const float4*>(t.lse + c * 32 + j);
+      const float neg[4] = {-l.x, -l.y, -l.z, -l.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        float v = exp2f(fmaf(__uint_as_float(x[c][j + k]), sl, neg[k]));
+        if (DIAG && first_col + c * 32 + j + k < t.r) v = 0.f;   // a query sees the keys up to its own row
+        p[c * 32 + j + k] = v;
       }
-      p[c * 32 + j] = p0;
-      p[c * 32 + j + 1] = p1;
-      __half2 hh = __floats2half2_rn(p0, p1);
-      packed[j >> 1] = *reinterpret_cast<uint32_t*>(&hh);
+#pragma unroll
+      for (int k = 0; k < 4; k += 2) {
+        __half2 hh = __floats2half2_rn(p[c * 32 + j + k], p[c * 32 + j + k + 1]);
+        packed[(j + k) >> 1] = *reinterpret_cast<uint32_t*>(&hh);
+      }
     }
     tmem_st_32x16(t.s_addr + c * 16, packed);
   }
@@ -518,26 +525,26 @@ __device__ __forceinline__ void probabilities(const ComputeTile& t, int first_co
 }
 
 __device__ __forceinline__ void score_gradients(const ComputeTile& t, const float (&p)[64]) {
+  uint8_t* row = t.ds_box + t.r * 128;
 #pragma unroll
   for (int c = 0; c < 2; ++c) {
     uint32_t y[32], packed[16];
     tmem_ld_32x32(t.dp_addr + c * 32, y);
     tmem_ld_wait_on(y);
 #pragma unroll
-    for (int j = 0; j < 32; j += 2) {
-      const float4 st = *reinterpret_cast<const float4*>(t.stats + c * 32 + j);
-      const float p0 = p[c * 32 + j], p1 = p[c * 32 + j + 1];
-      __half2 hh = __floats2half2_rn(p0 * (__uint_as_float(y[j]) - st.y), p1 * (__uint_as_float(y[j + 1]) - st.w));
-      packed[j >> 1] = *reinterpret_cast<uint32_t*>(&hh);
+    for (int j = 0; j < 32; j += 4) {
+      const float4 d = *reinterpret_cast<const float4*>(t.d + c * 32 + j);
+      const int at = c * 32 + j;
+      __half2 lo = __floats2half2_rn(p[at] * (__uint_as_float(y[j]) - d.x), p[at + 1] * (__uint_as_float(y[j + 1]) - d.y));
+      __half2 hi = __floats2half2_rn(p[at + 2] * (__uint_as_float(y[j + 2]) - d.z), p[at + 3] * (__uint_as_float(y[j + 3]) - d.w));
+      packed[j >> 1] = *reinterpret_cast<uint32_t*>(&lo);
+      packed[(j >> 1) + 1] = *reinterpret_cast<uint32_t*>(&hi);
     }
-    tmem_st_32x16(t.dp_addr + c * 16, packed);
-    uint8_t* row = t.ds_box + t.r * 128;
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       *reinterpret_cast<uint4*>(row + (((c * 4 + j) ^ (t.r & 7)) << 4)) =
           make_uint4(packed[4 * j], packed[4 * j + 1], packed[4 * j + 2], packed[4 * j + 3]);
   }
-  tmem_st_wait();
 }
 
 __global__ void __launch_bounds__(kBwdThreads, 1)
@@ -617,7 +624,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       const uint64_t v_k = make_smem_desc(smem_u32(s.v), 16, 1024);
       const uint64_t do_k = make_smem_desc(smem_u32(s.d_o), 16, 1024);
       const uint64_t do_mn = make_smem_desc(smem_u32(s.d_o), kBox, 1024);
-      const uint64_t ds_mn = make_smem_desc(smem_u32(s.ds), kBox, 1024);
+      const uint64_t ds_mn = make_smem_desc(smem_u32(s.ds), kBox, 1024), ds_k = make_smem_desc(smem_u32(s.ds), 16, 1024);
       auto wait = [&](uint64_t* bar, int turn, int code) {
         const bool got = mbar_wait(bar, turn & 1, abort_flag, a.status, code);
         tc_fence_after_sync();
@@ -660,13 +667,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         if (!ok) break;
         const uint64_t q_mn = make_smem_desc(smem_u32(s.q[i & 1]), kBox, 1024);
 #pragma unroll
-        for (int k8 = 0; k8 < 8; ++k8)
-          mma_f16_ts(tmem + kColDk, tmem + kColP + packed_col(k8), q_mn + k8 * (2048 >> 4), idesc_nt, (i | k8) != 0);
-        tc_commit(&s.q_empty[i & 1]);
-#pragma unroll
-        for (int k8 = 0; k8 < 8; ++k8)   // over the columns of dS^T, which the products above have read
+        for (int k8 = 0; k8 < 8; ++k8)   // over the columns of dP^T, which the compute warps have read
           mma_f16_ss(tmem + kColP, ds_mn + k8 * (2048 >> 4), k_mn + k8 * (2048 >> 4), idesc_tt, k8 != 0);
         tc_commit(&s.dq_full);
+#pragma unroll
+        for (int k8 = 0; k8 < 8; ++k8)   // while dQ is read out
+          mma_f16_ss(tmem + kColDk, ds_k + kstep(k8), q_mn + k8 * (2048 >> 4), idesc_nt, (i | k8) != 0);
+        tc_commit(&s.q_empty[i & 1]);
         if (more) {
           ok = wait(&s.do_full, i + 1, 70) && wait(&s.dq_free, i, 71);
           if (ok) d_prob();
@@ -684,7 +691,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       return i < n_q && token < tile.seg_end ? stats[token] : make_float2(INFINITY, 0.f);
     };
     auto put = [&](int i, float2 v) {
-      s.stats[i & 1][r] = v;
+      s.lse[i & 1][r] = v.x;
+      s.d[i & 1][r] = v.y;
       __syncwarp();
       if (lane == 0) mbar_arrive(&s.stats_full[i & 1]);
     };
@@ -736,7 +744,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const float sl = a.scale_log2;
     bool ok = true;
     for (int i = 0; i < n_q; ++i) {
-      t.stats = s.stats[i & 1] + wg * 64;
+      t.lse = s.lse[i & 1] + wg * 64;
+      t.d = s.d[i & 1] + wg * 64;
       ok = mbar_wait(&s.stats_full[i & 1], (i >> 1) & 1, abort_flag, a.status, 73) &&
            mbar_wait(&s.s_full, i & 1, abort_flag, a.status, 74);
       ok = __all_sync(0xffffffffu, ok);
