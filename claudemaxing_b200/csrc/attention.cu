@@ -10,7 +10,8 @@
 // 117 us for 9215 tokens in 4 segments, but the largest P is then no longer 1, which fp16 holds exactly,
 // and the output's error against float64 rises by up to a tenth on peaked rows.) The score product of
 // the next tile is issued right behind O += P V of this one; the commit that announces it also says that
-// O may be rescaled.
+// O may be rescaled, which happens behind the exponentials, when the scores' registers are free to hold the
+// whole row of O (ahead of them it went 16 columns at a time: 127.5 against 121.2 us).
 //
 // What bounds it: on long walks the exponentials (16 a clock and SM: 1024 clocks a tile) and the
 // two products (1024 clocks a tile) alternate, so two tiles must be in flight on an SM. NT = 2 does
@@ -168,28 +169,20 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, i
       mx[j & 3] = fmaxf(mx[j & 3], __uint_as_float(x[c][j]));
     }
   const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+  float f = 1.f;
+  bool rescale = false;   // of the whole warp
   if (first) {
     ref.set(top, scale, scale_far);
   } else {
     const bool grow = __fmul_rn(top, ref.sl) > ref.msl;
-    if (__any_sync(0xffffffffu, grow)) {
-      float f = 1.f;
+    rescale = __any_sync(0xffffffffu, grow);
+    if (rescale) {
       if (grow) {   // from one reference, as it was used, to the next; a far one is left behind by 2^4 at least
         const float old = fabsf(ref.msl) < kFarScore ? ref.msl : -INFINITY;
         ref.set(top, scale, scale_far);
         f = exp2f(fabsf(ref.msl) < kFarScore ? old - ref.msl : -fmaf(top, scale, -old));
       }
       l *= f;
-#pragma unroll 1
-      for (int c = 0; c < kD; c += 16) {
-        uint32_t o[16];
-        tmem_ld_32x16(o_addr + c, o);
-        tmem_ld_wait_on(o);
-#pragma unroll
-        for (int j = 0; j < 16; ++j) o[j] = __float_as_uint(__uint_as_float(o[j]) * f);
-        tmem_st_32x16(o_addr + c, o);
-      }
-      tmem_st_wait();
     }
   }
   float s[4] = {0.f, 0.f, 0.f, 0.f};
@@ -208,6 +201,18 @@ __device__ __forceinline__ void softmax_tile(uint32_t s_addr, uint32_t o_addr, i
     tmem_st_32x16(s_addr + c * 16, packed);
   }
   l += (s[0] + s[1]) + (s[2] + s[3]);
+  if (rescale) {   // the scores' registers are free now: all of O's row is on its way at once
+    uint32_t o[4][32];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) tmem_ld_32x32(o_addr + c * 32, o[c]);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      tmem_ld_wait_on(o[c]);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) o[c][j] = __float_as_uint(__uint_as_float(o[c][j]) * f);
+      tmem_st_32x32(o_addr + c * 32, o[c]);
+    }
+  }
   tmem_st_wait();
 }
 
