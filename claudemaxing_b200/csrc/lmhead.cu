@@ -62,8 +62,20 @@ constexpr int kBN = 256;          // columns per tile (vocabulary for logits, hi
 constexpr int kBK = 64;           // 64 16-bit elements = one 128-byte swizzle row
 constexpr int kABytes = kBM * kBK * 2;            // 16 KB: this CTA's rows of the A operand
 constexpr int kBHalfBytes = (kBN / 2) * kBK * 2;  // 16 KB: this CTA's half of the B operand
-constexpr int kStageBytes = kABytes + kBHalfBytes;
-constexpr int kStages = 6;
+constexpr int kRingBytes = 192 * 1024;
+// A row block of up to 128 rows runs on single CTAs (128 x 256 tiles, a whole B operand per stage): half of a
+// pair's tile would be padding, and with padding at 85 us of products a launch the weight's 72 us no
+// longer bound it (128 rows x 151936, a training pass: 278 -> 246 us). More rows take CTA pairs, which read
+// every operand byte half as often.
+template <bool PAIR>
+struct Unit {
+  static constexpr int kRows = PAIR ? 2 * kBM : kBM;    // rows of a tile
+  static constexpr int kCtas = PAIR ? 2 : 1;
+  static constexpr int kBBoxes = PAIR ? 1 : 2;          // 128-column (or -row) boxes of B per CTA
+  static constexpr int kStageBytes = kABytes + kBBoxes * kBHalfBytes;
+  static constexpr int kStages = kRingBytes / kStageBytes;   // 6 or 4
+};
+constexpr int kMaxStages = Unit<true>::kStages;
 constexpr int kThreadsGemm = 192;  // warp 0 TMA, warp 1 MMA, warps 2-5 epilogue
 constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kGradScale = 1024.0f;  // as GRAD_SCALE of the reference
@@ -75,8 +87,8 @@ constexpr int kEW = 16;                // accumulator columns per tcgen05.ld in 
 
 constexpr int kStageP = 4 * 2 * 4096;          // logits: per epilogue warp two 32 x 64 bf16 boxes
 constexpr int kStageT = 4 * 2 * 4096;          // gradient: per epilogue warp two 32 x 32 fp32 boxes
-constexpr int kSmemLogits = kStages * kStageBytes + kStageP + 1024 + 256;
-constexpr int kSmemGrad = kStages * kStageBytes + kStageT + 1024 + 256;
+constexpr int kSmemLogits = kRingBytes + kStageP + 1024 + 256;
+constexpr int kSmemGrad = kRingBytes + kStageT + 1024 + 256;
 
 // Waits until all of this thread's bulk stores have completed (written, not only read).
 __device__ __forceinline__ void tma_store_wait_done() {
@@ -98,19 +110,20 @@ __device__ __forceinline__ bool is_hot(float tile_max, float ref) {
   return tile_max > __fadd_rn(ref, kHot);
 }
 
+template <bool PAIR>
 struct PipeState {
   int stage = 0;
   uint32_t phase = 0;
   __device__ __forceinline__ void advance() {
-    if (++stage == kStages) { stage = 0; phase ^= 1u; }
+    if (++stage == Unit<PAIR>::kStages) { stage = 0; phase ^= 1u; }
   }
 };
 
 struct GemmSmem {
   uint8_t* tiles;        // 1024-byte aligned
   uint8_t* extra;        // kernel-specific staging area behind the stages
-  uint64_t* full;        // [kStages]  (used in the leader CTA)
-  uint64_t* empty;       // [kStages]
+  uint64_t* full;        // [kMaxStages]  (used in the leader CTA)
+  uint64_t* empty;       // [kMaxStages]
   uint64_t* acc_full;    // [2]
   uint64_t* acc_empty;   // [2]        (used in the leader CTA)
   uint32_t* tmem_base;
@@ -122,13 +135,13 @@ __device__ __forceinline__ GemmSmem carve_smem(uint8_t* raw) {
   GemmSmem s;
   const uintptr_t base = (reinterpret_cast<uintptr_t>(raw) + 1023u) & ~static_cast<uintptr_t>(1023u);
   s.tiles = reinterpret_cast<uint8_t*>(base);
-  s.extra = s.tiles + kStages * kStageBytes;  // 1024-byte aligned
+  s.extra = s.tiles + kRingBytes;  // 1024-byte aligned
   uint64_t* bars = reinterpret_cast<uint64_t*>(s.extra + EXTRA_BYTES);
   s.full = bars;
-  s.empty = bars + kStages;
-  s.acc_full = bars + 2 * kStages;
-  s.acc_empty = bars + 2 * kStages + 2;
-  s.tmem_base = reinterpret_cast<uint32_t*>(bars + 2 * kStages + 4);
+  s.empty = bars + kMaxStages;
+  s.acc_full = bars + 2 * kMaxStages;
+  s.acc_empty = bars + 2 * kMaxStages + 2;
+  s.tmem_base = reinterpret_cast<uint32_t*>(bars + 2 * kMaxStages + 4);
   s.abort_flag = reinterpret_cast<int*>(s.tmem_base + 1);
   return s;
 }
@@ -146,25 +159,36 @@ struct PairInit {
 
 // Barrier set-up, tensor-memory allocation and the agreement of both CTAs on whether to run at all
 // (an earlier kernel of the call may have given up). Every thread of both CTAs calls this.
-__device__ __forceinline__ PairInit init_pair(const GemmSmem& s, int warp, int lane, const int* status) {
+template <bool PAIR>
+__device__ __forceinline__ PairInit init_unit(const GemmSmem& s, int warp, int lane, const int* status) {
   PairInit r;
-  r.rank = cluster_ctarank();
+  r.rank = PAIR ? cluster_ctarank() : 0;
   if (warp == 0 && lane == 0) {
-    for (int i = 0; i < kStages; ++i) { mbar_init(&s.full[i], 1); mbar_init(&s.empty[i], 1); }
-    for (int i = 0; i < 2; ++i) { mbar_init(&s.acc_full[i], 1); mbar_init(&s.acc_empty[i], 8); }
+    for (int i = 0; i < Unit<PAIR>::kStages; ++i) { mbar_init(&s.full[i], 1); mbar_init(&s.empty[i], 1); }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s.acc_full[i], 1); mbar_init(&s.acc_empty[i], 4 * Unit<PAIR>::kCtas); }
     *s.abort_flag = *reinterpret_cast<const volatile int*>(status) != 0;
     fence_barrier_init();
   }
   __syncthreads();
-  cluster_sync_all();
-  // the leader's view decides for the pair
-  r.run = ld_shared_cluster_s32(mapa_u32(smem_u32(s.abort_flag), 0)) == 0;
-  cluster_sync_all();  // nobody leaves (or rewrites the flag) while the peer may still read it
+  if (PAIR) {
+    cluster_sync_all();
+    // the leader's view decides for the pair
+    r.run = ld_shared_cluster_s32(mapa_u32(smem_u32(s.abort_flag), 0)) == 0;
+    cluster_sync_all();  // nobody leaves (or rewrites the flag) while the peer may still read it
+  } else {
+    r.run = *reinterpret_cast<volatile int*>(s.abort_flag) == 0;
+    __syncthreads();
+  }
   if (!r.run) { r.tmem = 0; return r; }
   if (warp == 0 && lane == 0) *s.abort_flag = 0;
   if (warp == 1) {
-    tmem_alloc_pair(s.tmem_base, 512);
-    tmem_relinquish_pair();
+    if (PAIR) {
+      tmem_alloc_pair(s.tmem_base, 512);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(s.tmem_base, 512);
+      tmem_relinquish();
+    }
   }
   tc_fence_before_sync();
   __syncthreads();
@@ -173,7 +197,8 @@ __device__ __forceinline__ PairInit init_pair(const GemmSmem& s, int warp, int l
   return r;
 }
 
-__device__ __forceinline__ void finish_pair(const GemmSmem& s, int warp, uint32_t tmem, int* status,
+template <bool PAIR>
+__device__ __forceinline__ void finish_unit(const GemmSmem& s, int warp, uint32_t tmem, int* status,
                                             int* sticky) {
   tc_fence_before_sync();
   __syncthreads();
@@ -187,11 +212,35 @@ __device__ __forceinline__ void finish_pair(const GemmSmem& s, int warp, uint32_
   }
   // The leader's MMAs read the peer's shared memory and both CTAs signal each other's barriers:
   // neither may exit before the other is done.
-  cluster_sync_all();
+  if (PAIR) cluster_sync_all();
   if (warp == 1) {
     tc_fence_after_sync();
-    tmem_dealloc_pair(tmem, 512);
+    if (PAIR) tmem_dealloc_pair(tmem, 512);
+    else tmem_dealloc(tmem, 512);
   }
+}
+
+// A ring stage's barrier as the loads count on it (the leader's, for a pair), with its bytes announced.
+template <bool PAIR>
+__device__ __forceinline__ uint32_t announce_stage(uint64_t* full, uint32_t rank) {
+  if (rank == 0) mbar_expect_tx(full, Unit<PAIR>::kCtas * Unit<PAIR>::kStageBytes);
+  return PAIR ? mapa_u32(smem_u32(full), 0) : smem_u32(full);
+}
+template <bool PAIR>
+__device__ __forceinline__ void load_box(void* dst, const CUtensorMap* map, int c0, int c1, uint64_t* full,
+                                         uint32_t full_leader) {
+  if (PAIR) tma_load_2d_pair(dst, map, c0, c1, full_leader);
+  else tma_load_2d(dst, map, c0, c1, full);
+}
+template <bool PAIR>
+__device__ __forceinline__ void mma_step(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+  if (PAIR) mma_f16_ss_pair(d, da, db, idesc, accumulate);
+  else mma_f16_ss(d, da, db, idesc, accumulate);
+}
+template <bool PAIR>
+__device__ __forceinline__ void commit_to(uint64_t* bar) {   // in both CTAs of a pair
+  if (PAIR) tc_commit_pair(bar, 3);
+  else tc_commit(bar);
 }
 
 __device__ __forceinline__ void release_accumulator(const GemmSmem& s, int ab, uint32_t rank, int lane) {
@@ -418,11 +467,11 @@ __device__ __noinline__ void tile_ref_pass(uint32_t taddr, int n_valid, int labe
   arg_out = arg;
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsGemm, 1)
-lmhead_logits_kernel(const __grid_constant__ CUtensorMap map_h,
-                     const __grid_constant__ CUtensorMap map_w,
-                     const __grid_constant__ CUtensorMap map_p, const LogitsArgs a) {
+template <bool PAIR>
+__device__ __forceinline__ void logits_body(const CUtensorMap& map_h, const CUtensorMap& map_w,
+                                            const CUtensorMap& map_p, const LogitsArgs& a) {
   extern __shared__ uint8_t smem_raw[];
+  using U = Unit<PAIR>;
   const GemmSmem s = carve_smem<kStageP>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0 && lane == 0) {
@@ -430,42 +479,43 @@ lmhead_logits_kernel(const __grid_constant__ CUtensorMap map_h,
     prefetch_tensormap(&map_w);
     prefetch_tensormap(&map_p);
   }
-  const PairInit pi = init_pair(s, warp, lane, a.status);
+  const PairInit pi = init_unit<PAIR>(s, warp, lane, a.status);
   if (!pi.run) return;
   const uint32_t tmem = pi.tmem, rank = pi.rank;
-  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  const int pair = blockIdx.x / U::kCtas, n_pairs = gridDim.x / U::kCtas;
 
   // Tiles are ordered row-tile-fastest: the row tiles that share a weight tile run together, so
   // the weight streams from HBM once.
-  const int rt = (a.n_rows + 2 * kBM - 1) / (2 * kBM);   // 256-row tiles
+  const int rt = (a.n_rows + U::kRows - 1) / U::kRows;   // row tiles
   const int n_tiles = rt * a.ct;
   const int n_kb = (a.k_dim + kBK - 1) / kBK;
 
   if (warp == 0) {
     if (lane == 0) {
-      PipeState p;
+      PipeState<PAIR> p;
       bool ok = true;
       for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
         const int tr = tile % rt, tc = tile / rt;
-        const int row0 = a.row0 + tr * 2 * kBM + (int)rank * kBM;
+        const int row0 = a.row0 + tr * U::kRows + (int)rank * kBM;
         const int col0 = a.col0 + tc * kBN + (int)rank * (kBN / 2);
         for (int kb = 0; kb < n_kb; ++kb) {
           ok = mbar_wait(&s.empty[p.stage], p.phase ^ 1u, s.abort_flag, a.status, 11);
           if (!ok) break;
-          uint8_t* st = s.tiles + p.stage * kStageBytes;
-          // both CTAs' bytes are counted on the leader's barrier
-          const uint32_t full_leader = mapa_u32(smem_u32(&s.full[p.stage]), 0);
-          if (rank == 0) mbar_expect_tx(&s.full[p.stage], 2 * kStageBytes);
-          tma_load_2d_pair(st, &map_h, kb * kBK, row0, full_leader);
-          tma_load_2d_pair(st + kABytes, &map_w, kb * kBK, col0, full_leader);
+          uint8_t* st = s.tiles + p.stage * U::kStageBytes;
+          uint64_t* full = &s.full[p.stage];
+          const uint32_t full_leader = announce_stage<PAIR>(full, rank);
+          load_box<PAIR>(st, &map_h, kb * kBK, row0, full, full_leader);
+#pragma unroll
+          for (int j = 0; j < U::kBBoxes; ++j)
+            load_box<PAIR>(st + kABytes + j * kBHalfBytes, &map_w, kb * kBK, col0 + j * (kBN / 2), full, full_leader);
           p.advance();
         }
       }
     }
   } else if (warp == 1) {
     if (lane == 0 && rank == 0) {
-      constexpr uint32_t idesc = make_idesc_f16(2 * kBM, kBN, kFmtF16, kFmtF16, false, false);
-      PipeState p;
+      constexpr uint32_t idesc = make_idesc_f16(U::kRows, kBN, kFmtF16, kFmtF16, false, false);
+      PipeState<PAIR> p;
       bool ok = true;
       int it = 0;
       for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++it) {
@@ -479,16 +529,16 @@ lmhead_logits_kernel(const __grid_constant__ CUtensorMap map_h,
           ok = mbar_wait(&s.full[p.stage], p.phase, s.abort_flag, a.status, 13);
           if (!ok) break;
           tc_fence_after_sync();
-          const uint32_t a_addr = smem_u32(s.tiles + p.stage * kStageBytes);
+          const uint32_t a_addr = smem_u32(s.tiles + p.stage * U::kStageBytes);
           const uint64_t da = make_smem_desc(a_addr, 16, 1024);
           const uint64_t db = make_smem_desc(a_addr + kABytes, 16, 1024);
 #pragma unroll
           for (int k4 = 0; k4 < kBK / 16; ++k4)
-            mma_f16_ss_pair(d_tmem, da + k4 * 2, db + k4 * 2, idesc, (kb | k4) != 0);
-          tc_commit_pair(&s.empty[p.stage], 3);   // frees the stage in both CTAs
+            mma_step<PAIR>(d_tmem, da + k4 * 2, db + k4 * 2, idesc, (kb | k4) != 0);
+          commit_to<PAIR>(&s.empty[p.stage]);   // frees the stage
           p.advance();
         }
-        if (ok) tc_commit_pair(&s.acc_full[ab], 3);
+        if (ok) commit_to<PAIR>(&s.acc_full[ab]);
       }
     }
   } else {
@@ -504,7 +554,7 @@ lmhead_logits_kernel(const __grid_constant__ CUtensorMap map_h,
       ok = __all_sync(0xffffffffu, mbar_wait(&s.acc_full[ab], acc_phase, s.abort_flag, a.status, 14));
       if (!ok) break;
       tc_fence_after_sync();
-      const int p_row0 = tr * 2 * kBM + (int)rank * kBM + q * 32;   // row inside the row block
+      const int p_row0 = tr * U::kRows + (int)rank * kBM + q * 32;   // row inside the row block
       const int row = p_row0 + lane;
       const bool row_ok = row < a.n_rows;
       const int tile_col0 = a.col0 + tc * kBN;                      // column inside the shard
@@ -582,7 +632,18 @@ lmhead_logits_kernel(const __grid_constant__ CUtensorMap map_h,
     }
     if (lane == 0) tma_store_wait_read<0>();  // staging boxes fully read before shared memory goes away
   }
-  finish_pair(s, warp, tmem, a.status, a.sticky);
+  finish_unit<PAIR>(s, warp, tmem, a.status, a.sticky);
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsGemm, 1)
+lmhead_logits_kernel(const __grid_constant__ CUtensorMap map_h, const __grid_constant__ CUtensorMap map_w,
+                     const __grid_constant__ CUtensorMap map_p, const LogitsArgs a) {
+  logits_body<true>(map_h, map_w, map_p, a);
+}
+__global__ void __launch_bounds__(kThreadsGemm, 1)
+lmhead_logits_single_kernel(const __grid_constant__ CUtensorMap map_h, const __grid_constant__ CUtensorMap map_w,
+                            const __grid_constant__ CUtensorMap map_p, const LogitsArgs a) {
+  logits_body<false>(map_h, map_w, map_p, a);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -781,11 +842,11 @@ struct GradArgs {
   int* sticky;
 };
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsGemm, 1)
-lmhead_grad_kernel(const __grid_constant__ CUtensorMap map_p,
-                   const __grid_constant__ CUtensorMap map_w,
-                   const __grid_constant__ CUtensorMap map_dh, const GradArgs a) {
+template <bool PAIR>
+__device__ __forceinline__ void grad_body(const CUtensorMap& map_p, const CUtensorMap& map_w,
+                                          const CUtensorMap& map_dh, const GradArgs& a) {
   extern __shared__ uint8_t smem_raw[];
+  using U = Unit<PAIR>;
   const GemmSmem s = carve_smem<kStageT>(smem_raw);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (warp == 0 && lane == 0) {
@@ -793,12 +854,12 @@ lmhead_grad_kernel(const __grid_constant__ CUtensorMap map_p,
     prefetch_tensormap(&map_w);
     prefetch_tensormap(&map_dh);
   }
-  const PairInit pi = init_pair(s, warp, lane, a.status);
+  const PairInit pi = init_unit<PAIR>(s, warp, lane, a.status);
   if (!pi.run) return;
   const uint32_t tmem = pi.tmem, rank = pi.rank;
-  const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  const int pair = blockIdx.x / U::kCtas, n_pairs = gridDim.x / U::kCtas;
 
-  const int rt = (a.n_rows + 2 * kBM - 1) / (2 * kBM);
+  const int rt = (a.n_rows + U::kRows - 1) / U::kRows;
   const int nt = (a.k_dim + kBN - 1) / kBN;
   const int n_tiles = rt * nt;
   const int n_units = n_tiles * a.ksplit;
@@ -806,25 +867,24 @@ lmhead_grad_kernel(const __grid_constant__ CUtensorMap map_p,
 
   if (warp == 0) {
     if (lane == 0) {
-      PipeState p;
+      PipeState<PAIR> p;
       bool ok = true;
       for (int unit = pair; unit < n_units && ok; unit += n_pairs) {
         const int tile = unit % n_tiles, ks = unit / n_tiles;
         const int tr = tile % rt, tn = tile / rt;
-        const int row0 = tr * 2 * kBM + (int)rank * kBM;
+        const int row0 = tr * U::kRows + (int)rank * kBM;
         const int hcol0 = tn * kBN + (int)rank * (kBN / 2);
         const int kb_end = (a.n_kb * (ks + 1)) / a.ksplit;
         for (int kb = (a.n_kb * ks) / a.ksplit; kb < kb_end; ++kb) {
           ok = mbar_wait(&s.empty[p.stage], p.phase ^ 1u, s.abort_flag, a.status, 21);
           if (!ok) break;
-          uint8_t* st = s.tiles + p.stage * kStageBytes;
-          const uint32_t full_leader = mapa_u32(smem_u32(&s.full[p.stage]), 0);
-          if (rank == 0) mbar_expect_tx(&s.full[p.stage], 2 * kStageBytes);
-          tma_load_2d_pair(st, &map_p, kb * kBK, row0, full_leader);
+          uint8_t* st = s.tiles + p.stage * U::kStageBytes;
+          uint64_t* full = &s.full[p.stage];
+          const uint32_t full_leader = announce_stage<PAIR>(full, rank);
+          load_box<PAIR>(st, &map_p, kb * kBK, row0, full, full_leader);
 #pragma unroll
-          for (int j = 0; j < kBN / 2 / 64; ++j)
-            tma_load_2d_pair(st + kABytes + j * kBoxBytes, &map_w, hcol0 + j * 64, a.col0 + kb * kBK,
-                             full_leader);
+          for (int j = 0; j < U::kBBoxes * (kBN / 2 / 64); ++j)
+            load_box<PAIR>(st + kABytes + j * kBoxBytes, &map_w, hcol0 + j * 64, a.col0 + kb * kBK, full, full_leader);
           p.advance();
         }
       }
@@ -833,8 +893,8 @@ lmhead_grad_kernel(const __grid_constant__ CUtensorMap map_p,
     if (lane == 0 && rank == 0) {
       // A = P (K-major) and B = W (MN-major), both bf16: kind::f16 wants one element format for
       // both operands (a bf16 A with an fp16 B raises an illegal-instruction fault).
-      constexpr uint32_t idesc = make_idesc_f16(2 * kBM, kBN, kFmtBF16, kFmtBF16, false, true);
-      PipeState p;
+      constexpr uint32_t idesc = make_idesc_f16(U::kRows, kBN, kFmtBF16, kFmtBF16, false, true);
+      PipeState<PAIR> p;
       bool ok = true;
       int it = 0;
       for (int unit = pair; unit < n_units && ok; unit += n_pairs, ++it) {
@@ -850,19 +910,18 @@ lmhead_grad_kernel(const __grid_constant__ CUtensorMap map_p,
           ok = mbar_wait(&s.full[p.stage], p.phase, s.abort_flag, a.status, 23);
           if (!ok) break;
           tc_fence_after_sync();
-          const uint32_t a_addr = smem_u32(s.tiles + p.stage * kStageBytes);
+          const uint32_t a_addr = smem_u32(s.tiles + p.stage * U::kStageBytes);
           const uint64_t da = make_smem_desc(a_addr, 16, 1024);
           // MN-major B: the two 64-column boxes are kBoxBytes apart (leading offset), 8-k groups
           // 1024 bytes apart (stride offset); one MMA consumes 16 k = 2048 bytes.
           const uint64_t db = make_smem_desc(a_addr + kABytes, kBoxBytes, 1024);
 #pragma unroll
           for (int k4 = 0; k4 < kBK / 16; ++k4)
-            mma_f16_ss_pair(d_tmem, da + k4 * 2, db + k4 * (2048 >> 4), idesc,
-                            (kb != kb_begin) || k4 != 0);
-          tc_commit_pair(&s.empty[p.stage], 3);
+            mma_step<PAIR>(d_tmem, da + k4 * 2, db + k4 * (2048 >> 4), idesc, (kb != kb_begin) || k4 != 0);
+          commit_to<PAIR>(&s.empty[p.stage]);
           p.advance();
         }
-        if (ok) tc_commit_pair(&s.acc_full[ab], 3);
+        if (ok) commit_to<PAIR>(&s.acc_full[ab]);
       }
     }
   } else {
@@ -878,7 +937,7 @@ lmhead_grad_kernel(const __grid_constant__ CUtensorMap map_p,
       ok = __all_sync(0xffffffffu, mbar_wait(&s.acc_full[ab], acc_phase, s.abort_flag, a.status, 24));
       if (!ok) break;
       tc_fence_after_sync();
-      const int row_base = tr * 2 * kBM + (int)rank * kBM + q * 32;   // first of this warp's 32 rows
+      const int row_base = tr * U::kRows + (int)rank * kBM + q * 32;   // first of this warp's 32 rows
       const float my_mult = (row_base + lane < a.n_rows) ? a.mult[row_base + lane] : 0.f;
       const uint32_t taddr = tmem + (static_cast<uint32_t>(q * 32) << 16) + ab * kBN;
       const int col_base = tn * kBN;
@@ -910,7 +969,18 @@ lmhead_grad_kernel(const __grid_constant__ CUtensorMap map_p,
     }
     if (lane == 0) tma_store_wait_done();   // the sums have landed before the kernel ends
   }
-  finish_pair(s, warp, tmem, a.status, a.sticky);
+  finish_unit<PAIR>(s, warp, tmem, a.status, a.sticky);
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreadsGemm, 1)
+lmhead_grad_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_w,
+                   const __grid_constant__ CUtensorMap map_dh, const GradArgs a) {
+  grad_body<true>(map_p, map_w, map_dh, a);
+}
+__global__ void __launch_bounds__(kThreadsGemm, 1)
+lmhead_grad_single_kernel(const __grid_constant__ CUtensorMap map_p, const __grid_constant__ CUtensorMap map_w,
+                          const __grid_constant__ CUtensorMap map_dh, const GradArgs a) {
+  grad_body<false>(map_p, map_w, map_dh, a);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1256,12 +1326,10 @@ int ensure_smem_attr() {
   int major = 0;
   cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
   if (major != 10) return -2;
-  if (cudaFuncSetAttribute(lmhead_logits_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kSmemLogits) != cudaSuccess)
-    return -1;
-  if (cudaFuncSetAttribute(lmhead_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kSmemGrad) != cudaSuccess)
-    return -1;
+  for (const auto kernel : {lmhead_logits_kernel, lmhead_logits_single_kernel})
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLogits) != cudaSuccess) return -1;
+  for (const auto kernel : {lmhead_grad_kernel, lmhead_grad_single_kernel})
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemGrad) != cudaSuccess) return -1;
   g_attr_set[dev] = true;
   return 0;
 }
@@ -1406,7 +1474,9 @@ extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void
   LaunchTimer timer(s);
   for (int64_t r0 = 0; r0 < n; r0 += plan.row_block) {
     const int rows = (int)((n - r0) < plan.row_block ? (n - r0) : plan.row_block);
-    const int rt = (rows + 2 * kBM - 1) / (2 * kBM);
+    const bool single = rows <= kBM;
+    const int rt = (rows + 2 * kBM - 1) / (2 * kBM);   // one tile on single CTAs too
+    const int unit_ctas = single ? 1 : 2, workers = sms / unit_ctas;
     for (int t0 = 0; t0 < total_ct;) {
       const bool first = t0 == 0;
       const int want_ct = first ? plan.ct_first : plan.ct;
@@ -1428,11 +1498,12 @@ extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void
       la.status = ws.status;
       la.sticky = sticky;
       const int tiles1 = rt * ct;
-      const unsigned grid1 = 2u * (unsigned)(tiles1 < max_pairs ? tiles1 : max_pairs);
+      const unsigned grid1 = (unsigned)(unit_ctas * (tiles1 < workers ? tiles1 : workers));
 
       la.mode = first ? kModeTileMax : kModeCombined;
       timer.mark(0);
-      lmhead_logits_kernel<<<grid1, kThreadsGemm, kSmemLogits, s>>>(map_h, map_w_k, map_p_st, la);
+      (single ? lmhead_logits_single_kernel : lmhead_logits_kernel)<<<grid1, kThreadsGemm, kSmemLogits, s>>>(
+          map_h, map_w_k, map_p_st, la);
       timer.mark(0);
       SOUP_CHECK_LAUNCH("lmhead_logits");
 
@@ -1472,11 +1543,12 @@ extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void
         ga.status = ws.status;
         ga.sticky = sticky;
         const int tiles2 = rt * (int)((h + kBN - 1) / kBN);
-        ga.ksplit = pick_ksplit(tiles2, max_pairs, ga.n_kb, deterministic);
+        ga.ksplit = pick_ksplit(tiles2, workers, ga.n_kb, deterministic);
         const int units = tiles2 * ga.ksplit;
-        const unsigned grid2 = 2u * (unsigned)(units < max_pairs ? units : max_pairs);
+        const unsigned grid2 = (unsigned)(unit_ctas * (units < workers ? units : workers));
         timer.mark(2);
-        lmhead_grad_kernel<<<grid2, kThreadsGemm, kSmemGrad, s>>>(map_p_ld, map_w_mn, map_dh, ga);
+        (single ? lmhead_grad_single_kernel : lmhead_grad_kernel)<<<grid2, kThreadsGemm, kSmemGrad, s>>>(
+            map_p_ld, map_w_mn, map_dh, ga);
         timer.mark(2);
         SOUP_CHECK_LAUNCH("lmhead_grad");
       }
@@ -1509,11 +1581,11 @@ extern "C" int soup_lmhead_grad_units(int64_t n, int64_t h, int64_t v_shard, int
   const Plan p = make_plan(n, v_shard, sm_count(), (int)chunk_tiles);
   const int total_ct = (int)((v_shard + kBN - 1) / kBN), rest = total_ct - p.ct_first;
   const int tiles = (p.row_block + 2 * kBM - 1) / (2 * kBM) * (int)((h + kBN - 1) / kBN);
-  const int max_pairs = sm_count() / 2;
-  auto units = [&](int ct) { return ct > 0 ? tiles * pick_ksplit(tiles, max_pairs, ct * (kBN / kBK), false) : 0; };
+  const int workers = sm_count() / (p.row_block <= kBM ? 1 : 2);
+  auto units = [&](int ct) { return ct > 0 ? tiles * pick_ksplit(tiles, workers, ct * (kBN / kBK), false) : 0; };
   if (first_chunk) *first_chunk = units(p.ct_first);
   if (later_chunk) *later_chunk = units(rest < p.ct ? rest : p.ct);
-  if (pairs) *pairs = max_pairs;
+  if (pairs) *pairs = workers;
   return SOUP_OK;
 }
 

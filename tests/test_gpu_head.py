@@ -298,6 +298,13 @@ def test_gradient_at_the_edges_of_its_tiles(dims):
     check(*make(*dims, seed=31, drop=0.0 if dims[0] == 1 else 0.3))   # one unlabelled row: 0 / 0
 
 
+# Row blocks of up to 128 rows run on single CTAs: a full one, several units a CTA at ragged tiles, a
+# last block of 100 rows behind a block of 8192.
+@pytest.mark.parametrize("dims", [(128, 1536, 151936), (100, 2056, 60001), (8292, 64, 520)])
+def test_row_blocks_of_up_to_128_rows(dims):
+    check(*make(*dims, seed=36))
+
+
 @pytest.mark.parametrize("dims", [(1300, 1544, 40001), (1100, 2056, 30000)])
 def test_gradient_with_more_units_than_cta_pairs_at_ragged_tiles(dims):
     """A pair runs several units: both accumulators and both staging boxes are used again, at ragged
