@@ -26,6 +26,30 @@ int sm_count();
     if (e__ != cudaSuccess) SOUP_FAIL(SOUP_ERR_LAUNCH, "%s: %s", name, cudaGetErrorString(e__)); \
   } while (0)
 
+// Overlap of a launch with the end of the one before it on the stream (programmatic dependent launch): a kernel
+// lets the next one start as soon as it has room (pdl_trigger), and that one sets itself up and waits for the
+// kernels before it, and their memory, before it touches anything of theirs (pdl_wait). Every thread of a kernel
+// launched by launch_dependent passes pdl_wait, so that a kernel's end is also the end of all before it. (The head's
+// ten launches: 128 rows 245 -> 235 us, 1168 rows 1094 -> 1056, 2048 rows 1681 -> 1631.)
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <typename... Params, typename... Args>
+inline void launch_dependent(void (*kernel)(Params...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream,
+                             Args&&... args) {
+  cudaLaunchAttribute attribute = {};
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = grid;
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = &attribute;
+  config.numAttrs = 1;
+  cudaLaunchKernelEx(&config, kernel, Params(args)...);
+}
+
 inline bool is_float_dtype(int dt) { return dt == SOUP_F32 || dt == SOUP_F16 || dt == SOUP_BF16; }
 inline int dtype_size(int dt) { return dt == SOUP_F32 ? 4 : 2; }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }

@@ -157,30 +157,22 @@ struct PairInit {
   bool run;
 };
 
-// Barrier set-up, tensor-memory allocation and the agreement of both CTAs on whether to run at all
-// (an earlier kernel of the call may have given up). Every thread of both CTAs calls this.
+// Barrier set-up and tensor-memory allocation, which overlap the end of the kernel before, then the wait for it
+// and whether to run at all (an earlier kernel of the call may have given up). Every thread of both CTAs of a
+// pair calls this; both read the one status word, which nothing writes while they do.
 template <bool PAIR>
 __device__ __forceinline__ PairInit init_unit(const GemmSmem& s, int warp, int lane, const int* status) {
   PairInit r;
+  pdl_trigger();
   r.rank = PAIR ? cluster_ctarank() : 0;
   if (warp == 0 && lane == 0) {
     for (int i = 0; i < Unit<PAIR>::kStages; ++i) { mbar_init(&s.full[i], 1); mbar_init(&s.empty[i], 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(&s.acc_full[i], 1); mbar_init(&s.acc_empty[i], 4 * Unit<PAIR>::kCtas); }
-    *s.abort_flag = *reinterpret_cast<const volatile int*>(status) != 0;
+    *s.abort_flag = 0;
     fence_barrier_init();
   }
   __syncthreads();
-  if (PAIR) {
-    cluster_sync_all();
-    // the leader's view decides for the pair
-    r.run = ld_shared_cluster_s32(mapa_u32(smem_u32(s.abort_flag), 0)) == 0;
-    cluster_sync_all();  // nobody leaves (or rewrites the flag) while the peer may still read it
-  } else {
-    r.run = *reinterpret_cast<volatile int*>(s.abort_flag) == 0;
-    __syncthreads();
-  }
-  if (!r.run) { r.tmem = 0; return r; }
-  if (warp == 0 && lane == 0) *s.abort_flag = 0;
+  if (PAIR) cluster_sync_all();   // the peer's barriers are there before anything signals them
   if (warp == 1) {
     if (PAIR) {
       tmem_alloc_pair(s.tmem_base, 512);
@@ -194,6 +186,8 @@ __device__ __forceinline__ PairInit init_unit(const GemmSmem& s, int warp, int l
   __syncthreads();
   tc_fence_after_sync();
   r.tmem = *s.tmem_base;
+  pdl_wait();
+  r.run = *reinterpret_cast<const volatile int*>(status) == 0;
   return r;
 }
 
@@ -480,8 +474,11 @@ __device__ __forceinline__ void logits_body(const CUtensorMap& map_h, const CUte
     prefetch_tensormap(&map_p);
   }
   const PairInit pi = init_unit<PAIR>(s, warp, lane, a.status);
-  if (!pi.run) return;
   const uint32_t tmem = pi.tmem, rank = pi.rank;
+  if (!pi.run) {
+    finish_unit<PAIR>(s, warp, tmem, a.status, a.sticky);
+    return;
+  }
   const int pair = blockIdx.x / U::kCtas, n_pairs = gridDim.x / U::kCtas;
 
   // Tiles are ordered row-tile-fastest: the row tiles that share a weight tile run together, so
@@ -722,6 +719,8 @@ __global__ void __launch_bounds__(kRowThreads, 8) lmhead_row_kernel(const RowArg
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = blockIdx.x;
   const bool first = a.mode == kModeTileMax;
+  pdl_trigger();
+  pdl_wait();
   const float4* stats = a.tile_stats + (size_t)row * a.ct_stride;
   const float ref = a.run_max[row];   // lse so far (-inf before the first chunk)
   const float old_dot = a.run_dot[row];
@@ -855,8 +854,11 @@ __device__ __forceinline__ void grad_body(const CUtensorMap& map_p, const CUtens
     prefetch_tensormap(&map_dh);
   }
   const PairInit pi = init_unit<PAIR>(s, warp, lane, a.status);
-  if (!pi.run) return;
   const uint32_t tmem = pi.tmem, rank = pi.rank;
+  if (!pi.run) {
+    finish_unit<PAIR>(s, warp, tmem, a.status, a.sticky);
+    return;
+  }
   const int pair = blockIdx.x / U::kCtas, n_pairs = gridDim.x / U::kCtas;
 
   const int rt = (a.n_rows + U::kRows - 1) / U::kRows;
@@ -991,6 +993,7 @@ __global__ void __launch_bounds__(256)
 lmhead_init_kernel(float* run_max, float* run_sum, float* run_dot, int* best, float* best_val,
                    float* label_logit, float* grad_ref, int* status, float4* dh, int64_t dh_vec, int n) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_trigger();
   if (i == 0) *status = 0;
   if (i < n) {
     run_max[i] = -INFINITY;
@@ -1064,6 +1067,8 @@ constexpr int kFinishThreads = 128;
 template <bool VEC>
 __global__ void __launch_bounds__(kFinishThreads) lmhead_finish_kernel(const FinishArgs a) {
   const int row = blockIdx.x;
+  pdl_trigger();
+  pdl_wait();
   const float run_sum = a.run_sum[row], label_logit = a.label_logit[row];
   const float lse = a.run_max[row] + logf(run_sum);
   const long long tg = a.target[row];
@@ -1120,6 +1125,7 @@ lmhead_totals_kernel(const float* __restrict__ token_loss, const int* __restrict
                      float* grad_divisor, int64_t n) {
   __shared__ float s_loss[32];
   __shared__ int s_hits[32], s_lab[32];
+  pdl_wait();
   float sum = 0.f;
   int h = 0, l = 0;
   for (int64_t i = threadIdx.x; i < n; i += kTotalsThreads) {
@@ -1502,8 +1508,8 @@ extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void
 
       la.mode = first ? kModeTileMax : kModeCombined;
       timer.mark(0);
-      (single ? lmhead_logits_single_kernel : lmhead_logits_kernel)<<<grid1, kThreadsGemm, kSmemLogits, s>>>(
-          map_h, map_w_k, map_p_st, la);
+      launch_dependent(single ? lmhead_logits_single_kernel : lmhead_logits_kernel, grid1, kThreadsGemm, kSmemLogits, s,
+                       map_h, map_w_k, map_p_st, la);
       timer.mark(0);
       SOUP_CHECK_LAUNCH("lmhead_logits");
 
@@ -1528,7 +1534,7 @@ extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void
       ra.status = ws.status;
       ra.sticky = sticky;
       timer.mark(1);
-      lmhead_row_kernel<<<(unsigned)rows, kRowThreads, 0, s>>>(ra);
+      launch_dependent(lmhead_row_kernel, (unsigned)rows, kRowThreads, 0, s, ra);
       timer.mark(1);
       SOUP_CHECK_LAUNCH("lmhead_row");
 
@@ -1547,8 +1553,8 @@ extern "C" int soup_lmhead_ce(const void* hidden, const void* weight, const void
         const int units = tiles2 * ga.ksplit;
         const unsigned grid2 = (unsigned)(unit_ctas * (units < workers ? units : workers));
         timer.mark(2);
-        (single ? lmhead_grad_single_kernel : lmhead_grad_kernel)<<<grid2, kThreadsGemm, kSmemGrad, s>>>(
-            map_p_ld, map_w_mn, map_dh, ga);
+        launch_dependent(single ? lmhead_grad_single_kernel : lmhead_grad_kernel, grid2, kThreadsGemm, kSmemGrad, s,
+                         map_p_ld, map_w_mn, map_dh, ga);
         timer.mark(2);
         SOUP_CHECK_LAUNCH("lmhead_grad");
       }
@@ -1645,8 +1651,7 @@ extern "C" int soup_lmhead_finish_to(const float* run_max, const float* run_sum,
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const bool vec = h % 4 == 0 && (!dh || aligned16(dh)) && (!dh_out || aligned16(dh_out)) &&
                    (reinterpret_cast<uintptr_t>(weight) & 7u) == 0;
-  if (vec) lmhead_finish_kernel<true><<<(unsigned)n, kFinishThreads, 0, s>>>(a);
-  else lmhead_finish_kernel<false><<<(unsigned)n, kFinishThreads, 0, s>>>(a);
+  launch_dependent(vec ? lmhead_finish_kernel<true> : lmhead_finish_kernel<false>, (unsigned)n, kFinishThreads, 0, s, a);
   SOUP_CHECK_LAUNCH("lmhead_finish");
   return SOUP_OK;
 }
@@ -1671,8 +1676,8 @@ extern "C" int soup_lmhead_totals(const float* token_loss, const int* correct, c
     SOUP_FAIL(SOUP_ERR_ARG, "lmhead_totals: null pointer");
   if (divisor_kind < 0 || divisor_kind > 3 || (divisor_kind >= 2 && !divisor))
     SOUP_FAIL(SOUP_ERR_ARG, "lmhead_totals: divisor kind must be 0 (value), 1 (labelled rows), 2 (float*) or 3 (int64*)");
-  lmhead_totals_kernel<<<1, kTotalsThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      token_loss, correct, target, divisor, divisor_kind, divisor_value, loss, hits, labelled, grad_divisor, n);
+  launch_dependent(lmhead_totals_kernel, 1, kTotalsThreads, 0, reinterpret_cast<cudaStream_t>(stream), token_loss,
+                   correct, target, divisor, divisor_kind, divisor_value, loss, hits, labelled, grad_divisor, n);
   SOUP_CHECK_LAUNCH("lmhead_totals");
   return SOUP_OK;
 }
