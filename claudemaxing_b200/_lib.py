@@ -39,6 +39,9 @@ SIGNATURES = {
     "soup_lora_branch_workspace_bytes": [_L] * 3,
     "soup_lora_branch_bwd": [_P, _L] + [_P] * 8 + [_I] * 3 + [_F] * 3 + [_P] + [_L] * 5 + [_P],
     "soup_lora_cast": [_P] * 4 + [_L, _L, _I, _I, _P],
+    "soup_mlp_fwd": [_P] * 9 + [_L] * 3 + [_P],
+    "soup_mlp_bwd": [_P] * 9 + [_L] * 3 + [_P],
+    "soup_mlp_pays": [_L] * 3 + [_I],
     "soup_qkv_rope_fwd": [_P, _L] + [_P] * 7 + [_L] * 4 + [_P],
     "soup_qkv_rope_bwd": [_P] * 6 + [_L] * 5 + [_P],
     "soup_attn_bwd": [_P] * 11 + [_L] * 9 + [_F, _P],

@@ -8,6 +8,7 @@
 // and only then multiplied by up; dy*up is rounded the same way before it meets silu'.
 #include "common.cuh"
 #include "rowpipe.cuh"
+#include "silu.cuh"
 
 namespace soup {
 namespace {
@@ -15,9 +16,6 @@ namespace {
 constexpr int kThreads = 256;
 constexpr int kSteps = 2;      // forward: vectors per thread
 constexpr int kStepsBwd = 2;   // backward: same depth (4 vectors per thread measured slower: fewer CTAs fit)
-constexpr float kLog2e = 1.4426950408889634f;
-
-__device__ __forceinline__ float silu_denom(float g) { return 1.0f + exp2f(g * -kLog2e); }
 
 template <bool VEC>
 __global__ void __launch_bounds__(kThreads)
@@ -39,7 +37,7 @@ silu_mul_fwd_kernel(const void* __restrict__ gate, const void* __restrict__ up,
       float o[8];
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        float silu = __fdividef(g[s][k], silu_denom(g[s][k]));
+        float silu = silu_of(g[s][k]);
         if (round_silu) silu = round_through(silu, gdt);
         o[k] = silu * u[s][k];
       }
@@ -48,7 +46,7 @@ silu_mul_fwd_kernel(const void* __restrict__ gate, const void* __restrict__ up,
     if (blockIdx.x == 0) {  // ragged tail, at most 7 elements
       for (int64_t i = (n8 << 3) + threadIdx.x; i < n; i += kThreads) {
         const float gv = load1(gate, i, gdt);
-        float silu = __fdividef(gv, silu_denom(gv));
+        float silu = silu_of(gv);
         if (round_silu) silu = round_through(silu, gdt);
         store1(out, i, odt, silu * load1(up, i, udt));
       }
@@ -57,7 +55,7 @@ silu_mul_fwd_kernel(const void* __restrict__ gate, const void* __restrict__ up,
     for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n;
          i += (int64_t)gridDim.x * kThreads) {
       const float gv = load1(gate, i, gdt);
-      float silu = __fdividef(gv, silu_denom(gv));
+      float silu = silu_of(gv);
       if (round_silu) silu = round_through(silu, gdt);
       store1(out, i, odt, silu * load1(up, i, udt));
     }
@@ -74,7 +72,7 @@ __device__ __forceinline__ void bwd_elem(float dy, float g, float u, int gdt, in
     d_silu = round_through(d_silu, gdt);
   }
   d_up = dy * silu;
-  d_gate = d_silu * sig * (1.0f + g * (1.0f - sig));
+  d_gate = d_silu * silu_slope(g, sig);
 }
 
 template <bool VEC>

@@ -18,6 +18,9 @@ module computes the same block with those passes folded into the kernels next to
   product with A, backward in two launches where it adds into gradients that exist), their weights
   cast once per decoder forward;
 * o_proj and down_proj add the fp32 residual in the GEMM's epilogue and write fp32;
+* where their tiles fill the GPU the MLP's products take the elementwise passes next to them into their
+  epilogues (csrc/mlp_gemm.cu): gate, up and silu(gate) * up leave one kernel, and the gradient of the latter
+  never leaves tensor memory;
 * backward rotates dq and dk, and rounds dv, straight into one [tokens, q+k+v] fp16 buffer and
   forms the input gradient of the three projections in one GEMM with fp32 output; the MLP's two
   input gradients accumulate in one fp32 output as well;
@@ -403,6 +406,28 @@ class _ProjectAddResidual(torch.autograd.Function):
         return dy, (grad if ctx.needs_input_grad[1] else None), None
 
 
+def _mlp_kernels_cover(rows, weights, backward, *others):
+    """Whether csrc/mlp_gemm.cu takes these operands, fp16 [n, hidden] rows and (gate, up, down) weights, dense and
+    16-byte aligned (`others` too) with widths of whole 16-byte vectors, and is the faster way to their products
+    (`soup_mlp_pays`)."""
+    hidden, inter = rows.shape[-1], weights[0].shape[0]
+    return (rows.numel() > 0 and hidden % 8 == 0 and inter % 8 == 0
+            and all(w.dtype == F16 for w in (rows, *weights))
+            and [tuple(w.shape) for w in weights] == [(inter, hidden), (inter, hidden), (hidden, inter)]
+            and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (rows, *weights, *others))
+            and _lib.lib().soup_mlp_pays(rows.shape[0], hidden, inter, int(backward)) == 1)
+
+
+def _gate_and_up(rows, weights):
+    """The fp16 products with the gate and up weights, with the forward's bits."""
+    if not _mlp_kernels_cover(rows, weights, False):
+        return torch.mm(rows, weights[0].t()), torch.mm(rows, weights[1].t())
+    gate, up = (torch.empty(rows.shape[0], weights[0].shape[0], dtype=F16, device=rows.device) for _ in range(2))
+    _lib.call("soup_mlp_fwd", _lib.ptr(rows), None, _lib.ptr(weights[0]), _lib.ptr(weights[1]), None, _lib.ptr(gate),
+              _lib.ptr(up), None, None, rows.shape[0], rows.shape[1], gate.shape[1], _lib.stream_of(rows))
+    return gate, up
+
+
 class _GatedMLPAddResidual(torch.autograd.Function):
     """residual + down(silu(gate(x)) * up(x)) for frozen 4-bit projections, with the residual sum
     in down_proj's epilogue and the two input gradients in one fp32 accumulator. silu(gate) * up
@@ -417,14 +442,22 @@ class _GatedMLPAddResidual(torch.autograd.Function):
     @_plain_precision
     def forward(ctx, x, x16, residual, plan):
         rows = x16.reshape(-1, x16.shape[-1])
-        gate = torch.mm(rows, plan.gate.dequantized(F16).t())
-        up = torch.mm(rows, plan.up.dequantized(F16).t())
-        act = torch.empty_like(gate)
-        _silu_mul_fwd(gate, up, act, False)   # fp32 input, fp16 products: silu is not rounded first
-        h = residual.shape[-1]
-        out = torch.addmm(residual.reshape(-1, h), act, plan.down.dequantized(F16).t(),
-                          out_dtype=F32).view(residual.shape)
         ctx.kept = plan.keep_products
+        weights = [linear.dequantized(F16) for linear in (plan.gate, plan.up, plan.down)]
+        if (residual.dtype == F32 and residual.numel() == rows.numel()
+                and _mlp_kernels_cover(rows, weights, False, residual)):
+            n, h = rows.shape
+            inter = weights[0].shape[0]
+            gate, up, act = (torch.empty(n, inter, dtype=F16, device=rows.device) for _ in range(3))
+            out = torch.empty(residual.shape, dtype=F32, device=rows.device)
+            _lib.call("soup_mlp_fwd", _lib.ptr(rows), _lib.ptr(residual), *map(_lib.ptr, weights), _lib.ptr(gate),
+                      _lib.ptr(up), _lib.ptr(act), _lib.ptr(out), n, h, inter, _lib.stream_of(rows))
+        else:
+            gate, up = _gate_and_up(rows, weights)
+            act = torch.empty_like(gate)
+            _silu_mul_fwd(gate, up, act, False)   # fp32 input, fp16 products: silu is not rounded first
+            h = residual.shape[-1]
+            out = torch.addmm(residual.reshape(-1, h), act, weights[2].t(), out_dtype=F32).view(residual.shape)
         if ctx.kept:
             ctx.save_for_backward(gate, up)
         else:
@@ -439,17 +472,22 @@ class _GatedMLPAddResidual(torch.autograd.Function):
         dx = None
         if ctx.needs_input_grad[0]:
             g16 = _fp16_gradient_rows(grad)
-            d_act = torch.mm(g16, plan.down.dequantized(F16))
-            w_gate, w_up = plan.gate.dequantized(F16), plan.up.dequantized(F16)
+            weights = tuple(m.dequantized(F16) for m in (plan.gate, plan.up, plan.down))
+            w_gate, w_up, w_down = weights
             if ctx.kept:
                 gate, up = ctx.saved_tensors
                 d_gate, d_up = torch.empty_like(gate), torch.empty_like(up)
-                _silu_mul_bwd(d_act, gate, up, d_gate, d_up, False)
             else:
                 (x16,) = ctx.saved_tensors
-                rows = x16.reshape(-1, x16.shape[-1])
-                d_gate, d_up = torch.mm(rows, w_gate.t()), torch.mm(rows, w_up.t())
-                _silu_mul_bwd(d_act, d_gate, d_up, d_gate, d_up, False)   # over the recomputed pair
+                # the gradients go over the recomputed pair
+                gate, up = d_gate, d_up = _gate_and_up(x16.reshape(-1, x16.shape[-1]), weights)
+            if _mlp_kernels_cover(g16, weights, True, gate, up):
+                dx = torch.empty(ctx.x_shape, dtype=F32, device=gate.device)
+                _lib.call("soup_mlp_bwd", _lib.ptr(g16), _lib.ptr(gate), _lib.ptr(up), *map(_lib.ptr, weights),
+                          _lib.ptr(d_gate), _lib.ptr(d_up), _lib.ptr(dx), g16.shape[0], g16.shape[1], gate.shape[1],
+                          _lib.stream_of(g16))
+                return dx, None, (grad if ctx.needs_input_grad[2] else None), None
+            _silu_mul_bwd(torch.mm(g16, w_down), gate, up, d_gate, d_up, False)
             dx = torch.mm(d_gate, w_gate, out_dtype=F32)
             dx = torch.addmm(dx, d_up, w_up, out_dtype=F32).view(ctx.x_shape)
         return dx, None, (grad if ctx.needs_input_grad[2] else None), None

@@ -225,6 +225,24 @@ int soup_lora_branch_bwd(const void* g, int64_t g_pitch, const void* x16, const 
 int soup_lora_cast(const void* a, const void* b, void* a16, void* b16, int64_t n_a, int64_t n_b, int a_dtype,
                    int b_dtype, void* stream);
 
+/* The gated MLP of a block with frozen weights and its residual connection: gate = x16 w_gate^T and
+ * up = x16 w_up^T (fp16 [rows, inter], kept for backward), act = fp16(silu(gate) * up) and
+ * out = residual + act w_down^T (fp32 [rows, hidden]). x16 fp16 [rows, hidden], weights fp16 row-major
+ * ([inter, hidden] twice, [hidden, inter]), widths multiples of 8, everything dense and 16-byte aligned. Two
+ * launches for the projections and silu_mul_fwd_persistent of solution/swiglu_recompute.py:138-175. With out NULL
+ * (residual, w_down and act are not used then) only gate and up are formed, by the first launch. */
+int soup_mlp_fwd(const void* x16, const float* residual, const void* w_gate, const void* w_up, const void* w_down,
+                 void* gate, void* up, void* act, float* out, int64_t rows, int64_t hidden, int64_t inter,
+                 void* stream);
+/* 1 where these launches are faster than a library's products with the elementwise kernel between them. */
+int soup_mlp_pays(int64_t rows, int64_t hidden, int64_t inter, int backward);
+/* Its input gradient from dy16 (fp16 [rows, hidden]): d_act = fp16(dy16 w_down), d_gate and d_up (fp16, as
+ * silu_mul_bwd_recompute of solution/swiglu_recompute.py:60-79; they may be gate and up) and dx = d_gate w_gate +
+ * d_up w_up (fp32). Two launches; the results of both calls are the same in every run. */
+int soup_mlp_bwd(const void* dy16, const void* gate, const void* up, const void* w_gate, const void* w_up,
+                 const void* w_down, void* d_gate, void* d_up, float* dx, int64_t rows, int64_t hidden,
+                 int64_t inter, void* stream);
+
 /* The rows [q | k | v] of a q/k/v projection (fp16, row pitch qkv_pitch) as rotated q (+ add_q), rotated
  * k and v (+ add_v): fp16 [n, h, d] contiguous, sums and rotation in fp32, one rounding. add_q [n, hq*d]
  * and add_v [n, hk*d] fp16 contiguous or NULL; cos, sin fp32 [n, d]. One launch for what the reference

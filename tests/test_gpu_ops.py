@@ -805,6 +805,51 @@ def test_paired_lora_branches_are_the_two_single_branches():
         assert torch.equal(single, pair), name
 
 
+@pytest.mark.parametrize("rows", [1, 127, 129, 257, 700, 2560])
+@pytest.mark.parametrize("hidden,inter", [(8, 8), (72, 200), (520, 1096), (1536, 2048)])
+def test_mlp_products_with_their_elementwise_passes(rows, hidden, inter):
+    """`soup_mlp_fwd` / `soup_mlp_bwd`: row tiles, column tiles and K blocks with remainders, one and two K
+    splits (2560 x 1536 has 60 tiles, the others fewer), several tiles a CTA pair; gate and up alone. Each result
+    against float64 from the kernels' own operands of that step. Bounds: one fp16 ulp of the largest value (2^-10) where a sum rounds the other way, two where the
+    gradient of the activation does before the gradients are formed, 2e-5 for fp32 sums of fp16 products."""
+    from claudemaxing_b200 import _lib
+
+    gen = torch.Generator(device=DEV).manual_seed(rows + inter)
+
+    def rand(*shape, std=1.0, dtype=F16):
+        return (torch.randn(*shape, generator=gen, device=DEV) * std).to(dtype)
+
+    x, dy = rand(rows, hidden), rand(rows, hidden)
+    wg, wu, wd = (rand(*shape, std=hidden ** -0.5) for shape in ((inter, hidden), (inter, hidden), (hidden, inter)))
+    residual = rand(rows, hidden, dtype=F32)
+    P, stream = _lib.ptr, _lib.stream_of(x)
+    results = []
+    for _ in range(2):
+        gate, up, act, d_gate, d_up = (torch.full((rows, inter), float("nan"), dtype=F16, device=DEV) for _ in range(5))
+        out, dx = (torch.full((rows, hidden), float("nan"), device=DEV) for _ in range(2))
+        _lib.call("soup_mlp_fwd", P(x), P(residual), P(wg), P(wu), P(wd), P(gate), P(up), P(act), P(out), rows, hidden,
+                  inter, stream)
+        _lib.call("soup_mlp_bwd", P(dy), P(gate), P(up), P(wg), P(wu), P(wd), P(d_gate), P(d_up), P(dx), rows, hidden,
+                  inter, stream)
+        results.append((gate, up, act, out, d_gate, d_up, dx))
+    gate2, up2 = torch.empty_like(gate), torch.empty_like(up)
+    _lib.call("soup_mlp_fwd", P(x), None, P(wg), P(wu), None, P(gate2), P(up2), None, None, rows, hidden, inter, stream)
+    _lib.check_device_status()
+    for first, second in (*zip(*results), (gate2, gate), (up2, up)):
+        assert torch.equal(first, second)
+    f64 = lambda t: t.double()
+    g, u = f64(gate), f64(up)
+    sig = torch.sigmoid(g)
+    d_act = (f64(dy) @ f64(wd)).half().double()
+    for name, got, want, bound in (
+            ("gate", gate, f64(x) @ f64(wg).t(), 2 ** -10), ("up", up, f64(x) @ f64(wu).t(), 2 ** -10),
+            ("act", act, g * sig * u, 2 ** -10), ("out", out, f64(residual) + f64(act) @ f64(wd).t(), 2e-5),
+            ("d_up", d_up, d_act * g * sig, 2 ** -9),
+            ("d_gate", d_gate, d_act * u * sig * (1 + g * (1 - sig)), 2 ** -9),
+            ("dx", dx, f64(d_gate) @ f64(wg) + f64(d_up) @ f64(wu), 2e-5)):
+        assert_close_rel_max(got.float(), want.float(), bound, name)
+
+
 def test_ops_refuse_cpu_tensors():
     from claudemaxing_b200.rmsnorm import rmsnorm
     from claudemaxing_b200.swiglu_recompute import swiglu_recompute
