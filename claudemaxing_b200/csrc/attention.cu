@@ -25,6 +25,7 @@
 // The reference calls torch SDPA here (solution/attention.py:332-343) on a [1, 1, N, N] mask
 // built by its packing (solution/lm_head_loss.py:300-337); this kernel takes the segment offsets.
 #include <cfloat>
+#include <cmath>
 #include <cuda.h>
 
 #include "common.cuh"
@@ -391,9 +392,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 }
 
 // ------------------------------------------------------------------------------------------
-// Backward. A CTA owns one 128-token key/value tile of a segment and one query
-// head, keeps K, V and the accumulators dV and dK (tensor memory) and walks the query tiles from the
-// diagonal to the segment's end. Per query tile, everything transposed (lanes = key rows):
+// Backward. A CTA owns one 128-token key/value tile of a segment and one query head, or a few that share their
+// key/value head, keeps K, V and the accumulators dV and dK (tensor memory) and walks the query tiles from the
+// diagonal to the segment's end, head after head. Per query tile, everything transposed (lanes = key rows):
 //   S^T = K Q^T, dP^T = V dO^T               tensor-memory columns 0-127 / 128-255
 //   P^T = exp2(scale S^T - lse)              two compute warpgroups (64 query columns each), fp16 over S^T
 //   dV += P^T dO                             A from tensor memory, columns 256-383
@@ -406,12 +407,12 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 //
 // What bounds it: shared memory, at 128 B a clock. A tile's products read 288 KB of operands (S^T, dP^T, dQ and dK
 // both of theirs, dV one), loads, dS^T and the staging of dQ move 224 KB more and the rows' statistics 32: 4250
-// clocks by count, about 5200 measured between tiles (9215 tokens in 4 segments: 266 us), and the thread that
+// clocks by count, about 5200 measured between tiles (9215 tokens in 4 segments: 236 us), and the thread that
 // issues the products waits on none of the warps for long. The tensor core needs 2560. With dS^T in tensor memory as
 // dK's operand 32 KB fewer are read, but dQ, over the same columns, has to wait for dK and the next dP^T for both:
 // 5600 clocks, 290 us. (A query-stationary walk reads and moves 700 KB per tile: it stages and adds dK and dV, 128
 // KB, where this one adds dQ, 64 KB. It took 35.8 us for 1280 tokens in 5 segments, 12 / 2 heads, and 790 us for
-// 9215 tokens in 4; this one 20 and 266 us.)
+// 9215 tokens in 4; this one 20 and 236 us.)
 // ------------------------------------------------------------------------------------------
 constexpr int kBwdThreads = 448;   // warps 0-7 compute, 8-11 dQ, 12 loads, 13 products
 constexpr int kDqWarp = 8, kBwdLoadWarp = 12, kBwdMmaWarp = 13;
@@ -436,6 +437,7 @@ struct AttnKvArgs {
   const int32_t* cu;
   const float2* stats;   // [hq, n]
   int n, segments, hq, group;
+  int heads;             // query heads of a CTA, one after another: a divisor of group
   float scale_log2, scale;
   int* status;
 };
@@ -559,16 +561,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                    const __grid_constant__ CUtensorMap map_dv, const AttnKvArgs a) {
   extern __shared__ __align__(1024) uint8_t raw_kv[];
   Tile tile;
-  if (!locate_tile(a.cu, a.segments, blockIdx.x / a.hq, tile)) return;   // the whole CTA leaves
+  const int head_groups = a.hq / a.heads;
+  if (!locate_tile(a.cu, a.segments, blockIdx.x / head_groups, tile)) return;   // the whole CTA leaves
   KvSmem& s = *reinterpret_cast<KvSmem*>(raw_kv);
   if (smem_u32(raw_kv) & 1023) {   // the swizzled tiles and their descriptors want it; no room to align by hand
     if (threadIdx.x == 0) atomicCAS(a.status, 0, 60);
     return;
   }
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.x % a.hq, hk = h / a.group;
+  const int h0 = (blockIdx.x % head_groups) * a.heads, hk = h0 / a.group;
   // depth counts from the walk's end: the tile with the longest walk is the segment's first
-  const int n_q = tile.depth + 1;                                   // query tiles of the walk
+  const int n_q = tile.depth + 1;                                   // query tiles of a head's walk
+  const int n_it = n_q * a.heads;
   const int kv0 = tile.seg_begin + (tile.tiles - 1 - tile.depth) * kBKV;
   if (threadIdx.x == 0) {
     mbar_init(&s.k_full, 1);
@@ -609,11 +613,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         tma_load_2d(dst + kBox, map, col + 64, row, bar);
       };
       tile_in(s.k, &map_k, hk * kD, kv0, &s.k_full);
-      tile_in(s.q[0], &map_q, h * kD, kv0, &s.q_full[0]);
+      tile_in(s.q[0], &map_q, h0 * kD, kv0, &s.q_full[0]);
       tile_in(s.v, &map_v, hk * kD, kv0, &s.v_full);
-      tile_in(s.d_o, &map_do, h * kD, kv0, &s.do_full);
-      for (int i = 1; i < n_q; ++i) {
-        const int row = kv0 + i * kBQ;
+      tile_in(s.d_o, &map_do, h0 * kD, kv0, &s.do_full);
+      int step = 0, h = h0;
+      for (int i = 1; i < n_it; ++i) {
+        if (++step == n_q) { step = 0; ++h; }
+        const int row = kv0 + step * kBQ;
         if (i >= 2 && !mbar_wait(&s.q_empty[i & 1], ((i >> 1) & 1) ^ 1, abort_flag, a.status, 61)) break;
         tile_in(s.q[i & 1], &map_q, h * kD, row, &s.q_full[i & 1]);
         if (!mbar_wait(&s.do_empty, (i - 1) & 1, abort_flag, a.status, 62)) break;
@@ -655,8 +661,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (ok) scores(0);
       ok = ok && wait(&s.v_full, 0, 65) && wait(&s.do_full, 0, 66);
       if (ok) d_prob();
-      for (int i = 0; i < n_q && ok; ++i) {
-        const bool more = i + 1 < n_q;
+      for (int i = 0; i < n_it && ok; ++i) {
+        const bool more = i + 1 < n_it;
         ok = wait(&s.p_full, i, 67);
         if (!ok) break;
 #pragma unroll
@@ -690,10 +696,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     // ---------------------------------------------------------------- dQ, and the rows' statistics
     const int r = threadIdx.x - kDqWarp * 32;
     uint8_t* stage = s.stage[warp - kDqWarp];
-    const float2* stats = a.stats + (size_t)h * a.n;
-    auto fetch = [&](int i) {   // a query past the segment gets weight exp2(-inf) = 0
-      const int token = kv0 + i * kBQ + r;
-      return i < n_q && token < tile.seg_end ? stats[token] : make_float2(INFINITY, 0.f);
+    struct At {   // a step of the walk: query tile and head
+      int step, head;
+    };
+    auto after = [&](At at) { return at.step + 1 == n_q ? At{0, at.head + 1} : At{at.step + 1, at.head}; };
+    auto fetch = [&](At at) {   // a query past the segment gets weight exp2(-inf) = 0
+      const int token = kv0 + at.step * kBQ + r;
+      return at.head < h0 + a.heads && token < tile.seg_end ? a.stats[(size_t)at.head * a.n + token]
+                                                            : make_float2(INFINITY, 0.f);
     };
     auto put = [&](int i, float2 v) {
       s.lse[i & 1][r] = v.x;
@@ -701,17 +711,19 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       __syncwarp();
       if (lane == 0) mbar_arrive(&s.stats_full[i & 1]);
     };
-    put(0, fetch(0));
-    put(1, fetch(1));
+    At now = {0, h0}, next = after(now);
+    put(0, fetch(now));
+    put(1, fetch(next));
+    next = after(next);
     bool ok = true;
-    for (int i = 0; i < n_q; ++i) {
-      const float2 ahead = fetch(i + 2);
+    for (int i = 0; i < n_it; ++i, now = after(now), next = after(next)) {
+      const float2 ahead = fetch(next);
       ok = __all_sync(0xffffffffu, mbar_wait(&s.dq_full, i & 1, abort_flag, a.status, 72));
       if (!ok) break;
       tc_fence_after_sync();
       put(i + 2, ahead);   // dq_full(i): nobody reads the statistics of tile i any more
-      const bool keep = kv0 + i * kBQ + r < tile.seg_end;   // the tile's other rows belong to other segments
-      const int row0 = kv0 + i * kBQ + (warp - kDqWarp) * 32;
+      const bool keep = kv0 + now.step * kBQ + r < tile.seg_end;   // the tile's other rows belong to other segments
+      const int row0 = kv0 + now.step * kBQ + (warp - kDqWarp) * 32;
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
         uint32_t x[32], y[32];
@@ -731,8 +743,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && row0 < tile.seg_end) {
-          tma_reduce_add_2d(&map_dq, stage, h * kD + half * 64, row0);
-          tma_reduce_add_2d(&map_dq, stage + 4096, h * kD + half * 64 + 32, row0);
+          tma_reduce_add_2d(&map_dq, stage, now.head * kD + half * 64, row0);
+          tma_reduce_add_2d(&map_dq, stage + 4096, now.head * kD + half * 64 + 32, row0);
           tma_store_commit();
         }
       }
@@ -748,7 +760,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     t.ds_box = s.ds + wg * kBox;
     const float sl = a.scale_log2;
     bool ok = true;
-    for (int i = 0; i < n_q; ++i) {
+    int step = 0;
+    for (int i = 0; i < n_it; ++i) {
       t.lse = s.lse[i & 1] + wg * 64;
       t.d = s.d[i & 1] + wg * 64;
       ok = mbar_wait(&s.stats_full[i & 1], (i >> 1) & 1, abort_flag, a.status, 73) &&
@@ -757,8 +770,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (!ok) break;
       tc_fence_after_sync();
       float p[64];
-      if (i == 0) probabilities<true>(t, wg * 64, sl, p);
+      if (step == 0) probabilities<true>(t, wg * 64, sl, p);   // the tile on the diagonal
       else probabilities<false>(t, wg * 64, sl, p);
+      if (++step == n_q) step = 0;
       tc_fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(&s.p_full);
@@ -828,6 +842,29 @@ inline int forward_heads_per_cta(int64_t n_tokens, int64_t n_segments, int64_t h
   return tiles * walk * (double)hq > 14.0 * sm_count() ? 2 : 1;
 }
 
+// Query heads of a backward CTA, one after another on the same key/value tile: K, V, the prologue and the sums
+// of dK and dV are paid once for all of them. More heads make fewer and longer units, so the choice is the one
+// with the smallest estimate of the last SM's end, in steps of a walk: the SMs' share of all units (whole waves of
+// the mean one where they are few) or the longest unit, an end of 1.5 steps each. The segments' lengths are on the device: the longest is taken as 1.5 times
+// the mean. One, two and three heads, in us (both launches, 12 query and 2 key heads): 1280 tokens in 5 segments
+// 21.1, 26.6, 34.5; 4607 in 16 59.0, 47.2, 50.4; 8192 in 16 104, 93.7, 87.7; 4607 in 4 89.5, 102, 144; 9212 in 8
+// 170, 150, 157; 9215 in 4 276, 258, 284; 13496 in 8 338, 298, 284; 8192 in 1 572, 571, 553; 1200
+// in 30 28.1, 29.5, 20.1.
+inline int backward_heads_per_cta(int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk) {
+  const double depth = (double)((n_tokens + n_segments * kBQ - 1) / (n_segments * kBQ)), end = 1.5;
+  const double walk = (depth + 1.0) / 2.0, units = depth * (double)n_segments * (double)hq / sm_count();
+  int best = 1;
+  double best_cost = 0.0;
+  for (int heads = 1; heads <= 4 && heads <= hq / hk; ++heads) {
+    if ((hq / hk) % heads) continue;
+    const double waves = units / heads, share = (waves < 3.0 ? ceil(waves) : waves) * (heads * walk + end);
+    const double longest = 1.5 * heads * depth + end;
+    const double cost = share > longest ? share : longest;
+    if (heads == 1 || cost < best_cost) { best = heads; best_cost = cost; }
+  }
+  return best;
+}
+
 }  // namespace
 }  // namespace soup
 
@@ -893,7 +930,8 @@ extern "C" int soup_attn_bwd(const void* q, const void* k, const void* v, const 
   if (head_dim != kD) SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: head_dim must be 128");
   if (n_tokens < 0 || n_segments < 0 || hq <= 0 || hk <= 0 || hq % hk)
     SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: bad sizes (query heads must be a multiple of key heads)");
-  const int64_t ctas = tile_slots(n_tokens, n_segments) * hq;
+  const int heads = n_segments > 0 ? backward_heads_per_cta(n_tokens, n_segments, hq, hk) : 1;
+  const int64_t ctas = tile_slots(n_tokens, n_segments) * (hq / heads);
   if (n_tokens > (1 << 30) || n_segments > 65535 || hq > 65535 || ctas > INT32_MAX)
     SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: too many tokens, segments or heads");
   if (q_pitch < hq * kD || k_pitch < hk * kD || v_pitch < hk * kD || (q_pitch | k_pitch | v_pitch) & 7)
@@ -932,10 +970,20 @@ extern "C" int soup_attn_bwd(const void* q, const void* k, const void* v, const 
   a.segments = (int)n_segments;
   a.hq = (int)hq;
   a.group = (int)(hq / hk);
+  a.heads = heads;
   a.scale = scale;
   a.scale_log2 = scale * kLog2e;
   a.status = rowpipe::status_word();
   attn_bwd_kernel<<<(unsigned)ctas, kBwdThreads, sizeof(KvSmem), st>>>(mq, mdo, mk, mv, mdq, mdk, mdv, a);
   SOUP_CHECK_LAUNCH("attn_bwd");
+  return SOUP_OK;
+}
+
+extern "C" int soup_attn_plan(int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk, int* forward_heads,
+                              int* backward_heads) {
+  using namespace soup;
+  if (n_tokens <= 0 || n_segments <= 0 || hq <= 0 || hk <= 0 || hq % hk) SOUP_FAIL(SOUP_ERR_ARG, "attn_plan: bad sizes");
+  if (forward_heads) *forward_heads = forward_heads_per_cta(n_tokens, n_segments, hq, hk);
+  if (backward_heads) *backward_heads = backward_heads_per_cta(n_tokens, n_segments, hq, hk);
   return SOUP_OK;
 }

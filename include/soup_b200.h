@@ -188,6 +188,10 @@ int soup_rope_sum(const void* q, const void* q_add, const void* k, const void* c
                   int q_dtype, int q_add_dtype, int k_dtype, int cs_dtype, int q_out_dtype,
                   int k_out_dtype, int backward, void* stream);
 
+/* Query heads that a CTA of soup_attn_fwd and soup_attn_bwd works on at these sizes. */
+int soup_attn_plan(int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk, int* forward_heads,
+                   int* backward_heads);
+
 /* Backward of a block's two rank-16 adapters on one input (the reference's two LoRA branches,
  * solution/lora.py:94-134, with B scaled beforehand), in two launches. First, from the output gradients g
  * (fp16 [rows, out], row pitch in elements a multiple of 8, out of 16): gain[i] = fp16(g_i b_i), fp16

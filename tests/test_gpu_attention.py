@@ -279,3 +279,29 @@ def test_gradients_pass_through_the_views_of_a_decoder_block(pitch):
     assert seen == [True] * 3
     for x, w in zip(leaves, flat):   # sums of up to two tiles in any order
         assert (x.grad.float() - w.grad.float()).abs().max() <= 2e-3 * w.grad.float().abs().max()
+
+
+@pytest.mark.parametrize("heads,hq,hk,lens", [
+    (2, 12, 2, [513] * 19 + [1, 129, 0]),        # several units an SM, walks of up to five tiles
+    (3, 12, 2, [130] * 70),                      # more than 64 segments, walks of two tiles, one row in the last
+    (2, 4, 2, [40] * 200),                       # walks of one tile: every step begins another head
+    (4, 16, 4, [257] * 40),
+])
+def test_backward_of_several_heads_per_cta(heads, hq, hk, lens):
+    """A CTA that walks its key/value tile for one head after another: gradients of every head against float64.
+    Bound: fp16 P, dS and dO o O's rounding, as in the other tests here, 4e-3 of the largest."""
+    import ctypes
+
+    from claudemaxing_b200 import _lib
+    from oracle.attention import segment_attention_backward
+
+    n = sum(lens)
+    plan = ctypes.c_int()
+    _lib.call("soup_attn_plan", n, len(lens), hq, hk, None, ctypes.byref(plan))
+    assert plan.value == heads
+    gen = torch.Generator().manual_seed(heads)
+    q, k, v, g = (torch.randn(n, h, 128, generator=gen).half() for h in (hq, hk, hk, hq))
+    _, _, dq, dk, dv = _run(q.to(DEV), k.to(DEV), v.to(DEV), _cu(lens), g.to(DEV))
+    want = segment_attention_backward(q, k, v, _cu(lens), g)
+    for name, got, w in zip(("dq", "dk", "dv"), (dq, dk, dv), want):
+        assert_close_rel_max(got.float().cpu(), w.float(), 4e-3, name)
