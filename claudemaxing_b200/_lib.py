@@ -78,13 +78,6 @@ _RESTYPE = {"soup_lmhead_workspace_bytes": _L, "soup_lmhead_forward_workspace_by
             "soup_lora_branch_workspace_bytes": _L}
 SIGNATURES["soup_rmsnorm_bwd_partials"] = [_L, _L]
 
-class Nf4Item(ctypes.Structure):
-    """soup_nf4_item of include/soup_b200.h."""
-
-    _fields_ = [("packed", _P), ("absmax", _P), ("code2", _P), ("absmax2", _P), ("offset", _P),
-                ("out", _P), ("n_elems", _L)]
-
-
 class Nf4GemmItem(ctypes.Structure):
     """soup_nf4_gemm_item of include/soup_b200.h."""
 
@@ -206,6 +199,11 @@ _STATUS_MEANING = {
     22: "LM-head gradient accumulator: a bounded wait ran out",
     23: "LM-head gradient operand: a bounded wait ran out",
     24: "LM-head gradient epilogue: a bounded wait ran out",
+    111: "MLP operand loads: a bounded wait ran out",
+    112: "MLP accumulator: a bounded wait ran out",
+    113: "MLP operands: a bounded wait ran out",
+    114: "MLP epilogue: a bounded wait ran out",
+    115: "MLP epilogue's gate and up: a bounded wait ran out",
     90: "LM-head row merge: non-finite sum of exponentials",
     99: "bounded-wait self-test",
 }

@@ -21,7 +21,7 @@
 //
 // Roles per CTA: warp 0 loads the operands (a ring of five 32 KB stages), warp 1 of the leader issues the
 // products, warp 3 clears, warps 4-11 are the epilogue (two per quarter of the lanes) on one of two
-// accumulators while the products fill the other. Every wait is bounded (umma::mbar_wait), codes 111-116.
+// accumulators while the products fill the other. Every wait is bounded (umma::mbar_wait), codes 111-115.
 #include <cuda.h>
 
 #include "common.cuh"
