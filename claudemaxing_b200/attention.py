@@ -127,21 +127,22 @@ class SegmentAttention(torch.autograd.Function):
         inputs, ctx.batched = (q, k, v), q.dim() == 4
         q, k, v = map(_rows, inputs)
         n, hq, d = q.shape
-        out = torch.empty((n, hq, d), dtype=q.dtype, device=q.device)
+        # a tensor of its own, not a view: a caller may go on to change the output in place
+        out = torch.empty((1, n, hq, d) if ctx.batched else (n, hq, d), dtype=q.dtype, device=q.device)
         lse = torch.empty((hq, n), dtype=torch.float32, device=q.device)
         _lib.call("soup_attn_fwd", _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(cu_rows),
                   _lib.ptr(out), _lib.ptr(lse), n, cu_rows.numel() - 1, hq, k.shape[1], d,
                   q.stride(0), k.stride(0), v.stride(0), float(scale), _lib.stream_of(q))
         ctx.save_for_backward(*inputs, cu_rows, out, lse)
         ctx.longest, ctx.scale = int(longest), float(scale)
-        return out.unsqueeze(0) if ctx.batched else out
+        return out
 
     @staticmethod
     def backward(ctx, grad):
         *inputs, cu_rows, out, lse = ctx.saved_tensors
         q, k, v = map(_rows, inputs)
         if ctx.batched:
-            grad = grad[0]
+            grad, out = grad[0], out[0]
         if own_backward():
             # one rounding launch for all three: they are adjacent
             flat = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, ctx.scale).to(q.dtype)

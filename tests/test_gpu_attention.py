@@ -274,7 +274,7 @@ def test_gradients_pass_through_the_views_of_a_decoder_block(pitch):
     for x in views:
         x.register_hook(lambda g: seen.append(g.transpose(1, 2)[0].is_contiguous()))
     out = segment_attention(*views, cu, max(lens), 0.1)
-    assert out.shape == (1, n, heads[0], 128) and torch.equal(out[0], want)
+    assert out.shape == (1, n, heads[0], 128) and torch.equal(out[0], want) and not out._is_view()
     out.backward(grad)
     assert seen == [True] * 3
     for x, w in zip(leaves, flat):   # sums of up to two tiles in any order
