@@ -8,44 +8,37 @@
 // of mma.sync.m16n8k16, operands go from global memory to fragments without shared memory, and a
 // fragment's transpose is a movmatrix away, so that each [tokens, width] tensor is read once and the
 // only one written is the input gradient. (A tcgen05 tile would be 128 wide where these are 16.)
-// Bound by latency at the step's token counts: 8.2 + 6.3 us at 1280 tokens (hidden 1536, outputs 1536
-// and 256) where the eight launches take 37.2 us, 10.8 + 19.1 and 70.0 us at 4608.
+// Bound by latency at the step's token counts: 5.4 + 8.7 us at 1280 tokens (hidden 1536, outputs 1536
+// and 256; buffers larger than L2 in turn) where the eight launches take 37.2 us, 10.6 + 22.9 and 70.0 us at 4608.
 //
 // Roundings are those of the products they replace: fp32 accumulators, the rank-16 gradient and the
 // product back to the input's width rounded to fp16 once, weight gradients added in fp32 (by
 // reductions, in any order).
 #include "common.cuh"
 #include "rank16.cuh"
-#include "umma.cuh"
 
 namespace soup {
 namespace {
 
 using namespace rank16;
 
-// Adds `bytes` of fp32 values in shared memory to global memory (both 16-byte aligned).
-__device__ __forceinline__ void bulk_add(float* gdst, const float* ssrc, uint32_t bytes) {
-  asm volatile("cp.reduce.async.bulk.global.shared::cta.bulk_group.add.f32 [%0], [%1], %2;"
-               ::"l"(gdst), "r"(umma::smem_u32(ssrc)), "r"(bytes)
-               : "memory");
-}
 __device__ __forceinline__ void red_add4(float* p, float x, float y, float z, float w) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(x), "f"(y), "f"(z), "f"(w));
 }
 
 // ------------------------------------------------------------------------------------------
-// gain = g B (fp16 [rows, 16], B already scaled) and dB += alpha g^T a, for both adapters. A CTA owns 32
-// rows; its 16 warps take 32-column chunks of the gradients in turn: a chunk's fragments are an operand
-// of the first product as they are and, transposed, of the second. The warps' partial gains meet in
-// shared memory and are summed in a fixed order; a chunk's 32 x 16 values of dB are 2 KB in a row and are
-// added by the copy engine. A chain of a few dependent loads, 8.0 us at 128 rows as at 1280. (With the
-// plain order of columns, four-byte loads, 10.0 us; 128 rows per cluster of eight CTAs 18.1 us, the
-// partial gains crossing the cluster one value at a time.)
+// gain = g B (fp16 [rows, 16], B already scaled) and dB += alpha g^T a, for both adapters, by CTAs of two kinds that
+// do not wait for one another. One kind takes four strips of 32 output columns and a share of the rows, four
+// warps on each strip, whose sums meet in shared memory and leave as reductions. The other owns one or two
+// blocks of 16 rows; its 16 warps take 32-column chunks of the gradients in turn and their partial products meet
+// in shared memory, summed in a fixed order. Both read the gradients (one of them from L2), so that neither's
+// chain of loads waits for the other's. With both products in the CTAs that own the rows, and now: 128 rows 7.9 and
+// 3.5 us, 1280 8.4 and 5.4, 4608 12.1 and 10.6, 16384 38.4 and 28.3 (the first kind last in the grid: 8192 rows 22.0, now 16.6).
 // ------------------------------------------------------------------------------------------
-constexpr int kGainBlocks = 2, kGainRows = 16 * kGainBlocks, kGainWarps = 16, kChunk = 32;
-constexpr int kGainValues = kGainRows * kRank;   // of one adapter
-constexpr int kGainStage = kChunk * kRank;       // one chunk of dB; two per warp
-constexpr int kGainSmem = kGainWarps * (2 * kGainValues + 2 * kGainStage) * (int)sizeof(float);
+constexpr int kGainWarps = 16, kChunk = 32;
+constexpr int kGainValues = 16 * kRank;          // of one adapter and 16 rows
+constexpr int kDbStrips = 4, kDbGroups = 4;      // strips of a CTA, warps on each
+constexpr int kStripValues = kChunk * kRank;
 
 struct GainArgs {
   const __half* g[2];
@@ -57,104 +50,120 @@ struct GainArgs {
   float alpha[2];
   __half* gain;           // [2, rows, 16]
   int64_t rows;
+  int db_ctas, db_columns, blocks_per_share;   // CTAs of the first kind, along the strips; 16-row blocks of a share
 };
 
-__global__ void __launch_bounds__(kGainWarps * 32) lora_gain_kernel(const __grid_constant__ GainArgs p) {
-  extern __shared__ __align__(128) float s_gain[];   // [kGainWarps][2][kGainValues], then the warps' stages
+// 16 rows x 32 columns of a gradient: [row half][column block], rows past the end and columns past `left` zero.
+__device__ __forceinline__ void load_chunk(const __half* g, int64_t pitch, int64_t row0, int64_t rows, int left, int lane,
+                                           uint32_t (&f)[2][4]) {
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int64_t row = row0 + (lane >> 2) + half * 8;
+    const uint4 v = row < rows && 8 * (lane & 3) < left ? __ldg(reinterpret_cast<const uint4*>(g + row * pitch + 8 * (lane & 3)))
+                                                        : make_uint4(0u, 0u, 0u, 0u);
+    f[half][0] = v.x; f[half][1] = v.y; f[half][2] = v.z; f[half][3] = v.w;
+  }
+}
+
+// RB: 16-row blocks of a CTA of the second kind. Two share the fragments of B, as many bytes as a block's gradient,
+// once there are blocks enough for every SM.
+template <int RB>
+constexpr int kGainSmem = RB * 2 * kGainWarps * kGainValues * (int)sizeof(float);
+template <int RB>
+__global__ void __launch_bounds__(kGainWarps * 32, 2) lora_gain_kernel(const __grid_constant__ GainArgs p) {
+  extern __shared__ __align__(16) float s_sum[];   // either kind's partial sums
+  static_assert(2 * kGainWarps * kGainValues == kDbStrips * kDbGroups * kStripValues, "the first kind's fit");
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int64_t row0 = (int64_t)blockIdx.x * kGainRows;
-  float* stages = s_gain + kGainWarps * 2 * kGainValues + warp * 2 * kGainStage;
-  int turn = 0;
+  if ((int)blockIdx.x >= p.db_ctas) {   // the shorter chains start last
+    const int64_t row0 = (int64_t)(blockIdx.x - p.db_ctas) * (16 * RB);
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+      float gain[RB][2][4] = {};   // [row block][rank block]
 #pragma unroll 1
-  for (int w = 0; w < 2; ++w) {
-    // a, rows along the contraction: B fragments [16 rows x 8 ranks] of the row blocks
-    uint32_t ab[kGainBlocks][2][2];   // [row block][rank block][row half]
+      for (int col0 = warp * kChunk; col0 < p.out[w]; col0 += kGainWarps * kChunk) {
+        const int left = p.out[w] - col0;   // 16 in the last chunk of an odd number of sixteens
+        uint32_t gf[RB][2][4], bf[4][2];
 #pragma unroll
-    for (int rb = 0; rb < kGainBlocks; ++rb) {
-      uint32_t f[4];
-      load_rank_fragment(p.a + (int64_t)w * p.rows * kRank, row0 + rb * 16, p.rows, lane, f);
-      ab[rb][0][0] = transpose8x8(f[0]);
-      ab[rb][0][1] = transpose8x8(f[1]);
-      ab[rb][1][0] = transpose8x8(f[2]);
-      ab[rb][1][1] = transpose8x8(f[3]);
-    }
-    float gain[kGainBlocks][2][4] = {};   // [row block][rank block]
-    const int out = p.out[w];
-    const float al = p.alpha[w];
-#pragma unroll 2
-    for (int col0 = warp * kChunk; col0 < out; col0 += kGainWarps * kChunk) {
-      const int left = out - col0;   // 16 in the last chunk of an odd number of sixteens
-      uint32_t gf[kGainBlocks][2][4];   // [row block][row half][column block]
+        for (int rb = 0; rb < RB; ++rb) load_chunk(p.g[w] + col0, p.pitch[w], row0 + rb * 16, p.rows, left, lane, gf[rb]);
 #pragma unroll
-      for (int rb = 0; rb < kGainBlocks; ++rb)
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int64_t row = row0 + rb * 16 + g + half * 8;
-          const uint4 v = row < p.rows && 8 * t < left
-                              ? __ldg(reinterpret_cast<const uint4*>(p.g[w] + row * p.pitch[w] + col0 + 8 * t))
-                              : make_uint4(0u, 0u, 0u, 0u);
-          gf[rb][half][0] = v.x;
-          gf[rb][half][1] = v.y;
-          gf[rb][half][2] = v.z;
-          gf[rb][half][3] = v.w;
+        for (int j = 0; j < 4; ++j) {
+          const int col = column_of(j, g);
+          const uint2 v = col < left ? __ldg(reinterpret_cast<const uint2*>(p.b[w] + (int64_t)(col0 + col) * kRank + 4 * t))
+                                     : make_uint2(0u, 0u);
+          bf[j][0] = transpose8x8(v.x);
+          bf[j][1] = transpose8x8(v.y);
         }
-      uint32_t bf[4][2];   // [column block][rank block]
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int col = column_of(j, g);
-        const uint2 v = col < left ? __ldg(reinterpret_cast<const uint2*>(p.b[w] + (int64_t)(col0 + col) * kRank + 4 * t))
-                                   : make_uint2(0u, 0u);
-        bf[j][0] = transpose8x8(v.x);
-        bf[j][1] = transpose8x8(v.y);
+        for (int rb = 0; rb < RB; ++rb)
+#pragma unroll
+          for (int s = 0; s < 2; ++s) {
+            const uint32_t ga[4] = {gf[rb][0][2 * s], gf[rb][1][2 * s], gf[rb][0][2 * s + 1], gf[rb][1][2 * s + 1]};
+            mma16816(gain[rb][0], ga, bf[2 * s][0], bf[2 * s + 1][0]);
+            mma16816(gain[rb][1], ga, bf[2 * s][1], bf[2 * s + 1][1]);
+          }
       }
-      float db[2][2][4] = {};   // [16-column half][rank block]
 #pragma unroll
-      for (int rb = 0; rb < kGainBlocks; ++rb)
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-          const uint32_t ga[4] = {gf[rb][0][2 * s], gf[rb][1][2 * s], gf[rb][0][2 * s + 1], gf[rb][1][2 * s + 1]};
-          mma16816(gain[rb][0], ga, bf[2 * s][0], bf[2 * s + 1][0]);
-          mma16816(gain[rb][1], ga, bf[2 * s][1], bf[2 * s + 1][1]);
-          const uint32_t gt[4] = {transpose8x8(ga[0]), transpose8x8(ga[2]), transpose8x8(ga[1]), transpose8x8(ga[3])};
-          mma16816(db[s][0], gt, ab[rb][0][0], ab[rb][0][1]);
-          mma16816(db[s][1], gt, ab[rb][1][0], ab[rb][1][1]);
-        }
-      float* stage = stages + turn * kGainStage;
-      turn ^= 1;
-      if (lane == 0) umma::tma_store_wait_read<1>();   // the stage used two chunks ago has been read
-      __syncwarp();
-#pragma unroll
-      for (int s = 0; s < 2; ++s)
+      for (int rb = 0; rb < RB; ++rb)
 #pragma unroll
         for (int half = 0; half < 2; ++half)
-          *reinterpret_cast<float4*>(stage + column_of(2 * s + half, g) * kRank + 4 * t) =
-              make_float4(db[s][0][2 * half] * al, db[s][0][2 * half + 1] * al, db[s][1][2 * half] * al,
-                          db[s][1][2 * half + 1] * al);
-      umma::fence_proxy_async_smem();
-      __syncwarp();
-      if (lane == 0) {
-        bulk_add(p.db[w] + (int64_t)col0 * kRank, stage, min(left, kChunk) * kRank * sizeof(float));
-        umma::tma_store_commit();
-      }
+          *reinterpret_cast<float4*>(s_sum + ((warp * 2 + w) * RB + rb) * kGainValues + (g + half * 8) * kRank + 4 * t) =
+              make_float4(gain[rb][0][2 * half], gain[rb][0][2 * half + 1], gain[rb][1][2 * half],
+                          gain[rb][1][2 * half + 1]);
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < 2 * RB * kGainValues; i += kGainWarps * 32) {
+      const int w = i / (RB * kGainValues), e = i % (RB * kGainValues);
+      float sum = 0.f;   // in the warps' order: the same bits every time
 #pragma unroll
-    for (int rb = 0; rb < kGainBlocks; ++rb)
-#pragma unroll
-      for (int half = 0; half < 2; ++half)
-        *reinterpret_cast<float4*>(s_gain + (warp * 2 + w) * kGainValues + (rb * 16 + g + half * 8) * kRank + 4 * t) =
-            make_float4(gain[rb][0][2 * half], gain[rb][0][2 * half + 1], gain[rb][1][2 * half],
-                        gain[rb][1][2 * half + 1]);
+      for (int k = 0; k < kGainWarps; ++k) sum += s_sum[(k * 2 + w) * RB * kGainValues + e];
+      if (row0 + e / kRank < p.rows) p.gain[((int64_t)w * p.rows + row0) * kRank + e] = __float2half_rn(sum);
+    }
+    return;
   }
+  const int share = blockIdx.x / p.db_columns;
+  const int strips_first = (p.out[0] + kChunk - 1) / kChunk, strips = strips_first + (p.out[1] + kChunk - 1) / kChunk;
+  const int local = warp / kDbGroups, group = warp % kDbGroups;
+  const int strip = ((int)blockIdx.x - share * p.db_columns) * kDbStrips + local;
+  const int w = strip >= strips_first;
+  const int col0 = (w ? strip - strips_first : strip) * kChunk;
+  const int left = strip < strips ? p.out[w] - col0 : 0;
+  float db[2][2][4] = {};   // [16-column half][rank block]
+  const int64_t n_blocks = (p.rows + 15) / 16, begin = (int64_t)share * p.blocks_per_share;
+  const int64_t end = begin + p.blocks_per_share < n_blocks ? begin + p.blocks_per_share : n_blocks;
+#pragma unroll 2
+  for (int64_t rb = begin + group; rb < end; rb += kDbGroups) {
+    uint32_t gf[2][4], f[4];
+    load_chunk(p.g[w] + col0, p.pitch[w], rb * 16, p.rows, left, lane, gf);
+    load_rank_fragment(p.a + (int64_t)w * p.rows * kRank, rb * 16, p.rows, lane, f);
+    // a, rows along the contraction: B fragments [16 rows x 8 ranks]
+    const uint32_t ab[2][2] = {{transpose8x8(f[0]), transpose8x8(f[1])}, {transpose8x8(f[2]), transpose8x8(f[3])}};
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const uint32_t gt[4] = {transpose8x8(gf[0][2 * s]), transpose8x8(gf[0][2 * s + 1]), transpose8x8(gf[1][2 * s]),
+                              transpose8x8(gf[1][2 * s + 1])};
+      mma16816(db[s][0], gt, ab[0][0], ab[0][1]);
+      mma16816(db[s][1], gt, ab[1][0], ab[1][1]);
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < 2; ++s)
+#pragma unroll
+    for (int half = 0; half < 2; ++half)
+      *reinterpret_cast<float4*>(s_sum + warp * kStripValues + column_of(2 * s + half, g) * kRank + 4 * t) =
+          make_float4(db[s][0][2 * half], db[s][0][2 * half + 1], db[s][1][2 * half], db[s][1][2 * half + 1]);
   __syncthreads();
-  for (int i = threadIdx.x; i < 2 * kGainValues; i += kGainWarps * 32) {
-    float sum = 0.f;   // in the warps' order: the same bits every time
+  // the strip's four warps finish eight of its columns each: a lane four ranks of one
+  const int value = group * (kStripValues / kDbGroups) + lane * 4;
+  const float* sums = s_sum + local * kDbGroups * kStripValues + value;
+  float4 v = *reinterpret_cast<const float4*>(sums);
 #pragma unroll
-    for (int k = 0; k < kGainWarps; ++k) sum += s_gain[k * 2 * kGainValues + i];
-    const int w = i / kGainValues, e = i - w * kGainValues;
-    if (row0 + e / kRank < p.rows) p.gain[((int64_t)w * p.rows + row0) * kRank + e] = __float2half_rn(sum);
+  for (int k = 1; k < kDbGroups; ++k) {
+    const float4 o = *reinterpret_cast<const float4*>(sums + k * kStripValues);
+    v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
   }
-  if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");   // the sums have landed
+  const float al = p.alpha[w];
+  if (value / kRank < left) red_add4(p.db[w] + (int64_t)col0 * kRank + value, v.x * al, v.y * al, v.z * al, v.w * al);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -342,10 +351,26 @@ extern "C" int soup_lora_pair_gain(const void* g_first, int64_t pitch_first, int
   p.alpha[1] = alpha_second;
   p.gain = reinterpret_cast<__half*>(gain);
   p.rows = rows;
-  if (cudaFuncSetAttribute(lora_gain_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGainSmem) != cudaSuccess)
-    SOUP_FAIL(SOUP_ERR_LAUNCH, "lora_pair_gain: shared memory attribute");
-  lora_gain_kernel<<<(unsigned)((rows + kGainRows - 1) / kGainRows), kGainWarps * 32, kGainSmem,
-                     reinterpret_cast<cudaStream_t>(stream)>>>(p);
+  const int64_t n_blocks = (rows + 15) / 16;
+  const int64_t strips = (out_first + kChunk - 1) / kChunk + (out_second + kChunk - 1) / kChunk;
+  const int64_t columns = (strips + kDbStrips - 1) / kDbStrips;
+  // row blocks of a share, whole rounds of a strip's four warps, that leave about one CTA per SM
+  int64_t per = (columns * n_blocks + sm_count() - 1) / sm_count();
+  per = (per + kDbGroups - 1) / kDbGroups * kDbGroups;
+  const int rb = n_blocks >= sm_count() ? 2 : 1;
+  const int64_t db_ctas = columns * ((n_blocks + per - 1) / per), ctas = db_ctas + (n_blocks + rb - 1) / rb;
+  if (ctas > INT32_MAX || per > (1 << 30)) SOUP_FAIL(SOUP_ERR_ARG, "lora_pair_gain: too many rows");
+  p.db_ctas = (int)db_ctas;
+  p.db_columns = (int)columns;
+  p.blocks_per_share = (int)per;
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  if (rb == 1) {
+    lora_gain_kernel<1><<<(unsigned)ctas, kGainWarps * 32, kGainSmem<1>, st>>>(p);
+  } else {
+    if (cudaFuncSetAttribute(lora_gain_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGainSmem<2>) != cudaSuccess)
+      SOUP_FAIL(SOUP_ERR_LAUNCH, "lora_pair_gain: shared memory attribute");
+    lora_gain_kernel<2><<<(unsigned)ctas, kGainWarps * 32, kGainSmem<2>, st>>>(p);
+  }
   SOUP_CHECK_LAUNCH("lora_pair_gain");
   return SOUP_OK;
 }
