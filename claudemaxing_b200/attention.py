@@ -124,8 +124,8 @@ class SegmentAttention(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, cu_rows, longest, scale):
-        inputs, ctx.batched = (q, k, v), q.dim() == 4
-        q, k, v = map(_rows, inputs)
+        ctx.batched = q.dim() == 4
+        q, k, v = map(_rows, (q, k, v))
         n, hq, d = q.shape
         # a tensor of its own, not a view: a caller may go on to change the output in place
         out = torch.empty((1, n, hq, d) if ctx.batched else (n, hq, d), dtype=q.dtype, device=q.device)
@@ -133,14 +133,15 @@ class SegmentAttention(torch.autograd.Function):
         _lib.call("soup_attn_fwd", _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(cu_rows),
                   _lib.ptr(out), _lib.ptr(lse), n, cu_rows.numel() - 1, hq, k.shape[1], d,
                   q.stride(0), k.stride(0), v.stride(0), float(scale), _lib.stream_of(q))
-        ctx.save_for_backward(*inputs, cu_rows, out, lse)
+        # the token-major views: a saved-tensor hook may bring back a contiguous copy of what it was given, and
+        # one of [1, heads, tokens, 128] would have another layout
+        ctx.save_for_backward(q, k, v, cu_rows, out, lse)
         ctx.longest, ctx.scale = int(longest), float(scale)
         return out
 
     @staticmethod
     def backward(ctx, grad):
-        *inputs, cu_rows, out, lse = ctx.saved_tensors
-        q, k, v = map(_rows, inputs)
+        q, k, v, cu_rows, out, lse = ctx.saved_tensors
         if ctx.batched:
             grad, out = grad[0], out[0]
         if own_backward():

@@ -281,6 +281,29 @@ def test_gradients_pass_through_the_views_of_a_decoder_block(pitch):
         assert (x.grad.float() - w.grad.float()).abs().max() <= 2e-3 * w.grad.float().abs().max()
 
 
+def test_saved_tensors_may_come_back_as_contiguous_copies():
+    """Under a saved-tensor hook the gradients are those without one (with pinned memory `save_on_cpu` brings back
+    contiguous copies)."""
+    from claudemaxing_b200.attention import segment_attention
+
+    gen = torch.Generator().manual_seed(11)
+    lens, heads = [130, 1, 77], (4, 2, 2)
+    n = sum(lens)
+    cu = torch.tensor([0] + lens).cumsum(0).to(torch.int32).to(DEV)
+    rows = [torch.randn(n, h, 128, generator=gen).half().to(DEV).requires_grad_() for h in heads]
+    grad = torch.randn(1, n, heads[0], 128, generator=gen).half().to(DEV)
+
+    def gradients():
+        out = segment_attention(*(x.unsqueeze(0).transpose(1, 2) for x in rows), cu, max(lens), 0.1)
+        return torch.autograd.grad(out, rows, grad)
+
+    want = gradients()
+    with torch.autograd.graph.save_on_cpu(pin_memory=True):
+        got = gradients()
+    for x, w in zip(got, want):   # sums of up to two tiles in any order
+        assert (x.float() - w.float()).abs().max() <= 2e-3 * w.float().abs().max()
+
+
 @pytest.mark.parametrize("heads,hq,hk,lens", [
     (2, 12, 2, [513] * 19 + [1, 129, 0]),        # several units an SM, walks of up to five tiles
     (3, 12, 2, [130] * 70),                      # more than 64 segments, walks of two tiles, one row in the last
