@@ -414,17 +414,22 @@ inline int pick_splits(int64_t rows, int64_t hidden, int64_t kb_total) {
   return span(tiles, kb_total, 2) < span(tiles, kb_total, 1) ? 2 : 1;
 }
 
+// Sizes whose tile counts and coordinates stay far inside 32 bits.
+inline bool fits(int64_t rows, int64_t hidden, int64_t inter) {
+  return rows <= (1 << 22) && hidden <= (1 << 20) && inter <= (1 << 20);
+}
+
 int check(const char* name, int64_t rows, int64_t hidden, int64_t inter) {
   if (rows < 0 || hidden <= 0 || inter <= 0 || hidden % 8 || inter % 8)
     SOUP_FAIL(SOUP_ERR_ARG, "%s: the widths must be multiples of 8", name);
-  if (rows > (1 << 22) || hidden > (1 << 20) || inter > (1 << 20)) SOUP_FAIL(SOUP_ERR_ARG, "%s: too large", name);
+  if (!fits(rows, hidden, inter)) SOUP_FAIL(SOUP_ERR_ARG, "%s: too large", name);
   return SOUP_OK;
 }
 
 }  // namespace
 }  // namespace soup
 
-// Whether the two launches of a direction are faster than the library's products with the elementwise kernel
+// Whether the two launches of a direction take these sizes and are faster than the library's products with the elementwise kernel
 // between them: a question of how full the last wave of 256 x 256 tiles is. The share of the busiest pair's
 // K blocks that the rows need (in per cent), and the library's time over this file's, forward; backward, by
 // rows: hidden 1536, intermediate 8960: 512 51 0.83; 38 0.81, 896 66 0.96; 58 0.98, 1152 74 0.96; 67 0.97, 1280 83
@@ -433,7 +438,7 @@ int check(const char* name, int64_t rows, int64_t hidden, int64_t inter) {
 // 0.95; 61 0.90, 3072 93 1.05; 89 1.04.
 extern "C" int soup_mlp_pays(int64_t rows, int64_t hidden, int64_t inter, int backward) {
   using namespace soup;
-  if (rows <= 0 || hidden <= 0 || inter <= 0) return 0;
+  if (rows <= 0 || hidden <= 0 || inter <= 0 || !fits(rows, hidden, inter)) return 0;
   const int64_t kb_in = (hidden + kBK - 1) / kBK, kb_mid = (inter + kBK - 1) / kBK;
   const int64_t kb_out = backward ? 2 * kb_mid : kb_mid, outer = tiles_of(rows, hidden, kBN);
   const int64_t wide = tiles_of(rows, inter, backward ? kBN : kBN / 2);

@@ -238,7 +238,8 @@ int soup_lora_cast(const void* a, const void* b, void* a16, void* b16, int64_t n
 int soup_mlp_fwd(const void* x16, const float* residual, const void* w_gate, const void* w_up, const void* w_down,
                  void* gate, void* up, void* act, float* out, int64_t rows, int64_t hidden, int64_t inter,
                  void* stream);
-/* 1 where these launches are faster than a library's products with the elementwise kernel between them. */
+/* 1 where these launches take the sizes (up to 2^22 rows and widths of 2^20) and are faster than a library's
+ * products with the elementwise kernel between them. */
 int soup_mlp_pays(int64_t rows, int64_t hidden, int64_t inter, int backward);
 /* Its input gradient from dy16 (fp16 [rows, hidden]): d_act = fp16(dy16 w_down), d_gate and d_up (fp16, as
  * silu_mul_bwd_recompute of solution/swiglu_recompute.py:60-79; they may be gate and up) and dx = d_gate w_gate +

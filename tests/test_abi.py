@@ -55,6 +55,19 @@ def test_argument_errors_are_reported_not_fatal():
     assert _lib.lib().soup_last_error_string() is not None
 
 
+def test_mlp_products_never_pay_at_sizes_their_launches_refuse():
+    from claudemaxing_b200 import _lib
+
+    pays = _lib.lib().soup_mlp_pays
+    for backward in (0, 1):
+        assert pays(1 << 22, 256, 1024, backward) == 1
+        for size in (((1 << 22) + 1, 256, 1024), (5_000_000, 256, 1024), (2048, (1 << 20) + 8, 1024),
+                     (2048, 1024, (1 << 20) + 8)):
+            assert pays(*size, backward) == 0
+            with pytest.raises(RuntimeError, match="too large"):
+                _lib.call("soup_mlp_bwd" if backward else "soup_mlp_fwd", *[None] * 9, *size, None)
+
+
 def test_no_cpu_fallback():
     import torch
 
