@@ -408,11 +408,12 @@ class _ProjectAddResidual(torch.autograd.Function):
 
 def _mlp_kernels_cover(rows, weights, backward, *others):
     """Whether csrc/mlp_gemm.cu takes these operands, fp16 [n, hidden] rows and (gate, up, down) weights, dense and
-    16-byte aligned (`others` too) with widths of whole 16-byte vectors, and is the faster way to their products
-    (`soup_mlp_pays`)."""
+    16-byte aligned (`others` too) on one device, with widths of whole 16-byte vectors, and is the faster way to their
+    products (`soup_mlp_pays`)."""
     hidden, inter = rows.shape[-1], weights[0].shape[0]
     return (rows.numel() > 0 and hidden % 8 == 0 and inter % 8 == 0
             and all(w.dtype == F16 for w in (rows, *weights))
+            and all(t.device == rows.device for t in (*weights, *others))
             and [tuple(w.shape) for w in weights] == [(inter, hidden), (inter, hidden), (hidden, inter)]
             and all(t.is_contiguous() and t.data_ptr() % 16 == 0 for t in (rows, *weights, *others))
             and _lib.lib().soup_mlp_pays(rows.shape[0], hidden, inter, int(backward)) == 1)

@@ -172,3 +172,16 @@ def test_qkv_split_reads_adapter_terms_and_tables_of_its_own_shape_and_device_on
     launches.clear()
     _qkv(tables=((1, 5, 16), (1, 5, 8)))
     assert [name for name, _ in launches] == ["soup_rope_sum"]
+
+
+def test_mlp_kernels_take_operands_of_one_device_only():
+    """A launch reaches one device: operands of two go to the library's products, which refuse them."""
+    rows = torch.zeros(2944, 768, dtype=torch.float16)
+    weights = [torch.zeros(*shape, dtype=torch.float16) for shape in ((3072, 768), (3072, 768), (768, 3072))]
+    residual = torch.zeros(2944, 768)
+    away = torch.device("meta")
+    assert D._mlp_kernels_cover(rows, weights, False, residual)
+    assert not D._mlp_kernels_cover(rows, weights, False, residual.to(away))
+    for i in range(3):
+        mixed = [w.to(away) if i == j else w for j, w in enumerate(weights)]
+        assert not D._mlp_kernels_cover(rows, mixed, False, residual)
