@@ -445,7 +445,7 @@ class _GatedMLPAddResidual(torch.autograd.Function):
         rows = x16.reshape(-1, x16.shape[-1])
         ctx.kept = plan.keep_products
         weights = [linear.dequantized(F16) for linear in (plan.gate, plan.up, plan.down)]
-        if (residual.dtype == F32 and residual.numel() == rows.numel()
+        if (residual.dtype == F32 and residual.numel() == rows.numel() and residual.shape[-1] == rows.shape[-1]
                 and _mlp_kernels_cover(rows, weights, False, residual)):
             n, h = rows.shape
             inter = weights[0].shape[0]

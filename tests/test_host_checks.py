@@ -2,6 +2,7 @@
 launches replaced by a recorder, and the plans the library makes on the host."""
 
 import ctypes
+from types import SimpleNamespace
 
 import pytest
 import torch
@@ -185,3 +186,17 @@ def test_mlp_kernels_take_operands_of_one_device_only():
     for i in range(3):
         mixed = [w.to(away) if i == j else w for j, w in enumerate(weights)]
         assert not D._mlp_kernels_cover(rows, mixed, False, residual)
+
+
+def test_mlp_residual_is_as_wide_as_the_output(launches):
+    """As many elements in rows of another width: the library's product refuses them, no launch is made."""
+    weights = [torch.zeros(*shape, dtype=torch.float16) for shape in ((3072, 768), (3072, 768), (768, 3072))]
+    gate, up, down = (SimpleNamespace(dequantized=lambda dtype, w=w: w) for w in weights)
+    plan = SimpleNamespace(gate=gate, up=up, down=down, keep_products=True)
+    x = torch.zeros(1, 2944, 768)
+    D._GatedMLPAddResidual.apply(x, x.half(), torch.zeros(1, 2944, 768), plan)
+    assert [name for name, _ in launches] == ["soup_mlp_fwd"]
+    del launches[:]
+    with pytest.raises(RuntimeError):
+        D._GatedMLPAddResidual.apply(x, x.half(), torch.zeros(1, 1472, 1536), plan)
+    assert not any(args[8] is not None for name, args in launches if name == "soup_mlp_fwd")   # no output
