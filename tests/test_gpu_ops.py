@@ -773,6 +773,31 @@ def test_rank16_branch_at_the_edges_of_its_tiles(rows, width, out, scaling, give
     assert_close_rel_max(b.grad, (gs.t() @ low * (scaling if given else 1.0)).float(), 2 ** -10, "dB")
 
 
+@pytest.mark.parametrize("pair", [False, True])
+def test_lora_branch_frees_its_dropout_masks_before_its_outputs(pair):
+    """The forward's peak: the bool masks (a byte an element) are gone before the products, whose outputs are the
+    larger part here."""
+    from claudemaxing_b200.lora import LoRABranch, LoRABranchPair
+
+    rows, width, out = 4096, 256, 4096
+    x = torch.randn(1, rows, width, device=DEV)
+    x16 = x.half()
+    a, b = (torch.randn(2, *shape, device=DEV) * 0.05 for shape in ((16, width), (out, 16)))
+    a16, b16 = a.half(), b.half()
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    if pair:
+        kept = LoRABranchPair.apply(x, x16, a[0], b[0], a[1], b[1], 0.1, 0.1, 1.0, 1.0, a16, b16[0], b16[1])
+    else:
+        kept = LoRABranch.apply(x, x16, a[0], b[0], 0.1, 1.0, a16[0], b16[0], True)
+    n, branches = rows * width, 1 + pair
+    # outputs, dropped input, its bits and the product with A; half a mask of room for rounded allocations
+    want = branches * (2 * rows * out + 2 * n + n // 8 + 2 * rows * 16) + n // 2
+    assert torch.cuda.max_memory_allocated() - before <= want
+    del kept
+
+
 def test_paired_lora_branches_are_the_two_single_branches():
     """LoRABranchPair (one packing launch, one batched product with A, one unpacking launch that
     sums the input gradients) against two LoRABranch calls with the same dropout draws: outputs
