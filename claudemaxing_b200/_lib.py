@@ -45,7 +45,10 @@ SIGNATURES = {
     "soup_qkv_rope_fwd": [_P, _L] + [_P] * 7 + [_L] * 4 + [_P],
     "soup_qkv_rope_bwd": [_P] * 6 + [_L] * 5 + [_P],
     "soup_attn_bwd": [_P] * 11 + [_L] * 9 + [_F, _P],
+    "soup_attn_bwd_bounded": [_P] * 11 + [_L] * 10 + [_F, _P],
     "soup_attn_plan": [_L] * 4 + [_P] * 2,
+    "soup_attn_plan_bounded": [_L] * 5 + [_P] * 2,
+    "soup_attn_bound_matters": [_L] * 5,
     "soup_row_status": [_P, _P],
     "soup_device_status": [_P, _I, _P],
     "soup_wait_selftest": [_L, _P, _P, _P],

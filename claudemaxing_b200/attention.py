@@ -33,10 +33,11 @@ def own_backward():
     return OWN_BACKWARD and not torch.are_deterministic_algorithms_enabled()
 
 
-def attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, scale):
+def attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, scale, longest=0):
     """The fp32 gradients of the segment attention from this library's backward kernel
     (csrc/attention.cu) as one flat buffer: dq [n, hq, 128], dk [n, hk, 128], dv [n, hk, 128] one after
-    another (`gradient_parts`)."""
+    another (`gradient_parts`). `longest`: a bound on the longest segment's tokens that the launch is planned for
+    (0: not known)."""
     n, hq, d = q.shape
     hk = k.shape[1]
     grad = grad if grad.is_contiguous() else grad.contiguous()
@@ -44,9 +45,13 @@ def attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, scale):
     stats = torch.empty(n * hq * 2, dtype=torch.float32, device=q.device)
     dq = flat.data_ptr()
     dk = dq + 4 * n * hq * d
-    _lib.call("soup_attn_bwd", _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _lib.ptr(grad),
+    segments = cu_rows.numel() - 1
+    entry, bound = "soup_attn_bwd", ()
+    if longest > 0 and _lib.lib().soup_attn_bound_matters(n, segments, longest, hq, hk):
+        entry, bound = "soup_attn_bwd_bounded", (longest,)
+    _lib.call(entry, _lib.ptr(q), _lib.ptr(k), _lib.ptr(v), _lib.ptr(out), _lib.ptr(grad),
               _lib.ptr(lse), _lib.ptr(cu_rows), dq, dk, dk + 4 * n * hk * d, _lib.ptr(stats),
-              8 * n * hq, n, cu_rows.numel() - 1, hq, hk, d, q.stride(0), k.stride(0), v.stride(0),
+              8 * n * hq, n, segments, *bound, hq, hk, d, q.stride(0), k.stride(0), v.stride(0),
               float(scale), _lib.stream_of(q))
     return flat
 
@@ -59,9 +64,9 @@ def gradient_parts(flat, n, hq, hk, d):
             torch.as_strided(flat, (n, hk, d), (hk * d, d, 1), at + n * hk * d))
 
 
-def attention_gradients(q, k, v, out, lse, grad, cu_rows, scale):
+def attention_gradients(q, k, v, out, lse, grad, cu_rows, scale, longest=0):
     """`attention_gradients_f32` as three tensors, dq rounded to q's dtype: (dq, dk fp32, dv fp32)."""
-    flat = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, scale)
+    flat = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, scale, longest)
     dq, dk, dv = gradient_parts(flat, q.shape[0], q.shape[1], k.shape[1], q.shape[2])
     return dq.to(q.dtype), dk, dv
 
@@ -146,7 +151,7 @@ class SegmentAttention(torch.autograd.Function):
             grad, out = grad[0], out[0]
         if own_backward():
             # one rounding launch for all three: they are adjacent
-            flat = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, ctx.scale).to(q.dtype)
+            flat = attention_gradients_f32(q, k, v, out, lse, grad, cu_rows, ctx.scale, ctx.longest).to(q.dtype)
             grads = gradient_parts(flat, q.shape[0], q.shape[1], k.shape[1], q.shape[2])
         else:
             _varlen()   # registers the operator

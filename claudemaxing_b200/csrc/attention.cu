@@ -844,25 +844,57 @@ inline int forward_heads_per_cta(int64_t n_tokens, int64_t n_segments, int64_t h
 
 // Query heads of a backward CTA, one after another on the same key/value tile: K, V, the prologue and the sums
 // of dK and dV are paid once for all of them. More heads make fewer and longer units, so the choice is the one
-// with the smallest estimate of the last SM's end, in steps of a walk: the SMs' share of all units (whole waves of
-// the mean one where they are few) or the longest unit, an end of 1.5 steps each. The segments' lengths are on the device: the longest is taken as 1.5 times
-// the mean. One, two and three heads, in us (both launches, 12 query and 2 key heads): 1280 tokens in 5 segments
-// 21.1, 26.6, 34.5; 4607 in 16 59.0, 47.2, 50.4; 8192 in 16 104, 93.7, 87.7; 4607 in 4 89.5, 102, 144; 9212 in 8
-// 170, 150, 157; 9215 in 4 276, 258, 284; 13496 in 8 338, 298, 284; 8192 in 1 572, 571, 553; 1200
-// in 30 28.1, 29.5, 20.1.
-inline int backward_heads_per_cta(int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk) {
-  const double depth = (double)((n_tokens + n_segments * kBQ - 1) / (n_segments * kBQ)), end = 1.5;
-  const double walk = (depth + 1.0) / 2.0, units = depth * (double)n_segments * (double)hq / sm_count();
+// with the smallest estimate of the last SM's end, in steps of a walk (`cost` of a number of heads). One, two and three
+// heads, in us (both launches, 12 query and 2 key heads; "even": equal lengths, else falling to an eighth of the longest):
+// 1280 tokens in 5 24.6, 34.4, 44.6; 4607 in 16 62.8, 51.3, 54.2; 4607 in 4 93.2, 105, 146; 8192 in 16 118, 98.5, 94.8
+// and even 106, 84.9, 81.0; 8192 in 1 537, 556, 544; 9212 in 8 171, 150, 157; 9215 in 4 276, 257, 284; 13496 in 8 326,
+// 296, 286; 1200 in 30 even 30.7, 27.4, 22.6; one of 512 and 15 of 64 24.9, 35.2, 45.4; one of 2000 and 20 of 20 65.9, 101, 141;
+// one of 1024 and 30 of 100 55.1, 61.5, 81.8; one of 4096 and 100 of 20 220, 245, 280, and 16 of 512 257, 227, 289.
+template <class Cost>
+inline int cheapest_heads(int64_t hq, int64_t hk, Cost cost) {
   int best = 1;
-  double best_cost = 0.0;
-  for (int heads = 1; heads <= 4 && heads <= hq / hk; ++heads) {
+  double best_cost = cost(1.0);
+  for (int heads = 2; heads <= 4 && heads <= hq / hk; ++heads) {
     if ((hq / hk) % heads) continue;
-    const double waves = units / heads, share = (waves < 3.0 ? ceil(waves) : waves) * (heads * walk + end);
-    const double longest = 1.5 * heads * depth + end;
-    const double cost = share > longest ? share : longest;
-    if (heads == 1 || cost < best_cost) { best = heads; best_cost = cost; }
+    const double c = cost((double)heads);
+    if (c < best_cost) { best = heads; best_cost = c; }
   }
   return best;
+}
+
+// For segments of similar lengths (the lengths are on the device), the longest taken as 1.5 times the mean: the SMs'
+// share of all units (whole waves of the mean one where they are few) or the longest unit, an end of 1.5 steps each.
+inline int heads_for_similar_segments(int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk) {
+  const double depth = (double)((n_tokens + n_segments * kBQ - 1) / (n_segments * kBQ)), end = 1.5;
+  const double walk = (depth + 1.0) / 2.0, all = depth * (double)n_segments * (double)hq / sm_count();
+  return cheapest_heads(hq, hk, [&](double heads) {
+    const double units = all / heads, share = (units < 3.0 ? ceil(units) : units) * (heads * walk + end);
+    return fmax(share, 1.5 * heads * depth + end);
+  });
+}
+
+// With a bound on the longest segment (the others taken as equal): the SMs' share of all units or the unit on its
+// first tile, three steps each for what a unit pays besides its walk; both where the tiles are in plain order (more
+// than 64 segments), which starts the longest walks anywhere. A bound that is too large leaves heads apart that
+// could have gone together; one that is too small costs time, nothing else. Of 27 rows of 64 to 13496 tokens, 12 / 2 and 32 /
+// 8 heads, this takes the fastest number of heads or one at most 4 % slower; the rule above is up to 50 % slower on
+// rows of which one segment is long (2000 and 20 of 20: 99 us, this one 65).
+inline int heads_for_bounded_segments(int64_t n_tokens, int64_t n_segments, int64_t longest, int64_t hq, int64_t hk) {
+  auto tiles_of = [](double tokens) { return ceil(tokens / kBQ); };
+  if (longest > n_tokens) longest = n_tokens;
+  const double others = (double)(n_segments - 1), deep = tiles_of((double)longest), end = 3.0;
+  const double rest = others > 0.0 ? tiles_of((double)(n_tokens - longest) / others) : 0.0;
+  const double tiles = deep + others * rest, steps = (deep * (deep + 1.0) + others * rest * (rest + 1.0)) / 2.0;
+  return cheapest_heads(hq, hk, [&](double heads) {
+    const double share = (steps * heads + tiles * end) * ((double)hq / heads) / sm_count(), unit = heads * deep + end;
+    return n_segments > 64 ? share + unit : fmax(share, unit);
+  });
+}
+
+// longest 0: no bound is known.
+inline int backward_heads_per_cta(int64_t n_tokens, int64_t n_segments, int64_t longest, int64_t hq, int64_t hk) {
+  return longest > 0 ? heads_for_bounded_segments(n_tokens, n_segments, longest, hq, hk)
+                     : heads_for_similar_segments(n_tokens, n_segments, hq, hk);
 }
 
 }  // namespace
@@ -917,12 +949,12 @@ extern "C" int soup_attn_fwd(const void* q, const void* k, const void* v, const 
   return SOUP_OK;
 }
 
-extern "C" int soup_attn_bwd(const void* q, const void* k, const void* v, const void* out,
-                                 const void* d_out, const float* lse, const int32_t* cu_rows, float* dq,
-                                 float* dk, float* dv, void* workspace, int64_t workspace_bytes,
-                                 int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk,
-                                 int64_t head_dim, int64_t q_pitch, int64_t k_pitch, int64_t v_pitch,
-                                 float scale, void* stream) {
+extern "C" int soup_attn_bwd_bounded(const void* q, const void* k, const void* v, const void* out,
+                                     const void* d_out, const float* lse, const int32_t* cu_rows, float* dq,
+                                     float* dk, float* dv, void* workspace, int64_t workspace_bytes,
+                                     int64_t n_tokens, int64_t n_segments, int64_t longest, int64_t hq, int64_t hk,
+                                     int64_t head_dim, int64_t q_pitch, int64_t k_pitch, int64_t v_pitch,
+                                     float scale, void* stream) {
   using namespace soup;
   if (n_tokens == 0) return SOUP_OK;
   if (!q || !k || !v || !out || !d_out || !lse || !cu_rows || !dq || !dk || !dv || !workspace)
@@ -930,7 +962,8 @@ extern "C" int soup_attn_bwd(const void* q, const void* k, const void* v, const 
   if (head_dim != kD) SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: head_dim must be 128");
   if (n_tokens < 0 || n_segments < 0 || hq <= 0 || hk <= 0 || hq % hk)
     SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: bad sizes (query heads must be a multiple of key heads)");
-  const int heads = n_segments > 0 ? backward_heads_per_cta(n_tokens, n_segments, hq, hk) : 1;
+  if (longest < 0) SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: the longest segment's bound is negative");
+  const int heads = n_segments > 0 ? backward_heads_per_cta(n_tokens, n_segments, longest, hq, hk) : 1;
   const int64_t ctas = tile_slots(n_tokens, n_segments) * (hq / heads);
   if (n_tokens > (1 << 30) || n_segments > 65535 || hq > 65535 || ctas > INT32_MAX)
     SOUP_FAIL(SOUP_ERR_ARG, "attn_bwd: too many tokens, segments or heads");
@@ -979,11 +1012,33 @@ extern "C" int soup_attn_bwd(const void* q, const void* k, const void* v, const 
   return SOUP_OK;
 }
 
+extern "C" int soup_attn_bwd(const void* q, const void* k, const void* v, const void* out, const void* d_out,
+                             const float* lse, const int32_t* cu_rows, float* dq, float* dk, float* dv,
+                             void* workspace, int64_t workspace_bytes, int64_t n_tokens, int64_t n_segments,
+                             int64_t hq, int64_t hk, int64_t head_dim, int64_t q_pitch, int64_t k_pitch,
+                             int64_t v_pitch, float scale, void* stream) {
+  return soup_attn_bwd_bounded(q, k, v, out, d_out, lse, cu_rows, dq, dk, dv, workspace, workspace_bytes, n_tokens,
+                               n_segments, 0, hq, hk, head_dim, q_pitch, k_pitch, v_pitch, scale, stream);
+}
+
+extern "C" int soup_attn_plan_bounded(int64_t n_tokens, int64_t n_segments, int64_t longest, int64_t hq, int64_t hk,
+                                      int* forward_heads, int* backward_heads) {
+  using namespace soup;
+  if (n_tokens <= 0 || n_segments <= 0 || longest < 0 || hq <= 0 || hk <= 0 || hq % hk)
+    SOUP_FAIL(SOUP_ERR_ARG, "attn_plan: bad sizes");
+  if (forward_heads) *forward_heads = forward_heads_per_cta(n_tokens, n_segments, hq, hk);
+  if (backward_heads) *backward_heads = backward_heads_per_cta(n_tokens, n_segments, longest, hq, hk);
+  return SOUP_OK;
+}
+
 extern "C" int soup_attn_plan(int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk, int* forward_heads,
                               int* backward_heads) {
+  return soup_attn_plan_bounded(n_tokens, n_segments, 0, hq, hk, forward_heads, backward_heads);
+}
+
+extern "C" int soup_attn_bound_matters(int64_t n_tokens, int64_t n_segments, int64_t longest, int64_t hq, int64_t hk) {
   using namespace soup;
-  if (n_tokens <= 0 || n_segments <= 0 || hq <= 0 || hk <= 0 || hq % hk) SOUP_FAIL(SOUP_ERR_ARG, "attn_plan: bad sizes");
-  if (forward_heads) *forward_heads = forward_heads_per_cta(n_tokens, n_segments, hq, hk);
-  if (backward_heads) *backward_heads = backward_heads_per_cta(n_tokens, n_segments, hq, hk);
-  return SOUP_OK;
+  if (n_tokens <= 0 || n_segments <= 0 || longest <= 0 || hq <= 0 || hk <= 0 || hq % hk) return 0;
+  return backward_heads_per_cta(n_tokens, n_segments, longest, hq, hk) !=
+         backward_heads_per_cta(n_tokens, n_segments, 0, hq, hk);
 }

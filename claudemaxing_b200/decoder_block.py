@@ -293,13 +293,14 @@ class _QKVRope(torch.autograd.Function):
     """(x16 @ [Wq; Wk; Wv]^T + bias) split into q (+ adapter), k, v (+ adapter); q and k rotated;
     all three returned as fp16 [tokens, heads, head_dim]. With `cu_rows` (segment offsets of the
     packed row) the causal attention inside the segments runs here as well, on this library's
-    kernels, and its output [tokens, heads, head_dim] is what is returned: backward then hands the
-    attention kernel's fp32 gradients straight to the launch that rotates dq and dk back and writes the
-    projection's gradient (`soup_qkv_rope_bwd`)."""
+    kernels (the backward's planned for segments of at most `longest` tokens, 0: not known), and its output
+    [tokens, heads, head_dim] is what is returned: backward then hands the attention kernel's fp32
+    gradients straight to the launch that rotates dq and dk back and writes the projection's gradient
+    (`soup_qkv_rope_bwd`)."""
 
     @staticmethod
     @_plain_precision
-    def forward(ctx, x, x16, lora_q, lora_v, cos, sin, plan, cu_rows=None, scale=None):
+    def forward(ctx, x, x16, lora_q, lora_v, cos, sin, plan, cu_rows=None, scale=None, longest=0):
         _lib.require_cuda(x16, lora_q, lora_v, cos, sin)
         bases = [_base(m) for m in (plan.q, plan.k, plan.v)]
         n, d = x16.numel() // x16.shape[-1], plan.head_dim
@@ -342,7 +343,7 @@ class _QKVRope(torch.autograd.Function):
                   _lib.ptr(attended), _lib.ptr(lse), n, cu_rows.numel() - 1, hq, hk, d,
                   q_out.stride(0), k_out.stride(0), v_out.stride(0), float(scale), _lib.stream_of(q_out))
         ctx.save_for_backward(cos, sin, q_out, k_out, v_out, attended, lse, cu_rows)
-        ctx.scale = float(scale)
+        ctx.scale, ctx.longest = float(scale), longest
         return attended
 
     @staticmethod
@@ -352,7 +353,7 @@ class _QKVRope(torch.autograd.Function):
         if ctx.attends:
             cos, sin, q_out, k_out, v_out, attended, lse, cu_rows = ctx.saved_tensors
             flat = attention_gradients_f32(q_out, k_out, v_out, attended, lse, grads[0].reshape(n, hq, d),
-                                           cu_rows, ctx.scale)
+                                           cu_rows, ctx.scale, ctx.longest)
         else:
             cos, sin = ctx.saved_tensors
         dqkv = torch.empty(n, nq + 2 * nk, dtype=F16, device=cos.device)
@@ -380,7 +381,7 @@ class _QKVRope(torch.autograd.Function):
         return (dx, None,
                 None if q_shape is None else dqkv[:, :nq].view(q_shape),
                 None if v_shape is None else dqkv[:, nq + nk:].view(v_shape),
-                None, None, None, None, None)
+                None, None, None, None, None, None)
 
 
 class _ProjectAddResidual(torch.autograd.Function):
@@ -555,8 +556,10 @@ def fused_block_forward(layer, hidden_states, attention_mask=None, position_ids=
     scale = layer.self_attn.scaling
     if (plan.head_dim == 128 and attention_mod.OWN_FORWARD and attention_mod.own_backward()
             and cu.dtype == torch.int32 and cu.is_cuda):
+        longest = kwargs.get("max_length_q")
         attended = _QKVRope.apply(x, x16, branches[0], branches[2], cos.contiguous(), sin.contiguous(),
-                                  plan, cu, plan.head_dim ** -0.5 if scale is None else scale)
+                                  plan, cu, plan.head_dim ** -0.5 if scale is None else scale,
+                                  longest if isinstance(longest, int) else 0)
         n = attended.shape[0]
     else:
         q, k, v = _QKVRope.apply(x, x16, branches[0], branches[2], cos.contiguous(), sin.contiguous(), plan)

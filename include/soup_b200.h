@@ -188,9 +188,15 @@ int soup_rope_sum(const void* q, const void* q_add, const void* k, const void* c
                   int q_dtype, int q_add_dtype, int k_dtype, int cs_dtype, int q_out_dtype,
                   int k_out_dtype, int backward, void* stream);
 
-/* Query heads that a CTA of soup_attn_fwd and soup_attn_bwd works on at these sizes. */
+/* Query heads that a CTA of soup_attn_fwd and soup_attn_bwd works on at these sizes; _bounded: with a bound on the
+ * longest segment's tokens, as soup_attn_bwd_bounded takes it (0: not known). */
 int soup_attn_plan(int64_t n_tokens, int64_t n_segments, int64_t hq, int64_t hk, int* forward_heads,
                    int* backward_heads);
+int soup_attn_plan_bounded(int64_t n_tokens, int64_t n_segments, int64_t longest, int64_t hq, int64_t hk,
+                           int* forward_heads, int* backward_heads);
+/* 1 where that bound changes the backward's plan: soup_attn_bwd, which takes the segments for similarly long, would be
+ * the slower one. */
+int soup_attn_bound_matters(int64_t n_tokens, int64_t n_segments, int64_t longest, int64_t hq, int64_t hk);
 
 /* Backward of a block's two rank-16 adapters on one input (the reference's two LoRA branches,
  * solution/lora.py:94-134, with B scaled beforehand), in two launches. First, from the output gradients g
@@ -286,6 +292,13 @@ int soup_attn_bwd(const void* q, const void* k, const void* v, const void* out, 
                   void* workspace, int64_t workspace_bytes, int64_t n_tokens, int64_t n_segments,
                   int64_t hq, int64_t hk, int64_t head_dim, int64_t q_pitch, int64_t k_pitch,
                   int64_t v_pitch, float scale, void* stream);
+/* The same results, planned for a longest segment of at most `longest` tokens (0: not known): one long segment among
+ * short ones wants its heads apart. The plan is all that depends on it. */
+int soup_attn_bwd_bounded(const void* q, const void* k, const void* v, const void* out, const void* d_out,
+                          const float* lse, const int32_t* cu_rows, float* dq, float* dk, float* dv,
+                          void* workspace, int64_t workspace_bytes, int64_t n_tokens, int64_t n_segments,
+                          int64_t longest, int64_t hq, int64_t hk, int64_t head_dim, int64_t q_pitch,
+                          int64_t k_pitch, int64_t v_pitch, float scale, void* stream);
 
 /* out = round_out(round_gate?(silu(gate)) * up). Replaces silu_mul_fwd_persistent at
  * solution/swiglu_recompute.py:98-100 and :176-178 (kernel :36-48). */

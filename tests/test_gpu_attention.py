@@ -328,3 +328,39 @@ def test_backward_of_several_heads_per_cta(heads, hq, hk, lens):
     want = segment_attention_backward(q, k, v, _cu(lens), g)
     for name, got, w in zip(("dq", "dk", "dv"), (dq, dk, dv), want):
         assert_close_rel_max(got.float().cpu(), w.float(), 4e-3, name)
+
+
+@pytest.mark.parametrize("plain,bounded,hq,hk,lens", [
+    (3, 1, 12, 2, [4096] + [20] * 100),          # more than 64 segments
+    (2, 1, 12, 2, [20] * 10 + [2000] + [20] * 10),
+    (3, 2, 12, 2, [512] * 2 + [64] * 30),
+    (2, 3, 12, 2, [512] * 16),
+])
+def test_backward_planned_for_the_longest_segment(plain, bounded, hq, hk, lens):
+    """One long segment among short ones has its heads apart (a CTA that walked three of them one after another would
+    be the launch's end): the plan with the bound, and the same gradients. Bound: sums of up to 32 tiles in any
+    order, in fp32, rounded to fp16."""
+    import ctypes
+
+    from claudemaxing_b200 import _lib
+    from claudemaxing_b200.attention import SegmentAttention, attention_gradients
+
+    n, longest = sum(lens), max(lens)
+    heads = ctypes.c_int()
+    for bound, want in ((0, plain), (longest, bounded)):
+        _lib.call("soup_attn_plan_bounded", n, len(lens), bound, hq, hk, None, ctypes.byref(heads))
+        assert heads.value == want
+    gen = torch.Generator().manual_seed(len(lens))
+    q, k, v, g = (torch.randn(n, h, 128, generator=gen).half().to(DEV) for h in (hq, hk, hk, hq))
+    cu = _cu(lens).to(DEV)
+    out, lse = _forward(q, k, v, cu)
+    scale = 128 ** -0.5
+    apart = attention_gradients(q, k, v, out, lse, g, cu, scale)
+    together = attention_gradients(q, k, v, out, lse, g, cu, scale, longest)
+    leaves = [t.clone().requires_grad_() for t in (q, k, v)]
+    SegmentAttention.apply(*leaves, cu, longest, scale).backward(g)
+    _lib.check_device_status()
+    for a, b, leaf in zip(apart, together, leaves):
+        largest = a.float().abs().max()
+        assert (a.float() - b.float()).abs().max() <= 1e-3 * largest
+        assert (leaf.grad.float() - b.float()).abs().max() <= 1e-3 * largest

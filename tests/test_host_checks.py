@@ -200,3 +200,18 @@ def test_mlp_residual_is_as_wide_as_the_output(launches):
     with pytest.raises(RuntimeError):
         D._GatedMLPAddResidual.apply(x, x.half(), torch.zeros(1, 1472, 1536), plan)
     assert not any(args[8] is not None for name, args in launches if name == "soup_mlp_fwd")   # no output
+
+
+@pytest.mark.parametrize("longest,entry", [(4096, "soup_attn_bwd_bounded"), (0, "soup_attn_bwd")])
+def test_segment_attention_backward_knows_the_longest_segment(launches, longest, entry):
+    """The bound reaches the launch where it changes its plan (12 query heads, 2 key heads, a long segment among
+    a hundred short ones)."""
+    from claudemaxing_b200 import attention as A
+
+    n, cu = 6096, torch.tensor([0, 4096] + [4096 + 20 * (i + 1) for i in range(100)], dtype=torch.int32)
+    q, k, v = (torch.zeros(n, h, 128, dtype=torch.float16, requires_grad=True) for h in (12, 2, 2))
+    A.SegmentAttention.apply(q, k, v, cu, longest, 0.1).backward(torch.zeros(n, 12, 128, dtype=torch.float16))
+    name, args = launches[-1]
+    assert name == entry and args[12:14] == (n, 101)
+    if longest:
+        assert args[14] == longest
