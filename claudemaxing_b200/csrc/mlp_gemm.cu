@@ -429,13 +429,21 @@ int check(const char* name, int64_t rows, int64_t hidden, int64_t inter) {
 }  // namespace
 }  // namespace soup
 
-// Whether the two launches of a direction take these sizes and are faster than the library's products with the elementwise kernel
-// between them: a question of how full the last wave of 256 x 256 tiles is. The share of the busiest pair's
-// K blocks that the rows need (in per cent), and the library's time over this file's, forward; backward, by
-// rows: hidden 1536, intermediate 8960: 512 51 0.83; 38 0.81, 896 66 0.96; 58 0.98, 1152 74 0.96; 67 0.97, 1280 83
-// 1.06; 75 1.04, 1408 81 1.07; 82 1.14, 2048 78 1.02; 70 1.03, 3072 92 1.10; 93 1.14, 4608 93 1.07; 94 1.06, 8192 92
-// 1.05; 88 1.05; 896 / 4864: 1280 56 0.92; 45 0.85, 3072 68 1.08; 58 1.01; 2048 / 11008: 512 56 0.93; 44 0.84, 1280 73
-// 0.95; 61 0.90, 3072 93 1.05; 89 1.04.
+// Whether the two launches of a direction take these sizes and are faster than the library's products with the
+// elementwise kernel between them: a question of how full the last wave of 256 x 256 tiles is. The share of the busiest
+// pair's K blocks that the rows need (in per cent), and the library's time over this file's, forward; backward, by rows
+// (each the median of 9 to 15 replays in turn):
+//   896 / 4864     1280 56 0.90; 45 0.83, 2816 63 1.00; 56 1.04, 4096 83 1.12; 73 1.14, 8192 83 1.14; 78 1.15, 24576 1.05; 1.12
+//   1536 / 8960    512 51 0.83; 38 0.81, 1152 74 0.96; 67 0.97, 1280 83 1.06; 75 1.04, 2048 78 1.02; 70 1.02, 3072 92 1.13;
+//                  93 1.18, 4608 93 1.07; 94 1.06, 8192 92 1.11; 88 1.09, 16384 1.01; 1.10, 49152 1.03; 1.34
+//   2048 / 11008   512 56 0.93; 44 0.84, 1024 85 1.11; 79 1.05, 1280 73 0.94; 61 0.86, 1536 82 1.04; 69 0.97, 3072 93 1.15; 89 1.06
+//   2560 / 9728    2048 79 1.01; 73 0.95, 3072 92 1.17; 85 1.11
+//   3584 / 18944   512 87 0.99; 80 1.01, 768 78 0.93; 65 0.89, 896 77 0.96; 71 0.92, 1280 1.09; 1.08, 2048 1.06; 1.07, 8192 1.06; 1.19
+//   4096 / 14336   1152 76 0.91; 69 0.86, 1280 84 0.99; 77 0.98, 2048 1.08; 1.03, 8192 1.20; 1.21
+//   5120 / 27648   896 75 0.88; 68 0.82, 1024 86 0.98; 78 0.86, 1152 84 1.03; 81 0.95, 1280 1.08; 1.05, 4096 1.06; 1.07
+//   8192 / 28672   512 85 0.98; 82 0.96, 1152 82 0.93; 80 0.90, 1280 1.04; 1.02, 4096 1.21; 1.22
+// Up to a width of 2048 a share of 76, backward 69, per cent draws the line. Wider weights have tiles enough at any
+// number of rows, and the library's smaller tiles win where the rows are not: the line is five row tiles there.
 extern "C" int soup_mlp_pays(int64_t rows, int64_t hidden, int64_t inter, int backward) {
   using namespace soup;
   if (rows <= 0 || hidden <= 0 || inter <= 0 || !fits(rows, hidden, inter)) return 0;
@@ -445,7 +453,9 @@ extern "C" int soup_mlp_pays(int64_t rows, int64_t hidden, int64_t inter, int ba
   const int64_t busy = span(wide, kb_in, 1) + span(outer, kb_out, pick_splits(rows, hidden, kb_out));
   const double needed = 3.0 * (double)rows * (double)hidden * (double)inter /
                         ((double)(2 * kBM) * kBN * kBK * (double)(sm_count() / 2));
-  return needed >= (backward ? 0.68 : 0.76) * (double)busy;
+  const bool narrow = hidden <= 2048;
+  if (!narrow && rows < 5 * 2 * kBM) return 0;
+  return needed >= (backward && narrow ? 0.69 : 0.76) * (double)busy;
 }
 
 extern "C" int soup_mlp_fwd(const void* x16, const float* residual, const void* w_gate, const void* w_up,

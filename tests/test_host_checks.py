@@ -215,3 +215,18 @@ def test_segment_attention_backward_knows_the_longest_segment(launches, longest,
     assert name == entry and args[12:14] == (n, 101)
     if longest:
         assert args[14] == longest
+
+
+@pytest.mark.parametrize("hidden,inter,slower,faster", [
+    (1536, 8960, [512, 896, 1152], [1280, 1408, 3072, 4608, 16384]),
+    (2048, 11008, [512, 1280], [1024, 2048, 3072, 8192]),
+    (3584, 18944, [768, 896], [1280, 2304, 8192]),
+    (4096, 14336, [896, 1152], [2048, 8192]),
+    (5120, 27648, [896, 1024], [1280, 4096]),
+    (8192, 28672, [512, 1152], [1280, 4096]),
+])
+def test_mlp_launches_pay_where_both_directions_measured_faster(hidden, inter, slower, faster):
+    pays = _lib.lib().soup_mlp_pays
+    for backward in (0, 1):
+        assert [pays(rows, hidden, inter, backward) for rows in slower] == [0] * len(slower)
+        assert [pays(rows, hidden, inter, backward) for rows in faster] == [1] * len(faster)
