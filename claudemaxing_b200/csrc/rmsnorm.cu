@@ -959,6 +959,18 @@ inline bool row_kernel_covers(int64_t n_rows, int64_t n_cols, int dtype) {
   return dtype == SOUP_F32 || n_rows * threads <= 2ll * sm_count() * (threads == 32 ? 2048 : 1152);
 }
 
+// Whether the weight-gradient row kernel is the faster one. Rows of one warp stay with the kernel whose warps take a
+// row each. So do many fp32 rows of two or three warps: four CTAs leave an SM 256 or 384 threads, less in flight than
+// it takes (warp-per-row and row kernel, in us: 264 columns 22.2 and 17.9 at 8192 rows, 28.5 and 28.9 at 16384, 65.8 and
+// 87.0 at 65536; 512 columns 33.5 and 31.3 at 16384, 82.9 and 96.3 at 65536; 576 columns 60.1 and 57.9 at 32768, 99.6 and 106 at
+// 65536; 768 columns 69.1 and 63.3 at 32768, 212 and 223 at 131072). Wider rows and 16-bit ones gain at any number of rows:
+// fp32 896 x 65536 262 and 129, fp16 264 x 262144 267 and 243, 1024 x 32768 126 and 50.7, bf16 512 x 65536 94.6 and 75.3.
+inline bool dw_row_kernel_covers(int64_t n_rows, int64_t n_cols, int dtype) {
+  if (n_cols <= 256 || n_cols > kRowMaxThreads * 8) return false;
+  if (dtype != SOUP_F32 || n_cols > 768) return true;
+  return n_rows <= (n_cols <= 512 ? 16384 : 32768);
+}
+
 }  // namespace
 }  // namespace soup
 
@@ -1160,9 +1172,8 @@ int rmsnorm_bwd_any(const void* dy, const void* xin, const void* w, const float*
     else if (yb == 4) SOUP_RMS_BWD_P(4, 2, SOUP_F32, -1, -1, -1, -1);
     else SOUP_RMS_BWD_P(2, 2, -1, -1, -1, -1, -1);
 #undef SOUP_RMS_BWD_P
-  } else if (want_dw && n_cols > 256 && n_cols <= kRowMaxThreads * 8 && dy_dtype == xin_dtype &&
+  } else if (want_dw && dw_row_kernel_covers(n_rows, n_cols, dy_dtype) && dy_dtype == xin_dtype &&
              dy_dtype == w_dtype && dy_dtype == dx_dtype) {
-    // rows of one warp stay with the kernel whose warps take a row each
     const int64_t steps = (n_rows + kDwRows - 1) / kDwRows;
     if (steps < grid) grid = (unsigned)steps;
     const unsigned threads = row_block(n_cols).x;

@@ -193,6 +193,31 @@ def test_rmsnorm_weight_gradient_at_the_edges_of_its_kernels(cols, rows):
     assert torch.equal(leaves[1].grad, again[1].grad)   # a fixed order of additions
 
 
+@pytest.mark.parametrize("cols,last", [(264, 16384), (512, 16384), (520, 32768), (768, 32768)])
+def test_rmsnorm_weight_gradient_of_many_narrow_fp32_rows(cols, last):
+    """Up to `last` rows four CTAs an SM take a step of rows each, above them two CTAs of a row per warp, the faster
+    way there: the partial sums tell which ran, and both agree with float64. Bounds: fp32 sums over a row and over
+    all rows, against the largest value."""
+    from claudemaxing_b200 import _lib
+
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    for rows, ctas in ((last, 4 * sms), (last + 1, 2 * sms)):
+        gen = torch.Generator(device=DEV).manual_seed(rows)
+        x, dy = (torch.randn(rows, cols, generator=gen, device=DEV) for _ in range(2))
+        w = 1 + 0.5 * torch.randn(cols, generator=gen, device=DEV)
+        rstd = (x.square().mean(-1) + 1e-6).rsqrt()
+        partials = _lib.lib().soup_rmsnorm_bwd_partials(rows, cols)
+        part = torch.full((partials, cols), float("nan"), device=DEV)
+        dx, dw = torch.empty_like(x), torch.empty_like(w)
+        _lib.call("soup_rmsnorm_bwd", *map(_lib.ptr, (dy, x, w, rstd, dx, part, dw)), None, None, 0, rows, cols,
+                  *[_lib.F32] * 4, 0, _lib.stream_of(x))
+        assert part.isfinite().all(1).sum() == ctas
+        norm, gn = x.double() * rstd.double()[:, None], dy.double() * w.double()
+        want_dx = (gn - norm * (gn * norm).mean(-1, keepdim=True)) * rstd.double()[:, None]
+        assert_close_rel_max(dx, want_dx.float(), 1e-5, "dx")
+        assert_close_rel_max(dw, (dy.double() * norm).sum(0).float(), 1e-5, "dw")
+
+
 def test_rmsnorm_fp16_copy_path_and_tiny_weights():
     # fp32 x, frozen fp32 w: forward leaves an fp16 copy for the next layers, backward uses it;
     # a 2e5 "massive activation" channel and tiny / zero weights (tests_local/test_rmsnorm.py:197-277)
