@@ -29,8 +29,12 @@ int sm_count();
 // Overlap of a launch with the end of the one before it on the stream (programmatic dependent launch): a kernel
 // lets the next one start as soon as it has room (pdl_trigger), and that one sets itself up and waits for the
 // kernels before it, and their memory, before it touches anything of theirs (pdl_wait). Every thread of a kernel
-// launched by launch_dependent passes pdl_wait, so that a kernel's end is also the end of all before it. (The head's
-// ten launches: 128 rows 245 -> 235 us, 1168 rows 1094 -> 1056, 2048 rows 1681 -> 1631.)
+// launched by launch_dependent passes pdl_wait, so that a kernel's end is also the end of all before it. What a kernel
+// before it writes changes during the life of such a kernel: no __restrict__ or __ldg on it, which promise the compiler
+// that it does not. And a kernel that allocates tensor memory triggers before it does only where no other one fits
+// beside it on an SM (these take 220 KB of shared memory): the next kernel's allocation would wait for its end. (The
+// head's ten launches, captured, without and with: 24 rows 206.9 and 198.8 us, 128 rows 210.4 and 208.0, 129 rows 223.9
+// and 219.8; from 1168 rows on no difference beyond the noise of the power cap.)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

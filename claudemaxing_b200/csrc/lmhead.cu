@@ -1119,9 +1119,8 @@ __global__ void __launch_bounds__(kFinishThreads) lmhead_finish_kernel(const Fin
 // The divisor is the labelled count, or *divisor_ptr, or divisor_value. One CTA: a few 10 KB.
 constexpr int kTotalsThreads = 1024;
 __global__ void __launch_bounds__(kTotalsThreads)
-lmhead_totals_kernel(const float* __restrict__ token_loss, const int* __restrict__ correct,
-                     const int64_t* __restrict__ target, const void* divisor_ptr, int divisor_kind,
-                     float divisor_value, float* loss, int64_t* hits, int64_t* labelled,
+lmhead_totals_kernel(const float* token_loss, const int* correct, const int64_t* target, const void* divisor_ptr,
+                     int divisor_kind, float divisor_value, float* loss, int64_t* hits, int64_t* labelled,
                      float* grad_divisor, int64_t n) {
   __shared__ float s_loss[32];
   __shared__ int s_hits[32], s_lab[32];
