@@ -159,7 +159,8 @@ struct PairInit {
 
 // Barrier set-up and tensor-memory allocation, which overlap the end of the kernel before, then the wait for it
 // and whether to run at all (an earlier kernel of the call may have given up). Every thread of both CTAs of a
-// pair calls this; both read the one status word, which nothing writes while they do.
+// pair calls this. A unit of this launch that gives up may write the status word while a later one reads it: a warp
+// decides as one, and warps or CTAs that decide differently end in bounded waits.
 template <bool PAIR>
 __device__ __forceinline__ PairInit init_unit(const GemmSmem& s, int warp, int lane, const int* status) {
   PairInit r;
@@ -187,7 +188,7 @@ __device__ __forceinline__ PairInit init_unit(const GemmSmem& s, int warp, int l
   tc_fence_after_sync();
   r.tmem = *s.tmem_base;
   pdl_wait();
-  r.run = *reinterpret_cast<const volatile int*>(status) == 0;
+  r.run = __shfl_sync(0xffffffffu, *reinterpret_cast<const volatile int*>(status), 0) == 0;
   return r;
 }
 
