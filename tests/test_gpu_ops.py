@@ -2,6 +2,8 @@
 golden outputs of the reference's own kernels. NF4 and the dropout bits are compared bit for bit;
 the floating-point ops use the reference's own tolerances (tests_local/ of the reference)."""
 
+from types import SimpleNamespace
+
 import pytest
 import torch
 
@@ -424,7 +426,8 @@ def test_qkv_split_and_rotation_is_the_rotation_and_the_sums_it_replaces(dims, w
     assert torch.equal(got, want)
 
 
-@pytest.mark.parametrize("rows", [1, 16, 33, 1280])
+# From 148 row blocks of 16 on a CTA owns two of them: 2369 and 4609 rows leave the last one a single row of its first.
+@pytest.mark.parametrize("rows", [1, 16, 33, 1280, 2369, 4609])
 @pytest.mark.parametrize("hidden,outs", [(1536, (1536, 256)), (32, (16, 16)), (160, (48, 144))])
 def test_lora_pair_backward_in_two_launches(rows, hidden, outs):
     """`soup_lora_pair_gain` / `soup_lora_pair_input` against the products they replace in float64, with
@@ -761,7 +764,9 @@ def test_lora_branch_with_cast_scaled_weights_and_in_place_gradients(scaling, mo
         assert rel_norm(fast.float().cpu(), plain.float().cpu()) < 2e-3, name
 
 
-@pytest.mark.parametrize("rows", [1, 15, 17, 1000])
+# From 592 row blocks of 16 on a CTA owns two of them in the rank-16 gradient's launch (9473 rows: one row of the last
+# CTA's first block), and a warp of the output's launch walks three row tiles (520 columns, 16391 rows).
+@pytest.mark.parametrize("rows", [1, 15, 17, 1000, 9473, 16391])
 @pytest.mark.parametrize("width,out", [(32, 8), (96, 40), (1568, 520)])
 @pytest.mark.parametrize("scaling,given", [(2.0, False), (0.3, False), (0.3, True)])
 def test_rank16_branch_at_the_edges_of_its_tiles(rows, width, out, scaling, given):
@@ -898,6 +903,50 @@ def test_mlp_products_with_their_elementwise_passes(rows, hidden, inter):
             ("d_gate", d_gate, d_act * u * sig * (1 + g * (1 - sig)), 2 ** -9),
             ("dx", dx, f64(d_gate) @ f64(wg) + f64(d_up) @ f64(wu), 2e-5)):
         assert_close_rel_max(got.float(), want.float(), bound, name)
+
+
+@pytest.mark.parametrize("rows,hidden,inter,forward,backward", [
+    (1472, 1536, 3072, 1, 1),
+    (6464, 1536, 1024, 1, 0),
+    (4416, 512, 2048, 0, 1),
+    (257, 72, 200, 0, 0),
+])
+def test_gated_mlp_node_on_its_launches(rows, hidden, inter, forward, backward, monkeypatch):
+    """The fused block's MLP node where the launches pay in both directions, in one and in none: the entries it calls,
+    the numbers of the library's products, and the same bits whether gate and up are kept or formed again and
+    overwritten by their gradients. Bounds: gate, up and the activation's gradient may round the other way, 2^-10 of
+    their value each, in sums over them: 2^-9 of the largest."""
+    import importlib
+
+    block = importlib.import_module("claudemaxing_b200.decoder_block")
+    gen = torch.Generator(device=DEV).manual_seed(rows)
+    rand = lambda *shape, std=1.0: torch.randn(*shape, generator=gen, device=DEV) * std
+    weights = [rand(*shape, std=hidden ** -0.5).half() for shape in ((inter, hidden), (inter, hidden), (hidden, inter))]
+    x, residual, dy = (rand(1, rows, hidden) for _ in range(3))
+    names = []
+    real = block._lib.call
+    monkeypatch.setattr(block._lib, "call", lambda name, *args: (names.append(name), real(name, *args))[1])
+
+    def run(keep):
+        del names[:]
+        gate, up, down = (SimpleNamespace(dequantized=lambda dtype, w=w: w) for w in weights)
+        leaves = [x.clone().requires_grad_(), residual.clone().requires_grad_()]
+        out = block._GatedMLPAddResidual.apply(leaves[0], leaves[0].detach().half(), leaves[1],
+                                               SimpleNamespace(gate=gate, up=up, down=down, keep_products=keep))
+        out.backward(dy)
+        return out.detach(), leaves[0].grad, leaves[1].grad
+
+    kept = run(True)
+    assert (names.count("soup_mlp_fwd"), names.count("soup_mlp_bwd")) == (forward, backward)
+    again = run(False)
+    assert (names.count("soup_mlp_fwd"), names.count("soup_mlp_bwd")) == (2 * forward, backward)
+    block._lib.check_device_status()
+    for first, second in zip(kept, again):
+        assert torch.equal(first, second)
+    monkeypatch.setattr(block, "_mlp_kernels_cover", lambda *a: False)
+    for name, got, want in zip(("out", "dx", "dresidual"), kept, run(True)):
+        assert_close_rel_max(got, want, 2 ** -9, name)
+    assert "soup_mlp_fwd" not in names and "soup_mlp_bwd" not in names
 
 
 def test_ops_refuse_cpu_tensors():
