@@ -860,6 +860,39 @@ def test_paired_lora_branches_are_the_two_single_branches():
         assert torch.equal(single, pair), name
 
 
+def test_paired_lora_branches_of_many_elements_go_through_the_products(monkeypatch):
+    """Backward on either side of `lora.ONE_BY_ONE`: adapter by adapter up to it, the products of both beyond, with
+    the same numbers. Bounds: an fp16 rank-16 gradient or product that rounds the other way, 2^-10 of the largest
+    value each."""
+    import importlib
+
+    lora = importlib.import_module("claudemaxing_b200.lora")
+    names = []
+    real = lora._lib.call
+    monkeypatch.setattr(lora._lib, "call", lambda name, *args: (names.append(name), real(name, *args))[1])
+    hidden, outs = 4096, (256, 64)
+    most = lora.ONE_BY_ONE
+    for rows, one_by_one in ((most // hidden, True), (most // hidden + 1, False)):
+        gen = torch.Generator(device=DEV).manual_seed(rows)
+        rand = lambda *shape, std=1.0: torch.randn(*shape, generator=gen, device=DEV) * std
+        x = rand(1, rows, hidden)
+        ws = [rand(*shape, std=0.05) for shape in ((16, hidden), (outs[0], 16), (16, hidden), (outs[1], 16))]
+        grads = [rand(1, rows, o, std=0.1).half() for o in outs]
+        results = []
+        for limit, expected in ((most, one_by_one), (0 if one_by_one else 1 << 40, not one_by_one)):
+            monkeypatch.setattr(lora, "ONE_BY_ONE", limit)
+            torch.manual_seed(9)
+            leaves = [t.clone().requires_grad_() for t in (x, *ws)]
+            a16 = torch.stack([ws[0], ws[2]]).half()
+            out = lora.LoRABranchPair.apply(leaves[0], x.half(), *leaves[1:], 0.1, 0.25, 1.0, 1.0, a16, ws[1].half(),
+                                            ws[3].half())
+            del names[:]
+            results.append(torch.autograd.grad(out, leaves, grads))
+            assert ("soup_lora_branch_bwd" in names) == expected
+        for name, first, second in zip(("dx", "dA1", "dB1", "dA2", "dB2"), *results):
+            assert_close_rel_max(first, second, 2 ** -9, name)
+
+
 @pytest.mark.parametrize("rows", [1, 127, 129, 257, 700, 2560])
 @pytest.mark.parametrize("hidden,inter", [(8, 8), (72, 200), (520, 1096), (1536, 2048)])
 def test_mlp_products_with_their_elementwise_passes(rows, hidden, inter):
