@@ -10,9 +10,11 @@
 //
 // As library products with elementwise kernels between them a block of the 1.5B model (hidden 1536,
 // intermediate 8960) takes 202 us forward and backward at 1280 tokens and 656 at 4608, ten launches that write and
-// read d_act, gate, up and the residual once more than needed; here four and 193 and 617 us. What bounds it: the tiles'
-// operands come from L2, 128 flop a byte, at 9 to 11 TB/s (no tile is multicast); soup_mlp_pays has the sizes at
-// which the library's products, in other tile shapes, are faster all the same.
+// read d_act, gate, up and the residual once more than needed; here four and 193 and 617 us. What bounds it: at 4608
+// tokens, 1.2 PFLOP/s, the power cap: at the 1.55 GHz it leaves the tensor pipe is active 68 (kUp), 71 (kDown) and 51 % (kDact, whose
+// tiles are only 24 K blocks long) of the cycles, L2 moves 12 to 14 TB/s, 38 to 43 % of its peak, and the ports into the SMs are
+// busy 30 to 37 %. At 1280 tokens, 1.1 PFLOP/s, the last wave of tiles as well: the busiest pair walks 402 K blocks where 341 are
+// its share. soup_mlp_pays has the sizes at which the library's products, in other tile shapes, are faster.
 //
 // Tiles are 256 columns wide because shared memory serves the tensor core 128 bytes a clock: a 256 x 128
 // tile wants 96 for operands and 96 for the loads that replace them, a 256 x 256 tile 64 and 64. The two products

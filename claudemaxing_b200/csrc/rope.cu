@@ -230,8 +230,10 @@ rope_pipe_kernel(RopeArgs a, int stages, int* status) {
 // four elements of a head's first half and the matching four of its second half, keeps its position's cos /
 // sin (eight elements of each half would spill) and walks its share of the heads, a few of them in flight as
 // raw bits. Bound by memory; the dtype is a template constant because run-time codes, and operands unpacked
-// at the load, left the general kernel above half of its bytes in flight: 89.8 -> 24.8 us for 16384
-// positions of 14 fp16 heads of 128.
+// at the load, left the general kernel above half of its bytes in flight. General and this kernel, in us: 12 and 2
+// fp16 heads of 128 5.7 and 3.1 at 64 positions, 6.4 and 3.5 at 1024, 26.8 and 8.9 at 4096, 88.7 and 25.4 at 16384; fp32
+// 5.4 and 2.9, 6.7 and 5.7, 17.4 and 13.2, 50.7 and 44.0; 32 and 8 bf16 heads 64.5 and 18.5 at 4096; 16 and 2 fp16 heads of
+// 256 59.5 and 17.6; 8 and 8 of 16 5.5 and 3.2: the faster one at each of 336 sizes, so it takes every such call.
 __host__ __device__ constexpr int row_heads(int elem_size) { return 8 / elem_size; }   // 64 bytes of a thread in flight
 template <int DT>
 __global__ void __launch_bounds__(kThreads, 4) rope_rows_kernel(const RopeArgs a) {
