@@ -803,6 +803,26 @@ def test_rank16_branch_at_the_edges_of_its_tiles(rows, width, out, scaling, give
     assert_close_rel_max(b.grad, (gs.t() @ low * (scaling if given else 1.0)).float(), 2 ** -10, "dB")
 
 
+@pytest.mark.parametrize("extra", [0, 8])
+def test_rank16_branch_at_the_widest_output_its_launches_take(extra):
+    """2^24 columns run on the rank-16 launches, wider ones on the products. Both against the plain products (an fp16 ulp
+    of the largest value, 2^-10)."""
+    from claudemaxing_b200 import lora
+
+    out, gen = (1 << 24) + extra, torch.Generator(device=DEV).manual_seed(extra)
+    x = torch.randn(1, 1, 32, generator=gen, device=DEV)
+    a = torch.randn(16, 32, generator=gen, device=DEV) * 0.1
+    b = torch.randn(out, 16, generator=gen, device=DEV) * 0.1
+    assert lora._rank16_covers(x, x.half(), [(a, b)]) == (extra == 0)
+    torch.manual_seed(1)
+    got = lora.LoRABranch.apply(x, x.half(), a, b, 0.1, 2.0)
+    torch.manual_seed(1)
+    dropped = torch.native_dropout(x, 0.1, True)[0].half()
+    low = torch.nn.functional.linear(dropped, a.half())
+    want = torch.nn.functional.linear(low, b.half()) * 2.0
+    assert_close_rel_max(got, want, 2 ** -10, "out")
+
+
 @pytest.mark.parametrize("pair", [False, True])
 def test_lora_branch_frees_its_dropout_masks_before_its_outputs(pair):
     """The forward's peak: the bool masks (a byte an element) are gone before the products, whose outputs are the
